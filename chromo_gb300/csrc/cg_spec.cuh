@@ -146,121 +146,168 @@ struct ChainView {
         twist(!lean && rd.twist ? a.twist + rd.bead_off * 2 : nullptr) {}
 };
 
-// Lanes per bead of the position-move deposit; each lane takes 8 / kLanesPerBead
-// of the bead's trilinear corners.
 // Largest position move of the pooled voxel table: an entry gets at most 2 m
 // contributions of |d| < 2^42, which its two 32-bit split counters hold for
 // m < 512.
 constexpr int kPoolMaxBeads = 256;
 
+// Lanes that share one bead's trilinear corners in the block-wide deposit,
+// each with kCornersPerLane corners (two neighbours along x).
 constexpr int kLanesPerBead = 4;
 constexpr int kCornersPerLane = 8 / kLanesPerBead;
 
-// The bond to the fixed right neighbour of moved bead i (old r, t3, t2 and
-// new tr, tt3, tt2), with its twist term: the second bond of a one-bead move
-// when one lane takes the whole bead.
-template <typename Pos, typename Acc>
-static __device__ __noinline__ Acc right_bond_term(const ChainView<Pos>& cv, long long i, const Pos (&r)[3],
-                                                   const Pos (&tr)[3], const Pos (&t3)[3], const Pos (&tt3)[3],
-                                                   const Pos (&t2)[3], const Pos (&tt2)[3]) {
-  const V4<Pos> RN = cv.r4[i + 1], TN = cv.t34[i + 1];
-  const Bond<Pos> bn = bond_at(cv.bonds, cv.bonds32, i, (Pos)0);
-  const Pos rn[3] = {RN.x, RN.y, RN.z}, tn[3] = {TN.x, TN.y, TN.z};
-  Acc out = acc_zero<Acc>();
-  acc_add(out, pair_dE_rev(bn, r, tr, rn, t3, tt3, tn));
-  if (cv.twist) {
-    const Frame nb = frame_of(cv.t24[i + 1], TN), cur = frame_of(t2, t3), nw = frame_of(tt2, tt3);
-    acc_add_d(out, twist_pair_dE(cv.twist + 2 * i, cur, nb, nw, nb));
-  }
-  return out;
-}
-
-// Lane cl (0..kLanesPerBead-1) of bead k of a position move (transform M;
-// segment [ind0, indf) of m beads of a chain of N): transforms the bead,
-// stages its r, t3, t2 (lanes 0-2), takes the bond to a fixed left neighbour
-// (lane 0 of the first bead, `left`) or to a fixed right neighbour (lane 1 of
-// the last bead, `right`) into `pterm`, counts the confinement crossings
-// (lane 0), and returns the voxel-table contributions of its corners c =
-// cl * kCornersPerLane + j: q[2j] at vq[2j] (old weight removed; the weight
-// change when the old and new weights lie in the same eight voxels) and
-// q[2j+1] at vq[2j+1] (new weight otherwise), with the bead's binder states
-// in sw.  The neighbour beads and bond parameters are loaded with the moved
-// bead (in-range indices on every lane).
-template <typename Pos, typename Acc>
-__device__ __forceinline__ void bead_task(const RepDev& rd, const GridF& gf, const ChainView<Pos>& cv, int kind,
-                                          const Pos (&M)[3][4], long long N, long long ind0, long long indf,
-                                          long long m, long long k, int cl, V4<Pos>* stage, bool density,
-                                          bool conf, int (&vq)[2 * kCornersPerLane],
-                                          long long (&q)[2 * kCornersPerLane], unsigned& sw, unsigned& e,
-                                          bool& left, bool& right, Acc& pterm, int& oob) {
-  using Real = Pos;
-  const long long i = ind0 + k;
-  constexpr int kRightLane = kLanesPerBead > 1 ? 1 : 0;
-  left = cl == 0 && k == 0 && ind0 != 0;
-  right = cl == kRightLane && k == m - 1 && indf != N;
-  // with one lane per bead, a one-bead move's lane takes both bonds; else a
-  // lane takes at most one, and loads one neighbour
-  const bool two = kLanesPerBead == 1 && left && right;
-  const long long in = left ? i - 1 : (right ? i + 1 : i);
-  const V4<Pos> RN = cv.r4[in], TN = cv.t34[in];
-  const Bond<Real> bn = bond_at(cv.bonds, cv.bonds32, (right && !left) ? i : in, (Real)0);
-  const V4<Pos> R = cv.r4[i], T3 = cv.t34[i], T2 = cv.t24[i];
-  const unsigned swi = density ? cv.st[i] : 0u;
-  const Real r[3] = {R.x, R.y, R.z}, t3[3] = {T3.x, T3.y, T3.z}, t2[3] = {T2.x, T2.y, T2.z};
-  Real tr[3], tt3[3], tt2[3];
+// New position (and, but for a slide, which only translates, new tangents) of
+// a bead under a move's transform M.
+template <typename Pos>
+__device__ __forceinline__ void move_bead(int kind, const Pos (&M)[3][4], const Pos (&r)[3], const Pos (&t3)[3],
+                                          const Pos (&t2)[3], Pos (&tr)[3], Pos (&tt3)[3], Pos (&tt2)[3]) {
   if (kind == CG_SLIDE) {
     for (int j = 0; j < 3; j++) { tr[j] = r[j] + M[j][3]; tt3[j] = t3[j]; tt2[j] = t2[j]; }
   } else {
     for (int j = 0; j < 3; j++) {
-      Real er = 0, e3 = 0, e2 = 0;
-      for (int qq = 0; qq < 3; qq++) { er += M[j][qq] * r[qq]; e3 += M[j][qq] * t3[qq]; e2 += M[j][qq] * t2[qq]; }
+      Pos er = 0, e3 = 0, e2 = 0;
+      for (int q = 0; q < 3; q++) { er += M[j][q] * r[q]; e3 += M[j][q] * t3[q]; e2 += M[j][q] * t2[q]; }
       tr[j] = er + M[j][3]; tt3[j] = e3; tt2[j] = e2;
     }
   }
-  const bool fin = isfinite(tr[0]) && isfinite(tr[1]) && isfinite(tr[2]);
-  if (!fin) e |= E_NONFINITE;
-#pragma unroll
-  for (int w = cl; w < 3; w += kLanesPerBead) {  // lanes 0-2 stage r, t3, t2 (all three with fewer lanes)
-    Real o[3];
-    for (int j = 0; j < 3; j++) o[j] = w == 0 ? tr[j] : (w == 1 ? tt3[j] : tt2[j]);
-    stage[3 * k + w] = V4<Pos>{(Pos)o[0], (Pos)o[1], (Pos)o[2], (Pos)0};
+}
+
+template <typename Pos>
+__device__ __forceinline__ void load_transform(const MovePlan& P, Pos (&M)[3][4]) {
+  const Pos* Mp = reinterpret_cast<const Pos*>(P.M);
+  for (int i = 0; i < 3; i++)
+    for (int j = 0; j < 4; j++) M[i][j] = Mp[4 * i + j];
+}
+
+// Elastic (and twist) dE of one boundary bond of a position move: the bond to
+// the fixed neighbour left of the segment (side 0) or right of it (side 1);
+// zero where the segment ends the chain.  The move's plan holds its segment
+// and transform.
+template <typename Pos, typename Acc, bool LEAN>
+static __device__ __noinline__ Acc boundary_term(const KArgs& a, const RepDev& rd, const MovePlan& P, int kind,
+                                                 int side) {
+  const ChainView<Pos> cv(a, rd, LEAN);
+  const long long N = rd.n_beads;
+  Acc out = acc_zero<Acc>();
+  const long long i = side == 0 ? P.ind0 : P.indf - 1;
+  const long long in = side == 0 ? i - 1 : i + 1;
+  if (in < 0 || in >= N) return out;
+  Pos M[3][4];
+  load_transform(P, M);
+  const V4<Pos> R = cv.r4[i], T3 = cv.t34[i], RN = cv.r4[in], TN = cv.t34[in];
+  const Bond<Pos> bn = bond_at(cv.bonds, cv.bonds32, side == 0 ? in : i, (Pos)0);
+  const Pos r[3] = {R.x, R.y, R.z}, t3[3] = {T3.x, T3.y, T3.z};
+  const Pos rn[3] = {RN.x, RN.y, RN.z}, tn[3] = {TN.x, TN.y, TN.z};
+  Pos t2[3] = {0, 0, 0}, tr[3], tt3[3], tt2[3];
+  if (cv.twist) {
+    const V4<Pos> T2 = cv.t24[i];
+    t2[0] = T2.x; t2[1] = T2.y; t2[2] = T2.z;
   }
-  const Real rn[3] = {(Real)RN.x, (Real)RN.y, (Real)RN.z}, tn[3] = {(Real)TN.x, (Real)TN.y, (Real)TN.z};
-  pterm = acc_zero<Acc>();
-  if (left) acc_add(pterm, pair_dE_fwd(bn, rn, r, tr, tn, t3, tt3));
-  if (right && !two) acc_add(pterm, pair_dE_rev(bn, r, tr, rn, t3, tt3, tn));
-  if (cv.twist && (left || right) && !two) {  // SSTWLC: the bond's twist term
+  move_bead(kind, M, r, t3, t2, tr, tt3, tt2);
+  if (side == 0) acc_add(out, pair_dE_fwd(bn, rn, r, tr, tn, t3, tt3));
+  else acc_add(out, pair_dE_rev(bn, r, tr, rn, t3, tt3, tn));
+  if (cv.twist) {  // SSTWLC: the bond's twist term
     const Frame nb = frame_of(cv.t24[in], TN), cur = frame_of(t2, t3), nw = frame_of(tt2, tt3);
-    const double* tw = cv.twist + 2 * (left ? in : i);
-    acc_add_d(pterm, left ? twist_pair_dE(tw, nb, cur, nb, nw) : twist_pair_dE(tw, cur, nb, nw, nb));
+    const double* tw = cv.twist + 2 * (side == 0 ? in : i);
+    acc_add_d(out, side == 0 ? twist_pair_dE(tw, nb, cur, nb, nw) : twist_pair_dE(tw, cur, nb, nw, nb));
   }
-  if (two) {  // the right bond of a one-bead move (one lane per bead), out of line
-    acc_add(pterm, right_bond_term<Pos, Acc>(cv, i, r, tr, t3, tt3, t2, tt2));
-    if (cv.twist) {
-      const Frame nb = frame_of(cv.t24[in], TN), cur = frame_of(t2, t3), nw = frame_of(tt2, tt3);
-      acc_add_d(pterm, twist_pair_dE(cv.twist + 2 * in, nb, cur, nb, nw));
-    }
+  return out;
+}
+
+// Where one bead's weights lie before (0) and after (1) a move: the voxel of
+// the lowest corner, the axes on which the upper voxel wraps to 0 (bit j), and
+// the lower voxel's weight per axis.
+template <typename Pos>
+struct BeadCells {
+  int v0, v1;
+  unsigned wrap0, wrap1;
+  Pos wl0[3], wl1[3];
+};
+
+// One lane's bead i = ind0 + k of a position move (transform M): moves it,
+// stages its new vectors for the commit, counts the confinement crossings and
+// finds its cells.  Returns false (and E_NONFINITE in e) for a position that
+// is not finite.
+template <typename Pos>
+__device__ __forceinline__ bool place_bead(const RepDev& rd, const GridF& gf, const ChainView<Pos>& cv, int kind,
+                                           const Pos (&M)[3][4], long long i, V4<Pos>* stage, bool density,
+                                           bool conf, BeadCells<Pos>& c, unsigned& e, int& oob) {
+  const V4<Pos> R = cv.r4[i];
+  const Pos r[3] = {R.x, R.y, R.z};
+  Pos t3[3] = {0, 0, 0}, t2[3] = {0, 0, 0}, tr[3], tt3[3], tt2[3];
+  if (kind != CG_SLIDE) {
+    const V4<Pos> T3 = cv.t34[i], T2 = cv.t24[i];
+    t3[0] = T3.x; t3[1] = T3.y; t3[2] = T3.z;
+    t2[0] = T2.x; t2[1] = T2.y; t2[2] = T2.z;
   }
-  oob = 0;
-  if (cl == 0 && conf) oob = out_of_bounds(rd, tr, true) * 65536 + out_of_bounds(rd, r, false);
-  if (density && fin) {
-    Real wl0[3], wl1[3];
-    int lo0[3], hi0[3], lo1[3], hi1[3];
-    move_axes(rd, gf, r, wl0, lo0, hi0);
-    move_axes(rd, gf, tr, wl1, lo1, hi1);
-    const bool same = lo0[0] == lo1[0] && lo0[1] == lo1[1] && lo0[2] == lo1[2];
+  move_bead(kind, M, r, t3, t2, tr, tt3, tt2);
+  stage[0] = V4<Pos>{tr[0], tr[1], tr[2], (Pos)0};
+  if (kind != CG_SLIDE) {  // a slide's commit writes positions only
+    stage[1] = V4<Pos>{tt3[0], tt3[1], tt3[2], (Pos)0};
+    stage[2] = V4<Pos>{tt2[0], tt2[1], tt2[2], (Pos)0};
+  }
+  oob = conf ? out_of_bounds(rd, tr, true) * 65536 + out_of_bounds(rd, r, false) : 0;
+  if (!(isfinite(tr[0]) && isfinite(tr[1]) && isfinite(tr[2]))) {
+    e |= E_NONFINITE;
+    return false;
+  }
+  if (density) {
+    int lo[3], hi[3];
+    move_axes(rd, gf, r, c.wl0, lo, hi);
+    c.v0 = lo[0] + gf.nx * lo[1] + gf.nxy * lo[2];
+    c.wrap0 = (hi[0] == 0 ? 1u : 0u) | (hi[1] == 0 ? 2u : 0u) | (hi[2] == 0 ? 4u : 0u);
+    move_axes(rd, gf, tr, c.wl1, lo, hi);
+    c.v1 = lo[0] + gf.nx * lo[1] + gf.nxy * lo[2];
+    c.wrap1 = (hi[0] == 0 ? 1u : 0u) | (hi[1] == 0 ? 2u : 0u) | (hi[2] == 0 ? 4u : 0u);
+  }
+  return true;
+}
+
+// Voxels and fixed-point weights of the two corners (y, z bits of cl) a lane
+// takes of one set of cells.
+template <typename Pos>
+__device__ __forceinline__ void corner_pair(const GridF& gf, int v, unsigned wrap, const Pos (&wl)[3], int cl,
+                                            int& va, int& vb, long long& qa, long long& qb) {
+  const bool by = cl & 1, bz = cl & 2;
+  const Pos fy = by ? 1 - wl[1] : wl[1], fz = bz ? 1 - wl[2] : wl[2];
+  if (by) v += (wrap & 2u) ? gf.nx - gf.nxy : gf.nx;
+  if (bz) v += (wrap & 4u) ? gf.nxy - gf.nxy * gf.n[2] : gf.nxy;
+  va = v;
+  vb = v + ((wrap & 1u) ? 1 - gf.nx : 1);
+  qa = q40(wl[0] * fy * fz);
+  qb = q40((1 - wl[0]) * fy * fz);
+}
+
+// Voxel-table contributions of corners (cl, two along x) of a bead: q[2j] at
+// vq[2j] (old weight removed; the weight change when the old and new cells
+// are the same eight voxels) and q[2j+1] at vq[2j+1] (new weight otherwise).
+template <typename Pos>
+__device__ __forceinline__ void corner_terms(const GridF& gf, const BeadCells<Pos>& c, int cl,
+                                             int (&vq)[2 * kCornersPerLane], long long (&q)[2 * kCornersPerLane]) {
+  corner_pair(gf, c.v0, c.wrap0, c.wl0, cl, vq[0], vq[2], q[0], q[2]);
+  corner_pair(gf, c.v1, c.wrap1, c.wl1, cl, vq[1], vq[3], q[1], q[3]);
+  const bool same = c.v0 == c.v1;
 #pragma unroll
-    for (int j = 0; j < kCornersPerLane; j++) {
-      const int c = cl * kCornersPerLane + j;
-      Real w0, w1;
-      voxel_corner(gf, wl0, lo0, hi0, c, w0, vq[2 * j]);
-      voxel_corner(gf, wl1, lo1, hi1, c, w1, vq[2 * j + 1]);
-      const long long q0 = q40(w0), q1 = q40(w1);
-      q[2 * j] = same ? q1 - q0 : -q0;
-      q[2 * j + 1] = same ? 0 : q1;
-    }
-    sw = swi;
+  for (int j = 0; j < kCornersPerLane; j++) {
+    const long long qo = q[2 * j], qn = q[2 * j + 1];
+    q[2 * j] = same ? qn - qo : -qo;
+    q[2 * j + 1] = same ? 0 : qn;
   }
+}
+
+template <typename Pos>
+__device__ __forceinline__ BeadCells<Pos> shfl_cells(const BeadCells<Pos>& c, unsigned wraps, int src,
+                                                     unsigned& got_wraps) {
+  BeadCells<Pos> o;
+  o.v0 = __shfl_sync(kFull, c.v0, src);
+  o.v1 = __shfl_sync(kFull, c.v1, src);
+  got_wraps = __shfl_sync(kFull, wraps, src);
+#pragma unroll
+  for (int j = 0; j < 3; j++) {
+    o.wl0[j] = __shfl_sync(kFull, c.wl0[j], src);
+    o.wl1[j] = __shfl_sync(kFull, c.wl1[j], src);
+  }
+  return o;
 }
 
 // A bond term kept in a move plan (fixed-point part and FP64 part).
@@ -271,15 +318,24 @@ template <> __device__ __forceinline__ Fx load_acc<Fx>(long long q, double h) { 
 template <> __device__ __forceinline__ double load_acc<double>(long long, double h) { return h; }
 
 // Deposit of the batch's position moves that use a shared voxel table
-// (plan.blk), by every thread of the CTA: the moves' bead corners, in move
-// order, are dealt out to the threads (eight per bead), so a move of many
-// beads no longer holds the batch back while the other warps wait.  The
-// table is the CTA's pooled table (FP32 storage: keys voxel * 32 + slot, one
-// used list, claims appended once per warp) or the slot's own table (claims
-// appended once per warp and move).  The bond terms, confinement counts and
-// error bits go to the move's plan.  A move whose optimistic table overflows
-// (E_OVF: a pool or a table past 3/4 load) is skipped from then on; its
-// group deposits it again in its global table.  Called by every thread.
+// (plan.blk), by every thread of the CTA.  The moves' beads, in move order,
+// are dealt out to the warps in runs of at most 32.  Each warp first takes one
+// bead per lane (load, transform, staging, cells), then four lanes per bead:
+// the cells go round by shuffles and each lane adds two corners (old weights
+// out, new weights in) to the voxel table.  The last warp also takes the
+// moves' boundary bonds, one per lane.  (Four lanes per bead for the whole
+// task, each repeating the bead's transform and cells, issued three times the
+// instructions; the bonds, taken by the lanes of a segment's end beads, were
+// executed by nearly every warp.  256 chains of 2,000-20,000 beads, 20 MC steps
+// and the read-back: 20.9 -> 18.5 ms; one 10,000-bead chain, 10 steps: 3.71 ->
+// 3.46 ms; 64 SSTWLC chains of 2,000 beads, whose FP64 twist terms of a batch's
+// bonds now share their warp's issue, 10 steps: 18.2 -> 11.8 ms.)  The table is the CTA's pooled table (FP32
+// storage: keys voxel * 32 + slot, one used list, claims appended once per
+// warp) or the slot's own table (claims appended once per warp and move).  The
+// bond terms, confinement counts and error bits go to the move's plan.  A move
+// whose optimistic table overflows (E_OVF: a pool or a table past 3/4 load) is
+// skipped from then on; its group deposits it again in its global table.
+// Called by every thread.
 template <typename Pos, bool LEAN>
 __device__ void block_deposit(const KArgs& a, SpecShared& sh, int rep, int B, int kind) {
   using Acc = typename AccOf<Pos>::type;
@@ -287,78 +343,104 @@ __device__ void block_deposit(const KArgs& a, SpecShared& sh, int rep, int B, in
   const RepDev& rd = sh.ws.rd;
   const GridF& gf = sh.ws.gf;
   const ChainView<Pos> cv(a, rd, LEAN);
-  const long long N = rd.n_beads;
   const bool conf = rd.field_kind != 0 && rd.confine_kind;
   const int Hs = 1 << a.logH, hcol = a.hcol;
   const bool pool = a.pool_on != 0;
-  // lane j of every warp holds the end of move j's tasks in the batch's
-  // task list (kLanesPerBead per bead of the moves with plan.blk)
-  const int lane = (int)(threadIdx.x & 31u);
-  int end = (lane < B && sh.plan[lane].blk) ? kLanesPerBead * sh.plan[lane].m : 0;
+  const int lane = (int)(threadIdx.x & 31u), warp = (int)(threadIdx.x >> 5), W = (int)(blockDim.x >> 5);
+  // lane j of every warp holds the end of move j's beads in the batch's bead
+  // list (the moves with plan.blk)
+  int end = (lane < B && sh.plan[lane].blk) ? sh.plan[lane].m : 0;
 #pragma unroll
   for (int o = 1; o < 32; o <<= 1) {
     const int y = __shfl_up_sync(kFull, end, o);
     if (lane >= o) end += y;
   }
   const int total = __shfl_sync(kFull, end, 31);
-  for (int t0 = 0; t0 < total; t0 += (int)blockDim.x) {
-    const int t = t0 + (int)threadIdx.x;
-    // the task's move: the number of moves whose tasks end at or before t
+  // beads per warp and round: an even share, in whole passes of the corners
+  constexpr int BP = 32 / kLanesPerBead;
+  const int rounds = (total + 32 * W - 1) / (32 * W);
+  const int share = rounds > 0 ? (total + rounds * W - 1) / (rounds * W) : 0;
+  const int run = (share + BP - 1) / BP * BP;
+  for (int b0 = warp * run; b0 < total; b0 += W * run) {
+    const int b = b0 + lane;
+    // the bead's move: the number of moves whose beads end at or before b
     int s = 0;
-    for (int j = 0; j < B; j++) s += __shfl_sync(kFull, end, j) <= t ? 1 : 0;
-    const int before = __shfl_sync(kFull, end, s > 0 ? s - 1 : 0);
-    int base = s > 0 ? before : 0;
-    if (t >= total) s = base = 0;
-    MovePlan& P = sh.plan[s];
-    const bool act = t < total && !(P.derr & E_OVF);
-    const long long k = (t - base) / kLanesPerBead;
-    const int cl = (t - base) % kLanesPerBead;
-    unsigned char* wb = smem + a.spec_off_warps + (size_t)s * a.warp_smem;
-    int vq[2 * kCornersPerLane] = {};
-    long long q[2 * kCornersPerLane] = {};
-    unsigned sw = 0, e = 0;
-    if (act) {
+    for (int j = 0; j < B; j++) s += __shfl_sync(kFull, end, j) <= b ? 1 : 0;
+    int base = __shfl_sync(kFull, end, s > 0 ? s - 1 : 0);
+    if (s == 0) base = 0;
+    bool on = lane < run && b < total;
+    if (!on) s = 0;
+    BeadCells<Pos> c;
+    c.v0 = c.v1 = 0;
+    c.wrap0 = c.wrap1 = 0;
+    for (int j = 0; j < 3; j++) c.wl0[j] = c.wl1[j] = 0;
+    unsigned info = 0;  // states (three bytes), wrap bits of the cells before and after
+    if (on) {
+      MovePlan& P = sh.plan[s];
+      const long long k = b - base, i = P.ind0 + k;
       Pos M[3][4];
-      const Pos* Mp = reinterpret_cast<const Pos*>(P.M);
-      for (int i = 0; i < 3; i++)
-        for (int j = 0; j < 4; j++) M[i][j] = Mp[4 * i + j];
+      load_transform(P, M);
       V4<Pos>* stage = P.gstage ? reinterpret_cast<V4<Pos>*>(a.g_stage) +
                                       ((long long)rep * a.spec_s + s) * a.g_stage_cap * 3
-                                : reinterpret_cast<V4<Pos>*>(wb + a.off_stage);
-      bool left, right;
-      Acc pterm;
+                                : reinterpret_cast<V4<Pos>*>(smem + a.spec_off_warps + (size_t)s * a.warp_smem +
+                                                             a.off_stage);
+      const unsigned sw = cv.st[i];
+      unsigned e = 0;
       int oob;
-      bead_task<Pos, Acc>(rd, gf, cv, kind, M, N, P.ind0, P.indf, P.m, k, cl, stage, true, conf, vq, q, sw, e,
-                          left, right, pterm, oob);
-      if (left) store_acc(P.pq[0], P.ph[0], pterm);  // both bonds of a one-lane bead: in pq[0]
-      if (right && !left) store_acc(P.pq[1], P.ph[1], pterm);
+      on = place_bead(rd, gf, cv, kind, M, i, stage + 3 * k, true, conf, c, e, oob);
+      info = (sw & 0xFFFFFFu) | c.wrap0 << 24 | c.wrap1 << 27;
       if (oob) atomicAdd(&P.oob, oob);
+      if (e) atomicOr(&P.derr, e);
     }
-    // the pooled table (one used list for the whole CTA, keys voxel * 32 +
-    // slot), or the move's own table (one used list per move)
-    const unsigned peers = pool ? kFull : __match_any_sync(kFull, t < total ? s : -1);
-    int* keys = reinterpret_cast<int*>(pool ? smem + a.off_pkeys : wb + a.off_keys);
-    int* used = reinterpret_cast<int*>(pool ? smem + a.off_pused : wb + a.off_used);
-    long long* vals = reinterpret_cast<long long*>(pool ? smem + a.off_pvals : wb + a.off_vals);
-    bool want[2 * kCornersPerLane];
+    const int sl = on ? s : -1;
+    const int left = total - b0 < run ? total - b0 : run;
+    for (int p = 0; p < left; p += BP) {
+      const int src = p + lane / kLanesPerBead;
+      unsigned inf;
+      BeadCells<Pos> d = shfl_cells(c, info, src, inf);
+      const int t = __shfl_sync(kFull, sl, src);
+      d.wrap0 = (inf >> 24) & 7u;
+      d.wrap1 = (inf >> 27) & 7u;
+      const int tt = t < 0 ? 0 : t;
+      MovePlan& P = sh.plan[tt];
+      const bool act = t >= 0 && !(P.derr & E_OVF);
+      unsigned char* wb = smem + a.spec_off_warps + (size_t)tt * a.warp_smem;
+      int vq[2 * kCornersPerLane];
+      long long q[2 * kCornersPerLane];
+      corner_terms(gf, d, lane % kLanesPerBead, vq, q);
+      // the pooled table (one used list for the whole CTA, keys voxel * 32 +
+      // slot), or the move's own table (one used list per move)
+      const unsigned peers = pool ? kFull : __match_any_sync(kFull, t);
+      int* keys = reinterpret_cast<int*>(pool ? smem + a.off_pkeys : wb + a.off_keys);
+      int* used = reinterpret_cast<int*>(pool ? smem + a.off_pused : wb + a.off_used);
+      long long* vals = reinterpret_cast<long long*>(pool ? smem + a.off_pvals : wb + a.off_vals);
+      bool want[2 * kCornersPerLane];
 #pragma unroll
-    for (int j = 0; j < 2 * kCornersPerLane; j++) {
-      want[j] = q[j] != 0;
-      if (pool) vq[j] = vq[j] * 32 + s;
-    }
-    const bool sure = P.sure && !pool;
-    const unsigned full_bit = sure ? E_SPIN : E_OVF;
-    const int lh = pool ? a.pool_logH : a.logH;
-    int slot[2 * kCornersPerLane];
-    claim_slots<2 * kCornersPerLane>(keys, used, pool ? &sh.npool : &sh.nused[s], lh, vq, want, slot, e,
-                                     sure ? Hs : (3 << lh) / 4, full_bit, peers);
-    if (!(e & full_bit)) {
+      for (int j = 0; j < 2 * kCornersPerLane; j++) {
+        want[j] = act && q[j] != 0;
+        if (pool) vq[j] = vq[j] * 32 + tt;
+      }
+      const bool sure = P.sure && !pool;
+      const unsigned full_bit = sure ? E_SPIN : E_OVF;
+      const int lh = pool ? a.pool_logH : a.logH;
+      int slot[2 * kCornersPerLane];
+      unsigned e = 0;
+      claim_slots<2 * kCornersPerLane>(keys, used, pool ? &sh.npool : &sh.nused[tt], lh, vq, want, slot, e,
+                                       sure ? Hs : (3 << lh) / 4, full_bit, peers);
+      if (!(e & full_bit)) {
 #pragma unroll
-      for (int j = 0; j < 2 * kCornersPerLane; j++)
-        if (want[j]) add_corner(vals, hcol, slot[j], q[j], sw, rd.nb, true);
+        for (int j = 0; j < 2 * kCornersPerLane; j++)
+          if (want[j]) add_corner(vals, hcol, slot[j], q[j], inf, rd.nb, true);
+      }
+      if (e && t >= 0) atomicOr(&P.derr, e);
     }
-    if (e) atomicOr(&P.derr, e);
   }
+  // boundary bonds of the moves, two per move
+  if (warp == W - 1)
+    for (int j = lane; j < 2 * B; j += 32) {
+      MovePlan& P = sh.plan[j >> 1];
+      if (P.blk) store_acc(P.pq[j & 1], P.ph[j & 1], boundary_term<Pos, Acc, LEAN>(a, rd, P, kind, j & 1));
+    }
 }
 
 // Field dE and conflict registration of the batch's pooled voxel entries, by
@@ -694,39 +776,40 @@ __device__ void evaluate_move(const KArgs& a, SpecShared& sh, int rep, int s, in
       const int cap = gtab ? (1 << gm.logH) : (sure ? Hs : (3 * Hs) / 4);
       const unsigned full_bit = (gtab || sure) ? E_SPIN : E_OVF;
       unsigned e = 0;
-      // the group's own deposit: kLanesPerBead lanes per bead, lane gl
-      // taking part gl % kLanesPerBead of bead gl / kLanesPerBead of a pass
-      constexpr int BP = G / kLanesPerBead;
-      const int kc = gl / kLanesPerBead, cl = gl % kLanesPerBead;
-      for (long long kb = 0; __any_sync(kFull, run && kb < m && !(e & E_OVF)); kb += BP) {
-        const long long k = kb + kc;
-        const bool act = run && k < m && !(e & E_OVF);
-        int vq[2 * kCornersPerLane] = {};
-        long long q[2 * kCornersPerLane] = {};
+      // the group's own deposit: one bead per lane, its corners two by two,
+      // the boundary bonds on its first two lanes
+      for (long long kb = 0; __any_sync(kFull, run && kb < m && !(e & E_OVF)); kb += G) {
+        const long long k = kb + gl;
+        bool act = run && k < m && !(e & E_OVF);
+        BeadCells<Pos> c = {};
         unsigned sw = 0;
         if (act) {
-          bool left, right;
-          Acc pterm;
           int ob;
-          bead_task<Pos, Acc>(rd, gf, cv, kind, M, N, ind0, indf, m, k, cl, stage, density,
-                              check_field && rd.confine_kind, vq, q, sw, e, left, right, pterm, ob);
-          if (left || right) acc_add(part, pterm);
+          if (density) sw = st[ind0 + k];
+          act = place_bead(rd, gf, cv, kind, M, ind0 + k, stage + 3 * k, density, check_field && rd.confine_kind,
+                           c, e, ob);
           oob += ob;
         }
         if (density) {
-          bool want[2 * kCornersPerLane];
+          for (int cl = 0; cl < kLanesPerBead; cl++) {
+            int vq[2 * kCornersPerLane];
+            long long q[2 * kCornersPerLane];
+            corner_terms(gf, c, cl, vq, q);
+            bool want[2 * kCornersPerLane];
 #pragma unroll
-          for (int j = 0; j < 2 * kCornersPerLane; j++) want[j] = q[j] != 0;
-          int slot[2 * kCornersPerLane];
-          claim_slots<2 * kCornersPerLane>(S.keys, S.used, nused, S.logH, vq, want, slot, e, cap, full_bit, peers);
-          if (!(e & full_bit)) {
+            for (int j = 0; j < 2 * kCornersPerLane; j++) want[j] = act && q[j] != 0 && !(e & E_OVF);
+            int slot[2 * kCornersPerLane];
+            claim_slots<2 * kCornersPerLane>(S.keys, S.used, nused, S.logH, vq, want, slot, e, cap, full_bit, peers);
+            if (!(e & full_bit)) {
 #pragma unroll
-            for (int j = 0; j < 2 * kCornersPerLane; j++)
-              if (want[j]) add_corner(S.vals, hcol, slot[j], q[j], sw, rd.nb, !gtab);
+              for (int j = 0; j < 2 * kCornersPerLane; j++)
+                if (want[j]) add_corner(S.vals, hcol, slot[j], q[j], sw, rd.nb, !gtab);
+            }
           }
           e = gor<G>(e);  // a full table ends the group's passes together
         }
       }
+      if (run && m > 0 && gl < 2) acc_add(part, boundary_term<Pos, Acc, LEAN>(a, rd, P, kind, gl));
       e = gor<G>(e);
       if (run) ovf = (e & E_OVF) != 0;
       err |= e & ~E_OVF;
