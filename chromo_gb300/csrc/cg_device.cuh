@@ -586,9 +586,29 @@ __device__ __forceinline__ FF pair_dE_rev(const Bond<float>& b, const float r0[3
 // ---------------------------------------------------------------- density field
 // chromo/fields.pyx:1430-1673: eight trilinear weights and periodic voxel indices.
 
+// a mod b (Python's sign rule).  In a periodic box most beads of a long chain
+// lie outside [0, b), so the FP64 remainder (of a pipe at 1/64 of the FP32
+// rate) is on the hot path.  For b > 0 and |a| < 2^20 b: with q within one of
+// the quotient (an FP32 quotient, good to 2^-21 relative), |a| - q b in one FMA
+// is exact when it lies in [0, b), where it is the remainder (a multiple of the
+// smaller operand's last place below b), and has the right sign when it does
+// not, so one correction of q gives fmod's value bit for bit.  Other arguments
+// take fmod.  1,000 beads in FP64, 300 moves: 10.0 -> 9.7 ms with the voxel
+// widths of voxel_axes divided once on the host.  (The same for binary32 gave
+// nothing: 18.5 against 18.7 ms on 256 chains.)
 __device__ __forceinline__ double pymod(double a, double b) {
   if (a >= 0 && a < b) return a;  // fmod(a, b) == a exactly here
-  double m = fmod(a, b);
+  const double x = fabs(a);
+  double m;
+  if (b > 1e-30 && b < 1e30 && x < b * 1048576.0) {
+    const double q = (double)truncf(__fdividef((float)x, (float)b));
+    double r = __fma_rn(-q, b, x);
+    if (r < 0) r = __fma_rn(-(q - 1.0), b, x);
+    else if (r >= b) r = __fma_rn(-(q + 1.0), b, x);
+    m = a < 0 ? -r : r;
+  } else {
+    m = fmod(a, b);
+  }
   if (m != 0 && ((m < 0) != (b < 0))) m += b;
   return m;
 }
@@ -631,10 +651,11 @@ __device__ __forceinline__ void make_gridf(const RepDev& rd, GridF& gf) {
 __device__ __forceinline__ void voxel_axes(const RepDev& rd, const GridF&, const double pos[3],
                                            double wl[3], int lo[3], int hi[3]) {
   const double width[3] = {rd.wx, rd.wy, rd.wz};
+  const double dxyz[3] = {rd.dx, rd.dy, rd.dz};  // width / n, divided on the host
   const int n[3] = {rd.nx, rd.ny, rd.nz};
 #pragma unroll
   for (int j = 0; j < 3; j++) {
-    double d = width[j] / (double)n[j];
+    const double d = dxyz[j];
     double x = pymod(pos[j] + 0.5 * width[j], width[j]) - 0.5 * d;
     long long ind = (long long)floor(x / d);
     int li = ind == -1 ? n[j] - 1 : (int)ind;
