@@ -385,16 +385,20 @@ static int choose_shape(cg_sim* s, int w_req, int g_req) {
   const size_t budget = std::min<size_t>(smem_per_sm / ctas_per_sm - 1024, 220 * 1024);
   const int lhb = 10;
   const long long sc = G == 32 ? 48 : 32;
-  // FP32 storage: the position moves of a batch share one pooled voxel table
-  // (keys voxel * 32 + slot: grids below 2^26 voxels), as large as fits (up
-  // to 4,096 entries); the slots keep 64-entry tables for binding moves
-  int lhp = 0;
-  if (!s->fp64 && s->max_vox < (1LL << 26)) {
-    s->layout(6, sc);
-    for (int t = 12; t >= 8 && lhp == 0; t--)
-      if (s->cta_layout(lhb, W, G, t) <= budget) lhp = t;
+  // the position moves of a batch share one pooled voxel table (keys voxel *
+  // 32 + slot: grids below 2^26 voxels), as large as fits; the slots keep small
+  // tables for binding moves.  FP32 storage: up to 4,096 entries and 64-entry
+  // slot tables.  FP64 storage: up to 2,048 entries (its moves in flight touch
+  // ~50 voxels each) and, where they fit beside a pool of at least 1,024, slot
+  // tables of up to 256 entries.
+  int lhp = 0, lh = 6;
+  if (s->max_vox < (1LL << 26)) {
+    for (int t = s->fp64 ? 11 : 12; t >= 8 && lhp == 0; t--)
+      for (int l = s->fp64 && t >= 10 ? 8 : 6; l >= 6 && lhp == 0; l--) {
+        s->layout(l, sc);
+        if (s->cta_layout(lhb, W, G, t) <= budget) { lhp = t; lh = l; }
+      }
   }
-  int lh = 6;
   if (lhp == 0) {
     lh = 10;  // at most 1,024 slots: the 32-bit split counters of a shared table cannot overflow
     for (; lh > 6; lh--) {

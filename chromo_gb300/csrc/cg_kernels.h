@@ -51,11 +51,14 @@ struct MovePlan {
   long long pq[2];
   double ph[2];
   double M[12];  // the 3 x 4 transform, stored in the position type
-  // the CTA's pass over the pooled voxel table (FP32 position moves): the
-  // move's field dE in fixed point, its FP64 side sum, its exact 1e99 units,
-  // its touched voxels and a failed registration
+  // the CTA's pass over the pooled voxel table: the move's field dE in fixed
+  // point (fq plus limbs of 20 bits, summed by 32-bit shared atomics), its
+  // FP64 part, its exact 1e99 units, its touched voxels and a failed
+  // registration
   long long fq, fH;
   double fh;
+  unsigned fl0, fl1;
+  int fl2;
   int fn, freg;
 };
 
@@ -115,7 +118,7 @@ struct KArgs {
   // CTA layout: header, block voxel table, then one region per move slot;
   // spec_w warps of 32 / spec_g groups, spec_s = spec_w * 32 / spec_g slots
   int spec_w, spec_g, spec_s, spec_logHB, spec_off_bkeys, spec_off_bmask, spec_off_warps;
-  // pooled voxel table of the CTA (FP32 storage): 2^pool_logH entries keyed by
+  // pooled voxel table of the CTA: 2^pool_logH entries keyed by
   // voxel * 32 + move slot, shared by the position moves of a batch
   int pool_on, pool_logH, off_pkeys, off_pused, off_pvals;
   unsigned long long seed;

@@ -253,6 +253,39 @@ __device__ __forceinline__ double with_huge(double hard, long long huge) {
   return huge != 0 ? hard_with_huge(hard, huge) : hard;
 }
 
+// Field dE of one touched voxel v in FP64 arithmetic (row `d` of a voxel
+// table: the move's density deltas in, the voxel's post-move row out): added
+// to `part`; the 1e99 penalty of a voxel above vf_limit to `huge` (kHugeUnit
+// units).
+__device__ __forceinline__ void voxel_dE_f64(const RepDev& rd, const KArgs& a, const long long* grid, int v,
+                                             long long* d, bool split, double& part, long long& huge) {
+  long long row[4];
+  load_row(grid + (long long)v * a.ncol, a.ncol, row);
+  long long g0 = row[0], d0 = hash_delta(d, split);
+  double V = rd.has_access ? a.access_vol[rd.vox_off + v] : rd.vol_bin;
+  double c = 0, rho[CG_MAX_BINDERS], dd[CG_MAX_BINDERS];
+#pragma unroll
+  for (int b = 0; b < CG_MAX_BINDERS; b++) {
+    if (b >= rd.nb) break;
+    long long gb = row[1 + b], db = hash_delta(d + 1 + b, split);
+    rho[b] = ((double)gb * kFxInv) / V;
+    dd[b] = ((double)db * kFxInv) / V;
+    c += rd.pref[b] * (dd[b] * (2 * rho[b] + dd[b]));
+    d[1 + b] = gb + db;
+  }
+#pragma unroll
+  for (int b = 0; b < CG_MAX_BINDERS; b++)
+#pragma unroll
+    for (int e = 0; e < CG_MAX_BINDERS; e++)
+      if (b < rd.nb && e < rd.nb)
+        c += rd.xpref[b * CG_MAX_BINDERS + e] * (rho[b] * dd[e] + dd[b] * rho[e] + dd[b] * dd[e]);
+  const ChiSplit t = chi_term64(rd, V, g0, d0);
+  c += t.soft;
+  huge += t.huge;
+  d[0] = g0 + d0;
+  part += c;
+}
+
 // Field dE over the touched voxels (fixed-point grid), FP64 arithmetic; also
 // stores the post-move grid values into the hash values for the commit.  The
 // sum is added to `hard` (the FP64 part of the move's dE), nothing to `soft`;
@@ -269,34 +302,8 @@ static __device__ void field_dE_voxels(const WarpShared& ws, const KArgs& a, int
   long long hpart = 0;
   const long long* grid = a.grid + rd.vox_off * a.ncol;
   for (int i = lane; i < nused; i += G) {
-    int slot = used[i];
-    int v = keys[slot];
-    long long* d = vals + (long long)slot * hcol;
-    long long row[4];
-    load_row(grid + (long long)v * a.ncol, a.ncol, row);
-    long long g0 = row[0], d0 = hash_delta(d, split);
-    double V = rd.has_access ? a.access_vol[rd.vox_off + v] : rd.vol_bin;
-    double c = 0, rho[CG_MAX_BINDERS], dd[CG_MAX_BINDERS];
-#pragma unroll
-    for (int b = 0; b < CG_MAX_BINDERS; b++) {
-      if (b >= rd.nb) break;
-      long long gb = row[1 + b], db = hash_delta(d + 1 + b, split);
-      rho[b] = ((double)gb * kFxInv) / V;
-      dd[b] = ((double)db * kFxInv) / V;
-      c += rd.pref[b] * (dd[b] * (2 * rho[b] + dd[b]));
-      d[1 + b] = gb + db;
-    }
-#pragma unroll
-    for (int b = 0; b < CG_MAX_BINDERS; b++)
-#pragma unroll
-      for (int e = 0; e < CG_MAX_BINDERS; e++)
-        if (b < rd.nb && e < rd.nb)
-          c += rd.xpref[b * CG_MAX_BINDERS + e] * (rho[b] * dd[e] + dd[b] * rho[e] + dd[b] * dd[e]);
-    const ChiSplit t = chi_term64(rd, V, g0, d0);
-    c += t.soft;
-    hpart += t.huge;
-    d[0] = g0 + d0;
-    part += c;
+    const int slot = used[i];
+    voxel_dE_f64(rd, a, grid, keys[slot], vals + (long long)slot * hcol, split, part, hpart);
   }
   n_vox = nused;
   (void)soft;

@@ -110,12 +110,7 @@ struct SlotScratch {
   int logH;
   void* stage;
   int* idx;
-  unsigned* picked;
 };
-
-__device__ __forceinline__ void use_table(SlotScratch& S, const SlotScratch& from) {
-  S.keys = from.keys; S.used = from.used; S.bslot = from.bslot; S.vals = from.vals; S.logH = from.logH;
-}
 
 // Drop the entries a move left in a voxel table (keys, values, block slots).
 __device__ __forceinline__ void clear_table(const SlotScratch& T, int hcol, int nu, int gl, int G) {
@@ -443,19 +438,62 @@ __device__ void block_deposit(const KArgs& a, SpecShared& sh, int rep, int B, in
     }
 }
 
+// One pooled entry's field term: FP32 storage in fixed point, FP64 storage in
+// FP64.
+__device__ __forceinline__ void pool_voxel_dE(const WarpShared& ws, const KArgs& a, const long long* grid, int v,
+                                              long long* d, Fx& part, long long& huge) {
+  voxel_dE_f32(ws, a, grid, v, d, true, part, huge);
+}
+__device__ __forceinline__ void pool_voxel_dE(const WarpShared& ws, const KArgs& a, const long long* grid, int v,
+                                              long long* d, double& part, long long& huge) {
+  voxel_dE_f64(ws.rd, a, grid, v, d, true, part, huge);
+}
+
+// Add the warp's field terms to their moves' plans (s: this lane's move, -1 for
+// none).  Fixed point: q = l2 2^40 + l1 2^20 + l0 with l0, l1 in [0, 2^20);
+// the limbs of at most 4,096 entries sum within 32 bits (|q| < 2^51), so each
+// lane adds its own with four 32-bit shared atomics (a warp's entries belong to
+// a handful of moves; reducing them move by move first took longer: the field
+// phase of a batch of ~5 moves on 256 chains 12.0 k -> 8.5 k cycles).  FP64: a
+// warp reduces each move's terms first.
+__device__ __forceinline__ void add_pool_part(SpecShared& sh, int s, const Fx& part) {
+  if (s < 0) return;
+  MovePlan& P = sh.plan[s];
+  atomicAdd(&P.fl0, (unsigned)(part.q & 0xFFFFF));
+  atomicAdd(&P.fl1, (unsigned)((part.q >> 20) & 0xFFFFF));
+  atomicAdd(&P.fl2, (int)(part.q >> 40));
+  atomicAdd(&P.fn, 1);
+  if (!is_zero64(part.hard)) atomicAdd(&P.fh, part.hard);
+}
+__device__ __forceinline__ void add_pool_part(SpecShared& sh, int s, double part) {
+  const int lane = (int)(threadIdx.x & 31u);
+  unsigned todo = __ballot_sync(kFull, s >= 0);
+  while (todo) {
+    const int leader = __ffs((int)todo) - 1;
+    const int sl = __shfl_sync(kFull, s, leader);
+    const bool mine = s == sl;
+    const double sum = warp_sum(mine ? part : 0.0);
+    const unsigned who = __ballot_sync(kFull, mine);
+    if (lane == leader) {
+      atomicAdd(&sh.plan[sl].fh, sum);
+      atomicAdd(&sh.plan[sl].fn, __popc(who));
+    }
+    todo &= ~who;
+  }
+}
+
 // Field dE and conflict registration of the batch's pooled voxel entries, by
-// every thread of the CTA (FP32 storage): entry -> (voxel, move slot s);
-// the voxel's FP32 field term (voxel_dE_f32, which also leaves the voxel's
-// post-move row in the entry for the commit); its registration in the block
-// voxel table, whose atomicOr returns the moves that registered the voxel
-// first (an earlier one is a conflict of s, a later one learns of s through
-// its plan's mask).  Per move, the fixed-point terms are summed exactly (a
-// warp reduces each move's terms in three 21-bit limbs, one 64-bit atomic
-// per warp and move), so the sum does not depend on which thread took which
-// voxel.  Entries of moves that overflowed the pool are skipped (their
-// groups redo them in their global tables).  Called by every thread.
+// every thread of the CTA: entry -> (voxel, move slot s); the voxel's field
+// term (which also leaves the voxel's post-move row in the entry for the
+// commit); its registration in the block voxel table, whose atomicOr returns
+// the moves that registered the voxel first (an earlier one is a conflict of
+// s, a later one learns of s through its plan's mask).  Entries of moves that
+// overflowed the pool are skipped (their groups redo them in their global
+// tables).  Called by every thread.
+template <typename Pos>
 static __device__ void block_field_pool(const KArgs& a, SpecShared& sh, unsigned char* smem, int* bkeys,
                                  unsigned* bmask) {
+  using Acc = typename AccOf<Pos>::type;
   const WarpShared& ws = sh.ws;
   const RepDev& rd = ws.rd;
   const int* pkeys = reinterpret_cast<const int*>(smem + a.off_pkeys);
@@ -467,7 +505,7 @@ static __device__ void block_field_pool(const KArgs& a, SpecShared& sh, unsigned
   for (int e0 = (int)(threadIdx.x & ~31u); e0 < n; e0 += (int)blockDim.x) {
     const int e = e0 + lane;
     int s = -1;
-    Fx part = Fx{0, 0.0};
+    Acc part = acc_zero<Acc>();
     long long hp = 0;
     if (e < n) {
       const int slot = pused[e];
@@ -478,7 +516,7 @@ static __device__ void block_field_pool(const KArgs& a, SpecShared& sh, unsigned
       if (P.derr & E_OVF) {
         s = -1;
       } else {
-        voxel_dE_f32(ws, a, grid, v, pvals + (long long)slot * a.hcol, true, part, hp);
+        pool_voxel_dE(ws, a, grid, v, pvals + (long long)slot * a.hcol, part, hp);
         const int b = block_insert(bkeys, a.spec_logHB, v);
         if (b < 0) {
           atomicOr(&P.freg, 1);
@@ -489,29 +527,10 @@ static __device__ void block_field_pool(const KArgs& a, SpecShared& sh, unsigned
           for (unsigned later = prior & above; later; later &= later - 1)
             atomicOr(&sh.plan[__ffs((int)later) - 1].cmask, 1u << s);
         }
-        if (!is_zero64(part.hard)) atomicAdd(&P.fh, part.hard);
         if (hp) atomicAdd(reinterpret_cast<unsigned long long*>(&P.fH), (unsigned long long)hp);
       }
     }
-    // q = l2 2^42 + l1 2^21 + l0 with l0, l1 in [0, 2^21) (|q| < 2^50): each
-    // limb's sum over a warp fits 32 bits
-    unsigned todo = __ballot_sync(kFull, s >= 0);
-    while (todo) {
-      const int leader = __ffs((int)todo) - 1;
-      const int sl = __shfl_sync(kFull, s, leader);
-      const bool mine = s == sl;
-      const long long q = mine ? part.q : 0;
-      const unsigned l0 = __reduce_add_sync(kFull, (unsigned)(q & 0x1FFFFF));
-      const unsigned l1 = __reduce_add_sync(kFull, (unsigned)((q >> 21) & 0x1FFFFF));
-      const int l2 = __reduce_add_sync(kFull, (int)(q >> 42));
-      const unsigned who = __ballot_sync(kFull, mine);
-      if (lane == leader) {
-        const long long sum = (long long)l2 * 4398046511104LL + (long long)l1 * 2097152LL + (long long)l0;
-        atomicAdd(reinterpret_cast<unsigned long long*>(&sh.plan[sl].fq), (unsigned long long)sum);
-        atomicAdd(&sh.plan[sl].fn, __popc(who));
-      }
-      todo &= ~who;
-    }
+    add_pool_part(sh, s, part);
   }
 }
 
@@ -573,13 +592,182 @@ static __device__ __noinline__ void log_move(const KArgs& a, int rep, unsigned l
   a.mlog[(long long)rep * a.mlog_cap + (long long)k] = rec;
 }
 
-// The pooled pass's field terms of a move, added to its field dE.
-__device__ __forceinline__ void add_pool_terms(Fx& s, const MovePlan& P) {
-  s.q += P.fq;
-  if (!is_zero64(P.fh)) s.hard = add_hard(s.hard, P.fh);
+// A move's field dE from its plan: fixed point into `soft` (FP32 storage) or
+// FP64 into `hard`.
+__device__ __forceinline__ void plan_field(const MovePlan& P, Fx& soft, double&) {
+  soft.q = P.fq + (long long)P.fl2 * 1099511627776LL + (long long)P.fl1 * 1048576LL + (long long)P.fl0;
+  soft.hard = P.fh;
 }
-__device__ __forceinline__ void add_pool_terms(double& s, const MovePlan& P) {
-  s += (double)P.fq * kFxEInv + P.fh;
+__device__ __forceinline__ void plan_field(const MovePlan& P, double&, double& hard) { hard = P.fh; }
+
+// Scratch of move slot `slot`: its shared-memory region, or its region of the
+// global scratch (tables, staging and lists of any size the move can have).
+__device__ __forceinline__ SlotScratch shared_slot(const KArgs& a, SpecShared& sh, int slot) {
+  unsigned char* wb = reinterpret_cast<unsigned char*>(&sh) + a.spec_off_warps + (size_t)slot * a.warp_smem;
+  SlotScratch S;
+  S.keys = reinterpret_cast<int*>(wb + a.off_keys);
+  S.used = reinterpret_cast<int*>(wb + a.off_used);
+  S.bslot = reinterpret_cast<int*>(wb + a.off_bslot);
+  S.vals = reinterpret_cast<long long*>(wb + a.off_vals);
+  S.logH = a.logH;
+  S.stage = wb + a.off_stage;
+  S.idx = reinterpret_cast<int*>(wb + a.off_idx);
+  return S;
+}
+template <typename Pos>
+__device__ __forceinline__ SlotScratch global_slot(const KArgs& a, int rep, int slot) {
+  const long long gi = (long long)rep * a.spec_s + slot, Hg = 1LL << a.g_logH;
+  SlotScratch S;
+  S.keys = a.g_keys + gi * Hg;
+  S.used = a.g_used + gi * Hg;
+  S.bslot = a.g_bslot + gi * Hg;
+  S.vals = a.g_vals + gi * Hg * a.hcol;
+  S.logH = a.g_logH;
+  S.stage = reinterpret_cast<V4<Pos>*>(a.g_stage) + gi * a.g_stage_cap * 3;
+  S.idx = a.g_idx + gi * a.g_stage_cap;
+  return S;
+}
+
+// Field terms of a move left in its plan by own_path.
+__device__ __forceinline__ void store_field(MovePlan& P, const Fx& soft, double) { P.fq = soft.q; P.fh = soft.hard; }
+__device__ __forceinline__ void store_field(MovePlan& P, double, double hard) { P.fh = hard; }
+
+// A position move taken by its own group: its deposit (`dep`: the CTA did not
+// deposit it, or it overflowed the shared table it was deposited in) in its
+// shared or global table, the field dE over that table and the registration of
+// its voxels, all left in its plan.  The moves of the pooled table need it
+// only when they are long (over kPoolMaxBeads) or overflowed the pool; chains
+// in no density field take it for the bond terms.  Out of line: with the pooled
+// table it is rare, and inline it cost every batch ~3.6 k cycles of empty
+// passes and reductions (256 chains, 20 MC steps: 18.5 -> 16.4 ms with the
+// field sums in 32-bit limbs; 1,000 beads in FP64, whose moves over 64
+// beads took it before the pool served FP64: 9.7 -> 6.9 ms).  Called by the whole warp; `run` is false for groups
+// without such a move.
+template <typename Pos, int G, bool LEAN>
+static __device__ __noinline__ void own_path(const KArgs& a, SpecShared& sh, int rep, int s, int gl, bool run,
+                                             int kind, int* bkeys, unsigned* bmask) {
+  using Acc = typename AccOf<Pos>::type;
+  const RepDev& rd = sh.ws.rd;
+  const GridF& gf = sh.ws.gf;
+  const ChainView<Pos> cv(a, rd, LEAN);
+  MovePlan& P = sh.plan[s];
+  const int hcol = a.hcol;
+  const bool density = rd.field_kind == 2, check_field = rd.field_kind != 0;
+  const long long m = run ? P.m : 0, ind0 = run ? P.ind0 : 0;
+  const int Hs = 1 << a.logH;
+  const bool sure = run && P.sure;
+  int gtab = run ? P.gtab : 0;
+  bool ovf = run && (P.derr & E_OVF) != 0;
+  bool dep = run && (!P.blk || ovf);
+  int* nused = &sh.nused[s];
+  SlotScratch S = gtab ? global_slot<Pos>(a, rep, s) : shared_slot(a, sh, s);
+  V4<Pos>* stage = reinterpret_cast<V4<Pos>*>(run && P.gstage ? global_slot<Pos>(a, rep, s).stage
+                                                              : shared_slot(a, sh, s).stage);
+  Pos M[3][4];
+  load_transform(P, M);
+  const unsigned peers = group_mask<G>();
+  unsigned err = 0;
+  int oob = 0;
+  // pass 0: moves the CTA did not deposit; pass 1: overflowed ones
+  for (int pass = 0; pass < 2; pass++) {
+    if (pass == 1) {
+      if (!__any_sync(kFull, ovf)) break;
+      if (ovf && !gtab) clear_table(S, hcol, *nused, gl, G);
+      __syncwarp();
+      if (ovf) {
+        if (gl == 0) *nused = 0;
+        S = global_slot<Pos>(a, rep, s);
+        gtab = 1;
+        oob = 0;
+      }
+      __syncwarp();
+    }
+    const bool go = pass == 0 ? (dep && !ovf) : ovf;
+    const int cap = gtab ? (1 << a.g_logH) : (sure ? Hs : (3 * Hs) / 4);
+    const unsigned full_bit = (gtab || sure) ? E_SPIN : E_OVF;
+    unsigned e = 0;
+    // one bead per lane, its corners two by two
+    for (long long kb = 0; __any_sync(kFull, go && kb < m && !(e & E_OVF)); kb += G) {
+      const long long k = kb + gl;
+      bool act = go && k < m && !(e & E_OVF);
+      BeadCells<Pos> c = {};
+      unsigned sw = 0;
+      if (act) {
+        int ob;
+        if (density) sw = cv.st[ind0 + k];
+        act = place_bead(rd, gf, cv, kind, M, ind0 + k, stage + 3 * k, density, check_field && rd.confine_kind, c,
+                         e, ob);
+        oob += ob;
+      }
+      if (density) {
+        for (int cl = 0; cl < kLanesPerBead; cl++) {
+          int vq[2 * kCornersPerLane];
+          long long q[2 * kCornersPerLane];
+          corner_terms(gf, c, cl, vq, q);
+          bool want[2 * kCornersPerLane];
+#pragma unroll
+          for (int j = 0; j < 2 * kCornersPerLane; j++) want[j] = act && q[j] != 0 && !(e & E_OVF);
+          int slot[2 * kCornersPerLane];
+          claim_slots<2 * kCornersPerLane>(S.keys, S.used, nused, S.logH, vq, want, slot, e, cap, full_bit, peers);
+          if (!(e & full_bit)) {
+#pragma unroll
+            for (int j = 0; j < 2 * kCornersPerLane; j++)
+              if (want[j]) add_corner(S.vals, hcol, slot[j], q[j], sw, rd.nb, !gtab);
+          }
+        }
+        e = gor<G>(e);  // a full table ends the group's passes together
+      }
+    }
+    e = gor<G>(e);
+    if (go) ovf = pass == 0 && (e & E_OVF) != 0;
+    err |= e & ~E_OVF;
+  }
+  err = gor<G>(err);
+  oob = gsum<G>(oob);
+  __syncwarp();
+  Acc soft = acc_zero<Acc>();
+  double hard = 0;
+  long long huge = 0, nvox = 0;
+  unsigned cmb = 0;
+  int regfail = 0;
+  if (density) {
+    const int nu = run ? *nused : 0;
+    field_dE_voxels<G>(sh.ws, a, hcol, S.keys, S.used, S.vals, nu, gl, nvox, soft, hard, huge, !gtab);
+    // register the touched voxels for the conflict test: the moves that
+    // registered a voxel first are this move's conflicts if earlier in the
+    // batch; a later move that registered it first learns of this one through
+    // its plan's mask
+    const int nr = err ? 0 : nu;
+    const unsigned below = (1u << s) - 1u, above = ~((2u << s) - 1u);
+    for (int i = gl; i < nr; i += G) {
+      const int b = block_insert(bkeys, a.spec_logHB, S.keys[S.used[i]]);
+      S.bslot[i] = b;
+      if (b < 0) {
+        regfail = 1;
+      } else {
+        const unsigned prior = atomicOr(&bmask[b], 1u << s);
+        cmb |= prior & below;
+        for (unsigned later = prior & above; later; later &= later - 1)
+          atomicOr(&sh.plan[__ffs((int)later) - 1].cmask, 1u << s);
+      }
+    }
+    cmb = gor<G>(cmb);
+    regfail = (int)gor<G>((unsigned)regfail);
+  }
+  Acc bond = acc_zero<Acc>();
+  if (dep && gl < 2) bond = boundary_term<Pos, Acc, LEAN>(a, rd, P, kind, gl);
+  if (dep && gl < 2) store_acc(P.pq[gl], P.ph[gl], bond);
+  if (run && gl == 0) {
+    if (dep) P.oob = oob;
+    if (err) atomicOr(&P.derr, err);  // E_OVF stays: the pooled pass and commit skip this move's entries
+    P.gtab = gtab;
+    P.fn = (int)nvox;
+    P.fH = huge;
+    store_field(P, soft, hard);
+    if (cmb) atomicOr(&P.cmask, cmb);
+    P.freg = regfail;
+  }
+  __syncwarp();
 }
 
 // Evaluate move t of the batch in slot s (group lanes gl = 0..G-1); `live`
@@ -589,9 +777,8 @@ __device__ __forceinline__ void add_pool_terms(double& s, const MovePlan& P) {
 // around the block-wide deposit); B is the batch's number of moves.
 template <typename Pos, int G, bool LEAN>
 __device__ void evaluate_move(const KArgs& a, SpecShared& sh, int rep, int s, int gl, bool live, int kind,
-                              const cg_move_ctl& c, unsigned long long t, unsigned* draws,
-                              const SlotScratch& sm, const SlotScratch& gm, int* bkeys, unsigned* bmask,
-                              int logHB, int B) {
+                              const cg_move_ctl& c, unsigned long long t, unsigned* picked, int* bkeys,
+                              unsigned* bmask, int B) {
   using Real = Pos;
   using Acc = typename AccOf<Real>::type;
   const RepDev& rd = sh.ws.rd;
@@ -608,7 +795,10 @@ __device__ void evaluate_move(const KArgs& a, SpecShared& sh, int rep, int s, in
   const float* bonds32 = a.bonds32 + rd.bead_off * 8;
   MovePlan& P = sh.plan[s];
   MoveRng g;
-  if (__any_sync(kFull, live)) g.init<G>(a.seed, rep, t, draws, gl);
+  if (__any_sync(kFull, live))
+    g.init<G>(a.seed, rep, t,
+              reinterpret_cast<unsigned*>(reinterpret_cast<unsigned char*>(&sh) + a.spec_off_warps +
+                                          (size_t)s * a.warp_smem + a.off_draws), gl);
   unsigned err = 0;
   const bool check_field = rd.field_kind != 0 && kind != CG_TANGENT_ROTATION;
   const bool density = rd.field_kind == 2;
@@ -620,17 +810,13 @@ __device__ void evaluate_move(const KArgs& a, SpecShared& sh, int rep, int s, in
   long long dEH = 0;  // the exact 1e99 penalties, in kHugeUnit units
   long long nvox = 0;
   bool empty = !live;
-  int gtab = 0, gstage = 0;
-  unsigned cmb = 0;  // position moves: conflicts with earlier moves of the batch
-  SlotScratch S = sm;
-  int* nused = &sh.nused[s];
-  const int Hs = 1 << sm.logH;
+  int gtab = 0, gstage = 0, regfail = 0;
+  unsigned xm = 0;  // the Metropolis draw
+  const int Hs = 1 << a.logH;
   const bool pool = a.pool_on != 0;
-  bool pooled = false;  // a position move whose voxels the CTA's pooled pass evaluates
   if (threadIdx.x == 0) sh.npool = 0;  // every reader of the last batch's pool passed a barrier since
 
   if (kind <= CG_SLIDE) {
-    const ChainView<Pos> cv(a, rd, LEAN);
     Real M[3][4];
     for (int i = 0; i < 3; i++)
       for (int j = 0; j < 4; j++) M[i][j] = i == j ? (Real)1 : (Real)0;
@@ -690,23 +876,22 @@ __device__ void evaluate_move(const KArgs& a, SpecShared& sh, int rep, int s, in
     }
     m = (!live || err) ? 0 : indf - ind0;
     if (live && !err && m == 0) empty = true;
-    if (m > a.stage_cap) { S.stage = gm.stage; gstage = 1; }
-    // voxel table: with the CTA's pooled table (FP32 storage), every move of
-    // up to kPoolMaxBeads beads, optimistically (a pool past 3/4 load sends
-    // the move to its global table); else the slot's own table when the
-    // move's at most 16 m voxels surely fit, or optimistically up to m <=
-    // slots / 4 with the same fallback; global beyond
-    bool sure, blk;
+    if (live && !err && !empty) xm = g.next();  // drawn now: the stream's state is not kept over the deposit
+    if (m > a.stage_cap) gstage = 1;
+    // voxel table: the CTA's pooled table for every move of up to
+    // kPoolMaxBeads beads, optimistically (a pool past 3/4 load sends the move
+    // to its global table); without the pool (a grid of 2^26 voxels and more)
+    // the slot's own table when the move's at most 16 m voxels surely fit, or
+    // optimistically up to m <= slots / 4 with the same fallback; global beyond
+    bool sure = false, blk;
     if (pool) {
-      sure = false;
       blk = density && m > 0 && m <= kPoolMaxBeads;
-      if (density && m > 0 && !blk) { use_table(S, gm); gtab = 1; }
+      gtab = density && m > 0 && !blk;
     } else {
       sure = 16 * m <= Hs;
-      if (!sure && 4 * m > Hs) { use_table(S, gm); gtab = 1; }
+      gtab = !sure && 4 * m > Hs;
       blk = density && m > 0 && !gtab;  // moves with a shared table are deposited by the whole CTA
     }
-    V4<Pos>* stage = reinterpret_cast<V4<Pos>*>(S.stage);  // r, t3, t2 of each moved bead
     if (gl == 0 && live) {
       P.blk = blk ? 1 : 0;
       P.sure = sure ? 1 : 0;
@@ -714,6 +899,7 @@ __device__ void evaluate_move(const KArgs& a, SpecShared& sh, int rep, int s, in
       P.ind0 = (int)ind0;
       P.indf = (int)indf;
       P.gstage = gstage;
+      P.gtab = gtab;
       P.oob = 0;
       P.derr = 0;
       P.cmask = 0;
@@ -721,6 +907,8 @@ __device__ void evaluate_move(const KArgs& a, SpecShared& sh, int rep, int s, in
       P.ph[0] = P.ph[1] = 0;
       P.fq = P.fH = 0;
       P.fh = 0;
+      P.fl0 = P.fl1 = 0;
+      P.fl2 = 0;
       P.fn = P.freg = 0;
       Pos* Mp = reinterpret_cast<Pos*>(P.M);  // in the position type: no conversions
       for (int i = 0; i < 3; i++)
@@ -731,6 +919,7 @@ __device__ void evaluate_move(const KArgs& a, SpecShared& sh, int rep, int s, in
     // earlier moves u of the batch whose written beads [ind0, indf) meet the
     // beads this move reads (its segment and both neighbours); a move with no
     // beads (failed or empty) is never accepted, so it needs no exclusion
+    unsigned cmb = 0;
     for (int u0 = 0; u0 < B; u0 += G) {
       const int u = u0 + gl;
       bool hit = false;
@@ -741,88 +930,23 @@ __device__ void evaluate_move(const KArgs& a, SpecShared& sh, int rep, int s, in
       cmb |= gballot<G>(hit) << u0;
     }
     __syncthreads();
-    if (pool && density) block_field_pool(a, sh, reinterpret_cast<unsigned char*>(&sh), bkeys, bmask);
-    Acc part = acc_zero<Acc>();
-    int oob = 0;
-    bool ovf = false;
-    if (blk) {
-      const unsigned eb = P.derr;
-      ovf = (eb & E_OVF) != 0;
-      pooled = pool && !ovf;
-      err |= eb & ~E_OVF;
-      if (gl == 0) {
-        acc_add(part, load_acc<Acc>(P.pq[0], P.ph[0]));
-        acc_add(part, load_acc<Acc>(P.pq[1], P.ph[1]));
-        oob = P.oob;
-      }
-    }
-    const unsigned peers = group_mask<G>();
-    for (int pass = 0; pass < 2; pass++) {
-      if (pass == 1) {
-        if (!__any_sync(kFull, ovf)) break;
-        if (ovf) clear_table(S, hcol, *nused, gl, G);
-        __syncwarp();
-        if (ovf) {
-          if (gl == 0) *nused = 0;
-          use_table(S, gm);
-          gtab = 1;
-          part = acc_zero<Acc>();
-          oob = 0;
-        }
-        __syncwarp();
-      }
-      // pass 0: the moves the CTA did not deposit; pass 1: overflowed ones
-      const bool run = pass == 0 ? !blk : ovf;
-      const int cap = gtab ? (1 << gm.logH) : (sure ? Hs : (3 * Hs) / 4);
-      const unsigned full_bit = (gtab || sure) ? E_SPIN : E_OVF;
-      unsigned e = 0;
-      // the group's own deposit: one bead per lane, its corners two by two,
-      // the boundary bonds on its first two lanes
-      for (long long kb = 0; __any_sync(kFull, run && kb < m && !(e & E_OVF)); kb += G) {
-        const long long k = kb + gl;
-        bool act = run && k < m && !(e & E_OVF);
-        BeadCells<Pos> c = {};
-        unsigned sw = 0;
-        if (act) {
-          int ob;
-          if (density) sw = st[ind0 + k];
-          act = place_bead(rd, gf, cv, kind, M, ind0 + k, stage + 3 * k, density, check_field && rd.confine_kind,
-                           c, e, ob);
-          oob += ob;
-        }
-        if (density) {
-          for (int cl = 0; cl < kLanesPerBead; cl++) {
-            int vq[2 * kCornersPerLane];
-            long long q[2 * kCornersPerLane];
-            corner_terms(gf, c, cl, vq, q);
-            bool want[2 * kCornersPerLane];
-#pragma unroll
-            for (int j = 0; j < 2 * kCornersPerLane; j++) want[j] = act && q[j] != 0 && !(e & E_OVF);
-            int slot[2 * kCornersPerLane];
-            claim_slots<2 * kCornersPerLane>(S.keys, S.used, nused, S.logH, vq, want, slot, e, cap, full_bit, peers);
-            if (!(e & full_bit)) {
-#pragma unroll
-              for (int j = 0; j < 2 * kCornersPerLane; j++)
-                if (want[j]) add_corner(S.vals, hcol, slot[j], q[j], sw, rd.nb, !gtab);
-            }
-          }
-          e = gor<G>(e);  // a full table ends the group's passes together
-        }
-      }
-      if (run && m > 0 && gl < 2) acc_add(part, boundary_term<Pos, Acc, LEAN>(a, rd, P, kind, gl));
-      e = gor<G>(e);
-      if (run) ovf = (e & E_OVF) != 0;
-      err |= e & ~E_OVF;
-    }
-    err = gor<G>(err);
-    dEp = gsum<G>(part);
-    if (check_field && rd.confine_kind) {
-      int oo = gsum<G>(oob);
+    if (pool && density) block_field_pool<Pos>(a, sh, reinterpret_cast<unsigned char*>(&sh), bkeys, bmask);
+    const bool own = m > 0 && (!blk || !pool || (P.derr & E_OVF));
+    if (__any_sync(kFull, own)) own_path<Pos, G, LEAN>(a, sh, rep, s, gl, own, kind, bkeys, bmask);
+    if (gl == 0 && live && cmb) atomicOr(&P.cmask, cmb);
+    if (pool && density) __syncthreads();  // the pooled field pass is complete
+    if (m > 0) {  // the plan's results
+      acc_add(dEp, load_acc<Acc>(P.pq[0], P.ph[0]));
+      acc_add(dEp, load_acc<Acc>(P.pq[1], P.ph[1]));
+      plan_field(P, dEs, dEh);
+      dEH = P.fH;
+      const int oo = P.oob;
       dEH += ((long long)(oo >> 16) - (long long)(oo & 0xFFFF)) << 40;
+      err |= P.derr & ~E_OVF;
+      nvox = P.fn;
+      regfail = P.freg;
+      gtab = P.gtab;
     }
-    __syncwarp();
-    if (density)
-      field_dE_voxels<G>(ws, a, hcol, S.keys, S.used, S.vals, *nused, gl, nvox, dEs, dEh, dEH, !gtab);
   } else if (kind == CG_TANGENT_ROTATION) {
     Real ang = 0;
     long long n = 0;
@@ -832,7 +956,8 @@ __device__ void evaluate_move(const KArgs& a, SpecShared& sh, int rep, int s, in
       if (n > N) err |= E_WINDOW;
     }
     m = (!live || err) ? 0 : n;
-    if (m > a.stage_cap) { S.stage = gm.stage; S.idx = gm.idx; gstage = 1; }
+    if (m > a.stage_cap) gstage = 1;
+    const SlotScratch S = gstage ? global_slot<Pos>(a, rep, s) : shared_slot(a, sh, s);
     int* idx = S.idx;
     // n distinct random beads, drawn in order with redraws (get_inds): G
     // candidates per round, the first fresh ones taken in draw order.  Beads
@@ -852,14 +977,14 @@ __device__ void evaluate_move(const KArgs& a, SpecShared& sh, int rep, int s, in
       const unsigned grp = __match_any_sync(kFull, cand) & gmask;
       const unsigned gshift = G == 32 ? 0u : ((threadIdx.x & 31u) & ~(unsigned)(G - 1));
       const bool first = ((grp >> gshift) & lt) == 0;
-      const bool fresh = want && first && !(rounds > 0 && ((S.picked[cand >> 5] >> (cand & 31)) & 1u));
+      const bool fresh = want && first && !(rounds > 0 && ((picked[cand >> 5] >> (cand & 31)) & 1u));
       const unsigned bal = gballot<G>(fresh);
       const long long need = m - got;
       const int cnt = __popc(bal);
       const int rank = __popc(bal & lt);
       if (fresh && rank < need) {
         idx[got + rank] = (int)cand;
-        if (cnt < need) atomicOr(&S.picked[cand >> 5], 1u << (cand & 31));
+        if (cnt < need) atomicOr(&picked[cand >> 5], 1u << (cand & 31));
       }
       if (want) {
         rounds++;
@@ -932,7 +1057,7 @@ __device__ void evaluate_move(const KArgs& a, SpecShared& sh, int rep, int s, in
     // the picked marks only serve the redraws of this move
     for (long long k = gl; k < marked; k += G) {
       int i = idx[k];
-      atomicAnd(&S.picked[i >> 5], ~(1u << (i & 31)));
+      atomicAnd(&picked[i >> 5], ~(1u << (i & 31)));
     }
     __syncwarp();
     if (m > 0) {
@@ -949,9 +1074,11 @@ __device__ void evaluate_move(const KArgs& a, SpecShared& sh, int rep, int s, in
     }
     m = (!live || err) ? 0 : indf - ind0;
     const int nt = rd.sites[bsel];
-    if (m > a.stage_cap) { S.idx = gm.idx; gstage = 1; }
-    if (8 * m > Hs) { use_table(S, gm); gtab = 1; }
-    int* idx = S.idx;
+    if (m > a.stage_cap) gstage = 1;
+    if (8 * m > Hs) gtab = 1;
+    const SlotScratch S = gtab ? global_slot<Pos>(a, rep, s) : shared_slot(a, sh, s);
+    int* nused = &sh.nused[s];
+    int* idx = gstage ? global_slot<Pos>(a, rep, s).idx : shared_slot(a, sh, s).idx;
     Acc part = acc_zero<Acc>();
     int dbl = 0;
     // eight lanes per bead, one trilinear corner each: corner lane 0 takes
@@ -1010,48 +1137,24 @@ __device__ void evaluate_move(const KArgs& a, SpecShared& sh, int rep, int s, in
       if (m > 0) add_intra(ws, bsel, ddb, dEs, dEh);
     }
     if (gl == 0 && live) P.bsel = bsel;
+    // register the touched voxels for the conflict test
+    if (density) {
+      const int nu = (live && !err) ? *nused : 0;
+      for (int i = gl; i < nu; i += G) {
+        const int b = block_insert(bkeys, a.spec_logHB, S.keys[S.used[i]]);
+        S.bslot[i] = b;
+        if (b < 0) regfail = 1;
+        else atomicOr(&bmask[b], 1u << s);
+      }
+      regfail = (int)gor<G>((unsigned)regfail);
+    }
   }
   err = gor<G>(err);
-  // register the touched voxels for the conflict test
-  // (position moves: the moves that registered a voxel first are this
-  // move's conflicts if earlier in the batch; a later move that registered
-  // it first learns of this one through its plan's mask)
-  int regfail = 0;
-  if (density && check_field) {
-    const int nu = (live && !err && !empty) ? *nused : 0;
-    const unsigned below = (1u << s) - 1u, above = ~((2u << s) - 1u);
-    for (int i = gl; i < nu; i += G) {
-      int v = S.keys[S.used[i]];
-      int b = block_insert(bkeys, logHB, v);
-      S.bslot[i] = b;
-      if (b < 0) {
-        regfail = 1;
-      } else {
-        const unsigned prior = atomicOr(&bmask[b], 1u << s);
-        if (kind <= CG_SLIDE) {
-          cmb |= prior & below;
-          for (unsigned later = prior & above; later; later &= later - 1)
-            atomicOr(&sh.plan[__ffs((int)later) - 1].cmask, 1u << s);
-        }
-      }
-    }
-    regfail = (int)gor<G>((unsigned)regfail);
-  }
-  if (kind <= CG_SLIDE) {
-    cmb = gor<G>(cmb);
-    if (gl == 0 && live) atomicOr(&P.cmask, cmb);
-  }
-  if (kind <= CG_SLIDE && pool && density) {
-    __syncthreads();  // the pooled field pass is complete
-    if (pooled) {
-      add_pool_terms(dEs, P);
-      dEH += P.fH;
-      nvox = P.fn;
-      regfail |= P.freg;
-    }
-  }
   bool dec = false;
-  if (live && !err && !empty) dec = decide(g.next(), dEp, dEs, with_huge(dEh, dEH), gl == 0 ? &P.dE : nullptr);
+  if (live && !err && !empty) {
+    if (kind > CG_SLIDE) xm = g.next();
+    dec = decide(xm, dEp, dEs, with_huge(dEh, dEH), gl == 0 ? &P.dE : nullptr);
+  }
   if (gl == 0 && live) {
     P.kind = kind; P.m = (int)m; P.ind0 = (int)ind0; P.indf = (int)indf;
     P.empty = empty ? 1 : 0; P.err = (int)err; P.regfail = regfail; P.dec = dec ? 1 : 0;
@@ -1061,17 +1164,16 @@ __device__ void evaluate_move(const KArgs& a, SpecShared& sh, int rep, int s, in
 }
 
 // Bits of earlier moves of the batch (u < s) whose footprint meets move s's.
-template <int G>
+template <typename Pos, int G>
 __device__ void conflict_mask(const KArgs& a, SpecShared& sh, unsigned char* smem, int rep, int s, int gl,
-                              bool live, int kind, int B, const SlotScratch& sm, const SlotScratch& gm,
-                              const unsigned* bmask) {
+                              bool live, int kind, int B, const unsigned* bmask) {
   MovePlan& P = sh.plan[s];
   const RepDev& rd = sh.ws.rd;
   const bool act = live && !P.err && !P.empty;
   unsigned cm = 0;
   if (rd.field_kind == 2 && kind != CG_TANGENT_ROTATION) {
     const int nu = act ? sh.nused[s] : 0;
-    const int* bs = P.gtab ? gm.bslot : sm.bslot;
+    const int* bs = (P.gtab ? global_slot<Pos>(a, rep, s) : shared_slot(a, sh, s)).bslot;
     for (int i = gl; i < nu; i += G) {
       int b = bs[i];
       if (b >= 0) cm |= bmask[b];
@@ -1081,7 +1183,7 @@ __device__ void conflict_mask(const KArgs& a, SpecShared& sh, unsigned char* sme
   cm &= (1u << s) - 1u;
   if (kind == CG_TANGENT_ROTATION) {
     // rotated beads of u against those of s and their neighbours
-    const int* lw = P.gstage ? gm.idx : sm.idx;
+    const int* lw = (P.gstage ? global_slot<Pos>(a, rep, s) : shared_slot(a, sh, s)).idx;
     for (int u = 0; u < B; u++) {
       const MovePlan& U = sh.plan[u];
       int hit = 0;
@@ -1145,8 +1247,8 @@ __device__ __forceinline__ void update_amplitudes(cg_move_ctl& c) {
 }
 
 template <typename Pos, int G>
-__device__ void commit_and_clear(const KArgs& a, SpecShared& sh, int s, int gl, bool accept,
-                                 const SlotScratch& sm, const SlotScratch& gm, int* bkeys, unsigned* bmask) {
+__device__ void commit_and_clear(const KArgs& a, SpecShared& sh, int rep, int s, int gl, bool accept, int* bkeys,
+                                 unsigned* bmask) {
   const MovePlan& P = sh.plan[s];
   const RepDev& rd = sh.ws.rd;
   const int ncol = a.ncol, hcol = a.hcol;
@@ -1154,14 +1256,11 @@ __device__ void commit_and_clear(const KArgs& a, SpecShared& sh, int s, int gl, 
   V4<Pos>* t34w = reinterpret_cast<V4<Pos>*>(a.t34) + rd.bead_off;
   V4<Pos>* t24w = reinterpret_cast<V4<Pos>*>(a.t24) + rd.bead_off;
   unsigned* st = a.states + rd.bead_off;
-  const V4<Pos>* stage = reinterpret_cast<const V4<Pos>*>(P.gstage ? gm.stage : sm.stage);
-  const int* idx = P.gstage ? gm.idx : sm.idx;
-  int* keys = P.gtab ? gm.keys : sm.keys;
-  int* used = P.gtab ? gm.used : sm.used;
-  int* bslot = P.gtab ? gm.bslot : sm.bslot;
-  long long* vals = P.gtab ? gm.vals : sm.vals;
   const int m = P.m;
   if (accept) {
+    const SlotScratch S = P.gstage ? global_slot<Pos>(a, rep, s) : shared_slot(a, sh, s);
+    const V4<Pos>* stage = reinterpret_cast<const V4<Pos>*>(S.stage);
+    const int* idx = S.idx;
     if (P.kind <= CG_SLIDE) {
       for (int k = gl; k < m; k += G) {
         const long long i = (long long)P.ind0 + k;
@@ -1187,6 +1286,10 @@ __device__ void commit_and_clear(const KArgs& a, SpecShared& sh, int s, int gl, 
     }
   }
   const int nu = sh.nused[s];
+  if (nu == 0) return;  // no table of its own
+  const SlotScratch T = P.gtab ? global_slot<Pos>(a, rep, s) : shared_slot(a, sh, s);
+  int *keys = T.keys, *used = T.used, *bslot = T.bslot;
+  long long* vals = T.vals;
   long long* grid = a.grid + rd.vox_off * ncol;
   for (int i = gl; i < nu; i += G) {
     int slot = used[i];
@@ -1225,25 +1328,6 @@ __global__ void __maxnreg__(168) spec_kernel(KArgs a) {
   unsigned* bmask = reinterpret_cast<unsigned*>(smem + a.spec_off_bmask);
   const int HB = 1 << a.spec_logHB;
   const int hcol = a.hcol;
-  unsigned char* wb = smem + a.spec_off_warps + (size_t)slot * a.warp_smem;
-  unsigned* draws = reinterpret_cast<unsigned*>(wb + a.off_draws);
-  SlotScratch sm, gm;
-  sm.keys = reinterpret_cast<int*>(wb + a.off_keys);
-  sm.used = reinterpret_cast<int*>(wb + a.off_used);
-  sm.bslot = reinterpret_cast<int*>(wb + a.off_bslot);
-  sm.vals = reinterpret_cast<long long*>(wb + a.off_vals);
-  sm.logH = a.logH;
-  sm.stage = wb + a.off_stage;
-  sm.idx = reinterpret_cast<int*>(wb + a.off_idx);
-  const long long gi = (long long)rep * Sn + slot;
-  const long long Hg = 1LL << a.g_logH;
-  gm.keys = a.g_keys + gi * Hg;
-  gm.used = a.g_used + gi * Hg;
-  gm.bslot = a.g_bslot + gi * Hg;
-  gm.vals = a.g_vals + gi * Hg * hcol;
-  gm.logH = a.g_logH;
-  gm.stage = reinterpret_cast<V4<Pos>*>(a.g_stage) + gi * a.g_stage_cap * 3;
-  gm.idx = a.g_idx + gi * a.g_stage_cap;
   {
     const unsigned* src = reinterpret_cast<const unsigned*>(a.reps + rep);
     unsigned* dst = reinterpret_cast<unsigned*>(&sh.ws.rd);
@@ -1253,6 +1337,7 @@ __global__ void __maxnreg__(168) spec_kernel(KArgs a) {
     for (int i = tid; i < (int)(5 * sizeof(cg_move_ctl) / 4); i += blockDim.x) cd[i] = cs[i];
     for (int i = tid; i < HB; i += blockDim.x) { bkeys[i] = -1; bmask[i] = 0u; }
     for (int i = tid; i < 30; i += blockDim.x) sh.ws.tally[i] = 0;
+    const SlotScratch sm = shared_slot(a, sh, slot);
     for (int i = gl; i < (1 << a.logH); i += G) { sm.keys[i] = -1; sm.bslot[i] = -1; }
     for (int i = gl; i < (1 << a.logH) * hcol; i += G) sm.vals[i] = 0;
     if (gl == 0) sh.nused[slot] = 0;
@@ -1276,7 +1361,7 @@ __global__ void __maxnreg__(168) spec_kernel(KArgs a) {
   }
   __syncthreads();
   const long long words = (sh.ws.rd.n_beads + 31) / 32;
-  sm.picked = gm.picked = a.picked + a.picked_off[rep] + slot * words;
+  unsigned* picked = a.picked + a.picked_off[rep] + slot * words;
 
   for (long long step = 0; step < a.n_steps; step++) {
     for (int ci = 0; ci < a.n_ctl; ci++) {
@@ -1296,11 +1381,11 @@ __global__ void __maxnreg__(168) spec_kernel(KArgs a) {
           const int B = (int)(c.num_per_cycle - done < Sn ? c.num_per_cycle - done : Sn);
           const bool wlive = warp * GPW < B;  // the warp has a move of this batch
           const bool live = slot < B;
-          evaluate_move<Pos, G, LEAN>(a, sh, rep, slot, gl, live, kind, c, sh.t0 + (unsigned long long)slot, draws,
-                                sm, gm, bkeys, bmask, a.spec_logHB, B);
+          evaluate_move<Pos, G, LEAN>(a, sh, rep, slot, gl, live, kind, c, sh.t0 + (unsigned long long)slot, picked,
+                                      bkeys, bmask, B);
           __syncthreads();
           if (kind > CG_SLIDE) {  // position moves set their masks while evaluating
-            if (wlive) conflict_mask<G>(a, sh, smem, rep, slot, gl, live, kind, B, sm, gm, bmask);
+            if (wlive) conflict_mask<Pos, G>(a, sh, smem, rep, slot, gl, live, kind, B, bmask);
             __syncthreads();
           }
           // Resolve, computed by every warp from the plans (lane u reads move u):
@@ -1355,7 +1440,7 @@ __global__ void __maxnreg__(168) spec_kernel(KArgs a) {
             }
           }
           if (wlive && live)
-            commit_and_clear<Pos, G>(a, sh, slot, gl, slot < cut && ((acc >> slot) & 1u), sm, gm, bkeys, bmask);
+            commit_and_clear<Pos, G>(a, sh, rep, slot, gl, slot < cut && ((acc >> slot) & 1u), bkeys, bmask);
           __syncwarp();
           if (live && gl == 0) sh.nused[slot] = 0;
           if (kind <= CG_SLIDE && a.pool_on && sh.ws.rd.field_kind == 2)
