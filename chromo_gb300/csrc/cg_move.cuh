@@ -30,10 +30,11 @@ __device__ __forceinline__ void setup_f32(WarpShared& ws) {
 // Add d to column `col` of a hash entry.  Global-memory tables take one 64-bit
 // atomic.  Shared-memory tables (split = true) keep each column as two 32-bit
 // counters, d = hi * 2^21 + lo with lo in [0, 2^21): 32-bit shared atomics are
-// native and several times faster than 64-bit ones.  A shared table has at
-// most 1,024 slots and serves moves of m <= slots / 16 beads, so a column gets
-// at most 16 m <= 1,024 contributions of |d| < 2^42: |sum hi| < 2^10 * 3 * 2^19
-// and sum lo < 2^10 * 2^21, both below 2^31.
+// native and several times faster than 64-bit ones.  The low counter is read
+// unsigned.  A column gets at most 2 m contributions s (hi 2^21 + lo) with
+// s <= 3, |hi| <= 2^19 and m <= 256 beads (kPoolMaxBeads, and the moves a
+// 1,024-slot table takes): sum lo <= 512 * 3 * 2^21 < 2^32 and |sum hi| <= 512 *
+// 3 * 2^19 < 2^31.
 __device__ __forceinline__ void add_delta(long long* vals, int ncol, int slot, int col, long long d,
                                           bool split = false) {
   if (d == 0) return;
@@ -51,7 +52,7 @@ __device__ __forceinline__ void add_delta(long long* vals, int ncol, int slot, i
 __device__ __forceinline__ long long hash_delta(const long long* cell, bool split) {
   if (!split) return *cell;
   const int* half = reinterpret_cast<const int*>(cell);
-  return (long long)half[1] * 2097152LL + (long long)half[0];
+  return (long long)half[1] * 2097152LL + (long long)(unsigned)half[0];
 }
 
 // Linear probing for `key` after its home slot `start` was found taken by
@@ -151,6 +152,7 @@ __device__ __forceinline__ void claim_slots(int* keys, int* used, int* nused, in
                                             int cap, unsigned full_bit, unsigned peers) {
   int prev[NQ];
   bool fresh[NQ];
+  unsigned pend = 0;  // claims whose home slot holds another key
 #pragma unroll
   for (int j = 0; j < NQ; j++) {
     slot[j] = (int)(((unsigned)v[j] * 0x9E3779B1u) >> (32 - logH));
@@ -159,16 +161,28 @@ __device__ __forceinline__ void claim_slots(int* keys, int* used, int* nused, in
 #pragma unroll
   for (int j = 0; j < NQ; j++) {
     fresh[j] = prev[j] == -1;
-    if (!fresh[j] && prev[j] != v[j]) {
-      const int r = hash_probe_packed(keys, logH, v[j], slot[j]);
-      if (r < 0) {
-        err |= full_bit;
-        slot[j] = -1;
-      } else {
-        fresh[j] = (r >> 30) & 1;
-        slot[j] = r & ((1 << 30) - 1);
-      }
-    }
+    if (!fresh[j] && prev[j] != v[j]) pend |= 1u << j;
+  }
+  // linear probing of the displaced claims, one loop for all of a lane's: a
+  // warp nearly always holds a few, and a call per claim took 2.4 k cycles a
+  // pass with the claims (256 chains, 20 MC steps: 16.4 -> 14.1 ms together
+  // with the branch-free wrap of voxel_axes and the state times split halves of
+  // add_corner)
+  const int mask = (1 << logH) - 1;
+  for (int it = 1; pend; it++) {
+    const int j = __ffs((int)pend) - 1;
+    int key = v[0], h = slot[0];
+#pragma unroll
+    for (int i = 1; i < NQ; i++)
+      if (i == j) { key = v[i]; h = slot[i]; }
+    h = (h + 1) & mask;
+    const bool full = it > mask;  // every slot of the table seen
+    const int p = full ? key : atomicCAS(&keys[h], -1, key);
+    if (full) { h = -1; err |= full_bit; }
+#pragma unroll
+    for (int i = 0; i < NQ; i++)
+      if (i == j) { slot[i] = h; fresh[i] = p == -1; }
+    if (p == -1 || p == key) { pend &= pend - 1; it = 0; }
   }
   const unsigned lane = threadIdx.x & 31u, lt = (1u << lane) - 1u;
   const int leader = __ffs((int)peers) - 1;
@@ -200,10 +214,25 @@ __device__ __forceinline__ unsigned group_mask() {
 
 // Add a corner's contribution q to a voxel-table slot: the bead column, and
 // q times the bead's state for each binder column (states packed as bytes).
+// Split counters take the state times each half.
 __device__ __forceinline__ void add_corner(long long* vals, int hcol, int slot, long long q, unsigned sw, int nb,
                                            bool split) {
-  add_delta(vals, hcol, slot, 0, q, split);
-  for (int b = 0; b < nb; b++) add_delta(vals, hcol, slot, 1 + b, q * (long long)((sw >> (8 * b)) & 0xFF), split);
+  if (split) {
+    int* half = reinterpret_cast<int*>(vals + slot * hcol);
+    const int lo = (int)(q & 0x1FFFFF), hi = (int)(q >> 21);
+    atomicAdd(half, lo);
+    atomicAdd(half + 1, hi);
+    for (int b = 0; b < nb; b++) {
+      const int st = (int)((sw >> (8 * b)) & 0xFF);
+      if (st) {
+        atomicAdd(half + 2 * b + 2, st * lo);
+        atomicAdd(half + 2 * b + 3, st * hi);
+      }
+    }
+  } else {
+    add_delta(vals, hcol, slot, 0, q);
+    for (int b = 0; b < nb; b++) add_delta(vals, hcol, slot, 1 + b, q * (long long)((sw >> (8 * b)) & 0xFF));
+  }
 }
 
 // One voxel's grid row -- bead weight, then one column per binder -- with

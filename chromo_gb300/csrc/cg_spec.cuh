@@ -141,9 +141,9 @@ struct ChainView {
         twist(!lean && rd.twist ? a.twist + rd.bead_off * 2 : nullptr) {}
 };
 
-// Largest position move of the pooled voxel table: an entry gets at most 2 m
-// contributions of |d| < 2^42, which its two 32-bit split counters hold for
-// m < 512.
+// Largest position move of a shared voxel table (the split counters' bound,
+// see add_delta), halved for each axis of a single voxel, on which a bead's
+// lower and upper corners fall in the same voxel.
 constexpr int kPoolMaxBeads = 256;
 
 // Lanes that share one bead's trilinear corners in the block-wide deposit,
@@ -353,9 +353,11 @@ __device__ void block_deposit(const KArgs& a, SpecShared& sh, int rep, int B, in
   const int total = __shfl_sync(kFull, end, 31);
   // beads per warp and round: an even share, in whole passes of the corners
   constexpr int BP = 32 / kLanesPerBead;
-  const int rounds = (total + 32 * W - 1) / (32 * W);
-  const int share = rounds > 0 ? (total + rounds * W - 1) / (rounds * W) : 0;
-  const int run = (share + BP - 1) / BP * BP;
+  // (by steps: a batch has a few hundred beads)
+  int per = W;  // warps times rounds
+  while (32 * per < total) per += W;
+  int run = BP;
+  while (run * per < total) run += BP;
   for (int b0 = warp * run; b0 < total; b0 += W * run) {
     const int b = b0 + lane;
     // the bead's move: the number of moves whose beads end at or before b
@@ -884,12 +886,13 @@ __device__ void evaluate_move(const KArgs& a, SpecShared& sh, int rep, int s, in
     // the slot's own table when the move's at most 16 m voxels surely fit, or
     // optimistically up to m <= slots / 4 with the same fallback; global beyond
     bool sure = false, blk;
+    const int most = kPoolMaxBeads >> ((rd.nx == 1) + (rd.ny == 1) + (rd.nz == 1));
     if (pool) {
-      blk = density && m > 0 && m <= kPoolMaxBeads;
+      blk = density && m > 0 && m <= most;
       gtab = density && m > 0 && !blk;
     } else {
       sure = 16 * m <= Hs;
-      gtab = !sure && 4 * m > Hs;
+      gtab = (!sure && 4 * m > Hs) || m > most;
       blk = density && m > 0 && !gtab;  // moves with a shared table are deposited by the whole CTA
     }
     if (gl == 0 && live) {

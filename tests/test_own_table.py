@@ -1,7 +1,9 @@
-"""Position moves that leave the CTA's pooled voxel table: many long segments
-in flight (the pool overflows; segments over 256 beads never enter it) and a
-grid of 2^26 voxels (no pool: each slot's own table).  Several moves in flight
-equal one at a time bit for bit, and the grid equals its re-deposit."""
+"""Position moves at the edges of the CTA's pooled voxel table: many long
+segments in flight (the pool overflows; segments over 256 beads never enter it),
+a grid of 2^26 voxels (no pool: each slot's own table) and grids with axes of a
+single voxel (a bead's corners share it, the most that an entry's split counters
+hold).  Several moves in flight equal one at a time bit for bit, and the grid
+equals its re-deposit."""
 import numpy as np
 import pytest
 
@@ -23,7 +25,7 @@ def _sim(n, dims, amp, fp64, W):
     sim = nat.Sim([n], [dims], 1, pos_fp64=fp64, max_segment=amp + 2, max_tangent=n, warps_per_block=W)
     sim.set_chain(0, r=r, t3=t3, t2=t2, states=states, marks=marks, bonds=bonds_array(eb, g, ep, epp, eta))
     sim.set_field(0, field_params(field_kind=2, nxyz=dims, widths=tuple(40.0 * d for d in dims), n_binders=1,
-                                  chi=1.0, bead_vol=523.6, pref=[-100.0], intra=[-3.9]))
+                                  chi=1.0, vf_limit=1e6, bead_vol=523.6, pref=[-100.0], intra=[-3.9]))
     sim.set_binding(0, binding_params(sites=[2], e_mod=[-0.01], e_nomod=[1.52], mu=[-0.4]))
     sim.set_controllers(0, [move_ctl(m, amp_move=0.2 if m != "slide" else 2.0, amp_bead=amp, num_per_cycle=24,
                                      simple=False) for m in ("crank_shaft", "end_pivot", "slide")])
@@ -32,17 +34,21 @@ def _sim(n, dims, amp, fp64, W):
 
 
 @pytest.mark.parametrize("fp64", [False, True])
-@pytest.mark.parametrize("n,dims,amp", [(3000, (20, 21, 22), 600), (400, (30, 30, 30), 255), (500, (8192, 8192, 1), 120)])
+@pytest.mark.parametrize("n,dims,amp", [(3000, (20, 21, 22), 600), (400, (30, 30, 30), 255), (500, (8192, 8192, 1), 120),
+                                        (400, (1, 1, 1), 255), (400, (1, 40, 1), 200)])
 def test_long_moves_and_large_grids_equal_sequential(n, dims, amp, fp64):
     got = []
     for W in (1, 12):
         sim = _sim(n, dims, amp, fp64, W)
         sim.run(2, 99)
         sim.sync()
-        field = sim.energy(0)[2]
+        field, small = sim.energy(0)[2], np.prod(dims) < 1e6
+        grid = sim.density(0) if small else None
         chain = sim.get_chain(0)
         sim.deposit(-1)
         np.testing.assert_allclose(sim.energy(0)[2], field, rtol=1e-12)
+        if small:
+            np.testing.assert_array_equal(sim.density(0), grid)
         got.append(chain + (sim.tally(0),))
         sim.close()
     assert got[0][-1][:3, 1].sum() > 0  # moves were accepted
