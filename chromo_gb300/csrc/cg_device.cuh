@@ -753,8 +753,16 @@ static __device__ __noinline__ void fast_axes_ool(const RepDev& rd, const GridF&
 template <typename Real>
 __device__ __forceinline__ void move_axes(const RepDev& rd, const GridF& gf, const Real pos[3], Real wl[3],
                                           int lo[3], int hi[3]) {
-  if (rd.fast_n > 0) fast_axes_ool(rd, gf, pos, wl, lo, hi);
-  else voxel_axes(rd, gf, pos, wl, lo, hi);
+  if (rd.fast_n > 0) {
+    // through copies: arrays passed to a call live in local memory, on both paths
+    Real p[3], w[3];
+    int l[3], h[3];
+    for (int j = 0; j < 3; j++) p[j] = pos[j];
+    fast_axes_ool(rd, gf, p, w, l, h);
+    for (int j = 0; j < 3; j++) { wl[j] = w[j]; lo[j] = l[j]; hi[j] = h[j]; }
+  } else {
+    voxel_axes(rd, gf, pos, wl, lo, hi);
+  }
 }
 
 // Corner l (bit 0: x, bit 1: y, bit 2: z upper) of the eight trilinear
