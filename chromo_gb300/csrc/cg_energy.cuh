@@ -7,6 +7,8 @@
 // (chromo/polymers.pyx:1383-1538), and the field energy in the form whose
 // differences are the per-move field dE (chromo/fields.pyx:1675-1875).
 #pragma once
+#include <cooperative_groups.h>
+
 #include "cg_device.cuh"
 #include "cg_kernels.h"
 #include "cg_move.cuh"
@@ -67,6 +69,205 @@ __device__ __forceinline__ void voxel_energy(const KArgs& a, const RepDev& rd, l
   // it costs 1e99 vf, which does not depend on chi)
   if (!(vf > rd.vf_limit)) p.sx += sv;
   p.fe += vf > rd.vf_limit ? kEHugeField * vf : rd.chi * sv;
+}
+
+// ---------------------------------------------------------------- sums of one replica
+// The energies, the exchange's S and the derivative terms are sums over one
+// replica's beads and voxels.  A replica is taken by a cluster of kSumCtas
+// CTAs, whose partial sums meet in distributed shared memory and are added in
+// rank order: no workspace, the same bits every time, and 8 x R CTAs in flight
+// (one CTA per replica left most of the GPU idle below 152 replicas).  FP64
+// runs at 1/64 of the FP32 rate here, so the loops hold only the FP64
+// operations the sums need: rows of empty voxels are skipped (two thirds of a
+// 40^3 grid of a 5,000-bead chain), the volume factors are applied once to the
+// sums of products of fixed-point values (uniform volumes), vf > vf_limit is an
+// integer comparison, products are FMAs, and each bond's bead before it comes
+// from the neighbouring lane, already converted.  Upload, deposit and energies
+// of 256 chains of 2,000-20,000 beads: 7.06 -> 2.90 ms (the energies alone took
+// 4.6 ms with one CTA per replica and five divisions a voxel).
+constexpr int kSumCtas = 8;
+constexpr int kSumThreads = 256;
+
+// 16 sums over the CTAs of a cluster, valid in the first 16 threads of rank 0
+// (thread k: sum k).  Every thread of the cluster calls it.  Within a warp the
+// lanes halve the set of sums they carry at each step (16 FP64 additions
+// instead of 80).
+__device__ __forceinline__ double cluster_sums(double (&v)[16], double (*sh)[16]) {
+  namespace cgr = cooperative_groups;
+  cgr::cluster_group cl = cgr::this_cluster();
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+#pragma unroll
+  for (int h = 8, o = 16; h >= 1; h >>= 1, o >>= 1) {
+    const bool up = lane & o;
+#pragma unroll
+    for (int k = 0; k < h; k++) {
+      const double keep = up ? v[k + h] : v[k], give = up ? v[k] : v[k + h];
+      v[k] = keep + __shfl_xor_sync(kFull, give, o);
+    }
+  }
+  v[0] += __shfl_xor_sync(kFull, v[0], 1);
+  // lane l holds sum (bits 4, 3, 2, 1 of l as bits 3, 2, 1, 0)
+  if (!(lane & 1)) sh[warp][lane >> 1] = v[0];
+  __syncthreads();
+  double t = 0;
+  if (threadIdx.x < 16) {
+    for (int w = 0; w < kSumThreads / 32; w++) t += sh[w][threadIdx.x];
+    sh[0][threadIdx.x] = t;
+  }
+  cl.sync();
+  if (cl.block_rank() == 0 && threadIdx.x < 16)
+    for (int r = 1; r < kSumCtas; r++) t += cl.map_shared_rank(&sh[0][0], r)[threadIdx.x];
+  cl.sync();  // no CTA leaves while its sums are read
+  return t;
+}
+
+// Largest fixed-point bead weight of a voxel whose volume fraction, as the
+// FP64 expression of voxel_energy gives it, is not above vf_limit (that
+// expression does not decrease with the weight).  Uniform volumes.
+__device__ __forceinline__ long long weight_at_limit(const RepDev& rd) {
+  auto over = [&](long long n) { return ((double)n * kFxInv) / rd.vol_bin * rd.bead_vol > rd.vf_limit; };
+  const double est = rd.vf_limit / rd.bead_vol * rd.vol_bin * kFxScale;
+  if (!(est < 4e18)) return 0x7FFFFFFFFFFFFFFFLL;
+  if (!(est > 0)) return over(0) ? -1 : 0;  // limits of 0 and below: only empty voxels, or none
+  long long lo = (long long)(est * (1 - 4e-15)) - 2, hi = (long long)(est * (1 + 4e-15)) + 2;
+  if (lo < 0) lo = 0;
+  while (hi - lo > 1) {
+    const long long mid = lo + (hi - lo) / 2;
+    if (over(mid)) hi = mid;
+    else lo = mid;
+  }
+  return lo;
+}
+
+// One CTA's part of a replica's voxels: f(voxel, row) for its thread's rows, or
+// (SKIP) for those of them that are not empty.
+template <bool SKIP, class F>
+__device__ __forceinline__ void for_each_row(const KArgs& a, const RepDev& rd, int rank, const F& f) {
+  const long long* grid = a.grid + rd.vox_off * a.ncol;
+  const long long per = (rd.n_vox + kSumCtas - 1) / kSumCtas;
+  const long long v0 = rank * per, v1 = v0 + per < rd.n_vox ? v0 + per : rd.n_vox;
+  constexpr int U = 4;  // rows in flight per thread
+  for (long long v = v0 + threadIdx.x; v < v1; v += U * kSumThreads) {
+    long long row[U][4];
+#pragma unroll
+    for (int u = 0; u < U; u++) {
+      row[u][0] = row[u][1] = row[u][2] = row[u][3] = 0;
+      const long long w = v + u * kSumThreads;
+      if (w < v1) load_row(grid + w * a.ncol, a.ncol, row[u]);
+    }
+#pragma unroll
+    for (int u = 0; u < U; u++)
+      if (SKIP ? (row[u][0] | row[u][1] | row[u][2] | row[u][3]) != 0 : v + u * kSumThreads < v1)
+        f(v + u * kSumThreads, row[u]);
+  }
+}
+
+// Non-uniform volumes: an empty voxel adds nothing, unless its volume is not
+// positive (0 / 0 is the energy's value there).
+__device__ __forceinline__ bool empty_voxel(const KArgs& a, const RepDev& rd, long long v, const long long (&row)[4]) {
+  return (row[0] | row[1] | row[2] | row[3]) == 0 && a.access_vol[rd.vox_off + v] > 0;
+}
+
+// Sums of products of the fixed-point columns over a replica's voxels
+// (uniform volumes): bead weight squared at or below the limit and above it,
+// binder columns squared and in pairs (01, 02, 12), and the FP64 volume
+// fractions above the limit.
+struct GridSums {
+  double s00, s00_over, sbb[CG_MAX_BINDERS], sx[3], vf_over;
+};
+__device__ __forceinline__ void add_row(const RepDev& rd, long long gmax, const long long (&row)[4], GridSums& s) {
+  const double g0 = (double)row[0];
+  if (row[0] <= gmax) {
+    s.s00 = __fma_rn(g0, g0, s.s00);
+  } else {
+    s.s00_over = __fma_rn(g0, g0, s.s00_over);
+    s.vf_over += (g0 * kFxInv) / rd.vol_bin * rd.bead_vol;
+  }
+  double gb[CG_MAX_BINDERS] = {0, 0, 0};
+#pragma unroll
+  for (int b = 0; b < CG_MAX_BINDERS; b++)
+    if (row[1 + b]) {
+      gb[b] = (double)row[1 + b];
+      s.sbb[b] = __fma_rn(gb[b], gb[b], s.sbb[b]);
+    }
+  if (row[1] && row[2]) s.sx[0] = __fma_rn(gb[0], gb[1], s.sx[0]);
+  if (row[1] && row[3]) s.sx[1] = __fma_rn(gb[0], gb[2], s.sx[1]);
+  if (row[2] && row[3]) s.sx[2] = __fma_rn(gb[1], gb[2], s.sx[2]);
+}
+
+// Elastic energy of bond i - 1 -> i from the two beads' vectors in FP64.
+__device__ __forceinline__ double bond_energy(const double* b, const double r0[3], const double r1[3],
+                                              const double a0[3], const double a1[3]) {
+  const double2 q0 = *reinterpret_cast<const double2*>(b), q1 = *reinterpret_cast<const double2*>(b + 2);
+  const double eb = q0.x, g = q0.y, ep = q1.x, epp = q1.y, eta = b[4];
+  double dr[3], dp[3], bend[3];
+  for (int j = 0; j < 3; j++) dr[j] = r1[j] - r0[j];
+  const double par = __fma_rn(a0[2], dr[2], __fma_rn(a0[1], dr[1], a0[0] * dr[0]));
+  for (int j = 0; j < 3; j++) dp[j] = __fma_rn(-a0[j], par, dr[j]);
+  for (int j = 0; j < 3; j++) bend[j] = __fma_rn(-eta, dp[j], a1[j] - a0[j]);
+  const double b2 = __fma_rn(bend[2], bend[2], __fma_rn(bend[1], bend[1], bend[0] * bend[0]));
+  const double p2 = __fma_rn(dp[2], dp[2], __fma_rn(dp[1], dp[1], dp[0] * dp[0]));
+  const double x = par - g;
+  return 0.5 * __fma_rn(eb, b2, __fma_rn(ep, x * x, epp * p2));
+}
+
+// One CTA's part of a replica's beads: elastic (and twist) energy, binding free
+// energy from the replica's table `bf` ([binder][marks][state], the chemical
+// potential's term included), doubly bound beads per binder, and the sites
+// bound beyond max_binders.  A warp takes 31 bonds a pass: lane l holds bead
+// i0 + l, converted once, and its bond to lane l - 1's bead.
+template <typename Pos>
+__device__ __forceinline__ void bead_sums(const KArgs& a, const RepDev& rd, int rank, const double* bf, double& el,
+                                          double& bi, int (&dbl)[CG_MAX_BINDERS], long long& excess) {
+  const V4<Pos>* r4 = reinterpret_cast<const V4<Pos>*>(a.r4) + rd.bead_off;
+  const V4<Pos>* t34 = reinterpret_cast<const V4<Pos>*>(a.t34) + rd.bead_off;
+  const V4<Pos>* t24 = reinterpret_cast<const V4<Pos>*>(a.t24) + rd.bead_off;
+  const double* bonds = a.bonds + rd.bead_off * 6;
+  const long long N = rd.n_beads, per = (N + kSumCtas - 1) / kSumCtas;
+  const long long b0 = rank * per, b1 = b0 + per < N ? b0 + per : N;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  // lane 0's bead is the one before the pass's first
+  for (long long i0 = b0 - 1 + 31LL * warp; i0 + 1 < b1; i0 += 31LL * (kSumThreads / 32)) {
+    const long long i = i0 + lane;
+    const bool have = i >= 0 && i < b1;
+    double r[3] = {0, 0, 0}, t[3] = {0, 0, 0}, rp[3], tp[3];
+    if (have) {
+      ld3(r4, i, r);
+      ld3(t34, i, t);
+    }
+    for (int j = 0; j < 3; j++) {
+      rp[j] = __shfl_up_sync(kFull, r[j], 1);
+      tp[j] = __shfl_up_sync(kFull, t[j], 1);
+    }
+    if (!have || lane == 0) continue;
+    if (i > 0) {
+      el += bond_energy(bonds + 6 * (i - 1), rp, r, tp, t);
+      if (rd.twist)  // SSTWLC.compute_E, chromo/polymers.pyx:2250-2285
+        el += twist_bond_energy(a.twist + 2 * (rd.bead_off + i - 1), frame_of(t24[i - 1], t34[i - 1]),
+                                frame_of(t24[i], t34[i]));
+    }
+    const unsigned sw = a.states[rd.bead_off + i], mw = a.marks[rd.bead_off + i];
+    int tot = 0;
+#pragma unroll
+    for (int b = 0; b < CG_MAX_BINDERS; b++)
+      if (b < rd.nb) {
+        const int s = (int)((sw >> (8 * b)) & 0xFF), nm = (int)((mw >> (8 * b)) & 0xFF);
+        bi += bf[(b * (CG_MAX_MARK + 1) + nm) * (CG_MAX_MARK + 1) + s];
+        tot += s;
+        dbl[b] += s == 2;
+      }
+    if (rd.max_binders != -1 && tot > rd.max_binders) excess += tot - rd.max_binders;
+  }
+}
+
+// The replica's binding table with the chemical potential's term
+// (polymers.pyx:1494-1537), by the CTA's threads.
+__device__ __forceinline__ void fill_bind_table(const RepDev& rd, double* bf) {
+  for (int k = threadIdx.x; k < CG_MAX_BINDERS * (CG_MAX_MARK + 1) * (CG_MAX_MARK + 1); k += blockDim.x) {
+    const int b = k / ((CG_MAX_MARK + 1) * (CG_MAX_MARK + 1)), s = k % (CG_MAX_MARK + 1);
+    const double me = rd.mu[b] > 0 ? rd.mu[b] * (-rd.mu_adjust + 2) : rd.mu[b] * rd.mu_adjust;
+    bf[k] = rd.bind_f[k] - (double)s * me;
+  }
 }
 
 // one block; deterministic tree reduction, the total valid in warp 0

@@ -540,11 +540,12 @@ template <typename Pos>
 __global__ void deposit_kernel(KArgs a, int rep_only) {
   const int rep = rep_only >= 0 ? rep_only : blockIdx.y;
   const RepDev& rd = a.reps[rep];
-  if (rd.field_kind != 2) return;
+  if (rd.field_kind != 2 || blockIdx.x * (long long)blockDim.x >= rd.n_beads) return;
   const V4<Pos>* r4 = reinterpret_cast<const V4<Pos>*>(a.r4) + rd.bead_off;
   long long* grid = a.grid + rd.vox_off * a.ncol;
-  GridF gf;
-  make_gridf(rd, gf);
+  __shared__ GridF gf;  // once per CTA: its FP64 divisions took longer than the beads
+  if (threadIdx.x == 0) make_gridf(rd, gf);
+  __syncthreads();
   for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < rd.n_beads;
        i += (long long)gridDim.x * blockDim.x) {
     Pos p[3], w[8];
@@ -564,91 +565,108 @@ __global__ void deposit_kernel(KArgs a, int rep_only) {
 }
 
 // ---------------------------------------------------------------- FP64 energies
-// one block per replica; deterministic block tree reduction.
-__device__ double block_sum(double v, double* sh) {
-  v = warp_sum(v);
-  const int w = threadIdx.x >> 5, l = threadIdx.x & 31;
-  __syncthreads();
-  if (l == 0) sh[w] = v;
-  __syncthreads();
-  double t = 0;
-  if (threadIdx.x < 32) {
-    t = threadIdx.x < (blockDim.x >> 5) ? sh[threadIdx.x] : 0.0;
-    t = warp_sum(t);
-  }
-  return t;  // valid in warp 0
+// A cluster per replica (see cg_energy.cuh).
+//
+// S and the chi term of a replica with uniform voxel volumes: c the volume
+// fraction per fixed-point unit, S = (V / Vb) c^2 sum g0^2.
+__device__ __forceinline__ double chi_free_sum(const RepDev& rd, double s00) {
+  const double c = kFxInv / rd.vol_bin * rd.bead_vol;
+  return (rd.vol_bin / rd.bead_vol) * (c * c) * s00;
 }
 
 template <typename Pos>
-__global__ void energy_kernel(KArgs a, double* out) {
-  __shared__ double sh[32];
-  const int rep = blockIdx.x;
+__global__ void __cluster_dims__(kSumCtas, 1, 1) __launch_bounds__(kSumThreads)
+    energy_kernel(KArgs a, double* out) {
+  __shared__ double sh[kSumThreads / 32][16];
+  __shared__ double bf[CG_MAX_BINDERS * (CG_MAX_MARK + 1) * (CG_MAX_MARK + 1)];
+  __shared__ long long gmax_sh;
+  const int rep = blockIdx.x / kSumCtas, rank = blockIdx.x % kSumCtas;
   const RepDev& rd = a.reps[rep];
+  fill_bind_table(rd, bf);
+  const bool field = rd.field_kind == 2, uniform = field && !rd.has_access;
+  if (threadIdx.x == 0) gmax_sh = uniform ? weight_at_limit(rd) : 0;
+  __syncthreads();
+  double el = 0, bi = 0;
+  int dbl[CG_MAX_BINDERS] = {0, 0, 0};
+  long long excess = 0;
+  bead_sums<Pos>(a, rd, rank, bf, el, bi, dbl, excess);
+  GridSums g{};
   EnergyParts p{0.0, 0.0, 0.0, 0.0, {0, 0, 0}};
-  for (long long i = threadIdx.x; i < rd.n_beads; i += blockDim.x) bead_energy<Pos>(a, rd, i, p);
-  if (rd.field_kind == 2)
-    for (long long v = threadIdx.x; v < rd.n_vox; v += blockDim.x) voxel_energy(a, rd, v, p);
-  const double el = p.el, bi = p.bi, fe = p.fe, sx = p.sx;
-  const long long* dbl = p.dbl;
-  double t_el = block_sum(el, sh);
-  double t_bi = block_sum(bi, sh);
-  double t_fe = block_sum(fe, sh);
-  double t_sx = block_sum(sx, sh);
-  double t_db[CG_MAX_BINDERS];
-  for (int b = 0; b < CG_MAX_BINDERS; b++) t_db[b] = block_sum((double)dbl[b], sh);
-  if (threadIdx.x == 0) {
-    double intra = 0;
-    for (int b = 0; b < rd.nb; b++) intra += rd.intra[b] * t_db[b];
-    out[rep * 5 + 0] = t_el;
-    out[rep * 5 + 1] = t_bi;
-    out[rep * 5 + 2] = rd.field_kind == 2 ? t_fe + intra : 0.0;
-    out[rep * 5 + 3] = rd.run_dE;
-    out[rep * 5 + 4] = t_sx;
+  if (uniform) {
+    const long long gmax = gmax_sh;
+    for_each_row<true>(a, rd, rank, [&](long long, const long long (&row)[4]) { add_row(rd, gmax, row, g); });
+  } else if (field) {
+    for_each_row<false>(a, rd, rank, [&](long long v, const long long (&row)[4]) {
+      if (!empty_voxel(a, rd, v, row)) voxel_energy(a, rd, v, p);
+    });
   }
+  double v[16] = {el, bi, uniform ? g.s00 : p.sx, uniform ? g.vf_over : p.fe, g.sbb[0], g.sbb[1], g.sbb[2],
+                  g.sx[0], g.sx[1], g.sx[2], (double)dbl[0], (double)dbl[1], (double)dbl[2], (double)excess, 0.0, 0.0};
+  const double t = cluster_sums(v, sh);
+  if (rank != 0 || threadIdx.x >= 32) return;
+  double s[16];
+  for (int k = 0; k < 16; k++) s[k] = __shfl_sync(kFull, t, k);
+  if (threadIdx.x != 0) return;
+  double fe = 0, sx = 0;
+  if (uniform) {
+    const double u = kFxInv / rd.vol_bin, u2 = u * u;
+    sx = chi_free_sum(rd, s[2]);
+    for (int b = 0; b < rd.nb; b++) fe += rd.pref[b] * (u2 * s[4 + b]);
+    for (int b = 0; b < rd.nb; b++)
+      for (int e = 0; e < rd.nb; e++) fe += rd.xpref[b * CG_MAX_BINDERS + e] * (u2 * (b == e ? s[4 + b] : s[6 + b + e]));
+    fe += rd.chi * sx + kEHugeField * s[3];
+  } else if (field) {
+    sx = s[2];
+    fe = s[3];
+  }
+  double intra = 0;
+  for (int b = 0; b < rd.nb; b++) intra += rd.intra[b] * s[10 + b];
+  out[rep * 5 + 0] = s[0];
+  out[rep * 5 + 1] = s[1] + kEHugePoly * s[13];
+  out[rep * 5 + 2] = field ? fe + intra : 0.0;
+  out[rep * 5 + 3] = rd.run_dE;
+  out[rep * 5 + 4] = sx;
 }
 
-// The chi-free sums S_r alone (the input of the exchange): the same per-thread
-// order and block reduction as energy_kernel's out[5 r + 4], so the values are
-// identical, without the elastic, binding and binder-density terms.
-__global__ void chi_sum_kernel(KArgs a, double* out) {
-  __shared__ double sh[32];
-  const int rep = blockIdx.x;
+// The chi-free sums S_r alone (the input of the exchange): the same rows in the
+// same order as energy_kernel's out[5 r + 4], so the values are identical; and
+// with a mu ladder the bound sites of its binder (an exact integer sum).
+__global__ void __cluster_dims__(kSumCtas, 1, 1) __launch_bounds__(kSumThreads)
+    chi_sum_kernel(KArgs a, double* out) {
+  __shared__ double sh[kSumThreads / 32][16];
+  __shared__ long long gmax_sh;
+  const int rep = blockIdx.x / kSumCtas, rank = blockIdx.x % kSumCtas;
   const RepDev& rd = a.reps[rep];
+  const bool field = rd.field_kind == 2, uniform = field && !rd.has_access;
+  if (threadIdx.x == 0) gmax_sh = uniform ? weight_at_limit(rd) : 0;
+  __syncthreads();
   double sx = 0;
-  if (rd.field_kind == 2 && !rd.has_access) {
-    // uniform voxel volume: S = (V / Vb) c^2 sum g0^2 with c = 2^-40 Vb / V the
-    // volume fraction per fixed-point unit (no FP64 division per voxel); a
-    // voxel whose volume fraction may be above vf_limit takes the exact test
-    // of energy_kernel and is left out of S when above it
-    const long long* grid = a.grid + rd.vox_off * a.ncol;
-    const double c = kFxInv / rd.vol_bin * rd.bead_vol;
-    const double near = rd.vf_limit * (1.0 - 1e-9);
-    double s00 = 0;
-    for (long long v = threadIdx.x; v < rd.n_vox; v += blockDim.x) {
-      const long long n = grid[v * a.ncol];
-      const double g0 = (double)n;
-      if (g0 * c > near && ((double)n * kFxInv) / rd.vol_bin * rd.bead_vol > rd.vf_limit) continue;
-      s00 += g0 * g0;
-    }
-    sx = (rd.vol_bin / rd.bead_vol) * (c * c) * s00;
-  } else if (rd.field_kind == 2) {
-    const long long* grid = a.grid + rd.vox_off * a.ncol;
-    for (long long v = threadIdx.x; v < rd.n_vox; v += blockDim.x) {
-      double V = rd.has_access ? a.access_vol[rd.vox_off + v] : rd.vol_bin;
-      double vf = ((double)grid[v * a.ncol] * kFxInv) / V * rd.bead_vol;
-      if (!(vf > rd.vf_limit)) sx += (V / rd.bead_vol) * vf * vf;
-    }
+  if (uniform) {
+    const long long gmax = gmax_sh;
+    for_each_row<true>(a, rd, rank, [&](long long, const long long (&row)[4]) {
+      const double g0 = (double)row[0];
+      if (row[0] <= gmax) sx = __fma_rn(g0, g0, sx);
+    });
+  } else if (field) {
+    EnergyParts p{0.0, 0.0, 0.0, 0.0, {0, 0, 0}};
+    for_each_row<false>(a, rd, rank, [&](long long v, const long long (&row)[4]) {
+      if (!empty_voxel(a, rd, v, row)) voxel_energy(a, rd, v, p);
+    });
+    sx = p.sx;
   }
-  const double t = block_sum(sx, sh);
-  if (threadIdx.x == 0) out[rep * 5 + 4] = t;
-  if (a.mu_rungs > 1) {  // bound sites of the mu-ladder binder (exact integer sum)
+  long long nbl = 0;
+  if (a.mu_rungs > 1) {
     const unsigned* st = a.states + rd.bead_off;
     const int sh8 = 8 * a.mu_binder;
-    long long nbl = 0;
-    for (long long i = threadIdx.x; i < rd.n_beads; i += blockDim.x) nbl += (st[i] >> sh8) & 0xFFu;
-    const double nbt = block_sum((double)nbl, sh);
-    if (threadIdx.x == 0) a.nbound[rep] = nbt;
+    const long long per = (rd.n_beads + kSumCtas - 1) / kSumCtas;
+    const long long b1 = (rank + 1) * per < rd.n_beads ? (rank + 1) * per : rd.n_beads;
+    for (long long i = rank * per + threadIdx.x; i < b1; i += blockDim.x) nbl += (st[i] >> sh8) & 0xFFu;
   }
+  double v[16] = {sx, (double)nbl};
+  const double t = cluster_sums(v, sh);
+  if (rank != 0) return;
+  if (threadIdx.x == 0) out[rep * 5 + 4] = uniform ? chi_free_sum(rd, t) : t;
+  if (threadIdx.x == 1 && a.mu_rungs > 1) a.nbound[rep] = t;
 }
 
 // ---------------------------------------------------------------- replica exchange
@@ -782,12 +800,13 @@ void cg_launch_deposit(const cg::KArgs& a, bool fp64, int rep, int n_reps_launch
 }
 
 void cg_launch_energy(const cg::KArgs& a, bool fp64, double* out, cudaStream_t s) {
-  if (fp64) cg::energy_kernel<double><<<a.n_reps, 256, 0, s>>>(a, out);
-  else cg::energy_kernel<float><<<a.n_reps, 256, 0, s>>>(a, out);
+  const int blocks = a.n_reps * cg::kSumCtas;
+  if (fp64) cg::energy_kernel<double><<<blocks, cg::kSumThreads, 0, s>>>(a, out);
+  else cg::energy_kernel<float><<<blocks, cg::kSumThreads, 0, s>>>(a, out);
 }
 
 void cg_launch_chi_sum(const cg::KArgs& a, double* out, cudaStream_t s) {
-  cg::chi_sum_kernel<<<a.n_reps, 256, 0, s>>>(a, out);
+  cg::chi_sum_kernel<<<a.n_reps * cg::kSumCtas, cg::kSumThreads, 0, s>>>(a, out);
 }
 
 void cg_launch_exchange(const cg::KArgs& a, const double* eout, int n_rungs, long long round,
