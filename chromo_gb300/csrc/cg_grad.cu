@@ -18,239 +18,280 @@
 // products) to per-replica running sums over sampled configurations.
 #include <cuda_runtime.h>
 
-#include "cg_device.cuh"
-#include "cg_kernels.h"
+#include <algorithm>
+
+#include "cg_energy.cuh"
 
 namespace cg {
 
-// d E_pair / d dr of bond (bead j -> bead j+1), dr = r_{j+1} - r_j, a0 / a1
-// the t3 tangents at j / j+1.  With par = a0.dr, dp = P dr (P = I - a0 a0^T),
-// bend = a1 - a0 - eta dp:
-//   dE/ddr = -eta eb P bend + ep (par - gamma) a0 + epp P dp.
-__device__ __forceinline__ void bond_grad(const Bond<double>& b, const double a0[3], const double a1[3],
-                                          const double dr[3], double g[3]) {
-  const double par = a0[0] * dr[0] + a0[1] * dr[1] + a0[2] * dr[2];
-  double dp[3], bend[3];
-  for (int j = 0; j < 3; j++) dp[j] = dr[j] - a0[j] * par;
-  for (int j = 0; j < 3; j++) bend[j] = a1[j] + (-a0[j] - b.eta * dp[j]);
-  const double ab = a0[0] * bend[0] + a0[1] * bend[1] + a0[2] * bend[2];
-  const double ad = a0[0] * dp[0] + a0[1] * dp[1] + a0[2] * dp[2];
-  for (int j = 0; j < 3; j++)
-    g[j] = -b.eta * b.eb * (bend[j] - a0[j] * ab) + b.ep * (par - b.g) * a0[j] + b.epp * (dp[j] - a0[j] * ad);
-}
-
-// Trilinear weights of one position with their derivatives along x, y, z
-// (the construction of voxel_weights; d(lower)/dx = -1/dx, d(upper)/dx = 1/dx).
-__device__ __forceinline__ void weights_and_slopes(const RepDev& rd, const double pos[3], double w[8],
-                                                   double dw[8][3], int v[8]) {
-  const double width[3] = {rd.wx, rd.wy, rd.wz};
-  const int n[3] = {rd.nx, rd.ny, rd.nz};
-  double wl[3], inv[3];
-  int lo[3], hi[3];
-  for (int j = 0; j < 3; j++) {
-    const double d = width[j] / (double)n[j];
-    const double x = pymod(pos[j] + 0.5 * width[j], width[j]) - 0.5 * d;
-    const long long ind = (long long)floor(x / d);
-    const int li = ind == -1 ? n[j] - 1 : (int)ind;
-    lo[j] = li < 0 ? 0 : (li >= n[j] ? n[j] - 1 : li);
-    hi[j] = lo[j] + 1 == n[j] ? 0 : lo[j] + 1;
-    wl[j] = 1 - (x / d - (double)ind);
-    inv[j] = 1.0 / d;
-  }
-  for (int l = 0; l < 8; l++) {
-    const int bx = l & 1, by = (l >> 1) & 1, bz = (l >> 2) & 1;
-    const double f[3] = {bx ? 1 - wl[0] : wl[0], by ? 1 - wl[1] : wl[1], bz ? 1 - wl[2] : wl[2]};
-    const double s[3] = {bx ? inv[0] : -inv[0], by ? inv[1] : -inv[1], bz ? inv[2] : -inv[2]};
-    w[l] = f[0] * f[1] * f[2];
-    dw[l][0] = s[0] * f[1] * f[2];
-    dw[l][1] = f[0] * s[1] * f[2];
-    dw[l][2] = f[0] * f[1] * s[2];
-    v[l] = (bx ? hi[0] : lo[0]) + rd.nx * ((by ? hi[1] : lo[1]) + rd.ny * (bz ? hi[2] : lo[2]));
-  }
-}
-
-// d E_pair / d a0 and d E_pair / d a1 of bond (j -> j+1) (the t3 tangents at
-// j and j+1 taken as free vectors, as the energy's formula reads them):
+// Derivatives of E_pair of bond (bead j -> bead j+1), dr = r_{j+1} - r_j, a0 / a1
+// the t3 tangents at j / j+1 taken as free vectors.  With par = a0.dr,
+// dp = P dr (P = I - a0 a0^T), bend = a1 - a0 - eta dp:
+//   dE/ddr = -eta eb P bend + ep (par - gamma) a0 + epp P dp,
 //   dE/da1 = eb bend,
 //   dE/da0 = eb (eta (par bend + (a0.bend) dr) - bend) + ep (par - gamma) dr
 //            - epp (par dp + (a0.dp) dr).
-__device__ __forceinline__ void bond_tangent_grad(const Bond<double>& b, const double a0[3], const double a1[3],
-                                                  const double dr[3], double g0[3], double g1[3]) {
-  const double par = a0[0] * dr[0] + a0[1] * dr[1] + a0[2] * dr[2];
+__device__ __forceinline__ double dot3(const double a[3], const double b[3]) {
+  return __fma_rn(a[2], b[2], __fma_rn(a[1], b[1], a[0] * b[0]));
+}
+__device__ __forceinline__ void bond_grad(const double* bp, const double a0[3], const double a1[3],
+                                          const double dr[3], bool tangents, double g[3], double g0[3],
+                                          double g1[3]) {
+  const double2 q0 = *reinterpret_cast<const double2*>(bp), q1 = *reinterpret_cast<const double2*>(bp + 2);
+  const double eb = q0.x, gamma = q0.y, ep = q1.x, epp = q1.y, eta = bp[4];
+  const double par = dot3(a0, dr);
   double dp[3], bend[3];
-  for (int j = 0; j < 3; j++) dp[j] = dr[j] - a0[j] * par;
-  for (int j = 0; j < 3; j++) bend[j] = a1[j] + (-a0[j] - b.eta * dp[j]);
-  const double ab = a0[0] * bend[0] + a0[1] * bend[1] + a0[2] * bend[2];
-  const double ad = a0[0] * dp[0] + a0[1] * dp[1] + a0[2] * dp[2];
-  for (int j = 0; j < 3; j++) {
-    g1[j] = b.eb * bend[j];
-    g0[j] = b.eb * (b.eta * (par * bend[j] + ab * dr[j]) - bend[j]) + b.ep * (par - b.g) * dr[j] -
-            b.epp * (par * dp[j] + ad * dr[j]);
+  for (int j = 0; j < 3; j++) dp[j] = __fma_rn(-a0[j], par, dr[j]);
+  for (int j = 0; j < 3; j++) bend[j] = __fma_rn(-eta, dp[j], a1[j] - a0[j]);
+  const double ab = dot3(a0, bend), ad = dot3(a0, dp);
+  const double ee = eta * eb, px = ep * (par - gamma);
+  // -ee (bend - a0 ab) + px a0 + epp (dp - a0 ad) = -ee bend + epp dp + (ee ab + px - epp ad) a0
+  const double c = __fma_rn(ee, ab, __fma_rn(-epp, ad, px));
+  for (int j = 0; j < 3; j++) g[j] = __fma_rn(-ee, bend[j], __fma_rn(epp, dp[j], c * a0[j]));
+  if (tangents) {
+    const double cb = __fma_rn(ee, par, -eb), cp = -epp * par;
+    for (int j = 0; j < 3; j++) {
+      g1[j] = eb * bend[j];
+      g0[j] = __fma_rn(cb, bend[j], __fma_rn(c, dr[j], cp * dp[j]));
+    }
   }
 }
 
+// One coordinate's voxels (lower, upper) and its fraction of the way between
+// them, in FP64 (the construction of voxel_axes).  The quotient by the voxel
+// width is a product and an FMA remainder, corrected to floor(x / d): a
+// division runs ~10 operations of the FP64 pipe.
+__device__ __forceinline__ double cell_of(double pos, double width, double d, double inv, int n, int& lo, int& hi) {
+  const double x = pymod(pos + 0.5 * width, width) - 0.5 * d;
+  double q = floor(x * inv);
+  double r = __fma_rn(-q, d, x);
+  if (r < 0) {
+    q -= 1;
+    r = __fma_rn(-q, d, x);
+  } else if (r >= d) {
+    const double r1 = __fma_rn(-(q + 1), d, x);
+    if (r1 >= 0) { q += 1; r = r1; }
+  }
+  const int ind = (int)q;
+  const int li = ind == -1 ? n - 1 : ind;
+  lo = li < 0 ? 0 : (li >= n ? n - 1 : li);
+  hi = lo + 1 == n ? 0 : lo + 1;
+  return r * inv;
+}
+
+// dE_v/dw at one voxel of a replica with non-uniform volumes (states in sw).
+__device__ __forceinline__ double voxel_slope(const KArgs& a, const RepDev& rd, long long v, unsigned sw) {
+  const long long* row = a.grid + (rd.vox_off + v) * a.ncol;
+  const double V = a.access_vol[rd.vox_off + v];
+  double rho[CG_MAX_BINDERS];
+  for (int b = 0; b < rd.nb; b++) rho[b] = ((double)row[1 + b] * kFxInv) / V;
+  const double vf = ((double)row[0] * kFxInv) / V * rd.bead_vol;
+  double phi = vf > rd.vf_limit ? kEHugeField * rd.bead_vol / V : 2 * rd.chi * vf;
+  for (int b = 0; b < rd.nb; b++) {
+    const int s = (int)((sw >> (8 * b)) & 0xFF);
+    if (!s) continue;
+    double pb = 2 * rd.pref[b] * rho[b];
+    for (int c = 0; c < rd.nb; c++) pb += (rd.xpref[b * CG_MAX_BINDERS + c] + rd.xpref[c * CG_MAX_BINDERS + b]) * rho[c];
+    phi += (double)s * pb / V;
+  }
+  return phi;
+}
+
+// dE/dr (and dE/dt3) of every bead.  FP64 runs at 1/64 of the FP32 rate here, so
+// the kernel is bound by its FP64 operations (~150 a bead): a warp takes 30
+// beads a pass, each lane converting one bead and evaluating the bond to the
+// next lane's, whose derivatives come back by shuffles (every bond once); with
+// uniform volumes dE_v/dw is a linear combination of the voxel's fixed-point
+// columns whose coefficients depend on the bead's states only (a table of the
+// CTA), and the eight corners are contracted axis by axis.  Five divisions a
+// corner and every bond twice took 680 us for 64 chains of 5,000 beads with the
+// read-back (gradient and terms together: 1,086 -> 347 us).
 template <typename Pos, typename Out>
-__global__ void gradient_kernel(KArgs a, Out* out, Out* out_t3) {
+__global__ void __launch_bounds__(128) gradient_kernel(KArgs a, Out* out, Out* out_t3) {
+  __shared__ double tab[64][CG_MAX_BINDERS];  // binder columns' coefficients for packed states (2 bits each)
+  __shared__ double k0_sh, huge_sh, inv_sh[3];
+  __shared__ long long gmax_sh;
   const int rep = blockIdx.y;
   const RepDev& rd = a.reps[rep];
+  const long long N = rd.n_beads;
+  constexpr int kBeads = 30;  // beads a warp writes per pass
+  if (blockIdx.x * (long long)(blockDim.x / 32) * kBeads >= N) return;
+  const bool field = rd.field_kind == 2, uniform = field && !rd.has_access;
+  if (field) {
+    const double u = kFxInv / rd.vol_bin;
+    if (uniform)
+      for (int k = threadIdx.x; k < 64 * CG_MAX_BINDERS; k += blockDim.x) {
+        const int code = k / CG_MAX_BINDERS, c = k % CG_MAX_BINDERS;
+        double t = 0;
+        if (c < rd.nb)
+          for (int b = 0; b < rd.nb; b++) {
+            const int s = (code >> (2 * b)) & 3;
+            double pb = rd.xpref[b * CG_MAX_BINDERS + c] + rd.xpref[c * CG_MAX_BINDERS + b];
+            if (b == c) pb += 2 * rd.pref[b];
+            if (s) t += (double)s * pb;
+          }
+        tab[code][c] = t * u / rd.vol_bin;
+      }
+    if (threadIdx.x < 3) {
+      const double width[3] = {rd.wx, rd.wy, rd.wz};
+      const int n[3] = {rd.nx, rd.ny, rd.nz};
+      inv_sh[threadIdx.x] = (double)n[threadIdx.x] / width[threadIdx.x];
+    }
+    if (threadIdx.x == 32) {
+      k0_sh = 2 * rd.chi * rd.bead_vol * u;
+      huge_sh = kEHugeField * rd.bead_vol / rd.vol_bin;
+      gmax_sh = uniform ? weight_at_limit(rd) : 0;
+    }
+  }
+  __syncthreads();
   const V4<Pos>* r4 = reinterpret_cast<const V4<Pos>*>(a.r4) + rd.bead_off;
   const V4<Pos>* t34 = reinterpret_cast<const V4<Pos>*>(a.t34) + rd.bead_off;
   const double* bonds = a.bonds + rd.bead_off * 6;
   const unsigned* st = a.states + rd.bead_off;
   const long long* grid = a.grid + rd.vox_off * a.ncol;
-  const long long N = rd.n_beads;
-  for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < N;
-       i += (long long)gridDim.x * blockDim.x) {
-    double ri[3], ai[3], gr[3] = {0, 0, 0}, gt[3] = {0, 0, 0};
-    ld3(r4, i, ri);
-    ld3(t34, i, ai);
-    if (i > 0) {  // bond (i-1 -> i): + dE/ddr; dE/da1 for the tangent
-      double rp[3], ap[3], dr[3], g[3];
-      ld3(r4, i - 1, rp);
-      ld3(t34, i - 1, ap);
-      for (int j = 0; j < 3; j++) dr[j] = ri[j] - rp[j];
-      const Bond<double> b = load_bond<double>(bonds, i - 1);
-      bond_grad(b, ap, ai, dr, g);
-      for (int j = 0; j < 3; j++) gr[j] += g[j];
-      if (out_t3) {
-        double g0[3], g1[3];
-        bond_tangent_grad(b, ap, ai, dr, g0, g1);
-        for (int j = 0; j < 3; j++) gt[j] += g1[j];
-      }
+  const int lane = threadIdx.x & 31, wpb = blockDim.x >> 5;
+  const bool tangents = out_t3 != nullptr;
+  for (long long i0 = ((long long)blockIdx.x * wpb + (threadIdx.x >> 5)) * kBeads - 1; i0 + 1 < N;
+       i0 += (long long)gridDim.x * wpb * kBeads) {
+    const long long i = i0 + lane;
+    const bool have = i >= 0 && i < N;
+    double r[3] = {0, 0, 0}, t[3] = {0, 0, 0};
+    if (have) {
+      ld3(r4, i, r);
+      ld3(t34, i, t);
     }
-    if (i + 1 < N) {  // bond (i -> i+1): - dE/ddr; dE/da0 for the tangent
-      double rn[3], an[3], dr[3], g[3];
-      ld3(r4, i + 1, rn);
-      ld3(t34, i + 1, an);
-      for (int j = 0; j < 3; j++) dr[j] = rn[j] - ri[j];
-      const Bond<double> b = load_bond<double>(bonds, i);
-      bond_grad(b, ai, an, dr, g);
-      for (int j = 0; j < 3; j++) gr[j] -= g[j];
-      if (out_t3) {
-        double g0[3], g1[3];
-        bond_tangent_grad(b, ai, an, dr, g0, g1);
-        for (int j = 0; j < 3; j++) gt[j] += g0[j];
-      }
+    double dr[3], tn[3], g[3] = {0, 0, 0}, g0[3] = {0, 0, 0}, g1[3] = {0, 0, 0};
+    for (int j = 0; j < 3; j++) {
+      dr[j] = __shfl_down_sync(kFull, r[j], 1) - r[j];
+      tn[j] = __shfl_down_sync(kFull, t[j], 1);
     }
-    if (rd.field_kind == 2) {
-      double w[8], dw[8][3];
-      int v[8];
-      weights_and_slopes(rd, ri, w, dw, v);
+    if (have && lane < 31 && i + 1 < N) bond_grad(bonds + 6 * i, t, tn, dr, tangents, g, g0, g1);
+    // bond (i-1 -> i): + dE/ddr, dE/da1; bond (i -> i+1): - dE/ddr, dE/da0
+    double gr[3], gt[3];
+    for (int j = 0; j < 3; j++) {
+      gr[j] = __shfl_up_sync(kFull, g[j], 1) - g[j];
+      gt[j] = __shfl_up_sync(kFull, g1[j], 1) + g0[j];
+    }
+    if (!have || lane == 0 || lane > kBeads) continue;
+    if (field) {
+      int lo[3], hi[3];
+      const double inv[3] = {inv_sh[0], inv_sh[1], inv_sh[2]};
+      const double fx = cell_of(r[0], rd.wx, rd.dx, inv[0], rd.nx, lo[0], hi[0]);
+      const double fy = cell_of(r[1], rd.wy, rd.dy, inv[1], rd.ny, lo[1], hi[1]);
+      const double fz = cell_of(r[2], rd.wz, rd.dz, inv[2], rd.nz, lo[2], hi[2]);
       const unsigned sw = st[i];
+      const int code = (int)((sw & 3u) | ((sw >> 6) & 12u) | ((sw >> 12) & 48u));
+      double phi[8];
+#pragma unroll
       for (int l = 0; l < 8; l++) {
-        const long long* row = grid + (long long)v[l] * a.ncol;
-        const double V = rd.has_access ? a.access_vol[rd.vox_off + v[l]] : rd.vol_bin;
-        double rho[CG_MAX_BINDERS];
-        for (int b = 0; b < rd.nb; b++) rho[b] = ((double)row[1 + b] * kFxInv) / V;
-        const double vf = ((double)row[0] * kFxInv) / V * rd.bead_vol;
-        double phi = vf > rd.vf_limit ? kEHugeField * rd.bead_vol / V : 2 * rd.chi * vf;
-        for (int b = 0; b < rd.nb; b++) {
-          const int s = (int)((sw >> (8 * b)) & 0xFF);
-          if (!s) continue;
-          double pb = 2 * rd.pref[b] * rho[b];
-          for (int c = 0; c < rd.nb; c++)
-            pb += (rd.xpref[b * CG_MAX_BINDERS + c] + rd.xpref[c * CG_MAX_BINDERS + b]) * rho[c];
-          phi += (double)s * pb / V;
+        const long long v = (l & 1 ? hi[0] : lo[0]) +
+                            (long long)rd.nx * ((l & 2 ? hi[1] : lo[1]) + (long long)rd.ny * (l & 4 ? hi[2] : lo[2]));
+        if (uniform) {
+          long long row[4];
+          load_row(grid + v * a.ncol, a.ncol, row);
+          double p = row[0] > gmax_sh ? huge_sh : k0_sh * (double)row[0];
+#pragma unroll
+          for (int c = 0; c < CG_MAX_BINDERS; c++)
+            if (row[1 + c]) p = __fma_rn(tab[code][c], (double)row[1 + c], p);
+          phi[l] = p;
+        } else {
+          phi[l] = voxel_slope(a, rd, v, sw);
         }
-        for (int j = 0; j < 3; j++) gr[j] += phi * dw[l][j];
       }
+      // along x: slopes d and values e on the four (y, z) edges; then y, z
+      double d[4], e[4];
+#pragma unroll
+      for (int k = 0; k < 4; k++) {
+        d[k] = phi[2 * k + 1] - phi[2 * k];
+        e[k] = __fma_rn(fx, d[k], phi[2 * k]);
+      }
+      const double dx0 = __fma_rn(fy, d[1] - d[0], d[0]), dx1 = __fma_rn(fy, d[3] - d[2], d[2]);
+      const double ey0 = e[1] - e[0], ey1 = e[3] - e[2];
+      const double ez0 = __fma_rn(fy, ey0, e[0]), ez1 = __fma_rn(fy, ey1, e[2]);
+      gr[0] = __fma_rn(inv[0], __fma_rn(fz, dx1 - dx0, dx0), gr[0]);
+      gr[1] = __fma_rn(inv[1], __fma_rn(fz, ey1 - ey0, ey0), gr[1]);
+      gr[2] = __fma_rn(inv[2], ez1 - ez0, gr[2]);
     }
     Out* o = out + 3 * (rd.bead_off + i);
-    o[0] = (Out)gr[0];
-    o[1] = (Out)gr[1];
-    o[2] = (Out)gr[2];
-    if (out_t3) {
+    for (int j = 0; j < 3; j++) o[j] = (Out)gr[j];
+    if (tangents) {
       Out* ot = out_t3 + 3 * (rd.bead_off + i);
-      ot[0] = (Out)gt[0];
-      ot[1] = (Out)gt[1];
-      ot[2] = (Out)gt[2];
+      for (int j = 0; j < 3; j++) ot[j] = (Out)gt[j];
     }
   }
-}
-
-__device__ double grad_block_sum(double v, double* sh) {
-  v = warp_sum(v);
-  const int w = threadIdx.x >> 5, l = threadIdx.x & 31;
-  __syncthreads();
-  if (l == 0) sh[w] = v;
-  __syncthreads();
-  double t = 0;
-  if (threadIdx.x < 32) {
-    t = threadIdx.x < (blockDim.x >> 5) ? sh[threadIdx.x] : 0.0;
-    t = warp_sum(t);
-  }
-  return t;  // valid in warp 0
 }
 
 // Terms T[14] of one replica: [0] S = sum_(vf <= limit) (V / V_bead) vf^2,
 // [1..3] sum_v rho_b^2, [4..6] sum_v rho_0 rho_1, rho_0 rho_2, rho_1 rho_2,
 // [7..9] #(state_b == 2), [10..12] sum_i s_ib, [13] sum_v (W / V)^2 with W the
 // bead weight of the voxel.  acc (or null): running sums [T, T T^T, count].
-__global__ void terms_kernel(KArgs a, double* terms, double* acc) {
-  __shared__ double sh[32];
-  __shared__ double T[kTerms];
-  const int rep = blockIdx.x;
+// A cluster per replica (see cg_energy.cuh).
+__global__ void __cluster_dims__(kSumCtas, 1, 1) __launch_bounds__(kSumThreads)
+    terms_kernel(KArgs a, double* terms, double* acc) {
+  __shared__ double sh[kSumThreads / 32][16];
+  __shared__ double T[16];
+  __shared__ long long gmax_sh;
+  const int rep = blockIdx.x / kSumCtas, rank = blockIdx.x % kSumCtas;
   const RepDev& rd = a.reps[rep];
-  double loc[kTerms];
-  for (int k = 0; k < kTerms; k++) loc[k] = 0;
-  const unsigned* st = a.states + rd.bead_off;
-  for (long long i = threadIdx.x; i < rd.n_beads; i += blockDim.x) {
-    const unsigned sw = st[i];
-    for (int b = 0; b < rd.nb; b++) {
-      const int s = (int)((sw >> (8 * b)) & 0xFF);
-      loc[7 + b] += s == 2 ? 1.0 : 0.0;
-      loc[10 + b] += (double)s;
+  const bool field = rd.field_kind == 2, uniform = field && !rd.has_access;
+  if (threadIdx.x == 0) gmax_sh = uniform ? weight_at_limit(rd) : 0;
+  __syncthreads();
+  int dbl[CG_MAX_BINDERS] = {0, 0, 0};
+  long long sum[CG_MAX_BINDERS] = {0, 0, 0};
+  {
+    const unsigned* st = a.states + rd.bead_off;
+    const long long per = (rd.n_beads + kSumCtas - 1) / kSumCtas;
+    const long long b1 = (rank + 1) * per < rd.n_beads ? (rank + 1) * per : rd.n_beads;
+    for (long long i = rank * per + threadIdx.x; i < b1; i += blockDim.x) {
+      const unsigned sw = st[i];
+#pragma unroll
+      for (int b = 0; b < CG_MAX_BINDERS; b++)
+        if (b < rd.nb) {
+          const int s = (int)((sw >> (8 * b)) & 0xFF);
+          dbl[b] += s == 2;
+          sum[b] += s;
+        }
     }
   }
-  if (rd.field_kind == 2 && !rd.has_access) {
-    // Uniform voxel volume V: every term is a sum of products of fixed-point
-    // grid values times one constant, so the raw products are summed (no FP64
-    // division per voxel; GB300 runs FP64 at 1/64 of the FP32 rate) and
-    // scaled once.  vf <= vf_limit <=> g0 <= vf_limit / (2^-40 Vb / V).
-    const long long* grid = a.grid + rd.vox_off * a.ncol;
-    const double u = kFxInv / rd.vol_bin;          // density per fixed-point unit
-    const double c = u * rd.bead_vol;              // volume fraction per unit
-    const double gmax = rd.vf_limit / c;
-    double s00 = 0, s00_lim = 0, sbb[CG_MAX_BINDERS] = {0, 0, 0}, sx[3] = {0, 0, 0};
-    for (long long v = threadIdx.x; v < rd.n_vox; v += blockDim.x) {
-      const double g0 = (double)grid[v * a.ncol];
-      double gb[CG_MAX_BINDERS] = {0, 0, 0};
-      for (int b = 0; b < rd.nb; b++) gb[b] = (double)grid[v * a.ncol + 1 + b];
-      const double q = g0 * g0;
-      s00 += q;
-      if (g0 <= gmax) s00_lim += q;
-      for (int b = 0; b < CG_MAX_BINDERS; b++) sbb[b] += gb[b] * gb[b];
-      sx[0] += gb[0] * gb[1];
-      sx[1] += gb[0] * gb[2];
-      sx[2] += gb[1] * gb[2];
-    }
-    const double u2 = u * u;
-    loc[0] += (rd.vol_bin / rd.bead_vol) * (c * c) * s00_lim;
-    for (int b = 0; b < CG_MAX_BINDERS; b++) loc[1 + b] += u2 * sbb[b];
-    for (int k = 0; k < 3; k++) loc[4 + k] += u2 * sx[k];
-    loc[13] += u2 * s00;
-  } else if (rd.field_kind == 2) {
-    const long long* grid = a.grid + rd.vox_off * a.ncol;
-    for (long long v = threadIdx.x; v < rd.n_vox; v += blockDim.x) {
-      const double V = rd.has_access ? a.access_vol[rd.vox_off + v] : rd.vol_bin;
+  GridSums g{};
+  double dens2 = 0;
+  if (uniform) {
+    const long long gmax = gmax_sh;
+    for_each_row<true>(a, rd, rank, [&](long long, const long long (&row)[4]) { add_row(rd, gmax, row, g); });
+  } else if (field) {
+    for_each_row<false>(a, rd, rank, [&](long long v, const long long (&row)[4]) {
+      if (empty_voxel(a, rd, v, row)) return;
+      const double V = a.access_vol[rd.vox_off + v];
       double rho[CG_MAX_BINDERS] = {0, 0, 0};
-      for (int b = 0; b < rd.nb; b++) rho[b] = ((double)grid[v * a.ncol + 1 + b] * kFxInv) / V;
-      const double dens = ((double)grid[v * a.ncol] * kFxInv) / V;
+#pragma unroll
+      for (int b = 0; b < CG_MAX_BINDERS; b++)
+        if (b < rd.nb) rho[b] = ((double)row[1 + b] * kFxInv) / V;
+      const double dens = ((double)row[0] * kFxInv) / V;
       const double vf = dens * rd.bead_vol;
-      if (vf <= rd.vf_limit) loc[0] += (V / rd.bead_vol) * vf * vf;
-      for (int b = 0; b < CG_MAX_BINDERS; b++) loc[1 + b] += rho[b] * rho[b];
-      loc[4] += rho[0] * rho[1];
-      loc[5] += rho[0] * rho[2];
-      loc[6] += rho[1] * rho[2];
-      loc[13] += dens * dens;
-    }
+      if (vf <= rd.vf_limit) g.s00 += (V / rd.bead_vol) * vf * vf;
+      for (int b = 0; b < CG_MAX_BINDERS; b++) g.sbb[b] += rho[b] * rho[b];
+      g.sx[0] += rho[0] * rho[1];
+      g.sx[1] += rho[0] * rho[2];
+      g.sx[2] += rho[1] * rho[2];
+      dens2 += dens * dens;
+    });
   }
-  for (int k = 0; k < kTerms; k++) {
-    const double t = grad_block_sum(loc[k], sh);
-    if (threadIdx.x == 0) T[k] = t;
+  double v[16] = {g.s00, g.sbb[0], g.sbb[1], g.sbb[2], g.sx[0], g.sx[1], g.sx[2], (double)dbl[0], (double)dbl[1],
+                  (double)dbl[2], (double)sum[0], (double)sum[1], (double)sum[2],
+                  uniform ? g.s00 + g.s00_over : dens2, 0.0, 0.0};
+  double t = cluster_sums(v, sh);
+  if (rank != 0) return;
+  if (threadIdx.x < kTerms) {
+    const int k = threadIdx.x;
+    if (uniform) {
+      const double u = kFxInv / rd.vol_bin, c = u * rd.bead_vol;
+      if (k == 0) t *= (rd.vol_bin / rd.bead_vol) * (c * c);
+      else if (k < 7 || k == 13) t *= u * u;
+    }
+    T[k] = t;
+    if (terms) terms[rep * kTerms + k] = t;
   }
   __syncthreads();
-  if (terms && threadIdx.x < kTerms) terms[rep * kTerms + threadIdx.x] = T[threadIdx.x];
   if (acc) {
     double* A = acc + (long long)rep * kAccPerRep;
     if (threadIdx.x < kTerms) A[threadIdx.x] += T[threadIdx.x];
@@ -262,9 +303,12 @@ __global__ void terms_kernel(KArgs a, double* terms, double* acc) {
 
 }  // namespace cg
 
+// CTAs of 4 warps, 30 beads a warp and pass: enough to fill the GPU four times
+// over, at most one pass each.
 static dim3 gradient_grid(const cg::KArgs& a, long long max_beads) {
-  long long bx = (max_beads + 127) / 128;
-  if (bx > 64) bx = 64;
+  long long bx = (max_beads + 119) / 120;
+  const long long most = std::max<long long>(64, 152 * 16 / std::max(1, a.n_reps));
+  if (bx > most) bx = most;
   if (bx < 1) bx = 1;
   return dim3((unsigned)bx, (unsigned)a.n_reps);
 }
@@ -307,5 +351,5 @@ void cg_launch_store_chains(const cg::KArgs& a, bool fp64, long long total, cons
 }
 
 void cg_launch_terms(const cg::KArgs& a, double* terms, double* acc, cudaStream_t s) {
-  cg::terms_kernel<<<a.n_reps, 256, 0, s>>>(a, terms, acc);
+  cg::terms_kernel<<<a.n_reps * cg::kSumCtas, cg::kSumThreads, 0, s>>>(a, terms, acc);
 }
