@@ -674,7 +674,7 @@ static int steric_run(cg_sim* s, int rep, long long ind0, long long indf, const 
   const long long n = s->n_beads[rep];
   const long long m = r_trial ? indf - ind0 : 0;
   if (r_trial && (ind0 < 0 || indf > n || m < 1)) return fail(CG_ERR_ARG, "need 0 <= ind0 < indf <= n_beads");
-  const long long need = n + 3 * m + 1;
+  const long long need = n + 32 + 3 * m + 1;  // tile sums (at most n + 32), trial segment, total
   if (need > s->steric_cap) {
     if (s->steric_work) cudaFree(s->steric_work);
     s->steric_work = nullptr;
@@ -683,10 +683,10 @@ static int steric_run(cg_sim* s, int rep, long long ind0, long long indf, const 
     s->steric_cap = need;
   }
   double* rows = s->steric_work;
-  double* trial = r_trial ? rows + n : nullptr;
-  double* total = rows + n + 3 * m;
+  double* trial = r_trial ? rows + n + 32 : nullptr;
+  double* total = rows + n + 32 + 3 * m;
   if (trial) CUDA_TRY(cudaMemcpy(trial, r_trial, 8 * 3 * m, cudaMemcpyHostToDevice));
-  cg_launch_steric(s->args(), s->fp64 != 0, rep, r_trial ? m : n, ind0, indf, trial, e, V0, rows, total, 0);
+  cg_launch_steric(s->args(), s->fp64 != 0, rep, n, r_trial ? m : n, ind0, indf, trial, e, V0, rows, total, 0);
   CUDA_TRY(cudaGetLastError());
   CUDA_TRY(cudaMemcpy(out, total, 8, cudaMemcpyDeviceToHost));
   return CG_OK;
