@@ -164,12 +164,12 @@ struct cg_sim {
   int direct_host = 0;
   void* hio_tab = nullptr;
   unsigned* hio_flag = nullptr;
-  // replicas using SSTWLC twist (the MC kernel's full form); with none,
-  // launches take its lean form
+  // replicas using SSTWLC twist or fast_field (the MC kernel's full form); with
+  // none, launches take its lean form
   std::vector<unsigned char> full_of;
   long long n_full = 0;
   void note_features(int rep, const RepDev& d) {
-    const unsigned char f = d.twist != 0;
+    const unsigned char f = d.twist != 0 || d.fast_n > 0;
     if (f == full_of[rep]) return;
     const bool was_lean = n_full == 0;
     n_full += f ? 1 : -1;

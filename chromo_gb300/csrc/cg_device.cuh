@@ -687,8 +687,16 @@ __device__ __forceinline__ void voxel_axes(const RepDev&, const GridF& gf, const
     m[j] = a < 0 ? (r != 0 ? w - r : -r) : r;
     near = near && x < w * 1048576.0f && w > 1e-30f && w < 1e30f;
   }
-  if (!near)
-    for (int j = 0; j < 3; j++) m[j] = pymodf(pos[j] + gf.half_w[j], gf.w[j]);
+  if (!near) {  // one copy of fmodf's code for the three axes
+#pragma unroll 1
+    for (int j = 0; j < 3; j++) {
+      const float p = j == 0 ? pos[0] : j == 1 ? pos[1] : pos[2];
+      const float r = pymodf(p + gf.half_w[j], gf.w[j]);
+      if (j == 0) m[0] = r;
+      else if (j == 1) m[1] = r;
+      else m[2] = r;
+    }
+  }
 #pragma unroll
   for (int j = 0; j < 3; j++) {
     float x = m[j] - gf.half_d[j];
@@ -743,18 +751,19 @@ __device__ __forceinline__ void fast_axes(const RepDev&, const GridF& gf, const 
 }
 // Per-axis voxels and weights of a move's density change: the sub-bin ones
 // with fast_field, else the exact ones (full deposits always use the exact
-// ones, as the reference's update_all_densities does).  Out of line for
-// fast_field, which production runs leave off.
+// ones, as the reference's update_all_densities does).  EXACT: the caller's
+// instantiation serves no fast_field replica.  The sub-bin weights are out of
+// line, through copies of the arrays (arrays passed to a call live in local
+// memory, on both paths).
 template <typename Real>
 static __device__ __noinline__ void fast_axes_ool(const RepDev& rd, const GridF& gf, const Real pos[3],
                                                   Real wl[3], int lo[3], int hi[3]) {
   fast_axes(rd, gf, pos, wl, lo, hi);
 }
-template <typename Real>
+template <bool EXACT = false, typename Real>
 __device__ __forceinline__ void move_axes(const RepDev& rd, const GridF& gf, const Real pos[3], Real wl[3],
                                           int lo[3], int hi[3]) {
-  if (rd.fast_n > 0) {
-    // through copies: arrays passed to a call live in local memory, on both paths
+  if (!EXACT && rd.fast_n > 0) {
     Real p[3], w[3];
     int l[3], h[3];
     for (int j = 0; j < 3; j++) p[j] = pos[j];

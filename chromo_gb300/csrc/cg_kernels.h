@@ -48,6 +48,7 @@ struct MovePlan {
   // the two boundary bond terms, the confinement counts and the error bits out
   int blk, sure, oob;
   unsigned derr;
+  unsigned xm;  // the move's Metropolis draw
   long long pq[2];
   double ph[2];
   double M[12];  // the 3 x 4 transform, stored in the position type

@@ -139,17 +139,15 @@ __device__ __forceinline__ void deposit_bead(const RepDev& rd, int ncol, int* ke
   }
 }
 
-// Claim (or find) the slots of up to NQ voxels per lane (v[j] where
-// want[j]) in a table shared by the lanes `peers` (this lane's bit set); the
-// peers append their new slots to the used list with one counter update.
-// Every lane's home-slot claims are issued back to back; only a claim that
-// meets another key probes on.  A table that cannot take a new voxel (slot
-// -1), or whose count of voxels passes `cap` (every peer), sets `full_bit` in
-// err.  Called by the whole warp.
+// Claim (or find) the slots of up to NQ voxels per lane (v[j] where want[j]);
+// new slots are appended to the used list.  Every lane's home-slot claims are
+// issued back to back; only a claim that meets another key probes on.  A table
+// that cannot take a new voxel (slot -1), or whose count of voxels this lane
+// takes past `cap`, sets `full_bit` in err.
 template <int NQ>
 __device__ __forceinline__ void claim_slots(int* keys, int* used, int* nused, int logH, const int (&v)[NQ],
                                             const bool (&want)[NQ], int (&slot)[NQ], unsigned& err,
-                                            int cap, unsigned full_bit, unsigned peers) {
+                                            int cap, unsigned full_bit) {
   int prev[NQ];
   bool fresh[NQ];
   unsigned pend = 0;  // claims whose home slot holds another key
@@ -184,25 +182,16 @@ __device__ __forceinline__ void claim_slots(int* keys, int* used, int* nused, in
       if (i == j) { slot[i] = h; fresh[i] = p == -1; }
     if (p == -1 || p == key) { pend &= pend - 1; it = 0; }
   }
-  const unsigned lane = threadIdx.x & 31u, lt = (1u << lane) - 1u;
-  const int leader = __ffs((int)peers) - 1;
-  unsigned bal[NQ];
   int cnt = 0;
 #pragma unroll
-  for (int j = 0; j < NQ; j++) {
-    bal[j] = __ballot_sync(kFull, fresh[j]) & peers;
-    cnt += __popc(bal[j]);
-  }
-  int base = 0;
-  if ((int)lane == leader && cnt) base = atomicAdd(nused, cnt);
-  base = __shfl_sync(kFull, base, leader);
-  int at = base;
+  for (int j = 0; j < NQ; j++) cnt += fresh[j] ? 1 : 0;
+  if (cnt) {  // few lanes hold a new slot: a counter update each costs less than ballots over the warp
+    int at = atomicAdd(nused, cnt);
+    if (at + cnt > cap) err |= full_bit;
 #pragma unroll
-  for (int j = 0; j < NQ; j++) {
-    if (fresh[j]) used[at + __popc(bal[j] & lt)] = slot[j];
-    at += __popc(bal[j]);
+    for (int j = 0; j < NQ; j++)
+      if (fresh[j]) used[at++] = slot[j];
   }
-  if (at > cap) err |= full_bit;
 }
 
 // The lanes of this lane's aligned group of G lanes.
@@ -282,14 +271,12 @@ __device__ __forceinline__ double with_huge(double hard, long long huge) {
   return huge != 0 ? hard_with_huge(hard, huge) : hard;
 }
 
-// Field dE of one touched voxel v in FP64 arithmetic (row `d` of a voxel
+// Field dE of one touched voxel v (grid row `row`) in FP64 arithmetic (row `d` of a voxel
 // table: the move's density deltas in, the voxel's post-move row out): added
 // to `part`; the 1e99 penalty of a voxel above vf_limit to `huge` (kHugeUnit
 // units).
-__device__ __forceinline__ void voxel_dE_f64(const RepDev& rd, const KArgs& a, const long long* grid, int v,
+__device__ __forceinline__ void voxel_dE_f64(const RepDev& rd, const KArgs& a, const long long (&row)[4], int v,
                                              long long* d, bool split, double& part, long long& huge) {
-  long long row[4];
-  load_row(grid + (long long)v * a.ncol, a.ncol, row);
   long long g0 = row[0], d0 = hash_delta(d, split);
   double V = rd.has_access ? a.access_vol[rd.vox_off + v] : rd.vol_bin;
   double c = 0, rho[CG_MAX_BINDERS], dd[CG_MAX_BINDERS];
@@ -331,8 +318,10 @@ static __device__ void field_dE_voxels(const WarpShared& ws, const KArgs& a, int
   long long hpart = 0;
   const long long* grid = a.grid + rd.vox_off * a.ncol;
   for (int i = lane; i < nused; i += G) {
-    const int slot = used[i];
-    voxel_dE_f64(rd, a, grid, keys[slot], vals + (long long)slot * hcol, split, part, hpart);
+    const int slot = used[i], v = keys[slot];
+    long long row[4];
+    load_row(grid + (long long)v * a.ncol, a.ncol, row);
+    voxel_dE_f64(rd, a, row, v, vals + (long long)slot * hcol, split, part, hpart);
   }
   n_vox = nused;
   (void)soft;
@@ -354,11 +343,9 @@ __device__ __forceinline__ void acc_add_wide(Fx& s, double x) {
 // volume-fraction limit takes the FP64 branch (its chi term in fixed point or
 // the side sum, the 1e99 penalties exactly into `huge`), so which side of the
 // limit it lies on is decided as in FP64.
-__device__ __forceinline__ void voxel_dE_f32(const WarpShared& ws, const KArgs& a, const long long* grid, int v,
+__device__ __forceinline__ void voxel_dE_f32(const WarpShared& ws, const KArgs& a, const long long (&row)[4], int v,
                                              long long* d, bool split, Fx& part, long long& huge) {
   const RepDev& rd = ws.rd;
-  long long row[4];
-  load_row(grid + (long long)v * a.ncol, a.ncol, row);
   const long long g0 = row[0], d0 = hash_delta(d, split);
   float sc = ws.f_scale, k = ws.f_k;
   if (rd.has_access) {  // per-voxel factors precomputed from V (no FP64 division here)
@@ -407,8 +394,10 @@ static __device__ void field_dE_voxels(const WarpShared& ws, const KArgs& a, int
   const long long* grid = a.grid + rd.vox_off * a.ncol;
   (void)hard;
   for (int i = lane; i < nused; i += G) {
-    const int slot = used[i];
-    voxel_dE_f32(ws, a, grid, keys[slot], vals + (long long)slot * hcol, split, part, hpart);
+    const int slot = used[i], v = keys[slot];
+    long long row[4];
+    load_row(grid + (long long)v * a.ncol, a.ncol, row);
+    voxel_dE_f32(ws, a, row, v, vals + (long long)slot * hcol, split, part, hpart);
   }
   n_vox = nused;
   acc_add(soft, gsum<G>(part));

@@ -223,7 +223,7 @@ struct BeadCells {
 // stages its new vectors for the commit, counts the confinement crossings and
 // finds its cells.  Returns false (and E_NONFINITE in e) for a position that
 // is not finite.
-template <typename Pos>
+template <typename Pos, bool LEAN>
 __device__ __forceinline__ bool place_bead(const RepDev& rd, const GridF& gf, const ChainView<Pos>& cv, int kind,
                                            const Pos (&M)[3][4], long long i, V4<Pos>* stage, bool density,
                                            bool conf, BeadCells<Pos>& c, unsigned& e, int& oob) {
@@ -248,10 +248,10 @@ __device__ __forceinline__ bool place_bead(const RepDev& rd, const GridF& gf, co
   }
   if (density) {
     int lo[3], hi[3];
-    move_axes(rd, gf, r, c.wl0, lo, hi);
+    move_axes<LEAN>(rd, gf, r, c.wl0, lo, hi);
     c.v0 = lo[0] + gf.nx * lo[1] + gf.nxy * lo[2];
     c.wrap0 = (hi[0] == 0 ? 1u : 0u) | (hi[1] == 0 ? 2u : 0u) | (hi[2] == 0 ? 4u : 0u);
-    move_axes(rd, gf, tr, c.wl1, lo, hi);
+    move_axes<LEAN>(rd, gf, tr, c.wl1, lo, hi);
     c.v1 = lo[0] + gf.nx * lo[1] + gf.nxy * lo[2];
     c.wrap1 = (hi[0] == 0 ? 1u : 0u) | (hi[1] == 0 ? 2u : 0u) | (hi[2] == 0 ? 4u : 0u);
   }
@@ -325,8 +325,7 @@ template <> __device__ __forceinline__ double load_acc<double>(long long, double
 // and the read-back: 20.9 -> 18.5 ms; one 10,000-bead chain, 10 steps: 3.71 ->
 // 3.46 ms; 64 SSTWLC chains of 2,000 beads, whose FP64 twist terms of a batch's
 // bonds now share their warp's issue, 10 steps: 18.2 -> 11.8 ms.)  The table is the CTA's pooled table (FP32
-// storage: keys voxel * 32 + slot, one used list, claims appended once per
-// warp) or the slot's own table (claims appended once per warp and move).  The
+// storage: keys voxel * 32 + slot, one used list) or the slot's own table.  The
 // bond terms, confinement counts and error bits go to the move's plan.  A move
 // whose optimistic table overflows (E_OVF: a pool or a table past 3/4 load) is
 // skipped from then on; its group deposits it again in its global table.
@@ -384,7 +383,7 @@ __device__ void block_deposit(const KArgs& a, SpecShared& sh, int rep, int B, in
       const unsigned sw = cv.st[i];
       unsigned e = 0;
       int oob;
-      on = place_bead(rd, gf, cv, kind, M, i, stage + 3 * k, true, conf, c, e, oob);
+      on = place_bead<Pos, LEAN>(rd, gf, cv, kind, M, i, stage + 3 * k, true, conf, c, e, oob);
       info = (sw & 0xFFFFFFu) | c.wrap0 << 24 | c.wrap1 << 27;
       if (oob) atomicAdd(&P.oob, oob);
       if (e) atomicOr(&P.derr, e);
@@ -407,7 +406,6 @@ __device__ void block_deposit(const KArgs& a, SpecShared& sh, int rep, int B, in
       corner_terms(gf, d, lane % kLanesPerBead, vq, q);
       // the pooled table (one used list for the whole CTA, keys voxel * 32 +
       // slot), or the move's own table (one used list per move)
-      const unsigned peers = pool ? kFull : __match_any_sync(kFull, t);
       int* keys = reinterpret_cast<int*>(pool ? smem + a.off_pkeys : wb + a.off_keys);
       int* used = reinterpret_cast<int*>(pool ? smem + a.off_pused : wb + a.off_used);
       long long* vals = reinterpret_cast<long long*>(pool ? smem + a.off_pvals : wb + a.off_vals);
@@ -423,7 +421,7 @@ __device__ void block_deposit(const KArgs& a, SpecShared& sh, int rep, int B, in
       int slot[2 * kCornersPerLane];
       unsigned e = 0;
       claim_slots<2 * kCornersPerLane>(keys, used, pool ? &sh.npool : &sh.nused[tt], lh, vq, want, slot, e,
-                                       sure ? Hs : (3 << lh) / 4, full_bit, peers);
+                                       sure ? Hs : (3 << lh) / 4, full_bit);
       if (!(e & full_bit)) {
 #pragma unroll
         for (int j = 0; j < 2 * kCornersPerLane; j++)
@@ -442,13 +440,13 @@ __device__ void block_deposit(const KArgs& a, SpecShared& sh, int rep, int B, in
 
 // One pooled entry's field term: FP32 storage in fixed point, FP64 storage in
 // FP64.
-__device__ __forceinline__ void pool_voxel_dE(const WarpShared& ws, const KArgs& a, const long long* grid, int v,
+__device__ __forceinline__ void pool_voxel_dE(const WarpShared& ws, const KArgs& a, const long long (&row)[4], int v,
                                               long long* d, Fx& part, long long& huge) {
-  voxel_dE_f32(ws, a, grid, v, d, true, part, huge);
+  voxel_dE_f32(ws, a, row, v, d, true, part, huge);
 }
-__device__ __forceinline__ void pool_voxel_dE(const WarpShared& ws, const KArgs& a, const long long* grid, int v,
+__device__ __forceinline__ void pool_voxel_dE(const WarpShared& ws, const KArgs& a, const long long (&row)[4], int v,
                                               long long* d, double& part, long long& huge) {
-  voxel_dE_f64(ws.rd, a, grid, v, d, true, part, huge);
+  voxel_dE_f64(ws.rd, a, row, v, d, true, part, huge);
 }
 
 // Add the warp's field terms to their moves' plans (s: this lane's move, -1 for
@@ -504,33 +502,42 @@ static __device__ void block_field_pool(const KArgs& a, SpecShared& sh, unsigned
   const long long* grid = a.grid + rd.vox_off * a.ncol;
   const int n = sh.npool;
   const int lane = (int)(threadIdx.x & 31u);
-  for (int e0 = (int)(threadIdx.x & ~31u); e0 < n; e0 += (int)blockDim.x) {
-    const int e = e0 + lane;
-    int s = -1;
-    Acc part = acc_zero<Acc>();
-    long long hp = 0;
+  // entry e's slot and key (-1: none, or of a move that overflowed) and its
+  // voxel's grid row
+  auto fetch = [&](int e, int& slot, int& key, long long (&row)[4]) {
+    key = -1;
+    slot = 0;
     if (e < n) {
-      const int slot = pused[e];
-      const int key = pkeys[slot];
-      s = key & 31;
+      slot = pused[e];
+      key = pkeys[slot];
+      if (sh.plan[key & 31].derr & E_OVF) key = -1;
+    }
+    if (key >= 0) load_row(grid + (long long)(key >> 5) * a.ncol, a.ncol, row);
+  };
+  // an entry's row is under way while its voxel is registered (fetching the next
+  // entry's ahead as well spilled registers and cost 1 %)
+  for (int e0 = (int)(threadIdx.x & ~31u); e0 < n; e0 += (int)blockDim.x) {
+    int slot, key;
+    long long row[4];
+    fetch(e0 + lane, slot, key, row);
+    const int s = key < 0 ? -1 : key & 31;
+    Acc part = acc_zero<Acc>();
+    if (key >= 0) {
       const int v = key >> 5;
       MovePlan& P = sh.plan[s];
-      if (P.derr & E_OVF) {
-        s = -1;
+      const int b = block_insert(bkeys, a.spec_logHB, v);
+      if (b < 0) {
+        atomicOr(&P.freg, 1);
       } else {
-        pool_voxel_dE(ws, a, grid, v, pvals + (long long)slot * a.hcol, part, hp);
-        const int b = block_insert(bkeys, a.spec_logHB, v);
-        if (b < 0) {
-          atomicOr(&P.freg, 1);
-        } else {
-          const unsigned prior = atomicOr(&bmask[b], 1u << s);
-          const unsigned below = (1u << s) - 1u, above = ~((2u << s) - 1u);
-          if (prior & below) atomicOr(&P.cmask, prior & below);
-          for (unsigned later = prior & above; later; later &= later - 1)
-            atomicOr(&sh.plan[__ffs((int)later) - 1].cmask, 1u << s);
-        }
-        if (hp) atomicAdd(reinterpret_cast<unsigned long long*>(&P.fH), (unsigned long long)hp);
+        const unsigned prior = atomicOr(&bmask[b], 1u << s);
+        const unsigned below = (1u << s) - 1u, above = ~((2u << s) - 1u);
+        if (prior & below) atomicOr(&P.cmask, prior & below);
+        for (unsigned later = prior & above; later; later &= later - 1)
+          atomicOr(&sh.plan[__ffs((int)later) - 1].cmask, 1u << s);
       }
+      long long hp = 0;
+      pool_voxel_dE(ws, a, row, v, pvals + (long long)slot * a.hcol, part, hp);
+      if (hp) atomicAdd(reinterpret_cast<unsigned long long*>(&P.fH), (unsigned long long)hp);
     }
     add_pool_part(sh, s, part);
   }
@@ -542,13 +549,17 @@ static __device__ void block_field_pool(const KArgs& a, SpecShared& sh, unsigned
 // is the block voxel table.
 static __device__ void block_commit_pool(const KArgs& a, SpecShared& sh, unsigned char* smem, int cut, unsigned acc,
                                   int* bkeys, unsigned* bmask) {
+  // warp 0 keeps the batch's books meanwhile (with one warp it does both)
+  const int skip = blockDim.x > 32 ? 32 : 0;
+  const int tid = (int)threadIdx.x - skip, nt = (int)blockDim.x - skip;
+  if (tid < 0) return;
   const RepDev& rd = sh.ws.rd;
   int* pkeys = reinterpret_cast<int*>(smem + a.off_pkeys);
   const int* pused = reinterpret_cast<const int*>(smem + a.off_pused);
   long long* pvals = reinterpret_cast<long long*>(smem + a.off_pvals);
   long long* grid = a.grid + rd.vox_off * a.ncol;
   const int n = sh.npool, hcol = a.hcol, ncol = a.ncol;
-  for (int e = (int)threadIdx.x; e < n; e += (int)blockDim.x) {
+  for (int e = tid; e < n; e += nt) {
     const int slot = pused[e];
     const int key = pkeys[slot];
     const int s = key & 31;
@@ -561,7 +572,7 @@ static __device__ void block_commit_pool(const KArgs& a, SpecShared& sh, unsigne
     pkeys[slot] = -1;
     for (int cc = 0; cc < hcol; cc++) src[cc] = 0;
   }
-  for (int i = (int)threadIdx.x; i < (1 << a.spec_logHB); i += (int)blockDim.x) {
+  for (int i = tid; i < (1 << a.spec_logHB); i += nt) {
     bkeys[i] = -1;
     bmask[i] = 0u;
   }
@@ -667,7 +678,6 @@ static __device__ __noinline__ void own_path(const KArgs& a, SpecShared& sh, int
                                                               : shared_slot(a, sh, s).stage);
   Pos M[3][4];
   load_transform(P, M);
-  const unsigned peers = group_mask<G>();
   unsigned err = 0;
   int oob = 0;
   // pass 0: moves the CTA did not deposit; pass 1: overflowed ones
@@ -697,7 +707,7 @@ static __device__ __noinline__ void own_path(const KArgs& a, SpecShared& sh, int
       if (act) {
         int ob;
         if (density) sw = cv.st[ind0 + k];
-        act = place_bead(rd, gf, cv, kind, M, ind0 + k, stage + 3 * k, density, check_field && rd.confine_kind, c,
+        act = place_bead<Pos, LEAN>(rd, gf, cv, kind, M, ind0 + k, stage + 3 * k, density, check_field && rd.confine_kind, c,
                          e, ob);
         oob += ob;
       }
@@ -710,7 +720,7 @@ static __device__ __noinline__ void own_path(const KArgs& a, SpecShared& sh, int
 #pragma unroll
           for (int j = 0; j < 2 * kCornersPerLane; j++) want[j] = act && q[j] != 0 && !(e & E_OVF);
           int slot[2 * kCornersPerLane];
-          claim_slots<2 * kCornersPerLane>(S.keys, S.used, nused, S.logH, vq, want, slot, e, cap, full_bit, peers);
+          claim_slots<2 * kCornersPerLane>(S.keys, S.used, nused, S.logH, vq, want, slot, e, cap, full_bit);
           if (!(e & full_bit)) {
 #pragma unroll
             for (int j = 0; j < 2 * kCornersPerLane; j++)
@@ -772,15 +782,447 @@ static __device__ __noinline__ void own_path(const KArgs& a, SpecShared& sh, int
   __syncwarp();
 }
 
-// Evaluate move t of the batch in slot s (group lanes gl = 0..G-1); `live`
-// is false for the groups of a partly filled batch and for the warps without
-// a move, which run the collectives and block barriers with empty work.
-// Every thread of the CTA calls it (position moves hold two block barriers
-// around the block-wide deposit); B is the batch's number of moves.
+// Tangent rotation of bead i about the axis of draws xa, xb (sine sa, cosine
+// ca): its new frame and the dE of its two bonds, the neighbours' frames as they
+// are.
+template <typename Pos, bool LEAN>
+__device__ __forceinline__ typename AccOf<Pos>::type rotate_tangent(const KArgs& a, const RepDev& rd, long long i,
+                                                                    unsigned xa, unsigned xb, Pos sa, Pos ca,
+                                                                    Pos (&tt3)[3], Pos (&tt2)[3]) {
+  using Real = Pos;
+  using Acc = typename AccOf<Real>::type;
+  const long long N = rd.n_beads;
+  const V4<Pos>* r4 = reinterpret_cast<const V4<Pos>*>(a.r4) + rd.bead_off;
+  const V4<Pos>* t34 = reinterpret_cast<const V4<Pos>*>(a.t34) + rd.bead_off;
+  const V4<Pos>* t24 = reinterpret_cast<const V4<Pos>*>(a.t24) + rd.bead_off;
+  const double* bonds = a.bonds + rd.bead_off * 6;
+  const float* bonds32 = a.bonds32 + rd.bead_off * 8;
+  // the bead, both neighbours and both bonds, loaded together (in-range
+  // indices at the chain ends, where the term is skipped)
+  const bool hl = i != 0, hr = i + 1 != N;
+  const long long il = hl ? i - 1 : i, ir = hr ? i + 1 : i;
+  Real r[3], t3[3], t2[3], r0[3], t30[3], r1[3], t31[3];
+  ld3(r4, i, r); ld3(t34, i, t3); ld3(t24, i, t2);
+  ld3(r4, il, r0); ld3(t34, il, t30); ld3(r4, ir, r1); ld3(t34, ir, t31);
+  const Bond<Real> bl = bond_at(bonds, bonds32, il, (Real)0), br = bond_at(bonds, bonds32, i, (Real)0);
+  Real axis[3];
+  sphere_from<Real>(xa, xb, axis);
+  const Real origin[3] = {0, 0, 0};
+  Real M[3][4];
+  axis_rotation_sc(axis, origin, sa, ca, M);
+  for (int j = 0; j < 3; j++) {
+    Real e3 = 0, e2 = 0;
+    for (int q = 0; q < 3; q++) { e3 += M[j][q] * t3[q]; e2 += M[j][q] * t2[q]; }
+    tt3[j] = e3; tt2[j] = e2;
+  }
+  Acc de = acc_zero<Acc>();
+  if (hl) acc_add(de, pair_dE_fwd(bl, r0, r, r, t30, t3, tt3));
+  if (hr) acc_add(de, pair_dE_rev(br, r, r, r1, t3, tt3, t31));
+  if (!LEAN && rd.twist) {  // SSTWLC: twist terms of both bonds
+    const double* tw = a.twist + rd.bead_off * 2;
+    const Frame cur = frame_of(t2, t3), nw = frame_of(tt2, tt3);
+    double dt = 0;
+    if (hl) {
+      const Frame l = frame_of(t24[il], t34[il]);
+      dt += twist_pair_dE(tw + 2 * il, l, cur, l, nw);
+    }
+    if (hr) {
+      const Frame rr = frame_of(t24[ir], t34[ir]);
+      dt += twist_pair_dE(tw + 2 * i, cur, rr, nw, rr);
+    }
+    acc_add_d(de, dt);
+  }
+  return de;
+}
+
+// ---------------------------------------------------------------- short tangent rotations
+// Batches of tangent rotations of few beads (SimpleControl settles at an
+// amplitude of ~13, a mean of 7 beads): GS = 8 or 16 lanes per move instead of
+// 32, so that 2-4 times as many moves are in flight on the same warps, and the
+// rotated beads registered in the block table (key: bead), so that a move finds
+// the earlier moves that rotate its beads or their neighbours by three look-ups
+// a bead instead of comparing lists.  A move's staging, index list and draws
+// fit its share of the slot regions for up to 2 GS beads (amplitudes up to 32;
+// longer ones take the path of 32 lanes).  One 10,000-bead chain, 10 MC steps:
+// 2.83 -> 2.62 ms; 64 SSTWLC chains of 2,000 beads, whose FP64 twist terms fill
+// their warps' lanes: 10.4 -> 9.1 ms (kernel only, with the phases' state kept
+// in the plans).
+//
+// Moves in flight: kShortSpan sqrt(N) / (amp + 1), at which about two of them
+// meet an earlier accepted one (3 and 4 measured alike, 6 and 9 were slower on
+// 2,000-bead chains).
+constexpr float kShortSpan = 4.0f;
+struct ShortTangent {
+  int GS, s, gl;
+  unsigned gmask;  // the group's lanes
+  int* idx;
+  float* stage;    // new t3, t2 of each bead: 6 floats
+  unsigned* draws;
+  int ndraw;
+  __device__ __forceinline__ ShortTangent(const KArgs& a, SpecShared& sh, int gs) : GS(gs) {
+    const int lane = (int)(threadIdx.x & 31u), per = 32 / GS;
+    const int warp = (int)(threadIdx.x >> 5), sub = lane / GS;
+    s = warp * per + sub;
+    gl = lane & (GS - 1);
+    gmask = (GS == 16 ? 0xFFFFu : 0xFFu) << (lane & ~(GS - 1));
+    unsigned char* base = reinterpret_cast<unsigned char*>(&sh) + a.spec_off_warps + (size_t)warp * a.warp_smem;
+    idx = reinterpret_cast<int*>(base + a.off_draws) + sub * 2 * GS;
+    const int room = ((a.off_idx - a.off_stage + 4 * (int)a.stage_cap) * GS / 32) & ~15;
+    unsigned char* q = base + a.off_stage + sub * room;
+    stage = reinterpret_cast<float*>(q);
+    draws = reinterpret_cast<unsigned*>(q + 48 * GS);  // 2 GS beads x 24 bytes
+    ndraw = (room - 48 * GS) / 16 * 4;
+  }
+};
+static_assert(4 * kDrawCache == 32 * 2 * 4, "the index lists share the draw buffer: 2 GS beads a group");
+
+__device__ __forceinline__ unsigned block_find(const int* bkeys, const unsigned* bmask, int logHB, int key) {
+  const unsigned mask = (1u << logHB) - 1u;
+  unsigned h = ((unsigned)key * 0x9E3779B1u) >> (32 - logHB);
+  for (int it = 0; it < 64; it++) {  // as far as block_insert probes
+    const int k = bkeys[h];
+    if (k == key) return bmask[h];
+    if (k == -1) return 0u;
+    h = (h + 1) & mask;
+  }
+  return 0u;
+}
+
+// Evaluate the batch's B moves (one per group of GS lanes) into their plans.
+template <bool LEAN>
+__device__ void short_tangent_evaluate(const KArgs& a, SpecShared& sh, int rep, const ShortTangent& T, int B,
+                                       const cg_move_ctl& c, int* bkeys, unsigned* bmask) {
+  const RepDev& rd = sh.ws.rd;
+  const int GS = T.GS, gl = T.gl, s = T.s;
+  const bool live = s < B;
+  if (!__any_sync(kFull, live)) return;
+  const unsigned N = (unsigned)rd.n_beads, amp = (unsigned)c.amp_bead;
+  const unsigned long long t = sh.t0 + (unsigned long long)s;
+  const uint2 key = make_uint2((unsigned)a.seed ^ (unsigned)rep * 0x85EBCA6Bu,
+                               (unsigned)(a.seed >> 32) ^ 0x1B873593u);
+  const unsigned tlo = (unsigned)t, thi = (unsigned)(t >> 32);
+  const int have = min(T.ndraw, (int)(3 * amp + 6) & ~3);  // angle, count, beads, axes, decision
+  for (int j = gl; 4 * j < have; j += GS)
+    reinterpret_cast<uint4*>(T.draws)[j] = philox(make_uint4((unsigned)j, tlo, thi, 0x2545F491u), key);
+  __syncwarp();
+  auto word = [&](int j) { return j < have ? T.draws[j] >> 1 : move_draw_slow(key, tlo, thi, (unsigned long long)j); };
+  const float ang = (float)c.amp_move * (uni<float>(word(0)) - 0.5f);
+  const int n = (int)(word(1) % amp) + 1;
+  unsigned err = n > (int)N ? E_WINDOW : 0u;
+  int m = live && !err ? n : 0;
+  // distinct random beads in draw order: nearly always the first m draws are
+  int mine[2] = {-1, -1};
+#pragma unroll
+  for (int p = 0; p < 2; p++) {
+    const int k = p * GS + gl;
+    if (k < m) T.idx[k] = mine[p] = (int)(word(2 + k) % N);
+  }
+  __syncwarp();
+  bool dup = false;
+  const int most = (int)__reduce_max_sync(kFull, (unsigned)m);
+  for (int q = 0; q + 1 < most; q++) {
+    const int v = q < m ? T.idx[q] : -2;
+    dup = dup || (v == mine[0] && q < gl) || (v == mine[1] && q < GS + gl);
+  }
+  const unsigned dups = __ballot_sync(kFull, dup);
+  int used = m;  // draws taken for the beads
+  if (dups) {    // with redraws: by the group's first lane
+    if ((dups & T.gmask) && gl == 0) {
+      int got = 0, pos = 0;
+      while (got < m) {
+        if (pos >= 32 * kMaxIter) { err |= E_SPIN; break; }
+        const int x = (int)(word(2 + pos++) % N);
+        bool seen = false;
+        for (int q = 0; q < got; q++) seen = seen || T.idx[q] == x;
+        if (!seen) T.idx[got++] = x;
+      }
+      used = pos;
+    }
+    const int first = __ffs((int)T.gmask) - 1;
+    used = __shfl_sync(kFull, used, first);
+    err |= __shfl_sync(kFull, err, first);
+    if (err) m = 0;
+    __syncwarp();
+  }
+  float sa, ca;
+  rsincos(ang, &sa, &ca);
+  Fx part = acc_zero<Fx>();
+  int regfail = 0;
+  for (int k = gl; k < m; k += GS) {
+    const int i = T.idx[k];
+    const unsigned xa = word(2 + used + 2 * k), xb = word(3 + used + 2 * k);
+    float tt3[3], tt2[3];
+    acc_add(part, rotate_tangent<float, LEAN>(a, rd, i, xa, xb, sa, ca, tt3, tt2));
+    for (int j = 0; j < 3; j++) {
+      T.stage[6 * k + j] = tt3[j];
+      T.stage[6 * k + 3 + j] = tt2[j];
+    }
+    const int b = block_insert(bkeys, a.spec_logHB, i);
+    if (b < 0) regfail = 1;
+    else atomicOr(&bmask[b], 1u << s);
+  }
+  for (int o = GS / 2; o > 0; o >>= 1) {
+    part.q += __shfl_xor_sync(kFull, part.q, o);
+    regfail |= __shfl_xor_sync(kFull, regfail, o);
+  }
+  if (__any_sync(kFull, !is_zero64(part.hard)))
+    for (int o = GS / 2; o > 0; o >>= 1) part.hard += __shfl_xor_sync(kFull, part.hard, o);
+  if (live && gl == 0) {
+    MovePlan& P = sh.plan[s];
+    P.kind = CG_TANGENT_ROTATION;
+    P.m = m;
+    P.ind0 = m > 0 ? T.idx[0] : 0;
+    P.indf = m > 0 ? P.ind0 + 1 : 0;
+    P.empty = 0;
+    P.err = (int)err;
+    P.regfail = regfail;
+    P.nvox = 0;
+    P.cmask = 0;
+    bool dec = false;
+    if (!err) dec = decide(word(2 + used + 2 * m), part, Fx{0, 0.0}, 0.0, &P.dE);
+    P.dec = dec ? 1 : 0;
+    if (!LEAN && a.mlog) log_terms(P, part, (unsigned long long)(2 + used + 2 * m + (err ? 0 : 1)));
+  }
+}
+
+// The earlier moves of the batch that rotate this move's beads or their
+// neighbours.
+static __device__ __forceinline__ void short_tangent_conflicts(const KArgs& a, SpecShared& sh, const ShortTangent& T, int B,
+                                                        const int* bkeys, const unsigned* bmask) {
+  const int s = T.s;
+  unsigned cm = 0;
+  const int m = s < B ? sh.plan[s].m : 0;
+  for (int k = T.gl; k < m; k += T.GS) {
+    const int i = T.idx[k];
+#pragma unroll
+    for (int d = -1; d <= 1; d++) cm |= block_find(bkeys, bmask, a.spec_logHB, i + d);
+  }
+  cm &= (1u << s) - 1u;
+  if (cm) atomicOr(&sh.plan[s].cmask, cm);
+}
+
+static __device__ __forceinline__ void short_tangent_commit(const KArgs& a, SpecShared& sh, const ShortTangent& T, int cut,
+                                                     unsigned acc, int* bkeys, unsigned* bmask) {
+  const RepDev& rd = sh.ws.rd;
+  const int s = T.s;
+  if (s < cut && ((acc >> s) & 1u)) {
+    V4<float>* t34w = reinterpret_cast<V4<float>*>(a.t34) + rd.bead_off;
+    V4<float>* t24w = reinterpret_cast<V4<float>*>(a.t24) + rd.bead_off;
+    const int m = sh.plan[s].m;
+    for (int k = T.gl; k < m; k += T.GS) {
+      const float* q = T.stage + 6 * k;
+      const int i = T.idx[k];
+      t34w[i] = V4<float>{q[0], q[1], q[2], 0.0f};
+      t24w[i] = V4<float>{q[3], q[4], q[5], 0.0f};
+    }
+  }
+  for (int i = (int)threadIdx.x; i < (1 << a.spec_logHB); i += (int)blockDim.x) {
+    bkeys[i] = -1;
+    bmask[i] = 0u;
+  }
+}
+
+__device__ __forceinline__ void segment_of(long long b0, long long b1, long long N, int& ind0, int& indf) {
+  long long i0, i1;
+  check_bead_bounds(b0, b1, N, i0, i1);
+  ind0 = (int)i0;
+  indf = (int)i1;
+}
+
+// A move's state between the phases of its batch is in its plan, so little is
+// held in registers over them (kept in registers, it was spilled around the
+// out-of-line own_path and cost every batch ~5 %).
+
+// Propose position move t of the batch in slot s (group lanes gl = 0..G-1):
+// its segment and transform, its table and its Metropolis draw go to its plan.
+// `live` is false for the groups of a partly filled batch.  Called by the whole
+// warp.
+template <typename Pos, int G, bool LEAN>
+__device__ void propose_position(const KArgs& a, SpecShared& sh, int rep, int s, int gl, bool live, int kind,
+                                 const cg_move_ctl& c, unsigned long long t) {
+  using Real = Pos;
+  const RepDev& rd = sh.ws.rd;
+  const long long N = rd.n_beads;
+  const V4<Pos>* r4 = reinterpret_cast<const V4<Pos>*>(a.r4) + rd.bead_off;
+  MovePlan& P = sh.plan[s];
+  MoveRng g;
+  if (!__any_sync(kFull, live)) return;
+  g.init<G>(a.seed, rep, t,
+            reinterpret_cast<unsigned*>(reinterpret_cast<unsigned char*>(&sh) + a.spec_off_warps +
+                                        (size_t)s * a.warp_smem + a.off_draws), gl);
+  unsigned err = 0;
+  const bool density = rd.field_kind == 2;
+  int ind0 = 0, indf = 0, m = 0, gstage = 0, gtab = 0;  // chains are limited to 2e9 beads
+  bool empty = !live;
+  const int Hs = 1 << a.logH;
+  const bool pool = a.pool_on != 0;
+  Real M[3][4];
+  for (int i = 0; i < 3; i++)
+    for (int j = 0; j < 4; j++) M[i][j] = i == j ? (Real)1 : (Real)0;
+  if (live) {
+    if (kind == CG_CRANK_SHAFT) {
+      Real ang = (Real)c.amp_move * (uni<Real>(g.next()) - (Real)0.5);
+      const unsigned xb0 = g.next();
+      long long b0 = sizeof(Real) == 4 ? scaled_index(xb0, N) : (long long)(int)(unif(xb0) * (double)N);
+      long long b1 = from_point(g, c.amp_bead, N, b0, err);
+      if (b1 < 1) b1 = 1;
+      segment_of(b0, b1, N, ind0, indf);
+      long long ia, ib;
+      if (ind0 == indf - 1 && ind0 == 0) { ia = indf; ib = ind0; }
+      else if (ind0 == indf - 1 && ind0 == N - 1) { ia = ind0; ib = ind0 - 1; }
+      else if (ind0 == 0 && indf == N) { ia = indf - 1; ib = ind0; }
+      else if (ind0 == 0) { ia = indf; ib = ind0; }
+      else if (indf == N) { ia = indf - 1; ib = ind0 - 1; }
+      else { ia = indf; ib = ind0 - 1; }
+      if (!err) {
+        Real pa[3], pb[3], dir[3], p[3];
+        long long ip;  // the fulcrum bead, loaded with the two axis beads
+        if (ind0 == 0 && indf != N) ip = indf;
+        else if (ind0 != 0 && indf == N) ip = ind0 - 1;
+        else if (ind0 == 0 && indf == N) ip = ind0;
+        else ip = ind0 - 1;
+        ld3(r4, ia, pa); ld3(r4, ib, pb); ld3(r4, ip, p);
+        for (int i = 0; i < 3; i++) dir[i] = pa[i] - pb[i];
+        Real mag = rsqrt_(dir[0] * dir[0] + dir[1] * dir[1] + dir[2] * dir[2]);
+        if (mag < (Real)1E-5) sphere<Real>(g, dir);
+        else { Real sc = (Real)1 / mag; for (int i = 0; i < 3; i++) dir[i] = dir[i] * sc; }
+        axis_rotation(dir, p, ang, M);
+      }
+    } else if (kind == CG_END_PIVOT) {
+      Real ang = (Real)c.amp_move * (uni<Real>(g.next()) - (Real)0.5);
+      long long lhs = g.next() & 1u;
+      if (lhs == 1) { ind0 = 0; indf = (int)from_left(g, c.amp_bead, N, err) + 1; }
+      else { ind0 = (int)(N - from_left(g, c.amp_bead, N, err)); indf = (int)N; }
+      Real axis[3], p[3];
+      sphere<Real>(g, axis);
+      long long ip;
+      if (ind0 == 0 && indf != N) ip = indf;
+      else if (ind0 != 0 && indf == N) ip = ind0 - 1;
+      else if (ind0 == 0 && indf == N && lhs == 1) ip = indf - 1;
+      else ip = ind0;
+      if (!err) {
+        ld3(r4, ip, p);
+        axis_rotation(axis, p, ang, M);
+      }
+    } else {
+      Real amp = (Real)c.amp_move * uni<Real>(g.next()), d[3];
+      sphere<Real>(g, d);
+      for (int i = 0; i < 3; i++) M[i][3] = d[i] * amp;
+      long long b0 = g.next() % (unsigned)N;
+      long long b1 = from_point(g, c.amp_bead, N, b0, err);
+      segment_of(b0, b1, N, ind0, indf);
+    }
+  }
+  m = (!live || err) ? 0 : indf - ind0;
+  if (live && !err && m == 0) empty = true;
+  // the Metropolis draw, taken now: the plan holds all of the move's state from here
+  unsigned xm = 0;
+  if (live && !err && !empty) xm = g.next();
+  if (m > a.stage_cap) gstage = 1;
+  // voxel table: the CTA's pooled table for every move of up to
+  // kPoolMaxBeads beads, optimistically (a pool past 3/4 load sends the move
+  // to its global table); without the pool (a grid of 2^26 voxels and more)
+  // the slot's own table when the move's at most 16 m voxels surely fit, or
+  // optimistically up to m <= slots / 4 with the same fallback; global beyond
+  bool sure = false, blk;
+  const int most = kPoolMaxBeads >> ((rd.nx == 1) + (rd.ny == 1) + (rd.nz == 1));
+  if (pool) {
+    blk = density && m > 0 && m <= most;
+    gtab = density && m > 0 && !blk;
+  } else {
+    sure = 16 * m <= Hs;
+    gtab = (!sure && 4 * m > Hs) || m > most;
+    blk = density && m > 0 && !gtab;  // moves with a shared table are deposited by the whole CTA
+  }
+  if (gl == 0 && live) {
+    P.blk = blk ? 1 : 0;
+    P.sure = sure ? 1 : 0;
+    P.kind = kind;
+    P.m = m;
+    P.ind0 = ind0;
+    P.indf = indf;
+    P.empty = empty ? 1 : 0;
+    P.err = (int)err;
+    P.xm = xm;
+    if (!LEAN) P.ndraw = (int)g.pos;
+    P.gstage = gstage;
+    P.gtab = gtab;
+    P.oob = 0;
+    P.derr = 0;
+    P.cmask = 0;
+    P.pq[0] = P.pq[1] = 0;
+    P.ph[0] = P.ph[1] = 0;
+    P.fq = P.fH = 0;
+    P.fh = 0;
+    P.fl0 = P.fl1 = 0;
+    P.fl2 = 0;
+    P.fn = P.freg = 0;
+    Pos* Mp = reinterpret_cast<Pos*>(P.M);  // in the position type: no conversions
+    for (int i = 0; i < 3; i++)
+      for (int j = 0; j < 4; j++) Mp[4 * i + j] = M[i][j];
+  }
+}
+
+// Earlier moves u of the batch whose written beads [ind0, indf) meet the beads
+// a position move reads (its segment and both neighbours), added to its mask; a
+// move with no beads (failed or empty) is never accepted, so it needs no
+// exclusion.  Called by the whole warp.
+template <int G>
+__device__ __forceinline__ void bead_conflicts(SpecShared& sh, int s, int gl, bool live, int B) {
+  MovePlan& P = sh.plan[s];
+  const int m = live ? P.m : 0, ind0 = P.ind0, indf = P.indf;
+  unsigned cmb = 0;
+  for (int u0 = 0; u0 < B; u0 += G) {
+    const int u = u0 + gl;
+    bool hit = false;
+    if (m > 0 && u < s) {
+      const MovePlan& U = sh.plan[u];
+      hit = U.m > 0 && U.ind0 <= indf && ind0 <= U.indf;
+    }
+    cmb |= gballot<G>(hit) << u0;
+  }
+  if (gl == 0 && live && cmb) atomicOr(&P.cmask, cmb);
+}
+
+// The decision on a position move from the results in its plan.
+template <typename Pos, int G, bool LEAN>
+__device__ __forceinline__ void decide_position(const KArgs& a, SpecShared& sh, int s, int gl, bool live) {
+  using Acc = typename AccOf<Pos>::type;
+  if (!live) return;
+  MovePlan& P = sh.plan[s];
+  Acc dEp = acc_zero<Acc>(), dEs = acc_zero<Acc>();
+  double dEh = 0;
+  long long dEH = 0;  // the exact 1e99 penalties, in kHugeUnit units
+  unsigned err = (unsigned)P.err;
+  int nvox = 0, regfail = 0;
+  if (P.m > 0) {
+    acc_add(dEp, load_acc<Acc>(P.pq[0], P.ph[0]));
+    acc_add(dEp, load_acc<Acc>(P.pq[1], P.ph[1]));
+    plan_field(P, dEs, dEh);
+    const int oo = P.oob;
+    dEH = P.fH + (((long long)(oo >> 16) - (long long)(oo & 0xFFFF)) << 40);
+    err |= P.derr & ~E_OVF;
+    nvox = P.fn;
+    regfail = P.freg;
+  }
+  bool dec = false;
+  if (!err && !P.empty) dec = decide(P.xm, dEp, dEs, with_huge(dEh, dEH), gl == 0 ? &P.dE : nullptr);
+  __syncwarp(group_mask<G>());  // every lane has read the plan
+  if (gl == 0) {
+    P.err = (int)err;
+    P.regfail = regfail;
+    P.dec = dec ? 1 : 0;
+    P.nvox = nvox;
+    if (!LEAN && a.mlog) log_terms(P, dEp, (unsigned long long)P.ndraw);
+  }
+}
+
+// Evaluate tangent rotation or binding move t of the batch in slot s (group
+// lanes gl = 0..G-1); `live` is false for the groups of a partly filled batch.
+// Called by the whole warp.
 template <typename Pos, int G, bool LEAN>
 __device__ void evaluate_move(const KArgs& a, SpecShared& sh, int rep, int s, int gl, bool live, int kind,
-                              const cg_move_ctl& c, unsigned long long t, unsigned* picked, int* bkeys,
-                              unsigned* bmask, int B) {
+                              const cg_move_ctl& c, unsigned long long t, int* bkeys, unsigned* bmask) {
   using Real = Pos;
   using Acc = typename AccOf<Real>::type;
   const RepDev& rd = sh.ws.rd;
@@ -789,168 +1231,29 @@ __device__ void evaluate_move(const KArgs& a, SpecShared& sh, int rep, int s, in
   const long long N = rd.n_beads;
   const int hcol = a.hcol;  // stride of the voxel-table values
   const V4<Pos>* r4 = reinterpret_cast<const V4<Pos>*>(a.r4) + rd.bead_off;
-  const V4<Pos>* t34 = reinterpret_cast<const V4<Pos>*>(a.t34) + rd.bead_off;
-  const V4<Pos>* t24 = reinterpret_cast<const V4<Pos>*>(a.t24) + rd.bead_off;
   const unsigned* st = a.states + rd.bead_off;
   const unsigned* mk = a.marks + rd.bead_off;
-  const double* bonds = a.bonds + rd.bead_off * 6;
-  const float* bonds32 = a.bonds32 + rd.bead_off * 8;
   MovePlan& P = sh.plan[s];
   MoveRng g;
-  if (__any_sync(kFull, live))
-    g.init<G>(a.seed, rep, t,
-              reinterpret_cast<unsigned*>(reinterpret_cast<unsigned char*>(&sh) + a.spec_off_warps +
-                                          (size_t)s * a.warp_smem + a.off_draws), gl);
+  if (!__any_sync(kFull, live)) return;
+  g.init<G>(a.seed, rep, t,
+            reinterpret_cast<unsigned*>(reinterpret_cast<unsigned char*>(&sh) + a.spec_off_warps +
+                                        (size_t)s * a.warp_smem + a.off_draws), gl);
   unsigned err = 0;
   const bool check_field = rd.field_kind != 0 && kind != CG_TANGENT_ROTATION;
   const bool density = rd.field_kind == 2;
-  long long ind0 = 0, indf = 0, m = 0;
+  int ind0 = 0, indf = 0, m = 0;  // chains are limited to 2e9 beads
   // dE = dEp (polymer) + dEs (field; fixed point for FP32 storage) + dEh (the
   // FP64 part: confinement penalties, and the whole field dE for FP64 storage)
   Acc dEp = acc_zero<Acc>(), dEs = acc_zero<Acc>();
   double dEh = 0;
   long long dEH = 0;  // the exact 1e99 penalties, in kHugeUnit units
-  long long nvox = 0;
-  bool empty = !live;
+  int nvox = 0;
+  const bool empty = !live;
   int gtab = 0, gstage = 0, regfail = 0;
-  unsigned xm = 0;  // the Metropolis draw
   const int Hs = 1 << a.logH;
-  const bool pool = a.pool_on != 0;
-  if (threadIdx.x == 0) sh.npool = 0;  // every reader of the last batch's pool passed a barrier since
 
-  if (kind <= CG_SLIDE) {
-    Real M[3][4];
-    for (int i = 0; i < 3; i++)
-      for (int j = 0; j < 4; j++) M[i][j] = i == j ? (Real)1 : (Real)0;
-    if (live) {
-      if (kind == CG_CRANK_SHAFT) {
-        Real ang = (Real)c.amp_move * (uni<Real>(g.next()) - (Real)0.5);
-        const unsigned xb0 = g.next();
-        long long b0 = sizeof(Real) == 4 ? scaled_index(xb0, N) : (long long)(int)(unif(xb0) * (double)N);
-        long long b1 = from_point(g, c.amp_bead, N, b0, err);
-        if (b1 < 1) b1 = 1;
-        check_bead_bounds(b0, b1, N, ind0, indf);
-        long long ia, ib;
-        if (ind0 == indf - 1 && ind0 == 0) { ia = indf; ib = ind0; }
-        else if (ind0 == indf - 1 && ind0 == N - 1) { ia = ind0; ib = ind0 - 1; }
-        else if (ind0 == 0 && indf == N) { ia = indf - 1; ib = ind0; }
-        else if (ind0 == 0) { ia = indf; ib = ind0; }
-        else if (indf == N) { ia = indf - 1; ib = ind0 - 1; }
-        else { ia = indf; ib = ind0 - 1; }
-        if (!err) {
-          Real pa[3], pb[3], dir[3], p[3];
-          long long ip;  // the fulcrum bead, loaded with the two axis beads
-          if (ind0 == 0 && indf != N) ip = indf;
-          else if (ind0 != 0 && indf == N) ip = ind0 - 1;
-          else if (ind0 == 0 && indf == N) ip = ind0;
-          else ip = ind0 - 1;
-          ld3(r4, ia, pa); ld3(r4, ib, pb); ld3(r4, ip, p);
-          for (int i = 0; i < 3; i++) dir[i] = pa[i] - pb[i];
-          Real mag = rsqrt_(dir[0] * dir[0] + dir[1] * dir[1] + dir[2] * dir[2]);
-          if (mag < (Real)1E-5) sphere<Real>(g, dir);
-          else { Real sc = (Real)1 / mag; for (int i = 0; i < 3; i++) dir[i] = dir[i] * sc; }
-          axis_rotation(dir, p, ang, M);
-        }
-      } else if (kind == CG_END_PIVOT) {
-        Real ang = (Real)c.amp_move * (uni<Real>(g.next()) - (Real)0.5);
-        long long lhs = g.next() & 1u;
-        if (lhs == 1) { ind0 = 0; indf = from_left(g, c.amp_bead, N, err) + 1; }
-        else { ind0 = N - from_left(g, c.amp_bead, N, err); indf = N; }
-        Real axis[3], p[3];
-        sphere<Real>(g, axis);
-        long long ip;
-        if (ind0 == 0 && indf != N) ip = indf;
-        else if (ind0 != 0 && indf == N) ip = ind0 - 1;
-        else if (ind0 == 0 && indf == N && lhs == 1) ip = indf - 1;
-        else ip = ind0;
-        if (!err) {
-          ld3(r4, ip, p);
-          axis_rotation(axis, p, ang, M);
-        }
-      } else {
-        Real amp = (Real)c.amp_move * uni<Real>(g.next()), d[3];
-        sphere<Real>(g, d);
-        for (int i = 0; i < 3; i++) M[i][3] = d[i] * amp;
-        long long b0 = g.next() % (unsigned)N;
-        long long b1 = from_point(g, c.amp_bead, N, b0, err);
-        check_bead_bounds(b0, b1, N, ind0, indf);
-      }
-    }
-    m = (!live || err) ? 0 : indf - ind0;
-    if (live && !err && m == 0) empty = true;
-    if (live && !err && !empty) xm = g.next();  // drawn now: the stream's state is not kept over the deposit
-    if (m > a.stage_cap) gstage = 1;
-    // voxel table: the CTA's pooled table for every move of up to
-    // kPoolMaxBeads beads, optimistically (a pool past 3/4 load sends the move
-    // to its global table); without the pool (a grid of 2^26 voxels and more)
-    // the slot's own table when the move's at most 16 m voxels surely fit, or
-    // optimistically up to m <= slots / 4 with the same fallback; global beyond
-    bool sure = false, blk;
-    const int most = kPoolMaxBeads >> ((rd.nx == 1) + (rd.ny == 1) + (rd.nz == 1));
-    if (pool) {
-      blk = density && m > 0 && m <= most;
-      gtab = density && m > 0 && !blk;
-    } else {
-      sure = 16 * m <= Hs;
-      gtab = (!sure && 4 * m > Hs) || m > most;
-      blk = density && m > 0 && !gtab;  // moves with a shared table are deposited by the whole CTA
-    }
-    if (gl == 0 && live) {
-      P.blk = blk ? 1 : 0;
-      P.sure = sure ? 1 : 0;
-      P.m = (int)m;
-      P.ind0 = (int)ind0;
-      P.indf = (int)indf;
-      P.gstage = gstage;
-      P.gtab = gtab;
-      P.oob = 0;
-      P.derr = 0;
-      P.cmask = 0;
-      P.pq[0] = P.pq[1] = 0;
-      P.ph[0] = P.ph[1] = 0;
-      P.fq = P.fH = 0;
-      P.fh = 0;
-      P.fl0 = P.fl1 = 0;
-      P.fl2 = 0;
-      P.fn = P.freg = 0;
-      Pos* Mp = reinterpret_cast<Pos*>(P.M);  // in the position type: no conversions
-      for (int i = 0; i < 3; i++)
-        for (int j = 0; j < 4; j++) Mp[4 * i + j] = M[i][j];
-    }
-    __syncthreads();
-    block_deposit<Pos, LEAN>(a, sh, rep, B, kind);
-    // earlier moves u of the batch whose written beads [ind0, indf) meet the
-    // beads this move reads (its segment and both neighbours); a move with no
-    // beads (failed or empty) is never accepted, so it needs no exclusion
-    unsigned cmb = 0;
-    for (int u0 = 0; u0 < B; u0 += G) {
-      const int u = u0 + gl;
-      bool hit = false;
-      if (m > 0 && u < s) {
-        const MovePlan& U = sh.plan[u];
-        hit = U.m > 0 && (long long)U.ind0 <= indf && ind0 - 1 <= (long long)U.indf - 1;
-      }
-      cmb |= gballot<G>(hit) << u0;
-    }
-    __syncthreads();
-    if (pool && density) block_field_pool<Pos>(a, sh, reinterpret_cast<unsigned char*>(&sh), bkeys, bmask);
-    const bool own = m > 0 && (!blk || !pool || (P.derr & E_OVF));
-    if (__any_sync(kFull, own)) own_path<Pos, G, LEAN>(a, sh, rep, s, gl, own, kind, bkeys, bmask);
-    if (gl == 0 && live && cmb) atomicOr(&P.cmask, cmb);
-    if (pool && density) __syncthreads();  // the pooled field pass is complete
-    if (m > 0) {  // the plan's results
-      acc_add(dEp, load_acc<Acc>(P.pq[0], P.ph[0]));
-      acc_add(dEp, load_acc<Acc>(P.pq[1], P.ph[1]));
-      plan_field(P, dEs, dEh);
-      dEH = P.fH;
-      const int oo = P.oob;
-      dEH += ((long long)(oo >> 16) - (long long)(oo & 0xFFFF)) << 40;
-      err |= P.derr & ~E_OVF;
-      nvox = P.fn;
-      regfail = P.freg;
-      gtab = P.gtab;
-    }
-  } else if (kind == CG_TANGENT_ROTATION) {
+  if (kind == CG_TANGENT_ROTATION) {
     Real ang = 0;
     long long n = 0;
     if (live) {
@@ -958,10 +1261,11 @@ __device__ void evaluate_move(const KArgs& a, SpecShared& sh, int rep, int s, in
       n = (long long)(g.next() % (unsigned)c.amp_bead) + 1;
       if (n > N) err |= E_WINDOW;
     }
-    m = (!live || err) ? 0 : n;
+    m = (!live || err) ? 0 : (int)n;
     if (m > a.stage_cap) gstage = 1;
     const SlotScratch S = gstage ? global_slot<Pos>(a, rep, s) : shared_slot(a, sh, s);
     int* idx = S.idx;
+    unsigned* picked = a.picked + a.picked_off[rep] + s * ((N + 31) / 32);
     // n distinct random beads, drawn in order with redraws (get_inds): G
     // candidates per round, the first fresh ones taken in draw order.  Beads
     // taken in a round that another round follows are marked in the slot's
@@ -1014,45 +1318,11 @@ __device__ void evaluate_move(const KArgs& a, SpecShared& sh, int rep, int s, in
     Real sa, ca;
     rsincos(ang, &sa, &ca);
     for (long long k = gl; k < m; k += G) {
-      const long long i = idx[k];
-      // the bead, both neighbours and both bonds, loaded together (in-range
-      // indices at the chain ends, where the term is skipped)
-      const bool hl = i != 0, hr = i + 1 != N;
-      const long long il = hl ? i - 1 : i, ir = hr ? i + 1 : i;
-      Real r[3], t3[3], t2[3], tt3[3], tt2[3], r0[3], t30[3], r1[3], t31[3];
-      ld3(r4, i, r); ld3(t34, i, t3); ld3(t24, i, t2);
-      ld3(r4, il, r0); ld3(t34, il, t30); ld3(r4, ir, r1); ld3(t34, ir, t31);
-      const Bond<Real> bl = bond_at(bonds, bonds32, il, (Real)0), br = bond_at(bonds, bonds32, i, (Real)0);
       const unsigned xa = g.word(axis_base + 2 * k), xb = g.word(axis_base + 2 * k + 1);
-      Real axis[3];
-      sphere_from<Real>(xa, xb, axis);
-      const Real origin[3] = {0, 0, 0};
-      Real M[3][4];
-      axis_rotation_sc(axis, origin, sa, ca, M);
-      for (int j = 0; j < 3; j++) {
-        Real e3 = 0, e2 = 0;
-        for (int q = 0; q < 3; q++) { e3 += M[j][q] * t3[q]; e2 += M[j][q] * t2[q]; }
-        tt3[j] = e3; tt2[j] = e2;
-      }
+      Real tt3[3], tt2[3];
+      const Acc de = rotate_tangent<Pos, LEAN>(a, rd, idx[k], xa, xb, sa, ca, tt3, tt2);
       stage[3 * k + 1] = V4<Pos>{(Pos)tt3[0], (Pos)tt3[1], (Pos)tt3[2], (Pos)0};
       stage[3 * k + 2] = V4<Pos>{(Pos)tt2[0], (Pos)tt2[1], (Pos)tt2[2], (Pos)0};
-      Acc de = acc_zero<Acc>();
-      if (hl) acc_add(de, pair_dE_fwd(bl, r0, r, r, t30, t3, tt3));
-      if (hr) acc_add(de, pair_dE_rev(br, r, r, r1, t3, tt3, t31));
-      if (!LEAN && rd.twist) {  // SSTWLC: twist terms of both bonds
-        const double* tw = a.twist + rd.bead_off * 2;
-        const Frame cur = frame_of(t2, t3), nw = frame_of(tt2, tt3);
-        double dt = 0;
-        if (hl) {
-          const Frame l = frame_of(t24[il], t34[il]);
-          dt += twist_pair_dE(tw + 2 * il, l, cur, l, nw);
-        }
-        if (hr) {
-          const Frame rr = frame_of(t24[ir], t34[ir]);
-          dt += twist_pair_dE(tw + 2 * i, cur, rr, nw, rr);
-        }
-        acc_add_d(de, dt);
-      }
       acc_add(part, de);
     }
     g.pos = axis_base + 2 * (unsigned long long)m;
@@ -1073,7 +1343,7 @@ __device__ void evaluate_move(const KArgs& a, SpecShared& sh, int rep, int s, in
       bsel = (int)(g.next() % (unsigned)rd.nb);
       long long b0 = g.next() % (unsigned)N;
       long long b1 = from_point(g, c.amp_bead, N, b0, err);
-      if (!err) check_bead_bounds(b0, b1, N, ind0, indf);
+      if (!err) segment_of(b0, b1, N, ind0, indf);
     }
     m = (!live || err) ? 0 : indf - ind0;
     const int nt = rd.sites[bsel];
@@ -1109,7 +1379,7 @@ __device__ void evaluate_move(const KArgs& a, SpecShared& sh, int rep, int s, in
           Real p[3], wl[3], w;
           int lo[3], hi[3];
           ld3(r4, i, p);
-          move_axes(rd, gf, p, wl, lo, hi);
+          move_axes<LEAN>(rd, gf, p, wl, lo, hi);
           voxel_corner(gf, wl, lo, hi, cl, w, vq[0]);
           q = q40(w) * (long long)(s_new - s_old);
           want[0] = true;
@@ -1117,7 +1387,7 @@ __device__ void evaluate_move(const KArgs& a, SpecShared& sh, int rep, int s, in
       }
       if (density) {
         int slot[1];
-        claim_slots<1>(S.keys, S.used, nused, S.logH, vq, want, slot, err, 1 << S.logH, E_SPIN, group_mask<G>());
+        claim_slots<1>(S.keys, S.used, nused, S.logH, vq, want, slot, err, 1 << S.logH, E_SPIN);
         if (want[0] && slot[0] >= 0) add_delta(S.vals, hcol, slot[0], 1 + bsel, q, !gtab);
       }
     }
@@ -1136,7 +1406,9 @@ __device__ void evaluate_move(const KArgs& a, SpecShared& sh, int rep, int s, in
     }
     __syncwarp();
     if (density) {
-      field_dE_voxels<G>(ws, a, hcol, S.keys, S.used, S.vals, *nused, gl, nvox, dEs, dEh, dEH, !gtab);
+      long long nv = 0;
+      field_dE_voxels<G>(ws, a, hcol, S.keys, S.used, S.vals, *nused, gl, nv, dEs, dEh, dEH, !gtab);
+      nvox = (int)nv;
       if (m > 0) add_intra(ws, bsel, ddb, dEs, dEh);
     }
     if (gl == 0 && live) P.bsel = bsel;
@@ -1155,8 +1427,7 @@ __device__ void evaluate_move(const KArgs& a, SpecShared& sh, int rep, int s, in
   err = gor<G>(err);
   bool dec = false;
   if (live && !err && !empty) {
-    if (kind > CG_SLIDE) xm = g.next();
-    dec = decide(xm, dEp, dEs, with_huge(dEh, dEH), gl == 0 ? &P.dE : nullptr);
+    dec = decide(g.next(), dEp, dEs, with_huge(dEh, dEH), gl == 0 ? &P.dE : nullptr);
   }
   if (gl == 0 && live) {
     P.kind = kind; P.m = (int)m; P.ind0 = (int)ind0; P.indf = (int)indf;
@@ -1363,8 +1634,6 @@ __global__ void __maxnreg__(168) spec_kernel(KArgs a) {
     sh.npool = 0;
   }
   __syncthreads();
-  const long long words = (sh.ws.rd.n_beads + 31) / 32;
-  unsigned* picked = a.picked + a.picked_off[rep] + slot * words;
 
   for (long long step = 0; step < a.n_steps; step++) {
     for (int ci = 0; ci < a.n_ctl; ci++) {
@@ -1381,13 +1650,50 @@ __global__ void __maxnreg__(168) spec_kernel(KArgs a) {
             __syncthreads();
             break;
           }
-          const int B = (int)(c.num_per_cycle - done < Sn ? c.num_per_cycle - done : Sn);
+          // short tangent rotations: groups of 8 or 16 lanes, and as many moves
+          // in flight as are likely to stand (a later move meets the ~3/2 (amp + 1)
+          // beads of each earlier accepted one with probability ~3/8 (amp + 1)^2 / N)
+          constexpr bool kShort = G == 32 && sizeof(Pos) == 4;
+          const bool brief = kShort && kind == CG_TANGENT_ROTATION && c.amp_bead >= 1 && c.amp_bead <= 32;
+          int most = Sn;
+          if (brief) {
+            const int room = min(kMaxS, (int)(blockDim.x >> 5) * (c.amp_bead <= 16 ? 4 : 2));
+            const int likely = (int)(kShortSpan * sqrtf((float)sh.ws.rd.n_beads) / (float)(c.amp_bead + 1));
+            most = min(room, max(Sn, likely));
+          }
+          const int B = (int)(c.num_per_cycle - done < most ? c.num_per_cycle - done : most);
           const bool wlive = warp * GPW < B;  // the warp has a move of this batch
           const bool live = slot < B;
-          evaluate_move<Pos, G, LEAN>(a, sh, rep, slot, gl, live, kind, c, sh.t0 + (unsigned long long)slot, picked,
-                                      bkeys, bmask, B);
-          __syncthreads();
-          if (kind > CG_SLIDE) {  // position moves set their masks while evaluating
+          if constexpr (kShort) {
+            if (brief) {
+              const ShortTangent T(a, sh, c.amp_bead <= 16 ? 8 : 16);
+              short_tangent_evaluate<LEAN>(a, sh, rep, T, B, c, bkeys, bmask);
+              __syncthreads();
+              short_tangent_conflicts(a, sh, T, B, bkeys, bmask);
+              __syncthreads();
+            }
+          }
+          if (kind <= CG_SLIDE) {
+            if (tid == 0) sh.npool = 0;  // every reader of the last batch's pool passed a barrier since
+            propose_position<Pos, G, LEAN>(a, sh, rep, slot, gl, live, kind, c, sh.t0 + (unsigned long long)slot);
+            __syncthreads();
+            block_deposit<Pos, LEAN>(a, sh, rep, B, kind);
+            bead_conflicts<G>(sh, slot, gl, live, B);
+            __syncthreads();
+            const bool pool = a.pool_on != 0, density = sh.ws.rd.field_kind == 2;
+            if (pool && density) block_field_pool<Pos>(a, sh, smem, bkeys, bmask);
+            {
+              const MovePlan& P = sh.plan[slot];
+              const bool own = live && P.m > 0 && (!P.blk || !pool || (P.derr & E_OVF));
+              if (__any_sync(kFull, own)) own_path<Pos, G, LEAN>(a, sh, rep, slot, gl, own, kind, bkeys, bmask);
+            }
+            if (pool && density) __syncthreads();  // the pooled field pass is complete
+            decide_position<Pos, G, LEAN>(a, sh, slot, gl, live);
+            __syncthreads();
+          } else if (!brief) {
+            evaluate_move<Pos, G, LEAN>(a, sh, rep, slot, gl, live, kind, c, sh.t0 + (unsigned long long)slot, bkeys,
+                                        bmask);
+            __syncthreads();
             if (wlive) conflict_mask<Pos, G>(a, sh, smem, rep, slot, gl, live, kind, B, bmask);
             __syncthreads();
           }
@@ -1442,10 +1748,14 @@ __global__ void __maxnreg__(168) spec_kernel(KArgs a) {
               if (cut == first_fail && first_fail < B && sh.plan[first_fail].err) sh.stop = sh.plan[first_fail].err;
             }
           }
-          if (wlive && live)
-            commit_and_clear<Pos, G>(a, sh, rep, slot, gl, slot < cut && ((acc >> slot) & 1u), bkeys, bmask);
-          __syncwarp();
-          if (live && gl == 0) sh.nused[slot] = 0;
+          if constexpr (kShort)
+            if (brief) short_tangent_commit(a, sh, ShortTangent(a, sh, c.amp_bead <= 16 ? 8 : 16), cut, acc, bkeys, bmask);
+          if (!brief) {
+            if (wlive && live)
+              commit_and_clear<Pos, G>(a, sh, rep, slot, gl, slot < cut && ((acc >> slot) & 1u), bkeys, bmask);
+            __syncwarp();
+            if (live && gl == 0) sh.nused[slot] = 0;
+          }
           if (kind <= CG_SLIDE && a.pool_on && sh.ws.rd.field_kind == 2)
             block_commit_pool(a, sh, smem, cut, acc, bkeys, bmask);
           __syncthreads();
