@@ -383,7 +383,11 @@ static int choose_shape(cg_sim* s, int w_req, int g_req) {
   const long long reg_ctas = std::max(1, cg_spec_warps_per_sm(s->fp64 != 0, G) / W);
   if (ctas_per_sm > reg_ctas) ctas_per_sm = reg_ctas;
   const size_t budget = std::min<size_t>(smem_per_sm / ctas_per_sm - 1024, 220 * 1024);
-  const int lhb = 10;
+  // block voxel table: moves in flight touch ~50 voxels each, so 1,024 entries
+  // serve 6 of them at a load of 0.25, but 12 at 0.55 (10,000-bead chain, 10 MC
+  // steps: 2.59 ms against 2.42 with 2,048; 4,096 would halve the pool of two
+  // binders on one CTA per SM)
+  const int lhb = W * (32 / G) > 8 ? 11 : 10;
   const long long sc = G == 32 ? 48 : 32;
   // the position moves of a batch share one pooled voxel table (keys voxel *
   // 32 + slot: grids below 2^26 voxels), as large as fits; the slots keep small

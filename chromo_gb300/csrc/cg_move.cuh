@@ -62,6 +62,7 @@ __device__ __forceinline__ long long hash_delta(const long long* cell, bool spli
 static __device__ __noinline__ int hash_probe_packed(int* keys, int logH, int key, int start) {
   const unsigned mask = (1u << logH) - 1u;
   unsigned h = ((unsigned)start + 1u) & mask;
+  #pragma unroll 1
   for (unsigned it = 1; it <= mask; it++) {
     int prev = atomicCAS(&keys[h], -1, key);
     if (prev == -1) return (int)h | (1 << 30);
@@ -167,6 +168,7 @@ __device__ __forceinline__ void claim_slots(int* keys, int* used, int* nused, in
   // with the branch-free wrap of voxel_axes and the state times split halves of
   // add_corner)
   const int mask = (1 << logH) - 1;
+  #pragma unroll 1
   for (int it = 1; pend; it++) {
     const int j = __ffs((int)pend) - 1;
     int key = v[0], h = slot[0];
@@ -317,6 +319,7 @@ static __device__ void field_dE_voxels(const WarpShared& ws, const KArgs& a, int
   double part = 0;
   long long hpart = 0;
   const long long* grid = a.grid + rd.vox_off * a.ncol;
+  #pragma unroll 1
   for (int i = lane; i < nused; i += G) {
     const int slot = used[i], v = keys[slot];
     long long row[4];
@@ -393,6 +396,7 @@ static __device__ void field_dE_voxels(const WarpShared& ws, const KArgs& a, int
   long long hpart = 0;
   const long long* grid = a.grid + rd.vox_off * a.ncol;
   (void)hard;
+  #pragma unroll 1
   for (int i = lane; i < nused; i += G) {
     const int slot = used[i], v = keys[slot];
     long long row[4];

@@ -33,6 +33,13 @@
 // instruction serves 2 or 4 moves.  Every warp-collective operation below is
 // executed by the whole warp with per-group masks, so groups may diverge only
 // in code without collectives.
+//
+// Loops of run-time length are not unrolled: the kernel is large and few warps
+// share an SM, and a fifth of its instruction fetches missed the first cache
+// (256 chains of 2,000-20,000 beads, 20 MC steps, kernel only: 11.5 -> 10.4 ms;
+// one 10,000-bead chain, 10 steps: 2.62 -> 2.44 ms with the larger block table
+// above 8 moves in flight).  Exceptions, measured: the binder columns of
+// add_corner.
 #pragma once
 #include <cuda_runtime.h>
 
@@ -69,6 +76,7 @@ struct MoveRng {
     tlo = (unsigned)t;
     thi = (unsigned)(t >> 32);
     pos = 0; bpos = 0; fail = false;
+    #pragma unroll 1
     for (int j = gl; j < kDrawCache / 4; j += G) {
       uint4 o = philox(make_uint4((unsigned)j, tlo, thi, 0x2545F491u), key);
       reinterpret_cast<uint4*>(draws)[j] = o;
@@ -92,12 +100,24 @@ struct MoveRng {
 __device__ __forceinline__ int block_insert(int* bkeys, int logHB, int key) {
   const unsigned mask = (1u << logHB) - 1u;
   unsigned h = ((unsigned)key * 0x9E3779B1u) >> (32 - logHB);
+  #pragma unroll 1
   for (int it = 0; it < 64; it++) {
     int prev = atomicCAS(&bkeys[h], -1, key);
     if (prev == -1 || prev == key) return (int)h;
     h = (h + 1) & mask;
   }
   return -1;
+}
+
+// Empty the block voxel table (thread tid of nt), 16 bytes a store.
+__device__ __forceinline__ void clear_block_table(int* bkeys, unsigned* bmask, int logHB, int tid, int nt) {
+  int4* k = reinterpret_cast<int4*>(bkeys);
+  int4* m = reinterpret_cast<int4*>(bmask);
+#pragma unroll 1
+  for (int i = tid; i < (1 << logHB) / 4; i += nt) {
+    k[i] = make_int4(-1, -1, -1, -1);
+    m[i] = make_int4(0, 0, 0, 0);
+  }
 }
 
 // Scratch of one move slot: its shared-memory region, or the slot's global
@@ -114,9 +134,11 @@ struct SlotScratch {
 
 // Drop the entries a move left in a voxel table (keys, values, block slots).
 __device__ __forceinline__ void clear_table(const SlotScratch& T, int hcol, int nu, int gl, int G) {
+  #pragma unroll 1
   for (int i = gl; i < nu; i += G) {
     const int slot = T.used[i];
     T.keys[slot] = -1;
+    #pragma unroll 1
     for (int cc = 0; cc < hcol; cc++) T.vals[(long long)slot * hcol + cc] = 0;
     T.bslot[i] = -1;
   }
@@ -357,10 +379,12 @@ __device__ void block_deposit(const KArgs& a, SpecShared& sh, int rep, int B, in
   while (32 * per < total) per += W;
   int run = BP;
   while (run * per < total) run += BP;
+  #pragma unroll 1
   for (int b0 = warp * run; b0 < total; b0 += W * run) {
     const int b = b0 + lane;
     // the bead's move: the number of moves whose beads end at or before b
     int s = 0;
+    #pragma unroll 1
     for (int j = 0; j < B; j++) s += __shfl_sync(kFull, end, j) <= b ? 1 : 0;
     int base = __shfl_sync(kFull, end, s > 0 ? s - 1 : 0);
     if (s == 0) base = 0;
@@ -390,6 +414,7 @@ __device__ void block_deposit(const KArgs& a, SpecShared& sh, int rep, int B, in
     }
     const int sl = on ? s : -1;
     const int left = total - b0 < run ? total - b0 : run;
+    #pragma unroll 1
     for (int p = 0; p < left; p += BP) {
       const int src = p + lane / kLanesPerBead;
       unsigned inf;
@@ -516,6 +541,7 @@ static __device__ void block_field_pool(const KArgs& a, SpecShared& sh, unsigned
   };
   // an entry's row is under way while its voxel is registered (fetching the next
   // entry's ahead as well spilled registers and cost 1 %)
+  #pragma unroll 1
   for (int e0 = (int)(threadIdx.x & ~31u); e0 < n; e0 += (int)blockDim.x) {
     int slot, key;
     long long row[4];
@@ -532,6 +558,7 @@ static __device__ void block_field_pool(const KArgs& a, SpecShared& sh, unsigned
         const unsigned prior = atomicOr(&bmask[b], 1u << s);
         const unsigned below = (1u << s) - 1u, above = ~((2u << s) - 1u);
         if (prior & below) atomicOr(&P.cmask, prior & below);
+        #pragma unroll 1
         for (unsigned later = prior & above; later; later &= later - 1)
           atomicOr(&sh.plan[__ffs((int)later) - 1].cmask, 1u << s);
       }
@@ -559,6 +586,7 @@ static __device__ void block_commit_pool(const KArgs& a, SpecShared& sh, unsigne
   long long* pvals = reinterpret_cast<long long*>(smem + a.off_pvals);
   long long* grid = a.grid + rd.vox_off * a.ncol;
   const int n = sh.npool, hcol = a.hcol, ncol = a.ncol;
+  #pragma unroll 1
   for (int e = tid; e < n; e += nt) {
     const int slot = pused[e];
     const int key = pkeys[slot];
@@ -570,12 +598,10 @@ static __device__ void block_commit_pool(const KArgs& a, SpecShared& sh, unsigne
       if (ncol == 4) dst[1] = make_longlong2(hcol > 2 ? src[2] : 0, hcol > 3 ? src[3] : 0);
     }
     pkeys[slot] = -1;
+    #pragma unroll 1
     for (int cc = 0; cc < hcol; cc++) src[cc] = 0;
   }
-  for (int i = tid; i < (1 << a.spec_logHB); i += nt) {
-    bkeys[i] = -1;
-    bmask[i] = 0u;
-  }
+  clear_block_table(bkeys, bmask, a.spec_logHB, tid, nt);
 }
 
 // Move-log terms of a plan (out of line: the log is off in production runs).
@@ -699,6 +725,7 @@ static __device__ __noinline__ void own_path(const KArgs& a, SpecShared& sh, int
     const unsigned full_bit = (gtab || sure) ? E_SPIN : E_OVF;
     unsigned e = 0;
     // one bead per lane, its corners two by two
+    #pragma unroll 1
     for (long long kb = 0; __any_sync(kFull, go && kb < m && !(e & E_OVF)); kb += G) {
       const long long k = kb + gl;
       bool act = go && k < m && !(e & E_OVF);
@@ -751,6 +778,7 @@ static __device__ __noinline__ void own_path(const KArgs& a, SpecShared& sh, int
     // its plan's mask
     const int nr = err ? 0 : nu;
     const unsigned below = (1u << s) - 1u, above = ~((2u << s) - 1u);
+    #pragma unroll 1
     for (int i = gl; i < nr; i += G) {
       const int b = block_insert(bkeys, a.spec_logHB, S.keys[S.used[i]]);
       S.bslot[i] = b;
@@ -759,6 +787,7 @@ static __device__ __noinline__ void own_path(const KArgs& a, SpecShared& sh, int
       } else {
         const unsigned prior = atomicOr(&bmask[b], 1u << s);
         cmb |= prior & below;
+        #pragma unroll 1
         for (unsigned later = prior & above; later; later &= later - 1)
           atomicOr(&sh.plan[__ffs((int)later) - 1].cmask, 1u << s);
       }
@@ -879,6 +908,7 @@ static_assert(4 * kDrawCache == 32 * 2 * 4, "the index lists share the draw buff
 __device__ __forceinline__ unsigned block_find(const int* bkeys, const unsigned* bmask, int logHB, int key) {
   const unsigned mask = (1u << logHB) - 1u;
   unsigned h = ((unsigned)key * 0x9E3779B1u) >> (32 - logHB);
+  #pragma unroll 1
   for (int it = 0; it < 64; it++) {  // as far as block_insert probes
     const int k = bkeys[h];
     if (k == key) return bmask[h];
@@ -902,6 +932,7 @@ __device__ void short_tangent_evaluate(const KArgs& a, SpecShared& sh, int rep, 
                                (unsigned)(a.seed >> 32) ^ 0x1B873593u);
   const unsigned tlo = (unsigned)t, thi = (unsigned)(t >> 32);
   const int have = min(T.ndraw, (int)(3 * amp + 6) & ~3);  // angle, count, beads, axes, decision
+  #pragma unroll 1
   for (int j = gl; 4 * j < have; j += GS)
     reinterpret_cast<uint4*>(T.draws)[j] = philox(make_uint4((unsigned)j, tlo, thi, 0x2545F491u), key);
   __syncwarp();
@@ -920,6 +951,7 @@ __device__ void short_tangent_evaluate(const KArgs& a, SpecShared& sh, int rep, 
   __syncwarp();
   bool dup = false;
   const int most = (int)__reduce_max_sync(kFull, (unsigned)m);
+  #pragma unroll 1
   for (int q = 0; q + 1 < most; q++) {
     const int v = q < m ? T.idx[q] : -2;
     dup = dup || (v == mine[0] && q < gl) || (v == mine[1] && q < GS + gl);
@@ -933,6 +965,7 @@ __device__ void short_tangent_evaluate(const KArgs& a, SpecShared& sh, int rep, 
         if (pos >= 32 * kMaxIter) { err |= E_SPIN; break; }
         const int x = (int)(word(2 + pos++) % N);
         bool seen = false;
+        #pragma unroll 1
         for (int q = 0; q < got; q++) seen = seen || T.idx[q] == x;
         if (!seen) T.idx[got++] = x;
       }
@@ -948,6 +981,7 @@ __device__ void short_tangent_evaluate(const KArgs& a, SpecShared& sh, int rep, 
   rsincos(ang, &sa, &ca);
   Fx part = acc_zero<Fx>();
   int regfail = 0;
+  #pragma unroll 1
   for (int k = gl; k < m; k += GS) {
     const int i = T.idx[k];
     const unsigned xa = word(2 + used + 2 * k), xb = word(3 + used + 2 * k);
@@ -961,11 +995,13 @@ __device__ void short_tangent_evaluate(const KArgs& a, SpecShared& sh, int rep, 
     if (b < 0) regfail = 1;
     else atomicOr(&bmask[b], 1u << s);
   }
+  #pragma unroll 1
   for (int o = GS / 2; o > 0; o >>= 1) {
     part.q += __shfl_xor_sync(kFull, part.q, o);
     regfail |= __shfl_xor_sync(kFull, regfail, o);
   }
   if (__any_sync(kFull, !is_zero64(part.hard)))
+    #pragma unroll 1
     for (int o = GS / 2; o > 0; o >>= 1) part.hard += __shfl_xor_sync(kFull, part.hard, o);
   if (live && gl == 0) {
     MovePlan& P = sh.plan[s];
@@ -992,6 +1028,7 @@ static __device__ __forceinline__ void short_tangent_conflicts(const KArgs& a, S
   const int s = T.s;
   unsigned cm = 0;
   const int m = s < B ? sh.plan[s].m : 0;
+  #pragma unroll 1
   for (int k = T.gl; k < m; k += T.GS) {
     const int i = T.idx[k];
 #pragma unroll
@@ -1009,6 +1046,7 @@ static __device__ __forceinline__ void short_tangent_commit(const KArgs& a, Spec
     V4<float>* t34w = reinterpret_cast<V4<float>*>(a.t34) + rd.bead_off;
     V4<float>* t24w = reinterpret_cast<V4<float>*>(a.t24) + rd.bead_off;
     const int m = sh.plan[s].m;
+    #pragma unroll 1
     for (int k = T.gl; k < m; k += T.GS) {
       const float* q = T.stage + 6 * k;
       const int i = T.idx[k];
@@ -1016,10 +1054,7 @@ static __device__ __forceinline__ void short_tangent_commit(const KArgs& a, Spec
       t24w[i] = V4<float>{q[3], q[4], q[5], 0.0f};
     }
   }
-  for (int i = (int)threadIdx.x; i < (1 << a.spec_logHB); i += (int)blockDim.x) {
-    bkeys[i] = -1;
-    bmask[i] = 0u;
-  }
+  clear_block_table(bkeys, bmask, a.spec_logHB, (int)threadIdx.x, (int)blockDim.x);
 }
 
 __device__ __forceinline__ void segment_of(long long b0, long long b1, long long N, int& ind0, int& indf) {
@@ -1172,6 +1207,7 @@ __device__ __forceinline__ void bead_conflicts(SpecShared& sh, int s, int gl, bo
   MovePlan& P = sh.plan[s];
   const int m = live ? P.m : 0, ind0 = P.ind0, indf = P.indf;
   unsigned cmb = 0;
+  #pragma unroll 1
   for (int u0 = 0; u0 < B; u0 += G) {
     const int u = u0 + gl;
     bool hit = false;
@@ -1298,6 +1334,7 @@ __device__ void evaluate_move(const KArgs& a, SpecShared& sh, int rep, int s, in
         long long consumed;
         if (cnt >= need) {
           unsigned b = bal;
+          #pragma unroll 1
           for (long long q = 1; q < need; q++) b &= b - 1;
           consumed = __ffs((int)b);
           got = m;
@@ -1317,6 +1354,7 @@ __device__ void evaluate_move(const KArgs& a, SpecShared& sh, int rep, int s, in
     Acc part = acc_zero<Acc>();
     Real sa, ca;
     rsincos(ang, &sa, &ca);
+    #pragma unroll 1
     for (long long k = gl; k < m; k += G) {
       const unsigned xa = g.word(axis_base + 2 * k), xb = g.word(axis_base + 2 * k + 1);
       Real tt3[3], tt2[3];
@@ -1328,6 +1366,7 @@ __device__ void evaluate_move(const KArgs& a, SpecShared& sh, int rep, int s, in
     g.pos = axis_base + 2 * (unsigned long long)m;
     dEp = gsum<G>(part);
     // the picked marks only serve the redraws of this move
+    #pragma unroll 1
     for (long long k = gl; k < marked; k += G) {
       int i = idx[k];
       atomicAnd(&picked[i >> 5], ~(1u << (i & 31)));
@@ -1359,6 +1398,7 @@ __device__ void evaluate_move(const KArgs& a, SpecShared& sh, int rep, int s, in
     // column
     constexpr int BP = G / 8;
     const int kc = gl >> 3, cl = gl & 7;
+    #pragma unroll 1
     for (long long kb = 0; __any_sync(kFull, kb < m); kb += BP) {
       const long long k = kb + kc;
       int vq[1] = {0};
@@ -1397,6 +1437,7 @@ __device__ void evaluate_move(const KArgs& a, SpecShared& sh, int rep, int s, in
     const int ddb = gsum<G>(dbl);
     if (check_field && rd.field_kind == 1 && rd.confine_kind == 2) {
       int oob = 0;
+      #pragma unroll 1
       for (long long k = gl; k < m; k += G) {
         double p[3];
         ld3(r4, ind0 + k, p);
@@ -1415,6 +1456,7 @@ __device__ void evaluate_move(const KArgs& a, SpecShared& sh, int rep, int s, in
     // register the touched voxels for the conflict test
     if (density) {
       const int nu = (live && !err) ? *nused : 0;
+      #pragma unroll 1
       for (int i = gl; i < nu; i += G) {
         const int b = block_insert(bkeys, a.spec_logHB, S.keys[S.used[i]]);
         S.bslot[i] = b;
@@ -1448,6 +1490,7 @@ __device__ void conflict_mask(const KArgs& a, SpecShared& sh, unsigned char* sme
   if (rd.field_kind == 2 && kind != CG_TANGENT_ROTATION) {
     const int nu = act ? sh.nused[s] : 0;
     const int* bs = (P.gtab ? global_slot<Pos>(a, rep, s) : shared_slot(a, sh, s)).bslot;
+    #pragma unroll 1
     for (int i = gl; i < nu; i += G) {
       int b = bs[i];
       if (b >= 0) cm |= bmask[b];
@@ -1458,6 +1501,7 @@ __device__ void conflict_mask(const KArgs& a, SpecShared& sh, unsigned char* sme
   if (kind == CG_TANGENT_ROTATION) {
     // rotated beads of u against those of s and their neighbours
     const int* lw = (P.gstage ? global_slot<Pos>(a, rep, s) : shared_slot(a, sh, s)).idx;
+    #pragma unroll 1
     for (int u = 0; u < B; u++) {
       const MovePlan& U = sh.plan[u];
       int hit = 0;
@@ -1465,8 +1509,10 @@ __device__ void conflict_mask(const KArgs& a, SpecShared& sh, unsigned char* sme
         const int* lu = U.gstage ? a.g_idx + ((long long)rep * a.spec_s + u) * a.g_stage_cap
                                  : reinterpret_cast<const int*>(smem + a.spec_off_warps +
                                                                 (size_t)u * a.warp_smem + a.off_idx);
+        #pragma unroll 1
         for (int k = gl; k < P.m && !hit; k += G) {
           int j = lw[k];
+          #pragma unroll 1
           for (int q = 0; q < U.m; q++) {
             int d = lu[q] - j;
             if (d >= -1 && d <= 1) { hit = 1; break; }
@@ -1479,6 +1525,7 @@ __device__ void conflict_mask(const KArgs& a, SpecShared& sh, unsigned char* sme
     // lane gl takes the earlier moves u = u0 + gl: beads written by u,
     // [ind0, indf), against the beads read by s -- the segment and, for
     // position moves, its two neighbours
+    #pragma unroll 1
     for (int u0 = 0; u0 < B; u0 += G) {
       const int u = u0 + gl;
       bool hit = false;
@@ -1536,6 +1583,7 @@ __device__ void commit_and_clear(const KArgs& a, SpecShared& sh, int rep, int s,
     const V4<Pos>* stage = reinterpret_cast<const V4<Pos>*>(S.stage);
     const int* idx = S.idx;
     if (P.kind <= CG_SLIDE) {
+      #pragma unroll 1
       for (int k = gl; k < m; k += G) {
         const long long i = (long long)P.ind0 + k;
         r4w[i] = stage[3 * k];
@@ -1545,12 +1593,14 @@ __device__ void commit_and_clear(const KArgs& a, SpecShared& sh, int rep, int s,
         }
       }
     } else if (P.kind == CG_TANGENT_ROTATION) {
+      #pragma unroll 1
       for (int k = gl; k < m; k += G) {
         const long long i = idx[k];
         t34w[i] = stage[3 * k + 1];
         t24w[i] = stage[3 * k + 2];
       }
     } else {
+      #pragma unroll 1
       for (int k = gl; k < m; k += G) {
         const long long i = (long long)P.ind0 + k;
         unsigned sw = st[i];
@@ -1565,6 +1615,7 @@ __device__ void commit_and_clear(const KArgs& a, SpecShared& sh, int rep, int s,
   int *keys = T.keys, *used = T.used, *bslot = T.bslot;
   long long* vals = T.vals;
   long long* grid = a.grid + rd.vox_off * ncol;
+  #pragma unroll 1
   for (int i = gl; i < nu; i += G) {
     int slot = used[i];
     if (accept) {  // the voxel's post-move row, stored with 16-byte stores (padding column stays 0)
@@ -1575,6 +1626,7 @@ __device__ void commit_and_clear(const KArgs& a, SpecShared& sh, int rep, int s,
       if (ncol == 4) dst[1] = make_longlong2(hcol > 2 ? src[2] : 0, hcol > 3 ? src[3] : 0);
     }
     keys[slot] = -1;
+    #pragma unroll 1
     for (int cc = 0; cc < hcol; cc++) vals[(long long)slot * hcol + cc] = 0;
     int b = bslot[i];
     if (b >= 0) { bkeys[b] = -1; bmask[b] = 0u; }
@@ -1735,6 +1787,7 @@ __global__ void __maxnreg__(168) spec_kernel(KArgs a) {
               // alpha * x is alpha or 0 exactly: one FP64 multiply-add chain
               double run = sh.run_dE, rate = c.acc_rate;
               const double alpha = c.alpha, beta = 1 - c.alpha;
+              #pragma unroll 1
               for (int w = 0; w < cut; w++) {
                 const MovePlan& P = sh.plan[w];
                 if (!LEAN && a.mlog) log_move(a, rep, sh.t0 + (unsigned long long)w - sh.tlog, P);
