@@ -49,8 +49,10 @@ class ReplicaEnergy(torch.autograd.Function):
         gr = torch.empty((n, 3), dtype=torch.float64, device=dev)
         gt = torch.empty((n, 3), dtype=torch.float64, device=dev) if want_t3 else None
         nat.check(L.cg_gradient_device(sim.h, gr.data_ptr(), None if gt is None else gt.data_ptr(), stream))
-        counts = torch.as_tensor(sim.n_beads, dtype=torch.int64, device=dev)
-        rep = torch.repeat_interleave(torch.arange(sim.R, device=dev), counts)
+        # the replica of each bead; neither call waits for the kernels above (the
+        # pinned copy is kept by its allocator until the transfer is done)
+        counts = torch.from_numpy(sim.n_beads).pin_memory().to(dev, non_blocking=True)
+        rep = torch.repeat_interleave(torch.arange(sim.R, device=dev), counts, output_size=n)
         ctx.want_t3 = want_t3
         ctx.save_for_backward(gr, gt if gt is not None else gr.new_empty(0), rep)
         return out[:, :3].sum(1)

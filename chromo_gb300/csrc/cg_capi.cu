@@ -57,7 +57,8 @@ struct cg_sim {
   long long max_segment = 0, max_tangent = 0, max_beads = 0, max_vox = 0;
   int n_ctl = 5;
   long long kernels = 0;
-  // device buffers
+  // device buffers (one allocation)
+  void* slab = nullptr;
   RepDev* reps = nullptr;
   cg_move_ctl* ctl = nullptr;
   unsigned long long* tally = nullptr;
@@ -155,8 +156,11 @@ struct cg_sim {
   float* grad = nullptr;
   double* terms = nullptr;
   double* acc = nullptr;
-  // pinned host staging for chain uploads / downloads
-  void* pinned = nullptr;
+  // host staging for chain uploads / downloads: pageable up to kPageable bytes
+  // (pinning and releasing a buffer took longer than a short chain's copies),
+  // pinned beyond
+  static constexpr size_t kPageable = size_t(1) << 18;
+  void *pinned = nullptr, *pageable = nullptr;
   size_t pinned_bytes = 0;
   // direct host access (cudaDevAttrPageableMemoryAccess): cg_set_chains /
   // cg_get_chains read and write the caller's arrays from the GPU; the
@@ -202,6 +206,10 @@ struct cg_sim {
   }
 
   unsigned char* staging(size_t bytes) {
+    if (bytes <= kPageable && bytes > pinned_bytes) {
+      if (!pageable) pageable = std::malloc(kPageable);
+      if (pageable) return static_cast<unsigned char*>(pageable);
+    }
     if (bytes > pinned_bytes) {
       if (pinned) cudaFreeHost(pinned);
       pinned = nullptr;
@@ -332,20 +340,15 @@ void cg_destroy(cg_sim* s) {
   if (s->pinned) cudaFreeHost(s->pinned);
   if (s->twist) cudaFree(s->twist);
   if (s->steric_work) cudaFree(s->steric_work);
-  if (s->hio_tab) cudaFree(s->hio_tab);
-  if (s->hio_flag) cudaFree(s->hio_flag);
   {
     void* stage[] = {s->hio_r4, s->hio_t34, s->hio_t24, s->hio_states};
     for (void* p : stage)
       if (p) cudaFree(p);
   }
-  void* ptrs[] = {s->reps, s->ctl, s->tally, s->r4, s->t34, s->t24, s->states, s->marks, s->bonds,
-                  s->bonds32, s->grid, s->access_vol, s->access_sc, s->access_vb, s->g_keys, s->g_used, s->g_bslot, s->g_vals, s->g_stage, s->g_idx,
-                  s->picked, s->d_picked_off, s->eout, s->aout, s->rep_of_rung, s->swaps,
-                  s->swap_attempts, s->xround, s->grad, s->terms, s->acc, s->nbound, s->mu_swaps,
-                  s->mu_swap_attempts};
+  void* ptrs[] = {s->slab, s->grad, s->terms, s->acc};
   for (void* p : ptrs)
     if (p) cudaFree(p);
+  if (s->pageable) std::free(s->pageable);
   delete s;
 }
 
@@ -481,40 +484,6 @@ int cg_create(const cg_config* cfg, cg_sim** out) {
     s->picked_off[r] = s->total_picked;
     s->total_picked += (long long)s->spec_s * ((s->n_beads[r] + 31) / 32);
   }
-  auto M = [&](void** p, size_t bytes) { return cudaMalloc(p, bytes == 0 ? 16 : bytes); };
-  cudaError_t e = cudaSuccess;
-#define ALLOC(ptr, bytes) if (e == cudaSuccess) e = M((void**)&(ptr), (bytes))
-  ALLOC(s->reps, sizeof(RepDev) * s->R);
-  ALLOC(s->ctl, sizeof(cg_move_ctl) * 5 * s->R);
-  ALLOC(s->tally, sizeof(unsigned long long) * 30 * s->R);
-  ALLOC(s->r4, s->pos_bytes() * s->total_beads);
-  ALLOC(s->t34, s->pos_bytes() * s->total_beads);
-  ALLOC(s->t24, s->pos_bytes() * s->total_beads);
-  ALLOC(s->states, 4 * s->total_beads);
-  ALLOC(s->marks, 4 * s->total_beads);
-  ALLOC(s->bonds, 6 * 8 * s->total_beads);
-  ALLOC(s->bonds32, 8 * 4 * s->total_beads);
-  ALLOC(s->grid, 8 * s->ncol * s->total_vox);
-  if (s->nonuniform) ALLOC(s->access_vol, 8 * s->total_vox);
-  if (s->nonuniform) ALLOC(s->access_sc, 4 * s->total_vox);
-  if (s->nonuniform) ALLOC(s->access_vb, 8 * s->total_vox);
-  ALLOC(s->g_keys, 4 * Hg * RW);
-  ALLOC(s->g_used, 4 * Hg * RW);
-  ALLOC(s->g_bslot, 4 * Hg * RW);
-  ALLOC(s->g_vals, 8 * Hg * (s->nb + 1) * RW);
-  ALLOC(s->g_stage, s->scal_bytes() * 12 * s->g_stage_cap * RW);
-  ALLOC(s->g_idx, 4 * s->g_stage_cap * RW);
-  ALLOC(s->picked, 4 * s->total_picked);
-  ALLOC(s->d_picked_off, 8 * s->R);
-  ALLOC(s->eout, 8 * 5 * s->R);
-  ALLOC(s->aout, 8 * 4);
-  ALLOC(s->rep_of_rung, 4 * s->R);
-  ALLOC(s->swaps, 8 * s->R);
-  ALLOC(s->swap_attempts, 8 * s->R);
-  ALLOC(s->xround, 8);
-  ALLOC(s->nbound, 8 * s->R);
-  ALLOC(s->mu_swaps, 8 * s->R);
-  ALLOC(s->mu_swap_attempts, 8 * s->R);
   {
     // chains move between the caller's arrays and the device in one kernel
     // pass where the GPU can address pageable host memory (Grace-Blackwell
@@ -524,34 +493,59 @@ int cg_create(const cg_config* cfg, cg_sim** out) {
     const char* env = std::getenv("CHROMO_GB300_STAGED_HOST_IO");
     s->direct_host = pageable == 1 && s->R <= 65535 && !(env && env[0] == '1');
   }
-  if (s->direct_host) ALLOC(s->hio_tab, 4 * sizeof(void*) * s->R);
-  if (s->direct_host) ALLOC(s->hio_flag, sizeof(unsigned));
-#undef ALLOC
+  // One allocation holds every buffer (a cudaMalloc and a cudaFree each took a
+  // third of a short mc_sim call): first those that start as zeros, then those
+  // that start as ones, then those written before they are read.
+  std::vector<std::pair<void**, size_t>> parts;
+  size_t slab = 0, zeros = 0, ones = 0;
+  auto add = [&](auto& ptr, size_t bytes) {
+    parts.emplace_back(reinterpret_cast<void**>(&ptr), slab);
+    slab += (std::max<size_t>(bytes, 16) + 255) & ~size_t(255);
+  };
+  add(s->reps, sizeof(RepDev) * s->R);
+  add(s->ctl, sizeof(cg_move_ctl) * 5 * s->R);
+  add(s->tally, sizeof(unsigned long long) * 30 * s->R);
+  add(s->r4, s->pos_bytes() * s->total_beads);
+  add(s->t34, s->pos_bytes() * s->total_beads);
+  add(s->t24, s->pos_bytes() * s->total_beads);
+  add(s->states, 4 * s->total_beads);
+  add(s->marks, 4 * s->total_beads);
+  add(s->bonds, 6 * 8 * s->total_beads);
+  add(s->bonds32, 8 * 4 * s->total_beads);
+  add(s->grid, 8 * s->ncol * s->total_vox);
+  add(s->g_vals, 8 * Hg * (s->nb + 1) * RW);
+  add(s->picked, 4 * s->total_picked);
+  add(s->swaps, 8 * s->R);
+  add(s->swap_attempts, 8 * s->R);
+  add(s->xround, 8);
+  add(s->nbound, 8 * s->R);
+  add(s->mu_swaps, 8 * s->R);
+  add(s->mu_swap_attempts, 8 * s->R);
+  zeros = slab;
+  add(s->g_keys, 4 * Hg * RW);
+  add(s->g_bslot, 4 * Hg * RW);
+  ones = slab - zeros;
+  if (s->nonuniform) add(s->access_vol, 8 * s->total_vox);
+  if (s->nonuniform) add(s->access_sc, 4 * s->total_vox);
+  if (s->nonuniform) add(s->access_vb, 8 * s->total_vox);
+  add(s->g_used, 4 * Hg * RW);
+  add(s->g_stage, s->scal_bytes() * 12 * s->g_stage_cap * RW);
+  add(s->g_idx, 4 * s->g_stage_cap * RW);
+  add(s->d_picked_off, 8 * s->R);
+  add(s->eout, 8 * 5 * s->R);
+  add(s->aout, 8 * 4);
+  add(s->rep_of_rung, 4 * s->R);
+  if (s->direct_host) add(s->hio_tab, 4 * sizeof(void*) * s->R);
+  if (s->direct_host) add(s->hio_flag, sizeof(unsigned));
+  cudaError_t e = cudaMalloc(&s->slab, slab);
   if (e != cudaSuccess) {
+    s->slab = nullptr;
     cg_destroy(s);
     return fail(CG_ERR_NOMEM, std::string("cudaMalloc: ") + cudaGetErrorString(e));
   }
-  cudaMemset(s->reps, 0, sizeof(RepDev) * s->R);
-  cudaMemset(s->ctl, 0, sizeof(cg_move_ctl) * 5 * s->R);
-  cudaMemset(s->tally, 0, 8 * 30 * s->R);
-  cudaMemset(s->r4, 0, s->pos_bytes() * s->total_beads);
-  cudaMemset(s->t34, 0, s->pos_bytes() * s->total_beads);
-  cudaMemset(s->t24, 0, s->pos_bytes() * s->total_beads);
-  cudaMemset(s->states, 0, 4 * s->total_beads);
-  cudaMemset(s->marks, 0, 4 * s->total_beads);
-  cudaMemset(s->bonds, 0, 48 * s->total_beads);
-  cudaMemset(s->bonds32, 0, 32 * s->total_beads);
-  cudaMemset(s->grid, 0, 8 * s->ncol * s->total_vox);
-  cudaMemset(s->g_keys, 0xFF, 4 * Hg * RW);
-  cudaMemset(s->g_bslot, 0xFF, 4 * Hg * RW);
-  cudaMemset(s->g_vals, 0, 8 * Hg * (s->nb + 1) * RW);
-  cudaMemset(s->picked, 0, 4 * s->total_picked);
-  cudaMemset(s->swaps, 0, 8 * s->R);
-  cudaMemset(s->swap_attempts, 0, 8 * s->R);
-  cudaMemset(s->xround, 0, 8);
-  cudaMemset(s->nbound, 0, 8 * s->R);
-  cudaMemset(s->mu_swaps, 0, 8 * s->R);
-  cudaMemset(s->mu_swap_attempts, 0, 8 * s->R);
+  for (auto& p : parts) *p.first = static_cast<unsigned char*>(s->slab) + p.second;
+  cudaMemsetAsync(s->slab, 0, zeros, 0);
+  cudaMemsetAsync(static_cast<unsigned char*>(s->slab) + zeros, 0xFF, ones, 0);
   cudaMemcpy(s->d_picked_off, s->picked_off.data(), 8 * s->R, cudaMemcpyHostToDevice);
   std::vector<int> ror(s->R);
   for (int r = 0; r < s->R; r++) ror[r] = r;

@@ -9,10 +9,10 @@
 * ``field_prefactors``: oligomerisation, intranucleosome and cross-talk
   prefactors of ``init_field_energy_prefactors`` (chromo/fields.pyx:687-712).
 """
+import math
 from pathlib import Path
 
 import numpy as np
-from scipy.special import comb
 
 from ._native import MAX_BINDERS, MAX_MARK
 
@@ -42,16 +42,19 @@ def dss_parameters(bead_length, lp):
 
 def binding_free_energy_table(sites, e_mod, e_nomod):
     """[MAX_BINDERS, MAX_MARK+1, MAX_MARK+1] table of -ln(site partition function)."""
+    def comb(n, k):  # scipy's comb on these few small integers took 0.3 ms a call
+        return float(math.comb(n, k)) if n >= k >= 0 else 0.0
+
     f = np.zeros((MAX_BINDERS, MAX_MARK + 1, MAX_MARK + 1))
     for b in range(len(sites)):
         Nn = int(sites[b])
         for Nm in range(MAX_MARK + 1):
             for s in range(MAX_MARK + 1):
                 i = np.arange(s + 1)
+                ways = np.array([comb(Nm, k) * comb(Nn - Nm, s - k) for k in range(s + 1)])
                 with np.errstate(divide="ignore"):
                     f[b, Nm, s] = -np.log(np.sum(
-                        comb(Nm, i) * comb(Nn - Nm, s - i)
-                        * np.exp(-(i * e_mod[b] + (s - i) * e_nomod[b]))))
+                        ways * np.exp(-(i * e_mod[b] + (s - i) * e_nomod[b]))))
     return f
 
 
