@@ -60,9 +60,10 @@ def candidates(n_replicas: int, n_sm: int, pos_fp64: bool, warps_per_sm: Dict[in
     When every replica has an SM to itself, a few small W at 32 lanes too: a
     chain whose controller cycles hold few moves (one with specific_moves)
     has few moves to put in flight, and fewer warps then shorten each
-    batch's barriers."""
+    batch's barriers.  W = 0 at 32 lanes is the library's own default, which
+    with FP32 storage takes more warps than moves in flight."""
     ctas = max(1, math.ceil(n_replicas / max(1, n_sm)))
-    out = []
+    out = [] if pos_fp64 else [(0, 32)]
     for G in ((32,) if pos_fp64 else (32, 16, 8)):
         wmax = min(MAX_WARPS, MAX_IN_FLIGHT * G // 32, max(1, warps_per_sm[G] // ctas))
         ws = {wmax, wmax - 1, wmax - 2, (wmax + 1) // 2}

@@ -271,10 +271,12 @@ struct cg_sim {
     return warp_smem;
   }
   // CTA layout: header, block voxel table (2^lhb entries), the pooled voxel
-  // table (2^lhp entries: keys, used list, nb + 1 split int64 values; none
-  // for lhp = 0), one region per move slot (W warps of 32 / G slots).
-  size_t cta_layout(int lhb, int W, int G, int lhp = 0) {
-    size_t o = align16(sizeof(cg::SpecShared));
+  // table (2^lhp entries: keys, 16-bit used list, nb + 1 split int64 values; none
+  // for lhp = 0), one region per move slot (S of them, W warps).
+  size_t cta_layout(int lhb, int W, int G, int S, int lhp = 0) {
+    // (short tangent rotations take up to four moves per slot of 32 lanes)
+    const int plans = !fp64 && G == 32 ? std::min(4 * S, (int)cg::kMaxS) : S;
+    size_t o = align16(offsetof(cg::SpecShared, plan) + sizeof(cg::MovePlan) * (size_t)plans);
     spec_off_bkeys = (int)o; o += 4 * (size_t(1) << lhb);
     spec_off_bmask = (int)o; o += 4 * (size_t(1) << lhb);
     o = align32(o);
@@ -284,7 +286,7 @@ struct cg_sim {
     if (lhp > 0) {
       const size_t HP = size_t(1) << lhp;
       off_pkeys = (int)o; o += 4 * HP;
-      off_pused = (int)o; o += 4 * HP;
+      off_pused = (int)o; o += 2 * HP;
       o = align16(o);
       off_pvals = (int)o; o += 8 * HP * (nb + 1);
       o = align32(o);
@@ -293,7 +295,7 @@ struct cg_sim {
     spec_logHB = lhb;
     spec_w = W;
     spec_g = G;
-    spec_s = W * (32 / G);
+    spec_s = S;
     return o + (size_t)spec_s * warp_smem;
   }
 };
@@ -370,6 +372,15 @@ static int default_warps(const cg_sim* s, int G) {
   return (int)std::min<long long>(wmax, std::max<long long>(1, W));
 }
 
+// Moves in flight per replica: W warps of 32 / G moves where the caller chose W;
+// by default, with FP32 storage and 32 lanes per move, three for four warps (the
+// deposit and field phases use every warp; 256 chains, 20 MC steps, kernel only,
+// 8 warps with 4 / 5 / 6 / 8 moves: 10.7 / 10.0 / 9.95 / 10.2 ms).
+static int moves_in_flight(const cg_sim* s, int w_req, int W, int G) {
+  if (w_req > 0 || s->fp64 || G != 32) return std::min(W * (32 / G), cg::kMaxS);
+  return (3 * W + 3) / 4;
+}
+
 static int choose_shape(cg_sim* s, int w_req, int g_req) {
   // One CTA per replica with W warps of 32 / G moves each.  The CTAs that can
   // be resident per SM -- those every replica needs to run at once, or fewer
@@ -383,6 +394,7 @@ static int choose_shape(cg_sim* s, int w_req, int g_req) {
   int W = w_req > 0 ? w_req : default_warps(s, G);
   if (W > cg::kMaxW) W = cg::kMaxW;
   if (W * (32 / G) > cg::kMaxS) W = cg::kMaxS / (32 / G);
+  const int S = moves_in_flight(s, w_req, W, G);
   const long long reg_ctas = std::max(1, cg_spec_warps_per_sm(s->fp64 != 0, G) / W);
   if (ctas_per_sm > reg_ctas) ctas_per_sm = reg_ctas;
   const size_t budget = std::min<size_t>(smem_per_sm / ctas_per_sm - 1024, 220 * 1024);
@@ -390,7 +402,7 @@ static int choose_shape(cg_sim* s, int w_req, int g_req) {
   // serve 6 of them at a load of 0.25, but 12 at 0.55 (10,000-bead chain, 10 MC
   // steps: 2.59 ms against 2.42 with 2,048; 4,096 would halve the pool of two
   // binders on one CTA per SM)
-  const int lhb = W * (32 / G) > 8 ? 11 : 10;
+  const int lhb = S > 8 ? 11 : 10;
   const long long sc = G == 32 ? 48 : 32;
   // the position moves of a batch share one pooled voxel table (keys voxel *
   // 32 + slot: grids below 2^26 voxels), as large as fits; the slots keep small
@@ -403,18 +415,18 @@ static int choose_shape(cg_sim* s, int w_req, int g_req) {
     for (int t = s->fp64 ? 11 : 12; t >= 8 && lhp == 0; t--)
       for (int l = s->fp64 && t >= 10 ? 8 : 6; l >= 6 && lhp == 0; l--) {
         s->layout(l, sc);
-        if (s->cta_layout(lhb, W, G, t) <= budget) { lhp = t; lh = l; }
+        if (s->cta_layout(lhb, W, G, S, t) <= budget) { lhp = t; lh = l; }
       }
   }
   if (lhp == 0) {
     lh = 10;  // at most 1,024 slots: the 32-bit split counters of a shared table cannot overflow
     for (; lh > 6; lh--) {
       s->layout(lh, sc);
-      if (s->cta_layout(lhb, W, G) <= budget) break;
+      if (s->cta_layout(lhb, W, G, S) <= budget) break;
     }
   }
   s->layout(lh, sc);
-  s->spec_bytes = s->cta_layout(lhb, W, G, lhp);
+  s->spec_bytes = s->cta_layout(lhb, W, G, S, lhp);
   s->wpb = 1;
   cudaError_t e = cg_set_spec_smem(s->fp64 != 0, G, (int)s->spec_bytes);
   if (e == cudaSuccess) e = cg_set_mc_smem(s->fp64 != 0, (int)(s->spec_off_warps + s->warp_smem));
@@ -465,7 +477,7 @@ int cg_create(const cg_config* cfg, cg_sim** out) {
     cg_destroy(s);
     return fail(CG_ERR_ARG, "lanes_per_move must be 8, 16 or 32 (32 with FP64 storage)");
   }
-  if (cfg->warps_per_block < 0 || cfg->warps_per_block > cg::kMaxW) {
+  if (cfg->warps_per_block < 0 || cfg->warps_per_block > cg::kUserMaxW) {
     cg_destroy(s);
     return fail(CG_ERR_ARG, "warps_per_block must be in 0..12");
   }
@@ -475,7 +487,7 @@ int cg_create(const cg_config* cfg, cg_sim** out) {
     if (W * (32 / G) > cg::kMaxS) W = cg::kMaxS / (32 / G);
     s->spec_w = W;
     s->spec_g = G;
-    s->spec_s = W * (32 / G);
+    s->spec_s = moves_in_flight(s, cfg->warps_per_block, W, G);
   }
   const long long RW = (long long)s->R * s->spec_s;
   // tangent-rotation bitmaps: one per (replica, move slot)
@@ -570,7 +582,7 @@ int cg_create(const cg_config* cfg, cg_sim** out) {
   cudaMemcpy(s->reps, rd.data(), sizeof(RepDev) * s->R, cudaMemcpyHostToDevice);
   e = cudaGetLastError();
   if (e != cudaSuccess) { cg_destroy(s); return fail(CG_ERR_CUDA, cudaGetErrorString(e)); }
-  int rc = choose_shape(s, s->spec_w, s->spec_g);
+  int rc = choose_shape(s, cfg->warps_per_block, s->spec_g);
   if (rc) { cg_destroy(s); return rc; }
   *out = s;
   return CG_OK;

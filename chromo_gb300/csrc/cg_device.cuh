@@ -583,6 +583,49 @@ __device__ __forceinline__ FF pair_dE_rev(const Bond<float>& b, const float r0[3
   return half_sum3(b.eb * e_bend, b.ep * e_par, b.epp * e_perp);
 }
 
+// pair_dE_fwd / pair_dE_rev of a rotated tangent (no bead moves), with the
+// terms of the zero displacement left out.  FP32: the same bits (adding or
+// multiplying those zeros changes nothing); FP64 takes the general form.
+__device__ __forceinline__ FF tangent_dE_fwd(const Bond<float>& b, const float r0[3], const float r1[3],
+                                             const float t30[3], const float t31[3], const float tt31[3]) {
+  float dr[3];
+  for (int i = 0; i < 3; i++) dr[i] = r1[i] - r0[i];
+  const float pc = t30[0] * dr[0] + t30[1] * dr[1] + t30[2] * dr[2];
+  float e_bend = 0;
+  for (int i = 0; i < 3; i++) {
+    const float sh = (dr[i] - t30[i] * pc) * b.eta;
+    e_bend += (tt31[i] - t31[i]) * ((tt31[i] - t30[i] - sh) + (t31[i] - t30[i] - sh));
+  }
+  return FF{0.5f * (b.eb * e_bend), 0.0f};
+}
+__device__ __forceinline__ FF tangent_dE_rev(const Bond<float>& b, const float r0[3], const float r1[3],
+                                             const float t30[3], const float tt30[3], const float t31[3]) {
+  float dr[3], dt[3];
+  for (int i = 0; i < 3; i++) { dr[i] = r1[i] - r0[i]; dt[i] = tt30[i] - t30[i]; }
+  const float pt = tt30[0] * dr[0] + tt30[1] * dr[1] + tt30[2] * dr[2];
+  const float pc = t30[0] * dr[0] + t30[1] * dr[1] + t30[2] * dr[2];
+  const float dpar = dt[0] * dr[0] + dt[1] * dr[1] + dt[2] * dr[2];
+  const float e_par = dpar * ((pt - b.g) + (pc - b.g));
+  float e_perp = 0, e_bend = 0;
+  for (int i = 0; i < 3; i++) {
+    const float dpt = dr[i] - tt30[i] * pt, dp = dr[i] - t30[i] * pc;
+    const float ddp = -(dt[i] * pt + t30[i] * dpar);
+    const float bt = t31[i] - tt30[i] - dpt * b.eta, bc = t31[i] - t30[i] - dp * b.eta;
+    const float db = -dt[i] - ddp * b.eta;
+    e_perp += ddp * (dpt + dp);
+    e_bend += db * (bt + bc);
+  }
+  return half_sum3(b.eb * e_bend, b.ep * e_par, b.epp * e_perp);
+}
+__device__ __forceinline__ double tangent_dE_fwd(const Bond<double>& b, const double r0[3], const double r1[3],
+                                                 const double t30[3], const double t31[3], const double tt31[3]) {
+  return pair_dE_fwd(b, r0, r1, r1, t30, t31, tt31);
+}
+__device__ __forceinline__ double tangent_dE_rev(const Bond<double>& b, const double r0[3], const double r1[3],
+                                                 const double t30[3], const double tt30[3], const double t31[3]) {
+  return pair_dE_rev(b, r0, r0, r1, t30, tt30, t31);
+}
+
 // ---------------------------------------------------------------- density field
 // chromo/fields.pyx:1430-1673: eight trilinear weights and periodic voxel indices.
 

@@ -32,7 +32,9 @@ struct WarpShared {
   int pad[3];
 };
 
-constexpr int kMaxW = 12;  // warps per replica CTA (12 x 32 threads x 168 registers fill one SM)
+constexpr int kMaxW = 16;  // warps per replica CTA: 16 x 32 threads x 128 registers fill one SM (FP32 storage),
+                           // 12 x 32 x 168 (FP64 storage)
+constexpr int kUserMaxW = 12;  // largest warps_per_block a caller may ask for
 constexpr int kMaxS = 32;  // moves in flight per replica (one bit each in 32-bit masks)
 
 // Outcome of one speculatively evaluated move.
@@ -41,7 +43,8 @@ struct MovePlan {
   int empty, err, regfail, dec;
   unsigned cmask;
   int nvox, gtab, gstage, bsel, ndraw;
-  double dE;
+  double dE;     // the FP64 part of dE (all of it for FP64 storage)
+  long long dq;  // the fixed-point part, in 2^-30 kT
   double dEp;  // polymer part of dE (written only when the move log is on)
   // block-wide deposit of a position move (its beads' corners spread over
   // every thread of the CTA): the proposal's transform and table kind in,
@@ -68,14 +71,20 @@ constexpr int kDrawCache = 64;  // first draws of each in-flight move, precomput
 
 struct SpecShared {
   WarpShared ws;
-  MovePlan plan[kMaxS];
   int nused[kMaxS];
   unsigned long long t0;   // move counter (selects each move's random sub-stream)
   unsigned long long tlog; // move counter at launch (index origin of the move log)
-  double run_dE;
+  double run_dE;   // running sum of accepted dE: its FP64 part
+  long long run_q;  // and its fixed-point part (FP32 storage), exact over the launch
   int cut, stop;
   unsigned accmask;
   int npool;  // entries of the pooled voxel table in use
+  // conflicts among the position moves of a batch, by kind (see batch_limit):
+  // decayed counts of batches cut short and of the pairs of moves they tested,
+  // and the moves in flight chosen from them
+  float met[3], pairs[3];
+  int limit[3];
+  MovePlan plan[kMaxS];  // last: a CTA holds those its moves in flight can use (cta_layout)
 };
 
 static_assert(sizeof(unsigned) * kDrawCache % 16 == 0, "the draw buffers are written with 16-byte stores");
@@ -117,7 +126,7 @@ struct KArgs {
   long long stage_cap;
   int warp_smem, off_draws, off_keys, off_used, off_bslot, off_vals, off_stage, off_idx;
   // CTA layout: header, block voxel table, then one region per move slot;
-  // spec_w warps of 32 / spec_g groups, spec_s = spec_w * 32 / spec_g slots
+  // spec_w warps of 32 / spec_g groups, spec_s <= spec_w * 32 / spec_g slots
   int spec_w, spec_g, spec_s, spec_logHB, spec_off_bkeys, spec_off_bmask, spec_off_warps;
   // pooled voxel table of the CTA: 2^pool_logH entries keyed by
   // voxel * 32 + move slot, shared by the position moves of a batch

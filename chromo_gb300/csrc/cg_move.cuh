@@ -145,8 +145,8 @@ __device__ __forceinline__ void deposit_bead(const RepDev& rd, int ncol, int* ke
 // issued back to back; only a claim that meets another key probes on.  A table
 // that cannot take a new voxel (slot -1), or whose count of voxels this lane
 // takes past `cap`, sets `full_bit` in err.
-template <int NQ>
-__device__ __forceinline__ void claim_slots(int* keys, int* used, int* nused, int logH, const int (&v)[NQ],
+template <int NQ, typename U>
+__device__ __forceinline__ void claim_slots(int* keys, U* used, int* nused, int logH, const int (&v)[NQ],
                                             const bool (&want)[NQ], int (&slot)[NQ], unsigned& err,
                                             int cap, unsigned full_bit) {
   int prev[NQ];
@@ -192,7 +192,7 @@ __device__ __forceinline__ void claim_slots(int* keys, int* used, int* nused, in
     if (at + cnt > cap) err |= full_bit;
 #pragma unroll
     for (int j = 0; j < NQ; j++)
-      if (fresh[j]) used[at++] = slot[j];
+      if (fresh[j]) used[at++] = (U)slot[j];
   }
 }
 
@@ -528,20 +528,32 @@ __device__ __forceinline__ void add_intra(const WarpShared& ws, int bsel, int dd
 // dE = (0 + dEp) + hard in FP64, as the reference sums polymer and field dE
 // (mc_sim.pyx:144-171).  FP32 storage: decided on the FF sum when the FP64
 // part is empty.  *dE_out (if given) receives dE in FP64.
-__device__ __forceinline__ bool decide(unsigned x, double dEp, double, double hard, double* dE_out) {
+// The production kernel takes dE as its parts: dE = q 2^-30 + hard (q = 0 for
+// FP64 storage); no FP64 instruction for an FP32 move without an FP64 part.
+__device__ __forceinline__ bool decide(unsigned x, double dEp, double, double hard, long long& q, double& h) {
   double dE = 0;
   dE += dEp;
   dE += hard;
-  if (dE_out) *dE_out = dE;
+  q = 0;
+  h = dE;
   return metropolis(x, -dE);
 }
-__device__ __forceinline__ bool decide(unsigned x, const Fx& dEp, const Fx& soft, double hard,
-                                       double* dE_out) {
-  const long long q = dEp.q + soft.q;
+__device__ __forceinline__ bool decide(unsigned x, const Fx& dEp, const Fx& soft, double hard, long long& q,
+                                       double& h) {
+  q = dEp.q + soft.q;
   if (!is_zero64(dEp.hard)) hard = add_hard(hard, dEp.hard);
   if (!is_zero64(soft.hard)) hard = add_hard(hard, soft.hard);
-  const bool d = metropolis_fx(x, q, hard);
-  if (dE_out) *dE_out = (double)q * kFxEInv + hard;
+  h = hard;
+  return metropolis_fx(x, q, hard);
+}
+__device__ __forceinline__ double dE_value(long long q, double h) { return (double)q * kFxEInv + h; }
+
+template <typename Acc>
+__device__ __forceinline__ bool decide(unsigned x, const Acc& dEp, const Acc& soft, double hard, double* dE_out) {
+  long long q;
+  double h;
+  const bool d = decide(x, dEp, soft, hard, q, h);
+  if (dE_out) *dE_out = dE_value(q, h);
   return d;
 }
 }  // namespace cg

@@ -201,7 +201,7 @@ __device__ __forceinline__ void load_transform(const MovePlan& P, Pos (&M)[3][4]
 // zero where the segment ends the chain.  The move's plan holds its segment
 // and transform.
 template <typename Pos, typename Acc, bool LEAN>
-static __device__ __noinline__ Acc boundary_term(const KArgs& a, const RepDev& rd, const MovePlan& P, int kind,
+static __device__ __forceinline__ Acc boundary_term(const KArgs& a, const RepDev& rd, const MovePlan& P, int kind,
                                                  int side) {
   const ChainView<Pos> cv(a, rd, LEAN);
   const long long N = rd.n_beads;
@@ -432,7 +432,8 @@ __device__ void block_deposit(const KArgs& a, SpecShared& sh, int rep, int B, in
       // the pooled table (one used list for the whole CTA, keys voxel * 32 +
       // slot), or the move's own table (one used list per move)
       int* keys = reinterpret_cast<int*>(pool ? smem + a.off_pkeys : wb + a.off_keys);
-      int* used = reinterpret_cast<int*>(pool ? smem + a.off_pused : wb + a.off_used);
+      int* used = reinterpret_cast<int*>(wb + a.off_used);
+      unsigned short* pu = reinterpret_cast<unsigned short*>(smem + a.off_pused);
       long long* vals = reinterpret_cast<long long*>(pool ? smem + a.off_pvals : wb + a.off_vals);
       bool want[2 * kCornersPerLane];
 #pragma unroll
@@ -445,8 +446,11 @@ __device__ void block_deposit(const KArgs& a, SpecShared& sh, int rep, int B, in
       const int lh = pool ? a.pool_logH : a.logH;
       int slot[2 * kCornersPerLane];
       unsigned e = 0;
-      claim_slots<2 * kCornersPerLane>(keys, used, pool ? &sh.npool : &sh.nused[tt], lh, vq, want, slot, e,
-                                       sure ? Hs : (3 << lh) / 4, full_bit);
+      if (pool)
+        claim_slots<2 * kCornersPerLane>(keys, pu, &sh.npool, lh, vq, want, slot, e, (3 << lh) / 4, full_bit);
+      else
+        claim_slots<2 * kCornersPerLane>(keys, used, &sh.nused[tt], lh, vq, want, slot, e,
+                                         sure ? Hs : (3 << lh) / 4, full_bit);
       if (!(e & full_bit)) {
 #pragma unroll
         for (int j = 0; j < 2 * kCornersPerLane; j++)
@@ -522,7 +526,7 @@ static __device__ void block_field_pool(const KArgs& a, SpecShared& sh, unsigned
   const WarpShared& ws = sh.ws;
   const RepDev& rd = ws.rd;
   const int* pkeys = reinterpret_cast<const int*>(smem + a.off_pkeys);
-  const int* pused = reinterpret_cast<const int*>(smem + a.off_pused);
+  const unsigned short* pused = reinterpret_cast<const unsigned short*>(smem + a.off_pused);
   long long* pvals = reinterpret_cast<long long*>(smem + a.off_pvals);
   const long long* grid = a.grid + rd.vox_off * a.ncol;
   const int n = sh.npool;
@@ -582,7 +586,7 @@ static __device__ void block_commit_pool(const KArgs& a, SpecShared& sh, unsigne
   if (tid < 0) return;
   const RepDev& rd = sh.ws.rd;
   int* pkeys = reinterpret_cast<int*>(smem + a.off_pkeys);
-  const int* pused = reinterpret_cast<const int*>(smem + a.off_pused);
+  const unsigned short* pused = reinterpret_cast<const unsigned short*>(smem + a.off_pused);
   long long* pvals = reinterpret_cast<long long*>(smem + a.off_pvals);
   long long* grid = a.grid + rd.vox_off * a.ncol;
   const int n = sh.npool, hcol = a.hcol, ncol = a.ncol;
@@ -625,7 +629,7 @@ static __device__ __noinline__ void log_move(const KArgs& a, int rep, unsigned l
   rec.ind0 = P.ind0;
   rec.indf = P.indf;
   rec.dE_poly = P.empty ? 0.0 : P.dEp;
-  rec.dE_field = P.empty ? 0.0 : P.dE - P.dEp;
+  rec.dE_field = P.empty ? 0.0 : dE_value(P.dq, P.dE) - P.dEp;
   rec.accepted = P.empty ? -1 : P.dec;
   rec.n_draws = P.ndraw;
   a.mlog[(long long)rep * a.mlog_cap + (long long)k] = rec;
@@ -845,8 +849,8 @@ __device__ __forceinline__ typename AccOf<Pos>::type rotate_tangent(const KArgs&
     tt3[j] = e3; tt2[j] = e2;
   }
   Acc de = acc_zero<Acc>();
-  if (hl) acc_add(de, pair_dE_fwd(bl, r0, r, r, t30, t3, tt3));
-  if (hr) acc_add(de, pair_dE_rev(br, r, r, r1, t3, tt3, t31));
+  if (hl) acc_add(de, tangent_dE_fwd(bl, r0, r, t30, t3, tt3));
+  if (hr) acc_add(de, tangent_dE_rev(br, r, r1, t3, tt3, t31));
   if (!LEAN && rd.twist) {  // SSTWLC: twist terms of both bonds
     const double* tw = a.twist + rd.bead_off * 2;
     const Frame cur = frame_of(t2, t3), nw = frame_of(tt2, tt3);
@@ -1015,7 +1019,7 @@ __device__ void short_tangent_evaluate(const KArgs& a, SpecShared& sh, int rep, 
     P.nvox = 0;
     P.cmask = 0;
     bool dec = false;
-    if (!err) dec = decide(word(2 + used + 2 * m), part, Fx{0, 0.0}, 0.0, &P.dE);
+    if (!err) dec = decide(word(2 + used + 2 * m), part, Fx{0, 0.0}, 0.0, P.dq, P.dE);
     P.dec = dec ? 1 : 0;
     if (!LEAN && a.mlog) log_terms(P, part, (unsigned long long)(2 + used + 2 * m + (err ? 0 : 1)));
   }
@@ -1242,9 +1246,13 @@ __device__ __forceinline__ void decide_position(const KArgs& a, SpecShared& sh, 
     regfail = P.freg;
   }
   bool dec = false;
-  if (!err && !P.empty) dec = decide(P.xm, dEp, dEs, with_huge(dEh, dEH), gl == 0 ? &P.dE : nullptr);
+  long long dq = 0;
+  double dh = 0;
+  if (!err && !P.empty) dec = decide(P.xm, dEp, dEs, with_huge(dEh, dEH), dq, dh);
   __syncwarp(group_mask<G>());  // every lane has read the plan
   if (gl == 0) {
+    P.dq = dq;
+    P.dE = dh;
     P.err = (int)err;
     P.regfail = regfail;
     P.dec = dec ? 1 : 0;
@@ -1468,10 +1476,14 @@ __device__ void evaluate_move(const KArgs& a, SpecShared& sh, int rep, int s, in
   }
   err = gor<G>(err);
   bool dec = false;
+  long long dq = 0;
+  double dh = 0;
   if (live && !err && !empty) {
-    dec = decide(g.next(), dEp, dEs, with_huge(dEh, dEH), gl == 0 ? &P.dE : nullptr);
+    dec = decide(g.next(), dEp, dEs, with_huge(dEh, dEH), dq, dh);
   }
   if (gl == 0 && live) {
+    P.dq = dq;
+    P.dE = dh;
     P.kind = kind; P.m = (int)m; P.ind0 = (int)ind0; P.indf = (int)indf;
     P.empty = empty ? 1 : 0; P.err = (int)err; P.regfail = regfail; P.dec = dec ? 1 : 0;
     P.nvox = (int)nvox; P.gtab = gtab; P.gstage = gstage;
@@ -1634,13 +1646,42 @@ __device__ void commit_and_clear(const KArgs& a, SpecShared& sh, int rep, int s,
   }
 }
 
-// 168 registers: two CTAs of 6 warps fit one SM's register file (measured
-// faster than 128 registers with 8 warps, which spills).  LEAN: the
-// instantiation for launches with no SSTWLC replica and no move log, whose
-// code for those is left out (it holds the batch loop's state in registers
-// without spills; the host picks it per launch, a.lean).
+// Moves in flight for the next cycle of a position move: a batch of B costs
+// about kBatchFixed + B (its phases' latencies, in units of one more move) and
+// stands up to the first move that meets an earlier accepted one.  With p the
+// chance of that per pair of moves, as the batches so far met it, E(B) = sum_k
+// prod_(j<k) (1 - j p) moves of the batch are expected to stand; the B with the
+// least (kBatchFixed + B) / E(B) is taken.  The outcome does not depend on it.
+// (128 confined chains of 3,000 beads, of whose 12 moves in flight 4.7 stood: 4.84
+// -> 4.16 ms; kBatchFixed of 10, 20 and 40 measured within 1 %.)
+constexpr float kBatchFixed = 20.0f;
+__device__ __forceinline__ int batch_limit(float met, float pairs, int most) {
+  const float p = pairs > 0.0f ? met / pairs : 0.0f;
+  float stand = 1.0f, E = 0.0f, best_e = 0.0f, best_c = 1.0f;
+  int best = 1;
+#pragma unroll 1
+  for (int B = 1; B <= most; B++) {
+    E += stand;
+    const float c = kBatchFixed + (float)B;
+    if (c * best_e < best_c * E) {
+      best = B;
+      best_e = E;
+      best_c = c;
+    }
+    stand = fmaxf(0.0f, stand * (1.0f - (float)B * p));
+  }
+  return best;
+}
+
+// FP32 storage: 128 registers, 16 warps per SM, in CTAs of more warps than
+// moves in flight (the block-wide phases use them all).  At 168 registers and 12
+// warps: 256 chains, 20 MC steps, kernel only, 10.3 against 9.95 ms, one
+// 10,000-bead chain, 10 steps, 2.40 against 2.23.  FP64 storage: 168 registers.
+// LEAN: the instantiation for launches with no SSTWLC or fast_field replica and
+// no move log, whose code for those is left out (the host picks it per launch,
+// a.lean).
 template <typename Pos, int G, bool LEAN>
-__global__ void __maxnreg__(168) spec_kernel(KArgs a) {
+__global__ void __maxnreg__(sizeof(Pos) == 4 ? 128 : 168) spec_kernel(KArgs a) {
   extern __shared__ __align__(32) unsigned char smem[];
   constexpr int GPW = 32 / G;  // move groups per warp
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
@@ -1663,10 +1704,12 @@ __global__ void __maxnreg__(168) spec_kernel(KArgs a) {
     for (int i = tid; i < (int)(5 * sizeof(cg_move_ctl) / 4); i += blockDim.x) cd[i] = cs[i];
     for (int i = tid; i < HB; i += blockDim.x) { bkeys[i] = -1; bmask[i] = 0u; }
     for (int i = tid; i < 30; i += blockDim.x) sh.ws.tally[i] = 0;
-    const SlotScratch sm = shared_slot(a, sh, slot);
-    for (int i = gl; i < (1 << a.logH); i += G) { sm.keys[i] = -1; sm.bslot[i] = -1; }
-    for (int i = gl; i < (1 << a.logH) * hcol; i += G) sm.vals[i] = 0;
-    if (gl == 0) sh.nused[slot] = 0;
+    if (slot < Sn) {
+      const SlotScratch sm = shared_slot(a, sh, slot);
+      for (int i = gl; i < (1 << a.logH); i += G) { sm.keys[i] = -1; sm.bslot[i] = -1; }
+      for (int i = gl; i < (1 << a.logH) * hcol; i += G) sm.vals[i] = 0;
+      if (gl == 0) sh.nused[slot] = 0;
+    }
     if (a.pool_on) {
       int* pk = reinterpret_cast<int*>(smem + a.off_pkeys);
       long long* pv = reinterpret_cast<long long*>(smem + a.off_pvals);
@@ -1681,6 +1724,11 @@ __global__ void __maxnreg__(168) spec_kernel(KArgs a) {
     sh.t0 = rd0.draw_pos;
     sh.tlog = rd0.draw_pos;
     sh.run_dE = rd0.run_dE;
+    sh.run_q = 0;
+    for (int k = 0; k < 3; k++) {
+      sh.met[k] = sh.pairs[k] = 0.0f;
+      sh.limit[k] = Sn;
+    }
     sh.stop = 0;
     sh.cut = 0;
     sh.npool = 0;
@@ -1707,9 +1755,9 @@ __global__ void __maxnreg__(168) spec_kernel(KArgs a) {
           // beads of each earlier accepted one with probability ~3/8 (amp + 1)^2 / N)
           constexpr bool kShort = G == 32 && sizeof(Pos) == 4;
           const bool brief = kShort && kind == CG_TANGENT_ROTATION && c.amp_bead >= 1 && c.amp_bead <= 32;
-          int most = Sn;
+          int most = kind <= CG_SLIDE ? sh.limit[kind] : Sn;
           if (brief) {
-            const int room = min(kMaxS, (int)(blockDim.x >> 5) * (c.amp_bead <= 16 ? 4 : 2));
+            const int room = min(kMaxS, Sn * 32 / (c.amp_bead <= 16 ? 8 : 16));
             const int likely = (int)(kShortSpan * sqrtf((float)sh.ws.rd.n_beads) / (float)(c.amp_bead + 1));
             most = min(room, max(Sn, likely));
           }
@@ -1772,6 +1820,25 @@ __global__ void __maxnreg__(168) spec_kernel(KArgs a) {
             const unsigned sm_v = __reduce_add_sync(kFull, stand ? (unsigned)Pl.nvox : 0u);
             const unsigned ac_m = __reduce_add_sync(kFull, took ? (unsigned)Pl.m : 0u);
             const unsigned ac_v = __reduce_add_sync(kFull, took ? (unsigned)Pl.nvox : 0u);
+            const unsigned empties = __ballot_sync(kFull, stand && Pl.empty);
+            // running sum of accepted dE, penalised moves left out: the
+            // fixed-point parts exactly (32-bit reductions of 16-bit pieces of
+            // the two's complement), moves with an FP64 part one by one
+            const unsigned hards = __ballot_sync(kFull, took && !is_zero64(Pl.dE));
+            if constexpr (sizeof(Pos) == 4) {
+              const unsigned long long q = took && !((hards >> lane) & 1u) ? (unsigned long long)Pl.dq : 0ull;
+              unsigned long long sum = 0;
+#pragma unroll
+              for (int k = 0; k < 4; k++)
+                sum += (unsigned long long)__reduce_add_sync(kFull, (unsigned)(q >> (16 * k)) & 0xFFFFu) << (16 * k);
+              if (lane == 0) {
+                sh.run_q += (long long)sum;
+                if (sh.run_q > (1LL << 61) || sh.run_q < -(1LL << 61)) {  // far from the int64 range
+                  sh.run_dE += (double)sh.run_q * kFxEInv;
+                  sh.run_q = 0;
+                }
+              }
+            }
             if (lane == 0) {
               const unsigned n_acc = (unsigned)__popc(acc);
               c.num_attempt += cut;
@@ -1783,20 +1850,30 @@ __global__ void __maxnreg__(168) spec_kernel(KArgs a) {
               t[3] += sm_v;
               t[4] += ac_m;
               t[5] += ac_v;
-              // acc = alpha * x + (1 - alpha) * acc with x in {0, 1}, where
-              // alpha * x is alpha or 0 exactly: one FP64 multiply-add chain
-              double run = sh.run_dE, rate = c.acc_rate;
-              const double alpha = c.alpha, beta = 1 - c.alpha;
-              #pragma unroll 1
-              for (int w = 0; w < cut; w++) {
-                const MovePlan& P = sh.plan[w];
-                if (!LEAN && a.mlog) log_move(a, rep, sh.t0 + (unsigned long long)w - sh.tlog, P);
-                if (P.empty) continue;
-                if (P.dec && soft_dE(P.dE)) run += P.dE;
-                rate = (P.dec ? alpha : 0.0) + beta * rate;
+#pragma unroll 1
+              for (unsigned left = hards; left; left &= left - 1) {
+                const MovePlan& P = sh.plan[__ffs((int)left) - 1];
+                const double dE = dE_value(P.dq, P.dE);
+                if (soft_dE(dE)) sh.run_dE += dE;
               }
-              sh.run_dE = run;
+              // acc = alpha * x + (1 - alpha) * acc with x in {0, 1}: one FP64
+              // multiply a move, and an add of alpha where it was accepted (a
+              // chain of FP64 operations, in move order)
+              double rate = c.acc_rate;
+              const double alpha = c.alpha, beta = 1 - c.alpha;
+#pragma unroll 1
+              for (int w = 0; w < cut; w++) {
+                if (!LEAN && a.mlog) log_move(a, rep, sh.t0 + (unsigned long long)w - sh.tlog, sh.plan[w]);
+                if ((empties >> w) & 1u) continue;
+                rate = beta * rate;
+                if ((D >> w) & 1u) rate = alpha + rate;
+              }
               c.acc_rate = rate;
+              if (kind <= CG_SLIDE) {
+                const bool met = first_fail < B;
+                sh.met[kind] = 0.9f * sh.met[kind] + (met ? 1.0f : 0.0f);
+                sh.pairs[kind] = 0.9f * sh.pairs[kind] + (float)(cut * (cut - 1) / 2 + (met ? cut : 0));
+              }
               sh.t0 += (unsigned long long)cut;
               if (cut == first_fail && first_fail < B && sh.plan[first_fail].err) sh.stop = sh.plan[first_fail].err;
             }
@@ -1817,7 +1894,10 @@ __global__ void __maxnreg__(168) spec_kernel(KArgs a) {
         }
       }
       if (sh.stop) break;
-      if (tid == 0) update_amplitudes(c);
+      if (tid == 0) {
+        update_amplitudes(c);
+        if (kind <= CG_SLIDE) sh.limit[kind] = batch_limit(sh.met[kind], sh.pairs[kind], Sn);
+      }
       __syncthreads();
     }
     if (sh.stop) break;
@@ -1831,7 +1911,7 @@ __global__ void __maxnreg__(168) spec_kernel(KArgs a) {
   if (tid == 0) {
     RepDev* out = a.reps + rep;
     out->draw_pos = sh.t0;
-    out->run_dE = sh.run_dE;
+    out->run_dE = sh.run_dE + (double)sh.run_q * kFxEInv;
     out->err = (unsigned)sh.stop;
     unsigned long long* t = a.tally + (long long)rep * 30;
     for (int i = 0; i < 30; i++) t[i] += sh.ws.tally[i];
