@@ -580,10 +580,10 @@ static __device__ void block_field_pool(const KArgs& a, SpecShared& sh, unsigned
 // is the block voxel table.
 static __device__ void block_commit_pool(const KArgs& a, SpecShared& sh, unsigned char* smem, int cut, unsigned acc,
                                   int* bkeys, unsigned* bmask) {
-  // warp 0 keeps the batch's books meanwhile (with one warp it does both)
-  const int skip = blockDim.x > 32 ? 32 : 0;
-  const int tid = (int)threadIdx.x - skip, nt = (int)blockDim.x - skip;
-  if (tid < 0) return;
+  // the last two warps keep the batch's books meanwhile (with two or fewer they
+  // do both)
+  const int tid = (int)threadIdx.x, nt = (int)blockDim.x > 64 ? (int)blockDim.x - 64 : (int)blockDim.x;
+  if (tid >= nt) return;
   const RepDev& rd = sh.ws.rd;
   int* pkeys = reinterpret_cast<int*>(smem + a.off_pkeys);
   const unsigned short* pused = reinterpret_cast<const unsigned short*>(smem + a.off_pused);
@@ -870,16 +870,17 @@ __device__ __forceinline__ typename AccOf<Pos>::type rotate_tangent(const KArgs&
 
 // ---------------------------------------------------------------- short tangent rotations
 // Batches of tangent rotations of few beads (SimpleControl settles at an
-// amplitude of ~13, a mean of 7 beads): GS = 8 or 16 lanes per move instead of
-// 32, so that 2-4 times as many moves are in flight on the same warps, and the
-// rotated beads registered in the block table (key: bead), so that a move finds
-// the earlier moves that rotate its beads or their neighbours by three look-ups
-// a bead instead of comparing lists.  A move's staging, index list and draws
-// fit its share of the slot regions for up to 2 GS beads (amplitudes up to 32;
-// longer ones take the path of 32 lanes).  One 10,000-bead chain, 10 MC steps:
-// 2.83 -> 2.62 ms; 64 SSTWLC chains of 2,000 beads, whose FP64 twist terms fill
-// their warps' lanes: 10.4 -> 9.1 ms (kernel only, with the phases' state kept
-// in the plans).
+// amplitude of ~13, a mean of 7 beads): 8 lanes per move up to 8 beads, 16 beyond,
+// instead of 32, so that 2-4 times as many moves are in flight on the same warps,
+// and the rotated beads registered in the block table (key: bead), so that a
+// move finds the earlier moves that rotate its beads or their neighbours by
+// three look-ups a bead instead of comparing lists.  A move's staging, index
+// list and draws fit a quarter of a slot's region for up to 16 beads, half of it
+// for up to 32 (longer ones take the path of 32 lanes).  One 10,000-bead chain,
+// 10 MC steps, kernel only: 2.83 -> 2.62 ms; 64 SSTWLC chains of 2,000 beads,
+// whose FP64 twist terms fill their warps' lanes: 10.4 -> 9.1 ms (with the
+// phases' state kept in the plans); 9-16 beads on 16 lanes instead of 8, one
+// pass instead of two: 256 chains 9.90 -> 9.53 ms, the SSTWLC chains 8.46 -> 7.60.
 //
 // Moves in flight: kShortSpan sqrt(N) / (amp + 1), at which about two of them
 // meet an earlier accepted one (3 and 4 measured alike, 6 and 9 were slower on
@@ -892,22 +893,25 @@ struct ShortTangent {
   float* stage;    // new t3, t2 of each bead: 6 floats
   unsigned* draws;
   int ndraw;
-  __device__ __forceinline__ ShortTangent(const KArgs& a, SpecShared& sh, int gs) : GS(gs) {
-    const int lane = (int)(threadIdx.x & 31u), per = 32 / GS;
-    const int warp = (int)(threadIdx.x >> 5), sub = lane / GS;
-    s = warp * per + sub;
-    gl = lane & (GS - 1);
-    gmask = (GS == 16 ? 0xFFFFu : 0xFFu) << (lane & ~(GS - 1));
-    unsigned char* base = reinterpret_cast<unsigned char*>(&sh) + a.spec_off_warps + (size_t)warp * a.warp_smem;
-    idx = reinterpret_cast<int*>(base + a.off_draws) + sub * 2 * GS;
-    const int room = ((a.off_idx - a.off_stage + 4 * (int)a.stage_cap) * GS / 32) & ~15;
+  // gs lanes a group; up to cap (16 or 32) beads a move, which take a quarter or
+  // a half of a slot's region
+  __device__ __forceinline__ ShortTangent(const KArgs& a, SpecShared& sh, int gs, int cap) : GS(gs) {
+    const int lane = (int)(threadIdx.x & 31u), per = 64 / cap;
+    s = (int)threadIdx.x / gs;
+    gl = lane & (gs - 1);
+    gmask = (gs == 16 ? 0xFFFFu : 0xFFu) << (lane & ~(gs - 1));
+    const int sub = s % per;
+    unsigned char* base =
+        reinterpret_cast<unsigned char*>(&sh) + a.spec_off_warps + (size_t)(s / per) * a.warp_smem;
+    idx = reinterpret_cast<int*>(base + a.off_draws) + sub * cap;
+    const int room = ((a.off_idx - a.off_stage + 4 * (int)a.stage_cap) / per) & ~15;
     unsigned char* q = base + a.off_stage + sub * room;
     stage = reinterpret_cast<float*>(q);
-    draws = reinterpret_cast<unsigned*>(q + 48 * GS);  // 2 GS beads x 24 bytes
-    ndraw = (room - 48 * GS) / 16 * 4;
+    draws = reinterpret_cast<unsigned*>(q + 24 * cap);
+    ndraw = (room - 24 * cap) / 16 * 4;
   }
 };
-static_assert(4 * kDrawCache == 32 * 2 * 4, "the index lists share the draw buffer: 2 GS beads a group");
+static_assert(kDrawCache == 64, "the index lists share a slot's draw buffer: four of 16 or two of 32 beads");
 
 __device__ __forceinline__ unsigned block_find(const int* bkeys, const unsigned* bmask, int logHB, int key) {
   const unsigned mask = (1u << logHB) - 1u;
@@ -1755,9 +1759,10 @@ __global__ void __maxnreg__(sizeof(Pos) == 4 ? 128 : 168) spec_kernel(KArgs a) {
           // beads of each earlier accepted one with probability ~3/8 (amp + 1)^2 / N)
           constexpr bool kShort = G == 32 && sizeof(Pos) == 4;
           const bool brief = kShort && kind == CG_TANGENT_ROTATION && c.amp_bead >= 1 && c.amp_bead <= 32;
+          const int gs = c.amp_bead <= 8 ? 8 : 16, cap = c.amp_bead <= 16 ? 16 : 32;  // of a short rotation
           int most = kind <= CG_SLIDE ? sh.limit[kind] : Sn;
           if (brief) {
-            const int room = min(kMaxS, Sn * 32 / (c.amp_bead <= 16 ? 8 : 16));
+            const int room = min(min(kMaxS, Sn * (64 / cap)), (int)blockDim.x / gs);
             const int likely = (int)(kShortSpan * sqrtf((float)sh.ws.rd.n_beads) / (float)(c.amp_bead + 1));
             most = min(room, max(Sn, likely));
           }
@@ -1766,7 +1771,7 @@ __global__ void __maxnreg__(sizeof(Pos) == 4 ? 128 : 168) spec_kernel(KArgs a) {
           const bool live = slot < B;
           if constexpr (kShort) {
             if (brief) {
-              const ShortTangent T(a, sh, c.amp_bead <= 16 ? 8 : 16);
+              const ShortTangent T(a, sh, gs, cap);
               short_tangent_evaluate<LEAN>(a, sh, rep, T, B, c, bkeys, bmask);
               __syncthreads();
               short_tangent_conflicts(a, sh, T, B, bkeys, bmask);
@@ -1812,53 +1817,17 @@ __global__ void __maxnreg__(sizeof(Pos) == 4 ? 128 : 168) spec_kernel(KArgs a) {
           int cut = first_fail;
           if (RF && __ffs((int)RF) < cut) cut = __ffs((int)RF);
           const unsigned acc = cut >= 32 ? D : (D & ((1u << cut) - 1u));
-          if (warp == 0) {
-            // bookkeeping of the standing moves, in move order where it is FP64
-            const bool stand = lane < cut;
-            const bool took = (acc >> lane) & 1u;
-            const unsigned sm_m = __reduce_add_sync(kFull, stand ? (unsigned)Pl.m : 0u);
-            const unsigned sm_v = __reduce_add_sync(kFull, stand ? (unsigned)Pl.nvox : 0u);
-            const unsigned ac_m = __reduce_add_sync(kFull, took ? (unsigned)Pl.m : 0u);
-            const unsigned ac_v = __reduce_add_sync(kFull, took ? (unsigned)Pl.nvox : 0u);
-            const unsigned empties = __ballot_sync(kFull, stand && Pl.empty);
-            // running sum of accepted dE, penalised moves left out: the
-            // fixed-point parts exactly (32-bit reductions of 16-bit pieces of
-            // the two's complement), moves with an FP64 part one by one
-            const unsigned hards = __ballot_sync(kFull, took && !is_zero64(Pl.dE));
-            if constexpr (sizeof(Pos) == 4) {
-              const unsigned long long q = took && !((hards >> lane) & 1u) ? (unsigned long long)Pl.dq : 0ull;
-              unsigned long long sum = 0;
-#pragma unroll
-              for (int k = 0; k < 4; k++)
-                sum += (unsigned long long)__reduce_add_sync(kFull, (unsigned)(q >> (16 * k)) & 0xFFFFu) << (16 * k);
-              if (lane == 0) {
-                sh.run_q += (long long)sum;
-                if (sh.run_q > (1LL << 61) || sh.run_q < -(1LL << 61)) {  // far from the int64 range
-                  sh.run_dE += (double)sh.run_q * kFxEInv;
-                  sh.run_q = 0;
-                }
-              }
-            }
+          // bookkeeping of the standing moves by the last two warps (which, with
+          // more warps than moves in flight, have no move to commit): one the
+          // acceptance rate, an FP64 chain in move order, the other the sums
+          const int last = (int)(blockDim.x >> 5) - 1;
+          if (warp == last) {
+            const unsigned empties = __ballot_sync(kFull, lane < cut && Pl.empty);
             if (lane == 0) {
-              const unsigned n_acc = (unsigned)__popc(acc);
               c.num_attempt += cut;
-              c.num_success += n_acc;
-              unsigned long long* t = sh.ws.tally + kind * 6;
-              t[0] += (unsigned long long)cut;
-              t[1] += n_acc;
-              t[2] += sm_m;
-              t[3] += sm_v;
-              t[4] += ac_m;
-              t[5] += ac_v;
-#pragma unroll 1
-              for (unsigned left = hards; left; left &= left - 1) {
-                const MovePlan& P = sh.plan[__ffs((int)left) - 1];
-                const double dE = dE_value(P.dq, P.dE);
-                if (soft_dE(dE)) sh.run_dE += dE;
-              }
+              c.num_success += __popc(acc);
               // acc = alpha * x + (1 - alpha) * acc with x in {0, 1}: one FP64
-              // multiply a move, and an add of alpha where it was accepted (a
-              // chain of FP64 operations, in move order)
+              // multiply a move, and an add of alpha where it was accepted
               double rate = c.acc_rate;
               const double alpha = c.alpha, beta = 1 - c.alpha;
 #pragma unroll 1
@@ -1878,8 +1847,49 @@ __global__ void __maxnreg__(sizeof(Pos) == 4 ? 128 : 168) spec_kernel(KArgs a) {
               if (cut == first_fail && first_fail < B && sh.plan[first_fail].err) sh.stop = sh.plan[first_fail].err;
             }
           }
+          if (warp == (last > 0 ? last - 1 : 0)) {
+            const bool stand = lane < cut;
+            const bool took = (acc >> lane) & 1u;
+            const unsigned sm_m = __reduce_add_sync(kFull, stand ? (unsigned)Pl.m : 0u);
+            const unsigned sm_v = __reduce_add_sync(kFull, stand ? (unsigned)Pl.nvox : 0u);
+            const unsigned ac_m = __reduce_add_sync(kFull, took ? (unsigned)Pl.m : 0u);
+            const unsigned ac_v = __reduce_add_sync(kFull, took ? (unsigned)Pl.nvox : 0u);
+            // running sum of accepted dE, penalised moves left out: the
+            // fixed-point parts exactly (32-bit reductions of 16-bit pieces of
+            // the two's complement), moves with an FP64 part one by one
+            const unsigned hards = __ballot_sync(kFull, took && !is_zero64(Pl.dE));
+            if constexpr (sizeof(Pos) == 4) {
+              const unsigned long long q = took && !((hards >> lane) & 1u) ? (unsigned long long)Pl.dq : 0ull;
+              unsigned long long sum = 0;
+#pragma unroll
+              for (int k = 0; k < 4; k++)
+                sum += (unsigned long long)__reduce_add_sync(kFull, (unsigned)(q >> (16 * k)) & 0xFFFFu) << (16 * k);
+              if (lane == 0) {
+                sh.run_q += (long long)sum;
+                if (sh.run_q > (1LL << 61) || sh.run_q < -(1LL << 61)) {  // far from the int64 range
+                  sh.run_dE += (double)sh.run_q * kFxEInv;
+                  sh.run_q = 0;
+                }
+              }
+            }
+            if (lane == 0) {
+              unsigned long long* t = sh.ws.tally + kind * 6;
+              t[0] += (unsigned long long)cut;
+              t[1] += (unsigned long long)__popc(acc);
+              t[2] += sm_m;
+              t[3] += sm_v;
+              t[4] += ac_m;
+              t[5] += ac_v;
+#pragma unroll 1
+              for (unsigned left = hards; left; left &= left - 1) {
+                const MovePlan& P = sh.plan[__ffs((int)left) - 1];
+                const double dE = dE_value(P.dq, P.dE);
+                if (soft_dE(dE)) sh.run_dE += dE;
+              }
+            }
+          }
           if constexpr (kShort)
-            if (brief) short_tangent_commit(a, sh, ShortTangent(a, sh, c.amp_bead <= 16 ? 8 : 16), cut, acc, bkeys, bmask);
+            if (brief) short_tangent_commit(a, sh, ShortTangent(a, sh, gs, cap), cut, acc, bkeys, bmask);
           if (!brief) {
             if (wlive && live)
               commit_and_clear<Pos, G>(a, sh, rep, slot, gl, slot < cut && ((acc >> slot) & 1u), bkeys, bmask);
