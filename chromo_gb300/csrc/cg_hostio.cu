@@ -28,11 +28,22 @@ struct HostRow {  // one replica's host arrays (NULL: not transferred)
   long long* st;
 };
 
-// The host arrays are walked flat (element j of replica rep's [n x 3] or
-// [n x nb] array on thread j), so every warp reads or writes 32 consecutive
-// 8-byte words of host memory: whole 256-byte lines over the link.  The
-// resident side takes the scattered accesses (HBM / L2).
+// The host arrays are walked flat (consecutive elements of replica rep's
+// [n x 3] or [n x nb] array on consecutive threads), and from the 128-byte line
+// that the array starts in, so that a warp reads or writes two whole lines over
+// the link: a part of an array, or one that malloc places 16 bytes into a page,
+// starts off a line, and warps that begin there split every line between two
+// requests.  Threads before the array's first element do nothing.  The resident
+// side takes the scattered accesses (HBM / L2).  The link bounds both
+// directions (192 GB/s to the host, 210 GB/s from it with whole lines).  Measured
+// for 32 chains of 100,000 beads in parts of one array: read-back 1.84 -> 1.47 ms
+// (153 -> 191 GB/s), upload 1.57 -> 1.44 ms (179 -> 196 GB/s).
 //
+// First thread index of element 0: the elements between the line and p.
+__device__ __forceinline__ long long line_lead(const void* p) {
+  return (long long)((reinterpret_cast<unsigned long long>(p) >> 3) & 15);
+}
+
 // mode 0: check only (flag bit 1: non-finite coordinate, bit 2: state out of
 // range); mode 1: write a's storage; mode 2: check and write.
 template <typename Pos>
@@ -46,10 +57,12 @@ __global__ void host_load_kernel(KArgs a, const HostRow* tab, int nb, unsigned* 
                  reinterpret_cast<Pos*>(reinterpret_cast<V4<Pos>*>(a.t34) + off),
                  reinterpret_cast<Pos*>(reinterpret_cast<V4<Pos>*>(a.t24) + off)};
   const long long stride = (long long)gridDim.x * blockDim.x;
+  const long long first = blockIdx.x * (long long)blockDim.x + threadIdx.x;
   unsigned bad = 0;
   for (int k = 0; k < 3; k++) {
     if (!src[k]) continue;
-    for (long long j = blockIdx.x * (long long)blockDim.x + threadIdx.x; j < 3 * n; j += stride) {
+    for (long long j = first - line_lead(src[k]); j < 3 * n; j += stride) {
+      if (j < 0) continue;
       const double x = src[k][j];
       if (mode != 1 && !isfinite(x)) bad |= 1u;
       if (mode != 0) dst[k][4 * (j / 3) + j % 3] = (Pos)x;  // the 4-vector's pad stays 0
@@ -57,7 +70,8 @@ __global__ void host_load_kernel(KArgs a, const HostRow* tab, int nb, unsigned* 
   }
   if (row.st) {
     unsigned char* sb = reinterpret_cast<unsigned char*>(a.states + off);
-    for (long long j = blockIdx.x * (long long)blockDim.x + threadIdx.x; j < n * nb; j += stride) {
+    for (long long j = first - line_lead(row.st); j < n * nb; j += stride) {
+      if (j < 0) continue;
       const long long v = row.st[j];
       if (v < 0 || v > CG_MAX_MARK) bad |= 2u;
       else if (mode != 0) sb[4 * (j / nb) + j % nb] = (unsigned char)v;  // byte b of bead i's word
@@ -100,15 +114,16 @@ __global__ void host_store_kernel(KArgs a, const HostRow* tab, int nb) {
                        reinterpret_cast<const Pos*>(reinterpret_cast<const V4<Pos>*>(a.t34) + off),
                        reinterpret_cast<const Pos*>(reinterpret_cast<const V4<Pos>*>(a.t24) + off)};
   const long long stride = (long long)gridDim.x * blockDim.x;
+  const long long first = blockIdx.x * (long long)blockDim.x + threadIdx.x;
   for (int k = 0; k < 3; k++) {
     if (!dst[k]) continue;
-    for (long long j = blockIdx.x * (long long)blockDim.x + threadIdx.x; j < 3 * n; j += stride)
-      dst[k][j] = (double)src[k][4 * (j / 3) + j % 3];
+    for (long long j = first - line_lead(dst[k]); j < 3 * n; j += stride)
+      if (j >= 0) dst[k][j] = (double)src[k][4 * (j / 3) + j % 3];
   }
   if (row.st) {
     const unsigned char* sb = reinterpret_cast<const unsigned char*>(a.states + off);
-    for (long long j = blockIdx.x * (long long)blockDim.x + threadIdx.x; j < n * nb; j += stride)
-      row.st[j] = (long long)sb[4 * (j / nb) + j % nb];
+    for (long long j = first - line_lead(row.st); j < n * nb; j += stride)
+      if (j >= 0) row.st[j] = (long long)sb[4 * (j / nb) + j % nb];
   }
 }
 
