@@ -196,10 +196,9 @@ __device__ __forceinline__ void load_transform(const MovePlan& P, Pos (&M)[3][4]
     for (int j = 0; j < 4; j++) M[i][j] = Mp[4 * i + j];
 }
 
-// Elastic (and twist) dE of one boundary bond of a position move: the bond to
-// the fixed neighbour left of the segment (side 0) or right of it (side 1);
-// zero where the segment ends the chain.  The move's plan holds its segment
-// and transform.
+// Elastic dE of one boundary bond of a position move: the bond to the fixed
+// neighbour left of the segment (side 0) or right of it (side 1); zero where the
+// segment ends the chain.  The move's plan holds its segment and transform.
 template <typename Pos, typename Acc, bool LEAN>
 static __device__ __forceinline__ Acc boundary_term(const KArgs& a, const RepDev& rd, const MovePlan& P, int kind,
                                                  int side) {
@@ -215,20 +214,37 @@ static __device__ __forceinline__ Acc boundary_term(const KArgs& a, const RepDev
   const Bond<Pos> bn = bond_at(cv.bonds, cv.bonds32, side == 0 ? in : i, (Pos)0);
   const Pos r[3] = {R.x, R.y, R.z}, t3[3] = {T3.x, T3.y, T3.z};
   const Pos rn[3] = {RN.x, RN.y, RN.z}, tn[3] = {TN.x, TN.y, TN.z};
-  Pos t2[3] = {0, 0, 0}, tr[3], tt3[3], tt2[3];
-  if (cv.twist) {
-    const V4<Pos> T2 = cv.t24[i];
-    t2[0] = T2.x; t2[1] = T2.y; t2[2] = T2.z;
-  }
+  const Pos t2[3] = {0, 0, 0};
+  Pos tr[3], tt3[3], tt2[3];
   move_bead(kind, M, r, t3, t2, tr, tt3, tt2);
   if (side == 0) acc_add(out, pair_dE_fwd(bn, rn, r, tr, tn, t3, tt3));
   else acc_add(out, pair_dE_rev(bn, r, tr, rn, t3, tt3, tn));
-  if (cv.twist) {  // SSTWLC: the bond's twist term
-    const Frame nb = frame_of(cv.t24[in], TN), cur = frame_of(t2, t3), nw = frame_of(tt2, tt3);
-    const double* tw = cv.twist + 2 * (side == 0 ? in : i);
-    acc_add_d(out, side == 0 ? twist_pair_dE(tw, nb, cur, nb, nw) : twist_pair_dE(tw, cur, nb, nw, nb));
-  }
   return out;
+}
+
+// SSTWLC: twist energy of the same bond before the move (after = false) or
+// after it.
+template <typename Pos>
+static __device__ __forceinline__ double boundary_twist(const KArgs& a, const RepDev& rd, const MovePlan& P, int kind,
+                                                  int side, bool after) {
+  const ChainView<Pos> cv(a, rd, false);
+  const long long i = side == 0 ? P.ind0 : P.indf - 1;
+  const long long in = side == 0 ? i - 1 : i + 1;
+  if (in < 0 || in >= rd.n_beads) return 0.0;
+  V4<Pos> T2 = cv.t24[i], T3 = cv.t34[i];
+  const V4<Pos> N2 = cv.t24[in], N3 = cv.t34[in];
+  if (after) {
+    Pos M[3][4];
+    load_transform(P, M);
+    const Pos r[3] = {0, 0, 0}, t3[3] = {T3.x, T3.y, T3.z}, t2[3] = {T2.x, T2.y, T2.z};
+    Pos tr[3], tt3[3], tt2[3];
+    move_bead(kind, M, r, t3, t2, tr, tt3, tt2);
+    T2.x = tt2[0]; T2.y = tt2[1]; T2.z = tt2[2];
+    T3.x = tt3[0]; T3.y = tt3[1]; T3.z = tt3[2];
+  }
+  const bool left = side == 0;
+  return twist_bond_energy(cv.twist + 2 * (left ? in : i), frame_of(left ? N2 : T2, left ? N3 : T3),
+                           frame_of(left ? T2 : N2, left ? T3 : N3));
 }
 
 // Where one bead's weights lie before (0) and after (1) a move: the voxel of
@@ -372,15 +388,19 @@ __device__ void block_deposit(const KArgs& a, SpecShared& sh, int rep, int B, in
     if (lane >= o) end += y;
   }
   const int total = __shfl_sync(kFull, end, 31);
+  // warps of the beads: all, without those of an SSTWLC batch's bonds (below)
+  // where at least half remain
+  const bool twist = !LEAN && cv.twist != nullptr;
+  const int tws = twist ? (4 * B + 31) >> 5 : 0, WD = 2 * tws <= W ? W - tws : W;
   // beads per warp and round: an even share, in whole passes of the corners
   constexpr int BP = 32 / kLanesPerBead;
   // (by steps: a batch has a few hundred beads)
-  int per = W;  // warps times rounds
-  while (32 * per < total) per += W;
+  int per = WD;  // warps times rounds
+  while (32 * per < total) per += WD;
   int run = BP;
   while (run * per < total) run += BP;
   #pragma unroll 1
-  for (int b0 = warp * run; b0 < total; b0 += W * run) {
+  for (int b0 = warp < WD ? warp * run : total; b0 < total; b0 += WD * run) {
     const int b = b0 + lane;
     // the bead's move: the number of moves whose beads end at or before b
     int s = 0;
@@ -460,7 +480,26 @@ __device__ void block_deposit(const KArgs& a, SpecShared& sh, int rep, int B, in
     }
   }
   // boundary bonds of the moves, two per move
-  if (warp == W - 1)
+  if (!LEAN && twist) {
+    // the twist energies before and after the move on two lanes each, by warps
+    // without beads: an energy is ~150 FP64 operations, which issue at 1/64 of
+    // the FP32 rate whatever the number of lanes, and a batch's deposit waited
+    // for the two energies of each bond (64 SSTWLC chains of 2,000 beads, 10
+    // steps, kernel only, with short_tangent_twist: 7.60 -> 4.82 ms)
+    #pragma unroll 1
+    for (int j0 = 32 * (W - 1 - warp); j0 < 4 * B; j0 += 32 * W) {
+      const int j = j0 + lane, side = (j >> 1) & 1;
+      MovePlan& P = sh.plan[j < 4 * B ? j >> 2 : 0];
+      const bool on = j < 4 * B && P.blk;
+      const double e = on ? boundary_twist<Pos>(a, rd, P, kind, side, j & 1) : 0.0;
+      const double after = __shfl_xor_sync(kFull, e, 1);
+      if (on && !(j & 1)) {
+        Acc t = boundary_term<Pos, Acc, LEAN>(a, rd, P, kind, side);
+        acc_add_d(t, after - e);
+        store_acc(P.pq[side], P.ph[side], t);
+      }
+    }
+  } else if (warp == W - 1)
     for (int j = lane; j < 2 * B; j += 32) {
       MovePlan& P = sh.plan[j >> 1];
       if (P.blk) store_acc(P.pq[j & 1], P.ph[j & 1], boundary_term<Pos, Acc, LEAN>(a, rd, P, kind, j & 1));
@@ -485,14 +524,17 @@ __device__ __forceinline__ void pool_voxel_dE(const WarpShared& ws, const KArgs&
 // a handful of moves; reducing them move by move first took longer: the field
 // phase of a batch of ~5 moves on 256 chains 12.0 k -> 8.5 k cycles).  FP64: a
 // warp reduces each move's terms first.
-__device__ __forceinline__ void add_pool_part(SpecShared& sh, int s, const Fx& part) {
-  if (s < 0) return;
-  MovePlan& P = sh.plan[s];
+__device__ __forceinline__ void add_plan_part(MovePlan& P, const Fx& part) {
   atomicAdd(&P.fl0, (unsigned)(part.q & 0xFFFFF));
   atomicAdd(&P.fl1, (unsigned)((part.q >> 20) & 0xFFFFF));
   atomicAdd(&P.fl2, (int)(part.q >> 40));
-  atomicAdd(&P.fn, 1);
   if (!is_zero64(part.hard)) atomicAdd(&P.fh, part.hard);
+}
+__device__ __forceinline__ void add_pool_part(SpecShared& sh, int s, const Fx& part) {
+  if (s < 0) return;
+  MovePlan& P = sh.plan[s];
+  add_plan_part(P, part);
+  atomicAdd(&P.fn, 1);
 }
 __device__ __forceinline__ void add_pool_part(SpecShared& sh, int s, double part) {
   const int lane = (int)(threadIdx.x & 31u);
@@ -800,7 +842,11 @@ static __device__ __noinline__ void own_path(const KArgs& a, SpecShared& sh, int
     regfail = (int)gor<G>((unsigned)regfail);
   }
   Acc bond = acc_zero<Acc>();
-  if (dep && gl < 2) bond = boundary_term<Pos, Acc, LEAN>(a, rd, P, kind, gl);
+  if (dep && gl < 2) {
+    bond = boundary_term<Pos, Acc, LEAN>(a, rd, P, kind, gl);
+    if (!LEAN && rd.twist)
+      acc_add_d(bond, boundary_twist<Pos>(a, rd, P, kind, gl, true) - boundary_twist<Pos>(a, rd, P, kind, gl, false));
+  }
   if (dep && gl < 2) store_acc(P.pq[gl], P.ph[gl], bond);
   if (run && gl == 0) {
     if (dep) P.oob = oob;
@@ -817,7 +863,7 @@ static __device__ __noinline__ void own_path(const KArgs& a, SpecShared& sh, int
 
 // Tangent rotation of bead i about the axis of draws xa, xb (sine sa, cosine
 // ca): its new frame and the dE of its two bonds, the neighbours' frames as they
-// are.
+// are.  Lean: without the twist terms.
 template <typename Pos, bool LEAN>
 __device__ __forceinline__ typename AccOf<Pos>::type rotate_tangent(const KArgs& a, const RepDev& rd, long long i,
                                                                     unsigned xa, unsigned xb, Pos sa, Pos ca,
@@ -900,15 +946,20 @@ struct ShortTangent {
     s = (int)threadIdx.x / gs;
     gl = lane & (gs - 1);
     gmask = (gs == 16 ? 0xFFFFu : 0xFFu) << (lane & ~(gs - 1));
-    const int sub = s % per;
+    const int room = ((a.off_idx - a.off_stage + 4 * (int)a.stage_cap) / per) & ~15;
+    place(a, sh, s, cap, idx, stage);
+    draws = reinterpret_cast<unsigned*>(stage + 6 * cap);
+    ndraw = (room - 24 * cap) / 16 * 4;
+  }
+  // index list and staging of move s
+  static __device__ __forceinline__ void place(const KArgs& a, SpecShared& sh, int s, int cap, int*& idx,
+                                               float*& stage) {
+    const int per = 64 / cap, sub = s % per;
     unsigned char* base =
         reinterpret_cast<unsigned char*>(&sh) + a.spec_off_warps + (size_t)(s / per) * a.warp_smem;
-    idx = reinterpret_cast<int*>(base + a.off_draws) + sub * cap;
     const int room = ((a.off_idx - a.off_stage + 4 * (int)a.stage_cap) / per) & ~15;
-    unsigned char* q = base + a.off_stage + sub * room;
-    stage = reinterpret_cast<float*>(q);
-    draws = reinterpret_cast<unsigned*>(q + 24 * cap);
-    ndraw = (room - 24 * cap) / 16 * 4;
+    idx = reinterpret_cast<int*>(base + a.off_draws) + sub * cap;
+    stage = reinterpret_cast<float*>(base + a.off_stage + sub * room);
   }
 };
 static_assert(kDrawCache == 64, "the index lists share a slot's draw buffer: four of 16 or two of 32 beads");
@@ -994,7 +1045,7 @@ __device__ void short_tangent_evaluate(const KArgs& a, SpecShared& sh, int rep, 
     const int i = T.idx[k];
     const unsigned xa = word(2 + used + 2 * k), xb = word(3 + used + 2 * k);
     float tt3[3], tt2[3];
-    acc_add(part, rotate_tangent<float, LEAN>(a, rd, i, xa, xb, sa, ca, tt3, tt2));
+    acc_add(part, rotate_tangent<float, true>(a, rd, i, xa, xb, sa, ca, tt3, tt2));
     for (int j = 0; j < 3; j++) {
       T.stage[6 * k + j] = tt3[j];
       T.stage[6 * k + 3 + j] = tt2[j];
@@ -1022,10 +1073,85 @@ __device__ void short_tangent_evaluate(const KArgs& a, SpecShared& sh, int rep, 
     P.regfail = regfail;
     P.nvox = 0;
     P.cmask = 0;
+    if (!LEAN && rd.twist) {  // decided by short_tangent_twist
+      P.xm = word(2 + used + 2 * m);
+      P.ndraw = 2 + used + 2 * m + (err ? 0 : 1);
+      P.fq = part.q;
+      P.fh = part.hard;
+      P.fl0 = P.fl1 = 0;
+      P.fl2 = 0;
+      return;
+    }
     bool dec = false;
     if (!err) dec = decide(word(2 + used + 2 * m), part, Fx{0, 0.0}, 0.0, P.dq, P.dE);
     P.dec = dec ? 1 : 0;
     if (!LEAN && a.mlog) log_terms(P, part, (unsigned long long)(2 + used + 2 * m + (err ? 0 : 1)));
+  }
+}
+
+// SSTWLC: twist terms of the batch's rotated beads, then the decisions.  A
+// bead's four bond energies (left and right bond, before and after) are taken by
+// four lanes, the batch's beads packed over the CTA's warps: one FP64 energy after
+// another in the bead's own lane were 43 k of a batch's 57 k cycles.  Called by
+// every thread, after a barrier.
+static __device__ __noinline__ void short_tangent_twist(const KArgs& a, SpecShared& sh, int B, int cap) {
+  const RepDev& rd = sh.ws.rd;
+  const ChainView<float> cv(a, rd, false);
+  const int lane = (int)(threadIdx.x & 31u);
+  int end = lane < B ? sh.plan[lane].m : 0;
+#pragma unroll
+  for (int o = 1; o < 32; o <<= 1) {
+    const int y = __shfl_up_sync(kFull, end, o);
+    if (lane >= o) end += y;
+  }
+  const int total = 4 * __shfl_sync(kFull, end, 31);
+  #pragma unroll 1
+  for (int j0 = (int)threadIdx.x - lane; j0 < total; j0 += (int)blockDim.x) {
+    const int j = j0 + lane;
+    int s = 0;
+    #pragma unroll 1
+    for (int u = 0; u < B; u++) s += __shfl_sync(kFull, end, u) <= (j >> 2) ? 1 : 0;
+    int base = __shfl_sync(kFull, end, s > 0 ? (s - 1) & 31 : 0);
+    if (s == 0) base = 0;
+    const bool on = j < total;
+    double e = 0.0;
+    if (on) {
+      int* idx;
+      float* stage;
+      ShortTangent::place(a, sh, s, cap, idx, stage);
+      const int k = (j >> 2) - base, i = idx[k];
+      const bool left = !(j & 2);
+      const int in = left ? i - 1 : i + 1;
+      if (in >= 0 && in < (int)rd.n_beads) {
+        V4<float> T2 = cv.t24[i], T3 = cv.t34[i];
+        const V4<float> N2 = cv.t24[in], N3 = cv.t34[in];
+        if (j & 1) {
+          const float* q = stage + 6 * k;
+          T3 = V4<float>{q[0], q[1], q[2], 0.0f};
+          T2 = V4<float>{q[3], q[4], q[5], 0.0f};
+        }
+        e = twist_bond_energy(cv.twist + 2 * (left ? in : i), frame_of(left ? N2 : T2, left ? N3 : T3),
+                              frame_of(left ? T2 : N2, left ? T3 : N3));
+      }
+    }
+    const double d = __shfl_xor_sync(kFull, e, 1) - e;       // lanes 0 and 2 of four
+    const double dt = d + __shfl_down_sync(kFull, d, 2);     // lane 0
+    if (on && !(j & 3)) {
+      Fx part = acc_zero<Fx>();
+      acc_add_d(part, dt);
+      add_plan_part(sh.plan[s], part);
+    }
+  }
+  __syncthreads();
+  if ((int)threadIdx.x < B) {
+    MovePlan& P = sh.plan[threadIdx.x];
+    Fx part;
+    double none = 0.0;
+    plan_field(P, part, none);
+    bool dec = false;
+    if (!P.err) dec = decide(P.xm, part, Fx{0, 0.0}, 0.0, P.dq, P.dE);
+    P.dec = dec ? 1 : 0;
+    if (a.mlog) log_terms(P, part, (unsigned long long)P.ndraw);
   }
 }
 
@@ -1774,6 +1900,7 @@ __global__ void __maxnreg__(sizeof(Pos) == 4 ? 128 : 168) spec_kernel(KArgs a) {
               const ShortTangent T(a, sh, gs, cap);
               short_tangent_evaluate<LEAN>(a, sh, rep, T, B, c, bkeys, bmask);
               __syncthreads();
+              if (!LEAN && sh.ws.rd.twist) short_tangent_twist(a, sh, B, cap);
               short_tangent_conflicts(a, sh, T, B, bkeys, bmask);
               __syncthreads();
             }
