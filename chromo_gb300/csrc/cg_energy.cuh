@@ -140,13 +140,14 @@ __device__ __forceinline__ long long weight_at_limit(const RepDev& rd) {
 }
 
 // One CTA's part of a replica's voxels: f(voxel, row) for its thread's rows, or
-// (SKIP) for those of them that are not empty.
-template <bool SKIP, class F>
-__device__ __forceinline__ void for_each_row(const KArgs& a, const RepDev& rd, int rank, const F& f) {
+// (SKIP) for those of them that are not empty; g() after every kRowsInFlight.
+constexpr int kRowsInFlight = 4;
+template <bool SKIP, class F, class G>
+__device__ __forceinline__ void for_each_row(const KArgs& a, const RepDev& rd, int rank, const F& f, const G& g) {
   const long long* grid = a.grid + rd.vox_off * a.ncol;
   const long long per = (rd.n_vox + kSumCtas - 1) / kSumCtas;
   const long long v0 = rank * per, v1 = v0 + per < rd.n_vox ? v0 + per : rd.n_vox;
-  constexpr int U = 4;  // rows in flight per thread
+  constexpr int U = kRowsInFlight;
   for (long long v = v0 + threadIdx.x; v < v1; v += U * kSumThreads) {
     long long row[U][4];
 #pragma unroll
@@ -159,7 +160,12 @@ __device__ __forceinline__ void for_each_row(const KArgs& a, const RepDev& rd, i
     for (int u = 0; u < U; u++)
       if (SKIP ? (row[u][0] | row[u][1] | row[u][2] | row[u][3]) != 0 : v + u * kSumThreads < v1)
         f(v + u * kSumThreads, row[u]);
+    g();
   }
+}
+template <bool SKIP, class F>
+__device__ __forceinline__ void for_each_row(const KArgs& a, const RepDev& rd, int rank, const F& f) {
+  for_each_row<SKIP>(a, rd, rank, f, [] {});
 }
 
 // Non-uniform volumes: an empty voxel adds nothing, unless its volume is not
@@ -168,31 +174,131 @@ __device__ __forceinline__ bool empty_voxel(const KArgs& a, const RepDev& rd, lo
   return (row[0] | row[1] | row[2] | row[3]) == 0 && a.access_vol[rd.vox_off + v] > 0;
 }
 
-// Sums of products of the fixed-point columns over a replica's voxels
-// (uniform volumes): bead weight squared at or below the limit and above it,
-// binder columns squared and in pairs (01, 02, 12), and the FP64 volume
-// fractions above the limit.
-struct GridSums {
-  double s00, s00_over, sbb[CG_MAX_BINDERS], sx[3], vf_over;
+// Sum of products x y of fixed-point values 0 <= x, y < 2^52, exactly: of the
+// products of their 26-bit halves, sum ll + lh 2^26 + hh 2^52 (squares: lh holds
+// x_l x_h once).  Three or four 32 x 32 + 64-bit integer multiply-adds, where
+// FP64 takes two conversions and an FMA, each ~65 cycles of a quarter SM.  The
+// 64-bit sums hold kFxRows products.  40^3 voxels, two binders, with the
+// read-back: derivative terms of 64 replicas 124 -> 64 us, energies of 256
+// replicas 523 -> 327 us (held to 84 registers, 3 CTAs per SM instead of 2: 98
+// and 343 us).
+struct FxSum {
+  unsigned long long ll, lh, hh;
 };
-__device__ __forceinline__ void add_row(const RepDev& rd, long long gmax, const long long (&row)[4], GridSums& s) {
-  const double g0 = (double)row[0];
-  if (row[0] <= gmax) {
-    s.s00 = __fma_rn(g0, g0, s.s00);
-  } else {
-    s.s00_over = __fma_rn(g0, g0, s.s00_over);
-    s.vf_over += (g0 * kFxInv) / rd.vol_bin * rd.bead_vol;
-  }
-  double gb[CG_MAX_BINDERS] = {0, 0, 0};
+constexpr int kFxRows = 2048;  // lh of x y: two products below 2^52 each
+__device__ __forceinline__ void fx_split(long long x, unsigned& l, unsigned& h) {
+  l = (unsigned)x & 0x3FFFFFFu;
+  h = (unsigned)((unsigned long long)x >> 26);
+}
+__device__ __forceinline__ void fx_square(FxSum& s, unsigned l, unsigned h) {
+  s.ll += (unsigned long long)l * l;
+  s.lh += (unsigned long long)l * h;
+  s.hh += (unsigned long long)h * h;
+}
+__device__ __forceinline__ void fx_product(FxSum& s, unsigned l0, unsigned h0, unsigned l1, unsigned h1) {
+  s.ll += (unsigned long long)l0 * l1;
+  s.lh += (unsigned long long)l0 * h1;
+  s.lh += (unsigned long long)h0 * l1;
+  s.hh += (unsigned long long)h0 * h1;
+}
+// The sum in FP64 (one conversion, of its leading 64 bits); `shift` is 26, or 27
+// for squares.
+__device__ __forceinline__ double fx_value(const FxSum& s, int shift) {
+  unsigned long long lo = s.ll, hi = s.lh >> (64 - shift), t = s.lh << shift;
+  lo += t;
+  hi += lo < t ? 1 : 0;
+  t = s.hh << 52;
+  lo += t;
+  hi += (s.hh >> 12) + (lo < t ? 1 : 0);
+  const int z = hi ? __clzll((long long)hi) : 64;
+  const unsigned long long top = z == 64 ? lo : (z ? hi << z | lo >> (64 - z) : hi);
+  const double d = __ull2double_rn(top);
+  return z == 64 ? d : __longlong_as_double(__double_as_longlong(d) + ((long long)(64 - z) << 52));
+}
+
+// Sums of products of the fixed-point columns over a replica's voxels
+// (uniform volumes): bead weight squared at or below the limit, binder columns
+// squared and in pairs (01, 02, 12).  What the integer sums cannot hold -- a
+// column of 2^52 (4,096 beads in one voxel) or more, full 64-bit sums -- and the
+// rows above the limit go to FP64 sums in shared memory, a column per thread.
+struct GridSums {
+  FxSum s00, sbb[CG_MAX_BINDERS], sx[3];
+  int left;    // outer iterations until the 64-bit sums are emptied
+  bool rest;   // the FP64 sums are in use
+};
+enum { kRest00, kRestBB, kRestX = kRestBB + CG_MAX_BINDERS, kRestOver = kRestX + 3, kRestVf, kRests };
+typedef double RestSums[kRests][kSumThreads];
+
+__device__ __forceinline__ void init_sums(GridSums& s, RestSums& rest) {
+  s = GridSums{};
+  s.left = kFxRows / kRowsInFlight;
+  for (int k = 0; k < kRests; k++) rest[k][threadIdx.x] = 0.0;
+}
+// The integer sums as FP64, in the order of kRest00 .. kRestX + 2.
+template <class F>
+__device__ __forceinline__ void sum_values(const GridSums& s, int nb, const F& f) {
+  f(kRest00, fx_value(s.s00, 27));
 #pragma unroll
-  for (int b = 0; b < CG_MAX_BINDERS; b++)
-    if (row[1 + b]) {
-      gb[b] = (double)row[1 + b];
-      s.sbb[b] = __fma_rn(gb[b], gb[b], s.sbb[b]);
-    }
-  if (row[1] && row[2]) s.sx[0] = __fma_rn(gb[0], gb[1], s.sx[0]);
-  if (row[1] && row[3]) s.sx[1] = __fma_rn(gb[0], gb[2], s.sx[1]);
-  if (row[2] && row[3]) s.sx[2] = __fma_rn(gb[1], gb[2], s.sx[2]);
+  for (int b = 0; b < CG_MAX_BINDERS; b++) f(kRestBB + b, b < nb ? fx_value(s.sbb[b], 27) : 0.0);
+  f(kRestX, nb > 1 ? fx_value(s.sx[0], 26) : 0.0);
+  f(kRestX + 1, nb > 2 ? fx_value(s.sx[1], 26) : 0.0);
+  f(kRestX + 2, nb > 2 ? fx_value(s.sx[2], 26) : 0.0);
+}
+static __device__ __noinline__ void add_row_f64(RestSums& rest, long long gmax, double vol, double bead_vol,
+                                                long long r0, long long r1, long long r2, long long r3) {
+  const int t = threadIdx.x;
+  const double g0 = (double)r0, g[3] = {(double)r1, (double)r2, (double)r3};
+  double& s00 = rest[r0 <= gmax ? kRest00 : kRestOver][t];
+  s00 = __fma_rn(g0, g0, s00);
+  if (r0 > gmax) rest[kRestVf][t] += (g0 * kFxInv) / vol * bead_vol;
+  for (int b = 0; b < 3; b++) rest[kRestBB + b][t] = __fma_rn(g[b], g[b], rest[kRestBB + b][t]);
+  rest[kRestX][t] = __fma_rn(g[0], g[1], rest[kRestX][t]);
+  rest[kRestX + 1][t] = __fma_rn(g[0], g[2], rest[kRestX + 1][t]);
+  rest[kRestX + 2][t] = __fma_rn(g[1], g[2], rest[kRestX + 2][t]);
+}
+__device__ __forceinline__ void add_row(const RepDev& rd, long long gmax, const long long (&row)[4], GridSums& s,
+                                        RestSums& rest) {
+  if (row[0] > gmax || (unsigned long long)(row[0] | row[1] | row[2] | row[3]) >> 52) {
+    add_row_f64(rest, gmax, rd.vol_bin, rd.bead_vol, row[0], row[1], row[2], row[3]);
+    s.rest = true;
+    return;
+  }
+  unsigned l[4], h[4];
+#pragma unroll
+  for (int k = 0; k < 4; k++) fx_split(row[k], l[k], h[k]);
+  fx_square(s.s00, l[0], h[0]);
+  fx_square(s.sbb[0], l[1], h[1]);
+  if (rd.nb > 1) {
+    fx_square(s.sbb[1], l[2], h[2]);
+    fx_product(s.sx[0], l[1], h[1], l[2], h[2]);
+  }
+  if (rd.nb > 2) {
+    fx_square(s.sbb[2], l[3], h[3]);
+    fx_product(s.sx[1], l[1], h[1], l[3], h[3]);
+    fx_product(s.sx[2], l[2], h[2], l[3], h[3]);
+  }
+}
+// Called after every outer iteration: empties full integer sums.
+__device__ __forceinline__ void drain_sums(int nb, GridSums& s, RestSums& rest) {
+  if (--s.left) return;
+  sum_values(s, nb, [&](int k, double x) { rest[k][threadIdx.x] += x; });
+  s = GridSums{};
+  s.left = kFxRows / kRowsInFlight;
+  s.rest = true;
+}
+// The sums of one CTA's part of a replica: out[kRest00 .. kRestVf].
+__device__ __forceinline__ void grid_sums(const KArgs& a, const RepDev& rd, int rank, long long gmax, RestSums& rest,
+                                          double (&out)[kRests]) {
+  GridSums s;
+  init_sums(s, rest);
+  const int nb = rd.nb;
+  for_each_row<true>(a, rd, rank, [&](long long, const long long (&row)[4]) { add_row(rd, gmax, row, s, rest); },
+                     [&] { drain_sums(nb, s, rest); });
+  out[kRestOver] = out[kRestVf] = 0.0;
+  sum_values(s, nb, [&](int k, double x) { out[k] = x; });
+  if (s.rest)
+#pragma unroll
+    for (int k = 0; k < kRests; k++) out[k] += rest[k][threadIdx.x];
 }
 
 // Elastic energy of bond i - 1 -> i from the two beads' vectors in FP64.

@@ -230,6 +230,7 @@ __global__ void __cluster_dims__(kSumCtas, 1, 1) __launch_bounds__(kSumThreads)
     terms_kernel(KArgs a, double* terms, double* acc) {
   __shared__ double sh[kSumThreads / 32][16];
   __shared__ double T[16];
+  __shared__ RestSums rest;
   __shared__ long long gmax_sh;
   const int rep = blockIdx.x / kSumCtas, rank = blockIdx.x % kSumCtas;
   const RepDev& rd = a.reps[rep];
@@ -253,11 +254,9 @@ __global__ void __cluster_dims__(kSumCtas, 1, 1) __launch_bounds__(kSumThreads)
         }
     }
   }
-  GridSums g{};
-  double dens2 = 0;
+  double g[kRests] = {}, dens2 = 0;
   if (uniform) {
-    const long long gmax = gmax_sh;
-    for_each_row<true>(a, rd, rank, [&](long long, const long long (&row)[4]) { add_row(rd, gmax, row, g); });
+    grid_sums(a, rd, rank, gmax_sh, rest, g);
   } else if (field) {
     for_each_row<false>(a, rd, rank, [&](long long v, const long long (&row)[4]) {
       if (empty_voxel(a, rd, v, row)) return;
@@ -268,17 +267,17 @@ __global__ void __cluster_dims__(kSumCtas, 1, 1) __launch_bounds__(kSumThreads)
         if (b < rd.nb) rho[b] = ((double)row[1 + b] * kFxInv) / V;
       const double dens = ((double)row[0] * kFxInv) / V;
       const double vf = dens * rd.bead_vol;
-      if (vf <= rd.vf_limit) g.s00 += (V / rd.bead_vol) * vf * vf;
-      for (int b = 0; b < CG_MAX_BINDERS; b++) g.sbb[b] += rho[b] * rho[b];
-      g.sx[0] += rho[0] * rho[1];
-      g.sx[1] += rho[0] * rho[2];
-      g.sx[2] += rho[1] * rho[2];
+      if (vf <= rd.vf_limit) g[kRest00] += (V / rd.bead_vol) * vf * vf;
+      for (int b = 0; b < CG_MAX_BINDERS; b++) g[kRestBB + b] += rho[b] * rho[b];
+      g[kRestX + 0] += rho[0] * rho[1];
+      g[kRestX + 1] += rho[0] * rho[2];
+      g[kRestX + 2] += rho[1] * rho[2];
       dens2 += dens * dens;
     });
   }
-  double v[16] = {g.s00, g.sbb[0], g.sbb[1], g.sbb[2], g.sx[0], g.sx[1], g.sx[2], (double)dbl[0], (double)dbl[1],
-                  (double)dbl[2], (double)sum[0], (double)sum[1], (double)sum[2],
-                  uniform ? g.s00 + g.s00_over : dens2, 0.0, 0.0};
+  double v[16] = {g[kRest00], g[kRestBB], g[kRestBB + 1], g[kRestBB + 2], g[kRestX], g[kRestX + 1], g[kRestX + 2],
+                  (double)dbl[0], (double)dbl[1], (double)dbl[2], (double)sum[0], (double)sum[1], (double)sum[2],
+                  uniform ? g[kRest00] + g[kRestOver] : dens2, 0.0, 0.0};
   double t = cluster_sums(v, sh);
   if (rank != 0) return;
   if (threadIdx.x < kTerms) {

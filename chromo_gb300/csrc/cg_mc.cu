@@ -579,6 +579,7 @@ __global__ void __cluster_dims__(kSumCtas, 1, 1) __launch_bounds__(kSumThreads)
     energy_kernel(KArgs a, double* out) {
   __shared__ double sh[kSumThreads / 32][16];
   __shared__ double bf[CG_MAX_BINDERS * (CG_MAX_MARK + 1) * (CG_MAX_MARK + 1)];
+  __shared__ RestSums rest;
   __shared__ long long gmax_sh;
   const int rep = blockIdx.x / kSumCtas, rank = blockIdx.x % kSumCtas;
   const RepDev& rd = a.reps[rep];
@@ -590,18 +591,17 @@ __global__ void __cluster_dims__(kSumCtas, 1, 1) __launch_bounds__(kSumThreads)
   int dbl[CG_MAX_BINDERS] = {0, 0, 0};
   long long excess = 0;
   bead_sums<Pos>(a, rd, rank, bf, el, bi, dbl, excess);
-  GridSums g{};
+  double g[kRests] = {};
   EnergyParts p{0.0, 0.0, 0.0, 0.0, {0, 0, 0}};
   if (uniform) {
-    const long long gmax = gmax_sh;
-    for_each_row<true>(a, rd, rank, [&](long long, const long long (&row)[4]) { add_row(rd, gmax, row, g); });
+    grid_sums(a, rd, rank, gmax_sh, rest, g);
   } else if (field) {
     for_each_row<false>(a, rd, rank, [&](long long v, const long long (&row)[4]) {
       if (!empty_voxel(a, rd, v, row)) voxel_energy(a, rd, v, p);
     });
   }
-  double v[16] = {el, bi, uniform ? g.s00 : p.sx, uniform ? g.vf_over : p.fe, g.sbb[0], g.sbb[1], g.sbb[2],
-                  g.sx[0], g.sx[1], g.sx[2], (double)dbl[0], (double)dbl[1], (double)dbl[2], (double)excess, 0.0, 0.0};
+  double v[16] = {el, bi, uniform ? g[kRest00] : p.sx, uniform ? g[kRestVf] : p.fe, g[kRestBB], g[kRestBB + 1],
+                  g[kRestBB + 2], g[kRestX], g[kRestX + 1], g[kRestX + 2], (double)dbl[0], (double)dbl[1], (double)dbl[2], (double)excess, 0.0, 0.0};
   const double t = cluster_sums(v, sh);
   if (rank != 0 || threadIdx.x >= 32) return;
   double s[16];
@@ -643,10 +643,27 @@ __global__ void __cluster_dims__(kSumCtas, 1, 1) __launch_bounds__(kSumThreads)
   double sx = 0;
   if (uniform) {
     const long long gmax = gmax_sh;
-    for_each_row<true>(a, rd, rank, [&](long long, const long long (&row)[4]) {
-      const double g0 = (double)row[0];
-      if (row[0] <= gmax) sx = __fma_rn(g0, g0, sx);
-    });
+    FxSum s{};
+    int left = kFxRows / kRowsInFlight;
+    for_each_row<true>(
+        a, rd, rank,
+        [&](long long, const long long (&row)[4]) {
+          if (row[0] > gmax) return;
+          if ((unsigned long long)row[0] >> 52) {
+            sx = __fma_rn((double)row[0], (double)row[0], sx);
+            return;
+          }
+          unsigned l, h;
+          fx_split(row[0], l, h);
+          fx_square(s, l, h);
+        },
+        [&] {
+          if (--left) return;
+          sx += fx_value(s, 27);
+          s = FxSum{};
+          left = kFxRows / kRowsInFlight;
+        });
+    sx += fx_value(s, 27);
   } else if (field) {
     EnergyParts p{0.0, 0.0, 0.0, 0.0, {0, 0, 0}};
     for_each_row<false>(a, rd, rank, [&](long long v, const long long (&row)[4]) {
