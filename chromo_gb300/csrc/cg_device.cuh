@@ -409,6 +409,40 @@ __device__ __forceinline__ void axis_rotation(const Real a[3], const Real p[3], 
   axis_rotation_sc(a, p, s, c, M);
 }
 
+// FP64: a proposal's three sines and cosines (of the two sphere angles and the
+// rotation's) on three lanes of one sincos (1,730 cycles a warp, whatever its
+// lanes), and the rotation's rows one per lane.  Called by the whole warp.
+__device__ __forceinline__ void sphere_and_angle(unsigned xphi, unsigned xtheta, double ang, double v[3], double& s,
+                                                 double& c) {
+  const int lane = (int)(threadIdx.x & 31u);
+  const double phi = uni<double>(xphi) * (2.0 * 3.141592653589793);
+  const double theta = acos(uni<double>(xtheta) * 2 - 1);
+  double sn, cs;
+  sincos(lane == 0 ? phi : lane == 1 ? theta : ang, &sn, &cs);
+  const double st = __shfl_sync(0xFFFFFFFFu, sn, 1);
+  v[0] = __shfl_sync(0xFFFFFFFFu, cs, 0) * st;
+  v[1] = __shfl_sync(0xFFFFFFFFu, sn, 0) * st;
+  v[2] = __shfl_sync(0xFFFFFFFFu, cs, 1);
+  s = __shfl_sync(0xFFFFFFFFu, sn, 2);
+  c = __shfl_sync(0xFFFFFFFFu, cs, 2);
+}
+// Row j (0, 1, 2) of axis_rotation_sc's matrix, in the order of its columns
+// j, j + 1, j + 2 (mod 3) and the translation: the same operations on the same
+// values.
+__device__ __forceinline__ void rotation_row(const double a[3], const double p[3], double s, double c, int j,
+                                             double R[4]) {
+  auto pick = [](const double x[3], int k) { return k == 0 ? x[0] : k == 1 ? x[1] : x[2]; };
+  const int j1 = j == 2 ? 0 : j + 1, j2 = j == 0 ? 2 : j - 1;
+  const double u = pick(a, j), v = pick(a, j1), w = pick(a, j2);
+  const double pu = pick(p, j), pv = pick(p, j1), pw = pick(p, j2);
+  const double oc = 1 - c, uu = u * u;
+  R[0] = uu + (v * v + w * w) * c;
+  R[1] = u * v * oc - w * s;
+  R[2] = u * w * oc + v * s;
+  R[3] = (pv * w - pw * v) * s;
+  R[3] += (pu * (1 - uu) - u * (pv * v + pw * w)) * oc;
+}
+
 template <typename Pos, typename Real>
 __device__ __forceinline__ void ld3(const V4<Pos>* a, long long i, Real v[3]) {
   V4<Pos> q = a[i];
@@ -643,9 +677,7 @@ __device__ __forceinline__ double tangent_dE_rev(const Bond<double>& b, const do
 // is exact when it lies in [0, b), where it is the remainder (a multiple of the
 // smaller operand's last place below b), and has the right sign when it does
 // not, so one correction of q gives fmod's value bit for bit.  Other arguments
-// take fmod.  1,000 beads in FP64, 300 moves: 10.0 -> 9.7 ms with the voxel
-// widths of voxel_axes divided once on the host.  (The same for binary32 gave
-// nothing: 18.5 against 18.7 ms on 256 chains.)
+// take fmod.  (wrap_near is the same in integer steps.)
 __device__ __forceinline__ double pymod(double a, double b) {
   if (a >= 0 && a < b) return a;  // fmod(a, b) == a exactly here
   const double x = fabs(a);
@@ -669,51 +701,150 @@ __device__ __forceinline__ float pymodf(float a, float b) {
   return m;
 }
 
+// ---------------------------------------------------------------- FP64 in integer steps
+// An FP64 operation of a warp holds its quarter of the SM for ~60 cycles, and so
+// does a conversion from or to FP64, a comparison or a rounding (70); a division
+// is nine of them.  The steps below that need no rounding work on the words of
+// the numbers instead, with the same results (1,000 beads in FP64, 300 moves,
+// kernel only: 6.65 -> 5.91 ms with the sines and rotation rows on lanes, 5.08
+// with the deposit's axes on lanes too).
+
+// (double)n for n >= 0.
+__device__ __forceinline__ double whole_double(int n) {
+  const int z = __clz(n) & 31;
+  const unsigned m = (unsigned)n << z;  // leading one at bit 31
+  const double d = __hiloint2double((1023 + 31 - z) << 20 | (int)((m << 1) >> 12), (int)(m << 21));
+  return n ? d : 0.0;
+}
+// floor(x) for -1 < x < 2^31.
+__device__ __forceinline__ int floor_index(double x) {
+  const int hi = __double2hiint(x), lo = __double2loint(x);
+  const int e = ((hi >> 20) & 0x7FF) - 1023;
+  const unsigned long long m = (unsigned long long)(unsigned)((hi & 0xFFFFF) | 0x100000) << 32 | (unsigned)lo;
+  const int t = e < 0 ? 0 : (int)(m >> ((52 - e) & 63));
+  return hi < 0 && ((hi & 0x7FFFFFFF) | lo) ? -1 : t;
+}
+// (double)g * kFxInv, a fixed-point value in FP64.
+__device__ __forceinline__ double fx_double(long long g) {
+  const unsigned long long u = g < 0 ? 0ull - (unsigned long long)g : (unsigned long long)g;
+  if (u >> 53) return (double)g * kFxInv;
+  const int z = __clzll((long long)u) & 63;
+  const unsigned long long m = u << z;  // leading one at bit 63
+  const unsigned long long d = (unsigned long long)(1023 + 63 - 40 - z) << 52 | (m << 1) >> 12 |
+                               (g < 0 ? 1ull << 63 : 0ull);
+  return u ? __longlong_as_double((long long)d) : 0.0;
+}
+// x / b, correctly rounded, for inv = 1 / b correctly rounded (0: divide): two
+// steps of q + inv (x - b q) with the remainder in one FMA, the first to within
+// one unit in the last place, the second exact (Markstein 1990).  x and x / b
+// away from the ends of the FP64 range.
+__device__ __forceinline__ double quotient(double x, double b, double inv) {
+  if (is_zero64(inv)) return x / b;
+  double q = x * inv;
+  q = __fma_rn(__fma_rn(-b, q, x), inv, q);
+  return __fma_rn(__fma_rn(-b, q, x), inv, q);
+}
+// A number that quotient() takes as b: within 10^+-100.
+__device__ __forceinline__ double inverse_or_zero(double b) { return b > 1e-100 && b < 1e100 ? 1.0 / b : 0.0; }
+
+// m = a mod w (Python's rule) in [0, w] for w in (1e-30, 1e30) and |a| < 2^20 w;
+// false elsewhere.  As pymod: an FP32 quotient within one of the quotient, the
+// remainder in one FMA, one correction.  iw: 1 / w.
+__device__ __forceinline__ bool wrap_near(double a, double w, float iw, double& m) {
+  const unsigned long long bw = (unsigned long long)__double_as_longlong(w);
+  const unsigned long long bx = (unsigned long long)__double_as_longlong(a) & 0x7FFFFFFFFFFFFFFFull;
+  const bool near = bw > (unsigned long long)__double_as_longlong(1e-30) &&
+                    bw < (unsigned long long)__double_as_longlong(1e30) && bx < bw + (20ull << 52);
+  if (!near) return false;
+  const double x = __longlong_as_double((long long)bx);
+  const int hx = __double2hiint(x);
+  // |a| in FP32, rounded down (0 below 2^-126)
+  const float xf = hx < 0x38100000 ? 0.0f : __int_as_float((hx - 0x38000000) << 3 | (int)((unsigned)__double2loint(x) >> 29));
+  const int q = (int)(xf * iw);
+  double r = __fma_rn(-whole_double(q), w, x);
+  const long long br = __double_as_longlong(r);
+  const int fix = br < 0 && (br << 1) != 0 ? -1 : (br >= (long long)bw ? 1 : 0);
+  if (fix) r = __fma_rn(-whole_double(q + fix), w, x);
+  m = r;
+  if (__double2hiint(a) < 0 && (__double_as_longlong(r) << 1) != 0) m = w - r;
+  return true;
+}
+
 // FP32 copies of the grid geometry, derived once per launch
 struct GridF {
+  double inv_dd[3];  // 1 / d (FP64 storage)
   float w[3], inv_w[3], half_w[3], half_d[3], inv_d[3];
   float sw[3], inv_sw[3], nsub[3], half_np;  // fast_field sub-bins (FP32 storage)
   int n[3], nx, nxy;
 };
 
-__device__ __forceinline__ void make_gridf(const RepDev& rd, GridF& gf) {
-  const double W[3] = {rd.wx, rd.wy, rd.wz};
-  const int n[3] = {rd.nx, rd.ny, rd.nz};
-  for (int j = 0; j < 3; j++) {
-    double d = W[j] / (double)n[j];
-    gf.w[j] = (float)W[j];
-    gf.inv_w[j] = (float)(1.0 / W[j]);
-    gf.half_w[j] = (float)(0.5 * W[j]);
-    gf.half_d[j] = (float)(0.5 * d);
-    gf.inv_d[j] = (float)(1.0 / d);
-    gf.n[j] = n[j];
-    const int np = rd.fast_n > 0 ? rd.fast_n : 1;
-    gf.sw[j] = (float)(d / (double)np);
-    gf.inv_sw[j] = (float)((double)np / d);
-    gf.nsub[j] = (float)((double)np * n[j]);
-  }
+__device__ __forceinline__ void make_gridf_axis(const RepDev& rd, GridF& gf, int j) {
+  const double W = j == 0 ? rd.wx : j == 1 ? rd.wy : rd.wz;
+  const int n = j == 0 ? rd.nx : j == 1 ? rd.ny : rd.nz;
+  const double d = W / (double)n;
+  gf.w[j] = (float)W;
+  gf.inv_w[j] = (float)(1.0 / W);
+  gf.half_w[j] = (float)(0.5 * W);
+  gf.half_d[j] = (float)(0.5 * d);
+  gf.inv_dd[j] = inverse_or_zero(d);
+  gf.inv_d[j] = (float)(1.0 / d);
+  gf.n[j] = n;
+  const int np = rd.fast_n > 0 ? rd.fast_n : 1;
+  gf.sw[j] = (float)(d / (double)np);
+  gf.inv_sw[j] = (float)((double)np / d);
+  gf.nsub[j] = (float)((double)np * n);
+}
+__device__ __forceinline__ void make_gridf_rest(const RepDev& rd, GridF& gf) {
   gf.half_np = (float)(0.5 * (rd.fast_n > 0 ? rd.fast_n : 1));
   gf.nx = rd.nx;
   gf.nxy = rd.nx * rd.ny;
 }
+__device__ __forceinline__ void make_gridf(const RepDev& rd, GridF& gf) {
+  for (int j = 0; j < 3; j++) make_gridf_axis(rd, gf, j);
+  make_gridf_rest(rd, gf);
+}
 
-// Per axis: the lower and upper voxel of a bead and the lower voxel's weight
-// (fields.pyx:1524-1673).  Exact reference arithmetic (FP64 storage).
-__device__ __forceinline__ void voxel_axes(const RepDev& rd, const GridF&, const double pos[3],
+// The quotient x / d of the coordinate p and its floor, by the reference's
+// arithmetic: for coordinates and boxes that wrap_near leaves out.
+struct AxisQuotient {
+  double q, fl;
+};
+static __device__ __noinline__ AxisQuotient axis_quotient(double p, double w, double d) {
+  const double x = pymod(p + 0.5 * w, w) - 0.5 * d;
+  return AxisQuotient{x / d, floor(x / d)};
+}
+
+// One axis: the lower and upper voxel of a bead's coordinate p and the lower
+// voxel's weight (fields.pyx:1524-1673), box width w, n voxels of d (iw, id: 1 / w,
+// 1 / d).  Exact reference arithmetic (FP64 storage), bound by the FP64 pipe: ~11
+// operations by the integer steps above, up to 40 with conversions, comparisons
+// and a division.
+__device__ __forceinline__ double voxel_axis(double p, double w, double d, float iw, double id, int n, int& lo,
+                                             int& hi) {
+  double q, m, wl;
+  int ind;
+  if (wrap_near(p + 0.5 * w, w, iw, m)) {
+    q = quotient(m - 0.5 * d, d, id);
+    ind = floor_index(q);  // -1/2 <= q < n
+    wl = 1 - (q - (ind < 0 ? -1.0 : whole_double(ind)));
+  } else {
+    const AxisQuotient t = axis_quotient(p, w, d);
+    const long long l = (long long)t.fl;
+    ind = (int)l;
+    wl = 1 - (t.q - (double)l);
+  }
+  const int li = ind == -1 ? n - 1 : ind;
+  lo = li < 0 ? 0 : (li >= n ? n - 1 : li);  // in range for finite x; guards the rest
+  hi = lo + 1 == n ? 0 : lo + 1;
+  return wl;
+}
+__device__ __forceinline__ void voxel_axes(const RepDev& rd, const GridF& gf, const double pos[3],
                                            double wl[3], int lo[3], int hi[3]) {
   const double width[3] = {rd.wx, rd.wy, rd.wz};
   const double dxyz[3] = {rd.dx, rd.dy, rd.dz};  // width / n, divided on the host
-  const int n[3] = {rd.nx, rd.ny, rd.nz};
 #pragma unroll
-  for (int j = 0; j < 3; j++) {
-    const double d = dxyz[j];
-    double x = pymod(pos[j] + 0.5 * width[j], width[j]) - 0.5 * d;
-    long long ind = (long long)floor(x / d);
-    int li = ind == -1 ? n[j] - 1 : (int)ind;
-    lo[j] = li < 0 ? 0 : (li >= n[j] ? n[j] - 1 : li);  // in range for finite x; guards the rest
-    hi[j] = lo[j] + 1 == n[j] ? 0 : lo[j] + 1;
-    wl[j] = 1 - (x / d - (double)ind);
-  }
+  for (int j = 0; j < 3; j++)
+    wl[j] = voxel_axis(pos[j], width[j], dxyz[j], gf.inv_w[j], gf.inv_dd[j], gf.n[j], lo[j], hi[j]);
 }
 
 // FP32 arithmetic (FP32 storage): same construction, one reciprocal multiply.

@@ -24,6 +24,7 @@ struct WarpShared {
   float f_vb;     // bead volume
   float f_k;      // chi * vol_bin / bead volume
   float f_lim;    // vf_limit
+  double d_inv_vol, d_k;  // FP64 storage: 1 / vol_bin (0: divide), chi * (vol_bin / bead volume)
   // FP32 copies of the binding constants: free energy table, effective
   // chemical potential (mu (2 - f) for mu > 0, else mu f), intranucleosome term
   float f_bind[CG_MAX_BINDERS * (CG_MAX_MARK + 1) * (CG_MAX_MARK + 1)];

@@ -544,7 +544,8 @@ __global__ void deposit_kernel(KArgs a, int rep_only) {
   const V4<Pos>* r4 = reinterpret_cast<const V4<Pos>*>(a.r4) + rd.bead_off;
   long long* grid = a.grid + rd.vox_off * a.ncol;
   __shared__ GridF gf;  // once per CTA: its FP64 divisions took longer than the beads
-  if (threadIdx.x == 0) make_gridf(rd, gf);
+  if (threadIdx.x < 3) make_gridf_axis(rd, gf, threadIdx.x);
+  if (threadIdx.x == 3) make_gridf_rest(rd, gf);
   __syncthreads();
   for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < rd.n_beads;
        i += (long long)gridDim.x * blockDim.x) {

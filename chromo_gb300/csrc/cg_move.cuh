@@ -8,7 +8,7 @@
 
 namespace cg {
 
-// FP32 copies of a replica's field and binding constants (one thread).
+// Copies of a replica's field and binding constants (one thread).
 __device__ __forceinline__ void setup_f32(WarpShared& ws) {
   const RepDev& rd = ws.rd;
   make_gridf(rd, ws.gf);
@@ -16,8 +16,10 @@ __device__ __forceinline__ void setup_f32(WarpShared& ws) {
   for (int b = 0; b < CG_MAX_BINDERS * CG_MAX_BINDERS; b++) ws.f_xpref[b] = (float)rd.xpref[b];
   ws.f_scale = (float)(kFxInv / rd.vol_bin);
   ws.f_vb = (float)rd.bead_vol;
-  ws.f_k = (float)(rd.chi * (rd.vol_bin / rd.bead_vol));
+  ws.d_k = rd.chi * (rd.vol_bin / rd.bead_vol);
+  ws.f_k = (float)ws.d_k;
   ws.f_lim = (float)rd.vf_limit;
+  ws.d_inv_vol = inverse_or_zero(rd.vol_bin);
   for (int i = 0; i < CG_MAX_BINDERS * (CG_MAX_MARK + 1) * (CG_MAX_MARK + 1); i++)
     ws.f_bind[i] = (float)rd.bind_f[i];
   for (int b = 0; b < CG_MAX_BINDERS; b++) {
@@ -273,21 +275,39 @@ __device__ __forceinline__ double with_huge(double hard, long long huge) {
   return huge != 0 ? hard_with_huge(hard, huge) : hard;
 }
 
+// The same for FP64 storage with the factors at hand: inv = 1 / V (0: divide),
+// k = chi (V / V_bead).
+__device__ __forceinline__ ChiSplit chi_term(const RepDev& rd, double V, double inv, double k, long long g0,
+                                             long long d0) {
+  const double vf0 = quotient(fx_double(g0), V, inv) * rd.bead_vol;
+  const double vf1 = quotient(fx_double(g0 + d0), V, inv) * rd.bead_vol;
+  if (vf1 > rd.vf_limit || vf0 > rd.vf_limit) return chi_term64(rd, V, g0, d0);
+  return ChiSplit{k * ((vf1 - vf0) * (vf1 + vf0)), 0};
+}
+
 // Field dE of one touched voxel v (grid row `row`) in FP64 arithmetic (row `d` of a voxel
 // table: the move's density deltas in, the voxel's post-move row out): added
 // to `part`; the 1e99 penalty of a voxel above vf_limit to `huge` (kHugeUnit
-// units).
-__device__ __forceinline__ void voxel_dE_f64(const RepDev& rd, const KArgs& a, const long long (&row)[4], int v,
+// units).  Bound by the FP64 pipe: ~35 operations with one binder, by the
+// integer steps of cg_device.cuh (76 with conversions and divisions); cross
+// terms with a zero coefficient are left out.
+__device__ __forceinline__ void voxel_dE_f64(const WarpShared& ws, const KArgs& a, const long long (&row)[4], int v,
                                              long long* d, bool split, double& part, long long& huge) {
+  const RepDev& rd = ws.rd;
   long long g0 = row[0], d0 = hash_delta(d, split);
-  double V = rd.has_access ? a.access_vol[rd.vox_off + v] : rd.vol_bin;
+  double V = rd.vol_bin, inv = ws.d_inv_vol, k = ws.d_k;
+  if (rd.has_access) {
+    V = a.access_vol[rd.vox_off + v];
+    inv = 0.0;
+    k = rd.chi * (V / rd.bead_vol);
+  }
   double c = 0, rho[CG_MAX_BINDERS], dd[CG_MAX_BINDERS];
 #pragma unroll
   for (int b = 0; b < CG_MAX_BINDERS; b++) {
     if (b >= rd.nb) break;
     long long gb = row[1 + b], db = hash_delta(d + 1 + b, split);
-    rho[b] = ((double)gb * kFxInv) / V;
-    dd[b] = ((double)db * kFxInv) / V;
+    rho[b] = quotient(fx_double(gb), V, inv);
+    dd[b] = quotient(fx_double(db), V, inv);
     c += rd.pref[b] * (dd[b] * (2 * rho[b] + dd[b]));
     d[1 + b] = gb + db;
   }
@@ -295,9 +315,9 @@ __device__ __forceinline__ void voxel_dE_f64(const RepDev& rd, const KArgs& a, c
   for (int b = 0; b < CG_MAX_BINDERS; b++)
 #pragma unroll
     for (int e = 0; e < CG_MAX_BINDERS; e++)
-      if (b < rd.nb && e < rd.nb)
+      if (b < rd.nb && e < rd.nb && !is_zero64(rd.xpref[b * CG_MAX_BINDERS + e]))
         c += rd.xpref[b * CG_MAX_BINDERS + e] * (rho[b] * dd[e] + dd[b] * rho[e] + dd[b] * dd[e]);
-  const ChiSplit t = chi_term64(rd, V, g0, d0);
+  const ChiSplit t = chi_term(rd, V, inv, k, g0, d0);
   c += t.soft;
   huge += t.huge;
   d[0] = g0 + d0;
@@ -324,7 +344,7 @@ static __device__ void field_dE_voxels(const WarpShared& ws, const KArgs& a, int
     const int slot = used[i], v = keys[slot];
     long long row[4];
     load_row(grid + (long long)v * a.ncol, a.ncol, row);
-    voxel_dE_f64(rd, a, row, v, vals + (long long)slot * hcol, split, part, hpart);
+    voxel_dE_f64(ws, a, row, v, vals + (long long)slot * hcol, split, part, hpart);
   }
   n_vox = nused;
   (void)soft;

@@ -388,95 +388,196 @@ __device__ void block_deposit(const KArgs& a, SpecShared& sh, int rep, int B, in
     if (lane >= o) end += y;
   }
   const int total = __shfl_sync(kFull, end, 31);
+  // One lane's two corners of a bead of move t (-1: none) with states inf.
+  auto corner_pass = [&](const BeadCells<Pos>& d, int t, unsigned inf) {
+    const int tt = t < 0 ? 0 : t;
+    MovePlan& P = sh.plan[tt];
+    const bool act = t >= 0 && !(P.derr & E_OVF);
+    unsigned char* wb = smem + a.spec_off_warps + (size_t)tt * a.warp_smem;
+    int vq[2 * kCornersPerLane];
+    long long q[2 * kCornersPerLane];
+    corner_terms(gf, d, lane % kLanesPerBead, vq, q);
+    // the pooled table (one used list for the whole CTA, keys voxel * 32 +
+    // slot), or the move's own table (one used list per move)
+    int* keys = reinterpret_cast<int*>(pool ? smem + a.off_pkeys : wb + a.off_keys);
+    int* used = reinterpret_cast<int*>(wb + a.off_used);
+    unsigned short* pu = reinterpret_cast<unsigned short*>(smem + a.off_pused);
+    long long* vals = reinterpret_cast<long long*>(pool ? smem + a.off_pvals : wb + a.off_vals);
+    bool want[2 * kCornersPerLane];
+#pragma unroll
+    for (int j = 0; j < 2 * kCornersPerLane; j++) {
+      want[j] = act && q[j] != 0;
+      if (pool) vq[j] = vq[j] * 32 + tt;
+    }
+    const bool sure = P.sure && !pool;
+    const unsigned full_bit = sure ? E_SPIN : E_OVF;
+    const int lh = pool ? a.pool_logH : a.logH;
+    int slot[2 * kCornersPerLane];
+    unsigned e = 0;
+    if (pool)
+      claim_slots<2 * kCornersPerLane>(keys, pu, &sh.npool, lh, vq, want, slot, e, (3 << lh) / 4, full_bit);
+    else
+      claim_slots<2 * kCornersPerLane>(keys, used, &sh.nused[tt], lh, vq, want, slot, e,
+                                       sure ? Hs : (3 << lh) / 4, full_bit);
+    if (!(e & full_bit)) {
+#pragma unroll
+      for (int j = 0; j < 2 * kCornersPerLane; j++)
+        if (want[j]) add_corner(vals, hcol, slot[j], q[j], inf, rd.nb, true);
+    }
+    if (e && t >= 0) atomicOr(&P.derr, e);
+  };
   // warps of the beads: all, without those of an SSTWLC batch's bonds (below)
   // where at least half remain
   const bool twist = !LEAN && cv.twist != nullptr;
   const int tws = twist ? (4 * B + 31) >> 5 : 0, WD = 2 * tws <= W ? W - tws : W;
-  // beads per warp and round: an even share, in whole passes of the corners
   constexpr int BP = 32 / kLanesPerBead;
-  // (by steps: a batch has a few hundred beads)
-  int per = WD;  // warps times rounds
-  while (32 * per < total) per += WD;
-  int run = BP;
-  while (run * per < total) run += BP;
-  #pragma unroll 1
-  for (int b0 = warp < WD ? warp * run : total; b0 < total; b0 += WD * run) {
-    const int b = b0 + lane;
-    // the bead's move: the number of moves whose beads end at or before b
-    int s = 0;
+  if constexpr (sizeof(Pos) == 8) {
+    // FP64 holds its pipe for ~60 cycles an operation whatever the number of
+    // lanes, so the four lanes of a bead take an axis each (the fourth repeats
+    // the third's), 8 beads a warp and pass: one row of the transform, one
+    // coordinate's cells.
     #pragma unroll 1
-    for (int j = 0; j < B; j++) s += __shfl_sync(kFull, end, j) <= b ? 1 : 0;
-    int base = __shfl_sync(kFull, end, s > 0 ? s - 1 : 0);
-    if (s == 0) base = 0;
-    bool on = lane < run && b < total;
-    if (!on) s = 0;
-    BeadCells<Pos> c;
-    c.v0 = c.v1 = 0;
-    c.wrap0 = c.wrap1 = 0;
-    for (int j = 0; j < 3; j++) c.wl0[j] = c.wl1[j] = 0;
-    unsigned info = 0;  // states (three bytes), wrap bits of the cells before and after
-    if (on) {
+    for (int b0 = warp < WD ? warp * BP : total; b0 < total; b0 += WD * BP) {
+      const int b = b0 + (lane >> 2), quad = lane & 28, ax = lane & 3, j = ax < 3 ? ax : 2;
+      int s = 0;
+      #pragma unroll 1
+      for (int u = 0; u < B; u++) s += __shfl_sync(kFull, end, u) <= b ? 1 : 0;
+      int base = __shfl_sync(kFull, end, s > 0 ? s - 1 : 0);
+      if (s == 0) base = 0;
+      bool on = b < total;
+      if (!on) s = 0;
       MovePlan& P = sh.plan[s];
-      const long long k = b - base, i = P.ind0 + k;
-      Pos M[3][4];
-      load_transform(P, M);
-      V4<Pos>* stage = P.gstage ? reinterpret_cast<V4<Pos>*>(a.g_stage) +
-                                      ((long long)rep * a.spec_s + s) * a.g_stage_cap * 3
-                                : reinterpret_cast<V4<Pos>*>(smem + a.spec_off_warps + (size_t)s * a.warp_smem +
-                                                             a.off_stage);
-      const unsigned sw = cv.st[i];
-      unsigned e = 0;
-      int oob;
-      on = place_bead<Pos, LEAN>(rd, gf, cv, kind, M, i, stage + 3 * k, true, conf, c, e, oob);
-      info = (sw & 0xFFFFFFu) | c.wrap0 << 24 | c.wrap1 << 27;
-      if (oob) atomicAdd(&P.oob, oob);
-      if (e) atomicOr(&P.derr, e);
+      double r[3] = {0, 0, 0}, tr = 0;
+      unsigned sw = 0;
+      if (on) {
+        const long long k = b - base, i = P.ind0 + k;
+        double* stage = reinterpret_cast<double*>(
+            (P.gstage ? reinterpret_cast<V4<Pos>*>(a.g_stage) + ((long long)rep * a.spec_s + s) * a.g_stage_cap * 3
+                      : reinterpret_cast<V4<Pos>*>(smem + a.spec_off_warps + (size_t)s * a.warp_smem + a.off_stage)) +
+            3 * k);
+        const double* M = reinterpret_cast<const double*>(P.M) + 4 * j;
+        sw = cv.st[i];
+        ld3(cv.r4, i, r);
+        if (kind == CG_SLIDE) {  // a slide's commit writes positions only
+          tr = (j == 0 ? r[0] : j == 1 ? r[1] : r[2]) + M[3];
+        } else {
+          double t3[3], t2[3];
+          ld3(cv.t34, i, t3);
+          ld3(cv.t24, i, t2);
+          tr = M[0] * r[0] + M[1] * r[1] + M[2] * r[2] + M[3];
+          const double tt3 = M[0] * t3[0] + M[1] * t3[1] + M[2] * t3[2];
+          const double tt2 = M[0] * t2[0] + M[1] * t2[1] + M[2] * t2[2];
+          stage[4 + ax] = ax < 3 ? tt3 : 0.0;
+          stage[8 + ax] = ax < 3 ? tt2 : 0.0;
+        }
+        stage[ax] = ax < 3 ? tr : 0.0;
+      }
+      const unsigned bad = __ballot_sync(kFull, !isfinite(tr)) >> quad & 15u;
+      const bool fast = !LEAN && rd.fast_n > 0;
+      double t[3] = {0, 0, 0};
+      if (conf || fast)
+        for (int q = 0; q < 3; q++) t[q] = __shfl_sync(kFull, tr, quad + q);
+      if (conf && on && ax == 0) {
+        const int oob = out_of_bounds(rd, t, true) * 65536 + out_of_bounds(rd, r, false);
+        if (oob) atomicAdd(&P.oob, oob);
+      }
+      if (bad) {
+        if (ax == 0) atomicOr(&P.derr, (unsigned)E_NONFINITE);
+        on = false;
+        tr = 0;
+      }
+      double w0, w1;
+      int lo0, hi0, lo1, hi1;
+      if (fast) {
+        if (bad) t[0] = t[1] = t[2] = 0;
+        double wa[3], wb[3];
+        int la[3], ha[3], lb[3], hb[3];
+        fast_axes_ool(rd, gf, r, wa, la, ha);
+        fast_axes_ool(rd, gf, t, wb, lb, hb);
+        w0 = j == 0 ? wa[0] : j == 1 ? wa[1] : wa[2];
+        w1 = j == 0 ? wb[0] : j == 1 ? wb[1] : wb[2];
+        lo0 = j == 0 ? la[0] : j == 1 ? la[1] : la[2];
+        lo1 = j == 0 ? lb[0] : j == 1 ? lb[1] : lb[2];
+        hi0 = j == 0 ? ha[0] : j == 1 ? ha[1] : ha[2];
+        hi1 = j == 0 ? hb[0] : j == 1 ? hb[1] : hb[2];
+      } else {
+        const double w = *(j == 0 ? &rd.wx : j == 1 ? &rd.wy : &rd.wz), d = *(j == 0 ? &rd.dx : j == 1 ? &rd.dy : &rd.dz);
+        const float iw = gf.inv_w[j];
+        const double id = gf.inv_dd[j];
+        const int n = gf.n[j];
+        w0 = voxel_axis(j == 0 ? r[0] : j == 1 ? r[1] : r[2], w, d, iw, id, n, lo0, hi0);
+        w1 = voxel_axis(tr, w, d, iw, id, n, lo1, hi1);
+      }
+      const int stride = ax == 0 ? 1 : ax == 1 ? gf.nx : ax == 2 ? gf.nxy : 0;
+      BeadCells<Pos> c;
+      c.v0 = lo0 * stride;
+      c.v1 = lo1 * stride;
+#pragma unroll
+      for (int o = 1; o <= 2; o <<= 1) {
+        c.v0 += __shfl_xor_sync(kFull, c.v0, o);
+        c.v1 += __shfl_xor_sync(kFull, c.v1, o);
+      }
+      c.wrap0 = __ballot_sync(kFull, hi0 == 0) >> quad & 7u;
+      c.wrap1 = __ballot_sync(kFull, hi1 == 0) >> quad & 7u;
+#pragma unroll
+      for (int q = 0; q < 3; q++) {
+        c.wl0[q] = __shfl_sync(kFull, w0, quad + q);
+        c.wl1[q] = __shfl_sync(kFull, w1, quad + q);
+      }
+      corner_pass(c, on ? s : -1, sw & 0xFFFFFFu);
     }
-    const int sl = on ? s : -1;
-    const int left = total - b0 < run ? total - b0 : run;
+  } else {
+    // beads per warp and round: an even share, in whole passes of the corners
+    // (by steps: a batch has a few hundred beads)
+    int per = WD;  // warps times rounds
+    while (32 * per < total) per += WD;
+    int run = BP;
+    while (run * per < total) run += BP;
     #pragma unroll 1
-    for (int p = 0; p < left; p += BP) {
-      const int src = p + lane / kLanesPerBead;
-      unsigned inf;
-      BeadCells<Pos> d = shfl_cells(c, info, src, inf);
-      const int t = __shfl_sync(kFull, sl, src);
-      d.wrap0 = (inf >> 24) & 7u;
-      d.wrap1 = (inf >> 27) & 7u;
-      const int tt = t < 0 ? 0 : t;
-      MovePlan& P = sh.plan[tt];
-      const bool act = t >= 0 && !(P.derr & E_OVF);
-      unsigned char* wb = smem + a.spec_off_warps + (size_t)tt * a.warp_smem;
-      int vq[2 * kCornersPerLane];
-      long long q[2 * kCornersPerLane];
-      corner_terms(gf, d, lane % kLanesPerBead, vq, q);
-      // the pooled table (one used list for the whole CTA, keys voxel * 32 +
-      // slot), or the move's own table (one used list per move)
-      int* keys = reinterpret_cast<int*>(pool ? smem + a.off_pkeys : wb + a.off_keys);
-      int* used = reinterpret_cast<int*>(wb + a.off_used);
-      unsigned short* pu = reinterpret_cast<unsigned short*>(smem + a.off_pused);
-      long long* vals = reinterpret_cast<long long*>(pool ? smem + a.off_pvals : wb + a.off_vals);
-      bool want[2 * kCornersPerLane];
-#pragma unroll
-      for (int j = 0; j < 2 * kCornersPerLane; j++) {
-        want[j] = act && q[j] != 0;
-        if (pool) vq[j] = vq[j] * 32 + tt;
+    for (int b0 = warp < WD ? warp * run : total; b0 < total; b0 += WD * run) {
+      const int b = b0 + lane;
+      // the bead's move: the number of moves whose beads end at or before b
+      int s = 0;
+      #pragma unroll 1
+      for (int j = 0; j < B; j++) s += __shfl_sync(kFull, end, j) <= b ? 1 : 0;
+      int base = __shfl_sync(kFull, end, s > 0 ? s - 1 : 0);
+      if (s == 0) base = 0;
+      bool on = lane < run && b < total;
+      if (!on) s = 0;
+      BeadCells<Pos> c;
+      c.v0 = c.v1 = 0;
+      c.wrap0 = c.wrap1 = 0;
+      for (int j = 0; j < 3; j++) c.wl0[j] = c.wl1[j] = 0;
+      unsigned info = 0;  // states (three bytes), wrap bits of the cells before and after
+      if (on) {
+        MovePlan& P = sh.plan[s];
+        const long long k = b - base, i = P.ind0 + k;
+        Pos M[3][4];
+        load_transform(P, M);
+        V4<Pos>* stage = P.gstage ? reinterpret_cast<V4<Pos>*>(a.g_stage) +
+                                        ((long long)rep * a.spec_s + s) * a.g_stage_cap * 3
+                                  : reinterpret_cast<V4<Pos>*>(smem + a.spec_off_warps + (size_t)s * a.warp_smem +
+                                                               a.off_stage);
+        const unsigned sw = cv.st[i];
+        unsigned e = 0;
+        int oob;
+        on = place_bead<Pos, LEAN>(rd, gf, cv, kind, M, i, stage + 3 * k, true, conf, c, e, oob);
+        info = (sw & 0xFFFFFFu) | c.wrap0 << 24 | c.wrap1 << 27;
+        if (oob) atomicAdd(&P.oob, oob);
+        if (e) atomicOr(&P.derr, e);
       }
-      const bool sure = P.sure && !pool;
-      const unsigned full_bit = sure ? E_SPIN : E_OVF;
-      const int lh = pool ? a.pool_logH : a.logH;
-      int slot[2 * kCornersPerLane];
-      unsigned e = 0;
-      if (pool)
-        claim_slots<2 * kCornersPerLane>(keys, pu, &sh.npool, lh, vq, want, slot, e, (3 << lh) / 4, full_bit);
-      else
-        claim_slots<2 * kCornersPerLane>(keys, used, &sh.nused[tt], lh, vq, want, slot, e,
-                                         sure ? Hs : (3 << lh) / 4, full_bit);
-      if (!(e & full_bit)) {
-#pragma unroll
-        for (int j = 0; j < 2 * kCornersPerLane; j++)
-          if (want[j]) add_corner(vals, hcol, slot[j], q[j], inf, rd.nb, true);
+      const int sl = on ? s : -1;
+      const int left = total - b0 < run ? total - b0 : run;
+      #pragma unroll 1
+      for (int p = 0; p < left; p += BP) {
+        const int src = p + lane / kLanesPerBead;
+        unsigned inf;
+        BeadCells<Pos> d = shfl_cells(c, info, src, inf);
+        const int t = __shfl_sync(kFull, sl, src);
+        d.wrap0 = (inf >> 24) & 7u;
+        d.wrap1 = (inf >> 27) & 7u;
+        corner_pass(d, t, inf);
       }
-      if (e && t >= 0) atomicOr(&P.derr, e);
     }
   }
   // boundary bonds of the moves, two per move
@@ -514,7 +615,7 @@ __device__ __forceinline__ void pool_voxel_dE(const WarpShared& ws, const KArgs&
 }
 __device__ __forceinline__ void pool_voxel_dE(const WarpShared& ws, const KArgs& a, const long long (&row)[4], int v,
                                               long long* d, double& part, long long& huge) {
-  voxel_dE_f64(ws.rd, a, row, v, d, true, part, huge);
+  voxel_dE_f64(ws, a, row, v, d, true, part, huge);
 }
 
 // Add the warp's field terms to their moves' plans (s: this lane's move, -1 for
@@ -1225,6 +1326,10 @@ __device__ void propose_position(const KArgs& a, SpecShared& sh, int rep, int s,
   bool empty = !live;
   const int Hs = 1 << a.logH;
   const bool pool = a.pool_on != 0;
+  // FP64: the sines and the rows of M on lanes of the warp (row gl here, from the
+  // column gl on)
+  constexpr bool kRows = sizeof(Pos) == 8 && G == 32;
+  double row[4] = {1.0, 0.0, 0.0, 0.0};
   Real M[3][4];
   for (int i = 0; i < 3; i++)
     for (int j = 0; j < 4; j++) M[i][j] = i == j ? (Real)1 : (Real)0;
@@ -1255,7 +1360,13 @@ __device__ void propose_position(const KArgs& a, SpecShared& sh, int rep, int s,
         Real mag = rsqrt_(dir[0] * dir[0] + dir[1] * dir[1] + dir[2] * dir[2]);
         if (mag < (Real)1E-5) sphere<Real>(g, dir);
         else { Real sc = (Real)1 / mag; for (int i = 0; i < 3; i++) dir[i] = dir[i] * sc; }
-        axis_rotation(dir, p, ang, M);
+        if constexpr (kRows) {
+          double sn, cs;
+          sincos(ang, &sn, &cs);
+          rotation_row(dir, p, sn, cs, gl < 3 ? gl : 0, row);
+        } else {
+          axis_rotation(dir, p, ang, M);
+        }
       }
     } else if (kind == CG_END_PIVOT) {
       Real ang = (Real)c.amp_move * (uni<Real>(g.next()) - (Real)0.5);
@@ -1263,7 +1374,13 @@ __device__ void propose_position(const KArgs& a, SpecShared& sh, int rep, int s,
       if (lhs == 1) { ind0 = 0; indf = (int)from_left(g, c.amp_bead, N, err) + 1; }
       else { ind0 = (int)(N - from_left(g, c.amp_bead, N, err)); indf = (int)N; }
       Real axis[3], p[3];
-      sphere<Real>(g, axis);
+      double sn, cs;
+      if constexpr (kRows) {
+        const unsigned xa = g.next(), xb = g.next();
+        sphere_and_angle(xa, xb, ang, axis, sn, cs);
+      } else {
+        sphere<Real>(g, axis);
+      }
       long long ip;
       if (ind0 == 0 && indf != N) ip = indf;
       else if (ind0 != 0 && indf == N) ip = ind0 - 1;
@@ -1271,12 +1388,20 @@ __device__ void propose_position(const KArgs& a, SpecShared& sh, int rep, int s,
       else ip = ind0;
       if (!err) {
         ld3(r4, ip, p);
-        axis_rotation(axis, p, ang, M);
+        if constexpr (kRows) rotation_row(axis, p, sn, cs, gl < 3 ? gl : 0, row);
+        else axis_rotation(axis, p, ang, M);
       }
     } else {
       Real amp = (Real)c.amp_move * uni<Real>(g.next()), d[3];
-      sphere<Real>(g, d);
-      for (int i = 0; i < 3; i++) M[i][3] = d[i] * amp;
+      if constexpr (kRows) {
+        const unsigned xa = g.next(), xb = g.next();
+        double sn, cs;
+        sphere_and_angle(xa, xb, 0.0, d, sn, cs);
+        row[3] = (gl == 0 ? d[0] : gl == 1 ? d[1] : d[2]) * amp;
+      } else {
+        sphere<Real>(g, d);
+        for (int i = 0; i < 3; i++) M[i][3] = d[i] * amp;
+      }
       long long b0 = g.next() % (unsigned)N;
       long long b1 = from_point(g, c.amp_bead, N, b0, err);
       segment_of(b0, b1, N, ind0, indf);
@@ -1326,10 +1451,20 @@ __device__ void propose_position(const KArgs& a, SpecShared& sh, int rep, int s,
     P.fl0 = P.fl1 = 0;
     P.fl2 = 0;
     P.fn = P.freg = 0;
-    Pos* Mp = reinterpret_cast<Pos*>(P.M);  // in the position type: no conversions
-    for (int i = 0; i < 3; i++)
-      for (int j = 0; j < 4; j++) Mp[4 * i + j] = M[i][j];
+    if constexpr (!kRows) {
+      Pos* Mp = reinterpret_cast<Pos*>(P.M);  // in the position type: no conversions
+      for (int i = 0; i < 3; i++)
+        for (int j = 0; j < 4; j++) Mp[4 * i + j] = M[i][j];
+    }
   }
+  if constexpr (kRows)
+    if (gl < 3 && live) {
+      double* Mp = reinterpret_cast<double*>(P.M) + 4 * gl;
+      Mp[gl] = row[0];
+      Mp[gl == 2 ? 0 : gl + 1] = row[1];
+      Mp[gl == 0 ? 2 : gl - 1] = row[2];
+      Mp[3] = row[3];
+    }
 }
 
 // Earlier moves u of the batch whose written beads [ind0, indf) meet the beads
