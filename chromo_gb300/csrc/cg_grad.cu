@@ -59,9 +59,14 @@ __device__ __forceinline__ void bond_grad(const double* bp, const double a0[3], 
 
 // One coordinate's voxels (lower, upper) and its fraction of the way between
 // them, in FP64 (the construction of voxel_axes).  The quotient by the voxel
-// width is a product and an FMA remainder, corrected to floor(x / d): a
-// division runs ~10 operations of the FP64 pipe.
-__device__ __forceinline__ double cell_of(double pos, double width, double d, double inv, int n, int& lo, int& hi) {
+// width is a product and an FMA remainder, corrected to floor(x / d), comparisons
+// and roundings in integer steps; coordinates and boxes that wrap_near leaves
+// out take the plain form.
+struct AxisCell {
+  double r;
+  int ind;
+};
+static __device__ __noinline__ AxisCell far_cell(double pos, double width, double d, double inv) {
   const double x = pymod(pos + 0.5 * width, width) - 0.5 * d;
   double q = floor(x * inv);
   double r = __fma_rn(-q, d, x);
@@ -72,11 +77,33 @@ __device__ __forceinline__ double cell_of(double pos, double width, double d, do
     const double r1 = __fma_rn(-(q + 1), d, x);
     if (r1 >= 0) { q += 1; r = r1; }
   }
-  const int ind = (int)q;
-  const int li = ind == -1 ? n - 1 : ind;
+  return AxisCell{r, (int)q};
+}
+__device__ __forceinline__ double cell_of(double pos, double width, double d, double inv, float iw, int n, int& lo,
+                                          int& hi) {
+  double m;
+  AxisCell c;
+  if (wrap_near(pos + 0.5 * width, width, iw, m)) {
+    const double x = m - 0.5 * d;  // -1/2 <= x / d < n
+    const int ind = floor_index(x * inv);
+    c.ind = ind;
+    c.r = __fma_rn(ind < 0 ? 1.0 : -whole_double(ind), d, x);
+    const long long bits = __double_as_longlong(c.r);
+    const int fix = bits < 0 && (bits << 1) != 0 ? -1 : (bits >= __double_as_longlong(d) ? 1 : 0);
+    if (fix) {
+      const double r1 = __fma_rn(-(double)(ind + fix), d, x);
+      if (fix < 0 || r1 >= 0) {
+        c.ind = ind + fix;
+        c.r = r1;
+      }
+    }
+  } else {
+    c = far_cell(pos, width, d, inv);
+  }
+  const int li = c.ind == -1 ? n - 1 : c.ind;
   lo = li < 0 ? 0 : (li >= n ? n - 1 : li);
   hi = lo + 1 == n ? 0 : lo + 1;
-  return r * inv;
+  return c.r * inv;
 }
 
 // dE_v/dw at one voxel of a replica with non-uniform volumes (states in sw).
@@ -105,11 +132,13 @@ __device__ __forceinline__ double voxel_slope(const KArgs& a, const RepDev& rd, 
 // columns whose coefficients depend on the bead's states only (a table of the
 // CTA), and the eight corners are contracted axis by axis.  Five divisions a
 // corner and every bond twice took 680 us for 64 chains of 5,000 beads with the
-// read-back (gradient and terms together: 1,086 -> 347 us).
+// read-back; one pass a warp and conversions, comparisons and roundings on the
+// FP64 pipe 229, now 183.
 template <typename Pos, typename Out>
 __global__ void __launch_bounds__(128) gradient_kernel(KArgs a, Out* out, Out* out_t3) {
   __shared__ double tab[64][CG_MAX_BINDERS];  // binder columns' coefficients for packed states (2 bits each)
   __shared__ double k0_sh, huge_sh, inv_sh[3];
+  __shared__ float iw_sh[3];
   __shared__ long long gmax_sh;
   const int rep = blockIdx.y;
   const RepDev& rd = a.reps[rep];
@@ -118,7 +147,7 @@ __global__ void __launch_bounds__(128) gradient_kernel(KArgs a, Out* out, Out* o
   if (blockIdx.x * (long long)(blockDim.x / 32) * kBeads >= N) return;
   const bool field = rd.field_kind == 2, uniform = field && !rd.has_access;
   if (field) {
-    const double u = kFxInv / rd.vol_bin;
+    const double u = 1.0 / rd.vol_bin;  // the columns as fx_double gives them
     if (uniform)
       for (int k = threadIdx.x; k < 64 * CG_MAX_BINDERS; k += blockDim.x) {
         const int code = k / CG_MAX_BINDERS, c = k % CG_MAX_BINDERS;
@@ -130,18 +159,19 @@ __global__ void __launch_bounds__(128) gradient_kernel(KArgs a, Out* out, Out* o
             if (b == c) pb += 2 * rd.pref[b];
             if (s) t += (double)s * pb;
           }
-        tab[code][c] = t * u / rd.vol_bin;
+        tab[code][c] = t * (u * u);
       }
     if (threadIdx.x < 3) {
       const double width[3] = {rd.wx, rd.wy, rd.wz};
       const int n[3] = {rd.nx, rd.ny, rd.nz};
       inv_sh[threadIdx.x] = (double)n[threadIdx.x] / width[threadIdx.x];
+      iw_sh[threadIdx.x] = (float)(1.0 / width[threadIdx.x]);
     }
-    if (threadIdx.x == 32) {
+    if (threadIdx.x == 64) {
       k0_sh = 2 * rd.chi * rd.bead_vol * u;
       huge_sh = kEHugeField * rd.bead_vol / rd.vol_bin;
-      gmax_sh = uniform ? weight_at_limit(rd) : 0;
     }
+    if (threadIdx.x == 96) gmax_sh = uniform ? weight_at_limit(rd) : 0;
   }
   __syncthreads();
   const V4<Pos>* r4 = reinterpret_cast<const V4<Pos>*>(a.r4) + rd.bead_off;
@@ -176,9 +206,9 @@ __global__ void __launch_bounds__(128) gradient_kernel(KArgs a, Out* out, Out* o
     if (field) {
       int lo[3], hi[3];
       const double inv[3] = {inv_sh[0], inv_sh[1], inv_sh[2]};
-      const double fx = cell_of(r[0], rd.wx, rd.dx, inv[0], rd.nx, lo[0], hi[0]);
-      const double fy = cell_of(r[1], rd.wy, rd.dy, inv[1], rd.ny, lo[1], hi[1]);
-      const double fz = cell_of(r[2], rd.wz, rd.dz, inv[2], rd.nz, lo[2], hi[2]);
+      const double fx = cell_of(r[0], rd.wx, rd.dx, inv[0], iw_sh[0], rd.nx, lo[0], hi[0]);
+      const double fy = cell_of(r[1], rd.wy, rd.dy, inv[1], iw_sh[1], rd.ny, lo[1], hi[1]);
+      const double fz = cell_of(r[2], rd.wz, rd.dz, inv[2], iw_sh[2], rd.nz, lo[2], hi[2]);
       const unsigned sw = st[i];
       const int code = (int)((sw & 3u) | ((sw >> 6) & 12u) | ((sw >> 12) & 48u));
       double phi[8];
@@ -189,10 +219,10 @@ __global__ void __launch_bounds__(128) gradient_kernel(KArgs a, Out* out, Out* o
         if (uniform) {
           long long row[4];
           load_row(grid + v * a.ncol, a.ncol, row);
-          double p = row[0] > gmax_sh ? huge_sh : k0_sh * (double)row[0];
+          double p = row[0] > gmax_sh ? huge_sh : k0_sh * fx_double(row[0]);
 #pragma unroll
           for (int c = 0; c < CG_MAX_BINDERS; c++)
-            if (row[1 + c]) p = __fma_rn(tab[code][c], (double)row[1 + c], p);
+            if (row[1 + c]) p = __fma_rn(tab[code][c], fx_double(row[1 + c]), p);
           phi[l] = p;
         } else {
           phi[l] = voxel_slope(a, rd, v, sw);
@@ -302,12 +332,14 @@ __global__ void __cluster_dims__(kSumCtas, 1, 1) __launch_bounds__(kSumThreads)
 
 }  // namespace cg
 
-// CTAs of 4 warps, 30 beads a warp and pass: enough to fill the GPU four times
-// over, at most one pass each.
+// CTAs of 4 warps, 30 beads a warp and pass; passes per warp so that about one
+// wave of CTAs (5 per SM) remains, up to 8: a CTA's constants take ~200 FP64
+// operations, a pass ~170 a warp.  64 chains of 5,000 beads with the read-back:
+// one pass a warp 210 us, two waves of CTAs 195, one 183.
 static dim3 gradient_grid(const cg::KArgs& a, long long max_beads) {
-  long long bx = (max_beads + 119) / 120;
-  const long long most = std::max<long long>(64, 152 * 16 / std::max(1, a.n_reps));
-  if (bx > most) bx = most;
+  const long long passes = (max_beads + 29) / 30;
+  const long long per = std::min<long long>(8, std::max<long long>(1, passes * a.n_reps / (4 * 5 * 152)));
+  long long bx = (passes + 4 * per - 1) / (4 * per);
   if (bx < 1) bx = 1;
   return dim3((unsigned)bx, (unsigned)a.n_reps);
 }
