@@ -495,6 +495,20 @@ __device__ __forceinline__ Real e_pair(const Bond<Real>& b, const Real bend[3], 
        + (Real)0.5 * b.epp * (dp[0] * dp[0] + dp[1] * dp[1] + dp[2] * dp[2]);
 }
 
+// Energy of bond (0 -> 1) in FP64: the terms of pair_dE_fwd / pair_dE_rev before
+// or after the move, by the same operations.
+__device__ __forceinline__ double bond_e(const Bond<double>& b, const double r0[3], const double r1[3],
+                                         const double t30[3], const double t31[3]) {
+  double dr[3], dp[3], bend[3];
+  for (int i = 0; i < 3; i++) dr[i] = r1[i] - r0[i];
+  const double par = t30[0] * dr[0] + t30[1] * dr[1] + t30[2] * dr[2];
+  for (int i = 0; i < 3; i++) {
+    dp[i] = dr[i] - t30[i] * par;
+    bend[i] = t31[i] - t30[i] - dp[i] * b.eta;
+  }
+  return e_pair(b, bend, par, dp);
+}
+
 // bond (0 -> 1) with bead 1 moved: bead_pair_dE_poly_forward (FP64 difference)
 template <typename Real>
 __device__ __forceinline__ double pair_dE_fwd(const Bond<Real>& b, const Real r0[3], const Real r1[3],

@@ -222,6 +222,34 @@ static __device__ __forceinline__ Acc boundary_term(const KArgs& a, const RepDev
   return out;
 }
 
+// FP64 storage: elastic energy of the same bond before the move (after = false)
+// or after it.
+static __device__ __forceinline__ double boundary_energy(const KArgs& a, const RepDev& rd, const MovePlan& P, int kind,
+                                                   int side, bool after) {
+  const ChainView<double> cv(a, rd, true);
+  const long long i = side == 0 ? P.ind0 : P.indf - 1;
+  const long long in = side == 0 ? i - 1 : i + 1;
+  if (in < 0 || in >= rd.n_beads) return 0.0;
+  double r[3], t3[3], rn[3], tn[3];
+  ld3(cv.r4, i, r); ld3(cv.t34, i, t3); ld3(cv.r4, in, rn); ld3(cv.t34, in, tn);
+  if (after) {
+    double M[3][4], tr[3], tt3[3], tt2[3];
+    const double t2[3] = {0, 0, 0};
+    load_transform(P, M);
+    move_bead(kind, M, r, t3, t2, tr, tt3, tt2);
+    for (int j = 0; j < 3; j++) { r[j] = tr[j]; t3[j] = tt3[j]; }
+  }
+  const bool left = side == 0;
+  double ra[3], rb[3], ta[3], tb[3];
+  for (int j = 0; j < 3; j++) {
+    ra[j] = left ? rn[j] : r[j];
+    rb[j] = left ? r[j] : rn[j];
+    ta[j] = left ? tn[j] : t3[j];
+    tb[j] = left ? t3[j] : tn[j];
+  }
+  return bond_e(load_bond<double>(cv.bonds, left ? in : i), ra, rb, ta, tb);
+}
+
 // SSTWLC: twist energy of the same bond before the move (after = false) or
 // after it.
 template <typename Pos>
@@ -581,24 +609,30 @@ __device__ void block_deposit(const KArgs& a, SpecShared& sh, int rep, int B, in
     }
   }
   // boundary bonds of the moves, two per move
-  if (!LEAN && twist) {
-    // the twist energies before and after the move on two lanes each, by warps
-    // without beads: an energy is ~150 FP64 operations, which issue at 1/64 of
-    // the FP32 rate whatever the number of lanes, and a batch's deposit waited
-    // for the two energies of each bond (64 SSTWLC chains of 2,000 beads, 10
-    // steps, kernel only, with short_tangent_twist: 7.60 -> 4.82 ms)
+  if (twist || sizeof(Pos) == 8) {
+    // a bond's energies before and after the move on two lanes each, four a move:
+    // an energy of FP64 storage is ~45 FP64 operations, a twist energy ~150, which
+    // issue at 1/64 of the FP32 rate whatever the number of lanes.  SSTWLC: by
+    // warps without beads, where a batch's deposit waited for the two twist
+    // energies of each bond (64 SSTWLC chains of 2,000 beads, 10 steps, kernel
+    // only, with short_tangent_twist: 7.60 -> 4.82 ms)
     #pragma unroll 1
     for (int j0 = 32 * (W - 1 - warp); j0 < 4 * B; j0 += 32 * W) {
       const int j = j0 + lane, side = (j >> 1) & 1;
       MovePlan& P = sh.plan[j < 4 * B ? j >> 2 : 0];
       const bool on = j < 4 * B && P.blk;
-      const double e = on ? boundary_twist<Pos>(a, rd, P, kind, side, j & 1) : 0.0;
-      const double after = __shfl_xor_sync(kFull, e, 1);
-      if (on && !(j & 1)) {
-        Acc t = boundary_term<Pos, Acc, LEAN>(a, rd, P, kind, side);
-        acc_add_d(t, after - e);
-        store_acc(P.pq[side], P.ph[side], t);
+      Acc t = acc_zero<Acc>();
+      if constexpr (sizeof(Pos) == 8) {
+        const double e = on ? boundary_energy(a, rd, P, kind, side, j & 1) : 0.0;
+        t = __shfl_xor_sync(kFull, e, 1) - e;
+      } else {
+        if (on && !(j & 1)) t = boundary_term<Pos, Acc, LEAN>(a, rd, P, kind, side);
       }
+      if (!LEAN && twist) {
+        const double e = on ? boundary_twist<Pos>(a, rd, P, kind, side, j & 1) : 0.0;
+        acc_add_d(t, __shfl_xor_sync(kFull, e, 1) - e);
+      }
+      if (on && !(j & 1)) store_acc(P.pq[side], P.ph[side], t);
     }
   } else if (warp == W - 1)
     for (int j = lane; j < 2 * B; j += 32) {
@@ -1625,16 +1659,80 @@ __device__ void evaluate_move(const KArgs& a, SpecShared& sh, int rep, int s, in
     const unsigned long long axis_base = g.pos;
     V4<Pos>* stage = reinterpret_cast<V4<Pos>*>(S.stage);
     Acc part = acc_zero<Acc>();
-    Real sa, ca;
-    rsincos(ang, &sa, &ca);
-    #pragma unroll 1
-    for (long long k = gl; k < m; k += G) {
-      const unsigned xa = g.word(axis_base + 2 * k), xb = g.word(axis_base + 2 * k + 1);
-      Real tt3[3], tt2[3];
-      const Acc de = rotate_tangent<Pos, LEAN>(a, rd, idx[k], xa, xb, sa, ca, tt3, tt2);
-      stage[3 * k + 1] = V4<Pos>{(Pos)tt3[0], (Pos)tt3[1], (Pos)tt3[2], (Pos)0};
-      stage[3 * k + 2] = V4<Pos>{(Pos)tt2[0], (Pos)tt2[1], (Pos)tt2[2], (Pos)0};
-      acc_add(part, de);
+    bool by_axes = false;
+    if constexpr (sizeof(Pos) == 8 && G == 32)
+      if (LEAN || !rd.twist) {
+        // FP64: four lanes a bead, 8 beads a pass (~110 FP64 operations instead of
+        // ~300): the sines of the sphere's angles and of the rotation, the rows of
+        // the rotation, and the two bonds' energies before and after it (1,000
+        // beads, 300 moves, kernel only, with block_deposit's bonds: 5.07 -> 4.66 ms)
+        by_axes = true;
+        #pragma unroll 1
+        for (int k0 = 0; k0 < m; k0 += 8) {
+          const int lane = gl, quad = lane & 28, ax = lane & 3, j = ax < 3 ? ax : 2;
+          const bool on = k0 + (lane >> 2) < m;
+          const int k = on ? k0 + (lane >> 2) : 0;
+          const long long i = idx[k], in = ax & 2 ? i + 1 : i - 1;
+          const unsigned xa = g.word(axis_base + 2 * k), xb = g.word(axis_base + 2 * k + 1);
+          const double u = uni<double>(ax == 0 ? xa : xb);
+          const double phi = u * (2.0 * 3.141592653589793), theta = acos(u * 2 - 1);
+          double sn, cs;
+          sincos(ax == 0 ? phi : ax == 1 ? theta : (double)ang, &sn, &cs);
+          const double st1 = __shfl_sync(kFull, sn, quad + 1);
+          const double axis[3] = {__shfl_sync(kFull, cs, quad) * st1, __shfl_sync(kFull, sn, quad) * st1,
+                                  __shfl_sync(kFull, cs, quad + 1)};
+          const double none[3] = {0, 0, 0};
+          double R[4], r[3], t3[3], t2[3];
+          rotation_row(axis, none, __shfl_sync(kFull, sn, quad + 2), __shfl_sync(kFull, cs, quad + 2), j, R);
+          const double m0 = j == 0 ? R[0] : j == 1 ? R[2] : R[1], m1 = j == 0 ? R[1] : j == 1 ? R[0] : R[2],
+                       m2 = j == 0 ? R[2] : j == 1 ? R[1] : R[0];
+          const V4<double>* q4 = reinterpret_cast<const V4<double>*>(a.t34) + rd.bead_off;
+          ld3(reinterpret_cast<const V4<double>*>(r4), i, r);
+          ld3(q4, i, t3);
+          ld3(reinterpret_cast<const V4<double>*>(a.t24) + rd.bead_off, i, t2);
+          const double tt3 = m0 * t3[0] + m1 * t3[1] + m2 * t3[2], tt2 = m0 * t2[0] + m1 * t2[1] + m2 * t2[2];
+          if (on) {
+            double* q = reinterpret_cast<double*>(stage + 3 * k);
+            q[4 + ax] = ax < 3 ? tt3 : 0.0;
+            q[8 + ax] = ax < 3 ? tt2 : 0.0;
+          }
+          double mine[3];  // the bead's tangent, before (even lanes) or after
+          for (int q = 0; q < 3; q++) {
+            const double moved = __shfl_sync(kFull, tt3, quad + q);
+            mine[q] = ax & 1 ? moved : t3[q];
+          }
+          double e = 0.0;
+          if (in >= 0 && in < N) {
+            const bool left = !(ax & 2);
+            double rn[3], tn[3], ra[3], rb[3], ta[3], tb[3];
+            ld3(reinterpret_cast<const V4<double>*>(r4), in, rn);
+            ld3(q4, in, tn);
+            for (int q = 0; q < 3; q++) {
+              ra[q] = left ? rn[q] : r[q];
+              rb[q] = left ? r[q] : rn[q];
+              ta[q] = left ? tn[q] : mine[q];
+              tb[q] = left ? mine[q] : tn[q];
+            }
+            e = bond_e(load_bond<double>(a.bonds + rd.bead_off * 6, left ? in : i), ra, rb, ta, tb);
+          }
+          const double d = __shfl_xor_sync(kFull, e, 1) - e;          // lanes 0 and 2 of four
+          const double de = d + __shfl_down_sync(kFull, d, 2);        // lane 0
+          const double of = __shfl_sync(kFull, de, 4 * (lane & 7));   // bead k0 + (lane & 7)
+          if ((lane >> 3) == ((k0 >> 3) & 3) && k0 + (lane & 7) < m) acc_add(part, of);
+        }
+      }
+    if (!by_axes) {
+      Real sa, ca;
+      rsincos(ang, &sa, &ca);
+      #pragma unroll 1
+      for (long long k = gl; k < m; k += G) {
+        const unsigned xa = g.word(axis_base + 2 * k), xb = g.word(axis_base + 2 * k + 1);
+        Real tt3[3], tt2[3];
+        const Acc de = rotate_tangent<Pos, LEAN>(a, rd, idx[k], xa, xb, sa, ca, tt3, tt2);
+        stage[3 * k + 1] = V4<Pos>{(Pos)tt3[0], (Pos)tt3[1], (Pos)tt3[2], (Pos)0};
+        stage[3 * k + 2] = V4<Pos>{(Pos)tt2[0], (Pos)tt2[1], (Pos)tt2[2], (Pos)0};
+        acc_add(part, de);
+      }
     }
     g.pos = axis_base + 2 * (unsigned long long)m;
     dEp = gsum<G>(part);
