@@ -15,7 +15,8 @@
 // within e and a margin above the test's error take the FP64 distance and
 // energy.  Every pair in FP64 with its square root, and the 10,000 row sums
 // added by one thread, took 2.57 ms for a 10,000-bead chain (with one segment's
-// change 2.75 ms, now 0.17 ms).
+// change 2.75 ms); tested one by one and summed where they are met 112 us (184
+// us), with the near pairs listed per tile 51 us (86 us).
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -25,7 +26,10 @@
 namespace cg {
 
 constexpr int kRows = 32;       // rows of a tile
-constexpr int kStericThr = 256; // threads of a tile: one column each
+constexpr int kStericThr = 256; // threads of a tile
+constexpr int kGroup = 8;       // rows between two tests
+constexpr int kList = 1024;     // near pairs a CTA lists (5 bits of row, 10 of column)
+static_assert(kRows == 32 && kRows % kGroup == 0, "a bit per row, groups of whole rows");
 
 __device__ __forceinline__ double clash_energy(double d, double e, double V0) {
   if (!(d < e)) return 0.0;
@@ -51,52 +55,89 @@ template <typename Pos>
 __device__ __forceinline__ float3 offset_of(const double* t, const V4<Pos>& o) {
   return make_float3((float)(t[0] - (double)o.x), (float)(t[1] - (double)o.y), (float)(t[2] - (double)o.z));
 }
-__device__ __forceinline__ float dist2(const float3& a, const float3& b) {
+__device__ __forceinline__ float dist2(const float4& a, const float3& b) {
   const float x = a.x - b.x, y = a.y - b.y, z = a.z - b.z;
-  return x * x + y * y + z * z;
+  return __fmaf_rn(z, z, __fmaf_rn(y, y, x * x));
 }
 
+// Sum over the CTA, valid in thread 0.  Most threads, and warps, hold zero: their
+// FP64 additions (~60 cycles of the pipe each) are left out.
 __device__ __forceinline__ double tile_total(double v, double* sh) {
-  for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(kFull, v, o);
+  if (__any_sync(kFull, !is_zero64(v)))
+    for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(kFull, v, o);
   if ((threadIdx.x & 31) == 0) sh[threadIdx.x >> 5] = v;
   __syncthreads();
   double t = 0;
   if (threadIdx.x == 0)
-    for (int w = 0; w < (int)(blockDim.x >> 5); w++) t += sh[w];
-  return t;  // valid in thread 0
+    #pragma unroll 1
+    for (int w = 0; w < (int)(blockDim.x >> 5); w++)
+      if (!is_zero64(sh[w])) t += sh[w];
+  return t;
+}
+
+// The FP64 term of beads i (a row) and j.
+template <typename Pos, bool TRIAL>
+static __device__ __noinline__ double pair_term(const V4<Pos>* r4, long long i, long long j, long long ind0,
+                                                long long indf, const double* trial, double e, double V0) {
+  double ri[3], rj[3];
+  ld3(r4, i, ri);
+  ld3(r4, j, rj);
+  const double before = clash_energy(dist3(ri, rj), e, V0);
+  if (!TRIAL) return before;
+  const double* ti = trial + 3 * (i - ind0);
+  const double t0[3] = {ti[0], ti[1], ti[2]};
+  if (j >= ind0 && j < indf)
+    for (int q = 0; q < 3; q++) rj[q] = trial[3 * (j - ind0) + q];
+  return clash_energy(dist3(t0, rj), e, V0) - before;
 }
 
 // Rows [kRows blockIdx.x, ...) against columns [blockIdx.y chunk, ...): the
-// pairs i < j of the resident chain, or with trial != null (positions of the
-// beads [ind0, indf), m x 3) the change of the pairs of the moved beads, those
-// of two moved beads counted once (j < i).  parts: one sum per tile, by row
-// tile and chunk.
-template <typename Pos>
+// pairs i < j of the resident chain, or (TRIAL) with positions `trial` of the
+// beads [ind0, indf) (m x 3) the change of the pairs of the moved beads, those of
+// two moved beads counted once (j < i).  parts: one sum per tile, by row tile and
+// chunk.  A thread holds COLS columns and takes the smallest squared distance of
+// kGroup rows before it branches, so that a pair costs seven FP32 instructions
+// and a quarter of a shared load; the near pairs are listed, and their FP64 terms
+// taken on consecutive threads (near pairs of a chain lie along the diagonal: row
+// by row, one lane at a time, a tile's took 70 k cycles).
+template <typename Pos, bool TRIAL, int COLS>
 __global__ void __launch_bounds__(kStericThr)
     steric_tile_kernel(KArgs a, int rep, long long n_rows, long long ind0, long long indf, long long chunk,
                        const double* trial, double e, double V0, double* parts) {
-  __shared__ float3 cur[kRows], tri[kRows];
+  __shared__ float4 cur[kRows], tri[TRIAL ? kRows : 1];
   __shared__ float far_sh;
+  __shared__ int found[kStericThr / 32];
+  __shared__ unsigned short list[kList];
   __shared__ double sh[kStericThr / 32];
   const RepDev& rd = a.reps[rep];
   const V4<Pos>* r4 = reinterpret_cast<const V4<Pos>*>(a.r4) + rd.bead_off;
   const long long N = rd.n_beads;
-  const long long first = trial ? ind0 : 0;  // bead of row 0
-  const long long k0 = (long long)blockIdx.x * kRows;
+  const int lane = (int)(threadIdx.x & 31u), warp = (int)(threadIdx.x >> 5);
+  const long long k0 = (long long)blockIdx.x * kRows, row0 = (TRIAL ? ind0 : 0) + k0;  // bead of row 0
   const int rows = (int)(n_rows - k0 < kRows ? n_rows - k0 : kRows);
-  const long long c0 = (long long)blockIdx.y * chunk, c1 = c0 + chunk < N ? c0 + chunk : N;
+  long long c0 = (long long)blockIdx.y * chunk;
+  const long long c1 = c0 + chunk < N ? c0 + chunk : N;
+  if (!TRIAL && c0 < k0 + 1) c0 = k0 + 1;  // pairs above the diagonal
+  if (c0 >= c1) {  // a chunk below the diagonal
+    if (threadIdx.x == 0) parts[(long long)blockIdx.x * gridDim.y + blockIdx.y] = 0.0;
+    return;
+  }
   double part = 0;
-  if (trial || c1 > k0 + 1) {  // a chunk below the diagonal has no pair
-    const V4<Pos> org = r4[first + k0];
+  {
+    const float inf = __int_as_float(0x7F800000);
+    const V4<Pos> org = r4[row0];
     if (threadIdx.x < 32) {
       float far = 0;
+      // rows past the last are nowhere near (inf - inf drops out of the minimum)
+      float3 c = make_float3(inf, inf, inf), t = c;
       if ((int)threadIdx.x < rows) {
-        const long long i = first + k0 + threadIdx.x;
-        const float3 c = offset_of(r4[i], org), t = trial ? offset_of(trial + 3 * (i - ind0), org) : c;
-        cur[threadIdx.x] = c;
-        tri[threadIdx.x] = t;
+        const long long i = row0 + threadIdx.x;
+        c = offset_of(r4[i], org);
+        t = TRIAL ? offset_of(trial + 3 * (i - ind0), org) : c;
         far = fmaxf(fmaxf(fabsf(c.x), fmaxf(fabsf(c.y), fabsf(c.z))), fmaxf(fabsf(t.x), fmaxf(fabsf(t.y), fabsf(t.z))));
       }
+      cur[threadIdx.x] = make_float4(c.x, c.y, c.z, 0.0f);
+      if (TRIAL) tri[threadIdx.x] = make_float4(t.x, t.y, t.z, 0.0f);
       for (int o = 16; o > 0; o >>= 1) far = fmaxf(far, __shfl_xor_sync(kFull, far, o));
       if (threadIdx.x == 0) far_sh = far;
     }
@@ -104,32 +145,93 @@ __global__ void __launch_bounds__(kStericThr)
     const float ef = (float)e;
     const float reach = ef + 4e-6f * (ef + 2.0f * far_sh) + 1e-30f;
     // beyond FP32's squares every pair takes the FP64 distance (NaN: no d2 is >= thr)
-    const float thr = reach < 1e18f ? reach * reach * 1.00001f : __int_as_float(0x7FFFFFFF);
-    for (long long j = c0 + threadIdx.x; j < c1; j += kStericThr) {
-      const float3 cj = offset_of(r4[j], org);
-      const bool moved = trial && j >= ind0 && j < indf;
-      const float3 tj = moved ? offset_of(trial + 3 * (j - ind0), org) : cj;
-      for (int k = 0; k < rows; k++) {
-        const long long i = first + k0 + k;
-        bool near = !(dist2(cur[k], cj) >= thr);
-        if (trial) near = (near || !(dist2(tri[k], tj) >= thr)) && !(moved && j >= i);
-        else near = near && j > i;
-        if (near) {
-          double ri[3], rj[3];
-          ld3(r4, i, ri);
-          ld3(r4, j, rj);
-          const double before = clash_energy(dist3(ri, rj), e, V0);
-          if (trial) {
-            const double* ti = trial + 3 * (i - ind0);
-            const double t0[3] = {ti[0], ti[1], ti[2]};
-            if (moved)
-              for (int q = 0; q < 3; q++) rj[q] = trial[3 * (j - ind0) + q];
-            part += clash_energy(dist3(t0, rj), e, V0) - before;
-          } else {
-            part += before;
+    const bool all = !(reach < 1e18f);
+    const float thr = all ? __int_as_float(0x7FFFFFFF) : reach * reach * 1.00001f;
+    #pragma unroll 1
+    for (long long jb = c0; jb < c1; jb += COLS * kStericThr) {
+      const long long j0 = jb + threadIdx.x;
+      float3 cj[COLS], tj[COLS];
+      bool moved[COLS];
+#pragma unroll
+      for (int u = 0; u < COLS; u++) {
+        const long long j = j0 + u * kStericThr;
+        cj[u] = j < c1 ? offset_of(r4[j], org) : make_float3(inf, inf, inf);
+        moved[u] = TRIAL && j >= ind0 && j < indf && j < c1;
+        tj[u] = moved[u] ? offset_of(trial + 3 * (j - ind0), org) : cj[u];
+      }
+      unsigned hit[COLS];
+#pragma unroll
+      for (int u = 0; u < COLS; u++) hit[u] = 0;
+      #pragma unroll 1
+      for (int g = 0; g < rows; g += kGroup) {
+        float low[COLS];
+#pragma unroll
+        for (int u = 0; u < COLS; u++) low[u] = inf;
+#pragma unroll
+        for (int q = 0; q < kGroup; q++) {
+          const float4 c = cur[g + q];
+#pragma unroll
+          for (int u = 0; u < COLS; u++) low[u] = fminf(low[u], dist2(c, cj[u]));
+          if (TRIAL) {
+            const float4 t = tri[g + q];
+#pragma unroll
+            for (int u = 0; u < COLS; u++) low[u] = fminf(low[u], dist2(t, tj[u]));
+          }
+        }
+#pragma unroll
+        for (int u = 0; u < COLS; u++) {
+          const long long j = j0 + u * kStericThr;
+          if (!(all || low[u] < thr) || j >= c1) continue;
+          #pragma unroll 1
+          for (int k = g; k < g + kGroup && k < rows; k++) {
+            const long long i = row0 + k;
+            bool near = !(dist2(cur[k], cj[u]) >= thr);
+            if (TRIAL) near = (near || !(dist2(tri[k], tj[u]) >= thr)) && !(moved[u] && j >= i);
+            else near = near && j > i;
+            if (near) hit[u] |= 1u << k;
           }
         }
       }
+      // the marked pairs, in thread order, as a list of the CTA: their FP64 terms on
+      // consecutive threads
+      int cnt = 0;
+#pragma unroll
+      for (int u = 0; u < COLS; u++) cnt += __popc(hit[u]);
+      int at = cnt;
+      for (int o = 1; o < 32; o <<= 1) {
+        const int y = __shfl_up_sync(kFull, at, o);
+        if (lane >= o) at += y;
+      }
+      if (lane == 31) found[warp] = at;
+      __syncthreads();
+      at -= cnt;
+      int total = 0;
+      for (int w = 0; w < kStericThr / 32; w++) {
+        if (w < warp) at += found[w];
+        total += found[w];
+      }
+      const bool listed = total <= kList;
+      #pragma unroll 1
+      while (cnt > 0) {
+        int u = 0;
+        unsigned h = 0;
+#pragma unroll
+        for (int v = COLS - 1; v >= 0; v--)
+          if (hit[v]) { u = v; h = hit[v]; }
+        const int k = __ffs((int)h) - 1;
+#pragma unroll
+        for (int v = 0; v < COLS; v++)
+          if (v == u) hit[v] &= hit[v] - 1;
+        cnt--;
+        if (listed) list[at++] = (unsigned short)((u * kStericThr + (int)threadIdx.x) << 5 | k);
+        else part += pair_term<Pos, TRIAL>(r4, row0 + k, j0 + u * kStericThr, ind0, indf, trial, e, V0);
+      }
+      __syncthreads();
+      if (listed)
+        #pragma unroll 1
+        for (int q = threadIdx.x; q < total; q += kStericThr)
+          part += pair_term<Pos, TRIAL>(r4, row0 + (list[q] & 31), jb + (list[q] >> 5), ind0, indf, trial, e, V0);
+      __syncthreads();  // the list is read
     }
   }
   const double t = tile_total(part, sh);
@@ -140,27 +242,41 @@ __global__ void __launch_bounds__(kStericThr)
 __global__ void __launch_bounds__(kStericThr) steric_sum_kernel(const double* parts, long long n, double* out) {
   __shared__ double sh[kStericThr / 32];
   double s = 0;
-  for (long long k = threadIdx.x; k < n; k += kStericThr) s += parts[k];
+  for (long long k = threadIdx.x; k < n; k += kStericThr) {
+    const double p = parts[k];
+    if (!is_zero64(p)) s += p;
+  }
   const double t = tile_total(s, sh);
   if (threadIdx.x == 0) out[0] = t;
 }
 
 }  // namespace cg
 
-// parts holds at least n_beads doubles: at most 32 chunks of columns.
+// parts holds at least n_beads + 32 doubles.  Columns in chunks of 1,024 (a pass
+// of a tile's threads), more where there would be over 32 chunks; in chunks of 256,
+// a column a thread, where fewer than two CTAs per SM would run: the FP64 terms of
+// the few near pairs, ~4 k cycles each, are then spread over more warps.
+template <typename Pos>
+static void launch_tiles(const cg::KArgs& a, dim3 grid, int rep, long long n_rows, long long ind0, long long indf,
+                         long long chunk, const double* trial, double e, double V0, double* parts, cudaStream_t s) {
+  auto run = [&](auto kernel) {
+    kernel<<<grid, cg::kStericThr, 0, s>>>(a, rep, n_rows, ind0, indf, chunk, trial, e, V0, parts);
+  };
+  const bool one = chunk == cg::kStericThr;
+  if (trial) run(one ? cg::steric_tile_kernel<Pos, true, 1> : cg::steric_tile_kernel<Pos, true, 4>);
+  else run(one ? cg::steric_tile_kernel<Pos, false, 1> : cg::steric_tile_kernel<Pos, false, 4>);
+}
 void cg_launch_steric(const cg::KArgs& a, bool fp64, int rep, long long n_beads, long long n_rows, long long ind0,
                       long long indf, const double* trial, double e, double V0, double* parts, double* out,
                       cudaStream_t s) {
   const long long tiles = (n_rows + cg::kRows - 1) / cg::kRows;
-  const long long chunk =
+  long long chunk =
       std::max<long long>(1024, ((n_beads + 31) / 32 + cg::kStericThr - 1) / cg::kStericThr * cg::kStericThr);
+  const long long narrow = (n_beads + cg::kStericThr - 1) / cg::kStericThr;
+  if (tiles * ((n_beads + chunk - 1) / chunk) < 304 && tiles * narrow <= n_beads + 32) chunk = cg::kStericThr;
   const long long chunks = (n_beads + chunk - 1) / chunk;
   const dim3 grid((unsigned)tiles, (unsigned)chunks);
-  if (fp64)
-    cg::steric_tile_kernel<double><<<grid, cg::kStericThr, 0, s>>>(a, rep, n_rows, ind0, indf, chunk, trial, e, V0,
-                                                                   parts);
-  else
-    cg::steric_tile_kernel<float><<<grid, cg::kStericThr, 0, s>>>(a, rep, n_rows, ind0, indf, chunk, trial, e, V0,
-                                                                  parts);
+  if (fp64) launch_tiles<double>(a, grid, rep, n_rows, ind0, indf, chunk, trial, e, V0, parts, s);
+  else launch_tiles<float>(a, grid, rep, n_rows, ind0, indf, chunk, trial, e, V0, parts, s);
   cg::steric_sum_kernel<<<1, cg::kStericThr, 0, s>>>(parts, tiles * chunks, out);
 }
