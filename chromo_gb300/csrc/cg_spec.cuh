@@ -1,10 +1,12 @@
 // cg_spec.cuh -- the production MC kernel: several moves of a replica in flight.
 //
 // One CTA per replica, W warps, each warp split into 32 / G groups of G lanes
-// (G = 8, 16 or 32).  Every group evaluates one move, so S = W * 32 / G moves
-// are in flight.  Within one controller's cycle (same move kind, fixed
-// amplitudes) the next S attempted moves are evaluated at once, group s taking
-// move t0 + s, all against the state before the batch.  Then:
+// (G = 8, 16 or 32).  A group evaluates one move, so up to S <= W * 32 / G moves
+// are in flight (the default FP32 shape has 3/4 as many moves as warps; short
+// tangent rotations take 8 or 16 lanes and more moves).  Within one controller's
+// cycle (same move kind, fixed amplitudes) the next B <= S attempted moves are
+// evaluated at once, group s taking move t0 + s, all against the state before
+// the batch.  Then:
 //
 //   * each move's read/write footprint -- the beads it reads or writes and
 //     the voxels it touches -- is compared with the footprints of the earlier
