@@ -77,7 +77,11 @@ struct SpecShared {
   unsigned long long tlog; // move counter at launch (index origin of the move log)
   double run_dE;   // running sum of accepted dE: its FP64 part
   long long run_q;  // and its fixed-point part (FP32 storage), exact over the launch
-  int cut, stop;
+  // move counter at the start of this controller cycle and of the next, by the
+  // parity of the cycle's number (a thread may still read the one while the other
+  // is written)
+  unsigned long long start[2];
+  int stop;
   unsigned accmask;
   int npool;  // entries of the pooled voxel table in use
   // conflicts among the position moves of a batch, by kind (see batch_limit):
