@@ -814,13 +814,16 @@ __device__ __forceinline__ void make_gridf_axis(const RepDev& rd, GridF& gf, int
   gf.inv_w[j] = (float)(1.0 / W);
   gf.half_w[j] = (float)(0.5 * W);
   gf.half_d[j] = (float)(0.5 * d);
-  gf.inv_dd[j] = inverse_or_zero(d);
-  gf.inv_d[j] = (float)(1.0 / d);
+  const double inv = 1.0 / d;
+  gf.inv_dd[j] = d > 1e-100 && d < 1e100 ? inv : 0.0;  // as inverse_or_zero
+  gf.inv_d[j] = (float)inv;
   gf.n[j] = n;
-  const int np = rd.fast_n > 0 ? rd.fast_n : 1;
-  gf.sw[j] = (float)(d / (double)np);
-  gf.inv_sw[j] = (float)((double)np / d);
-  gf.nsub[j] = (float)((double)np * n);
+  if (rd.fast_n > 0) {
+    const int np = rd.fast_n;
+    gf.sw[j] = (float)(d / (double)np);
+    gf.inv_sw[j] = (float)((double)np / d);
+    gf.nsub[j] = (float)((double)np * n);
+  }
 }
 __device__ __forceinline__ void make_gridf_rest(const RepDev& rd, GridF& gf) {
   gf.half_np = (float)(0.5 * (rd.fast_n > 0 ? rd.fast_n : 1));

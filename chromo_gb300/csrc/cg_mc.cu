@@ -58,7 +58,7 @@ __global__ void __launch_bounds__(128, 1) mc_kernel(KArgs a) {
     if (lane == 0) ws.nused = 0;
   }
   __syncwarp();
-  if (lane == 0) setup_f32(ws);
+  if (lane < kSetupParts) setup_part(ws, lane);
   __syncwarp();
   using Real = Pos;
   const RepDev& rd = ws.rd;

@@ -8,25 +8,38 @@
 
 namespace cg {
 
-// Copies of a replica's field and binding constants (one thread).
-__device__ __forceinline__ void setup_f32(WarpShared& ws) {
+// Copies of a replica's field and binding constants, in kSetupParts parts: FP64
+// divisions and conversions, ~9 k cycles by one thread.
+constexpr int kSetupParts = 8;
+__device__ __forceinline__ void setup_body(WarpShared& ws, int part) {
   const RepDev& rd = ws.rd;
-  make_gridf(rd, ws.gf);
-  for (int b = 0; b < CG_MAX_BINDERS; b++) ws.f_pref[b] = (float)rd.pref[b];
-  for (int b = 0; b < CG_MAX_BINDERS * CG_MAX_BINDERS; b++) ws.f_xpref[b] = (float)rd.xpref[b];
-  ws.f_scale = (float)(kFxInv / rd.vol_bin);
-  ws.f_vb = (float)rd.bead_vol;
-  ws.d_k = rd.chi * (rd.vol_bin / rd.bead_vol);
-  ws.f_k = (float)ws.d_k;
-  ws.f_lim = (float)rd.vf_limit;
-  ws.d_inv_vol = inverse_or_zero(rd.vol_bin);
-  for (int i = 0; i < CG_MAX_BINDERS * (CG_MAX_MARK + 1) * (CG_MAX_MARK + 1); i++)
-    ws.f_bind[i] = (float)rd.bind_f[i];
-  for (int b = 0; b < CG_MAX_BINDERS; b++) {
-    ws.f_me[b] = (float)(rd.mu[b] > 0 ? rd.mu[b] * (-rd.mu_adjust + 2) : rd.mu[b] * rd.mu_adjust);
-    ws.f_intra[b] = (float)rd.intra[b];
+  constexpr int kTab = CG_MAX_BINDERS * (CG_MAX_MARK + 1) * (CG_MAX_MARK + 1), kShare = (kTab + 2) / 3;
+  if (part < 3) {
+    make_gridf_axis(rd, ws.gf, part);
+  } else if (part < 6) {
+    #pragma unroll 1
+    for (int i = (part - 3) * kShare; i < (part - 2) * kShare && i < kTab; i++) ws.f_bind[i] = (float)rd.bind_f[i];
+  } else if (part == 6) {
+    make_gridf_rest(rd, ws.gf);
+    ws.f_scale = (float)(kFxInv / rd.vol_bin);
+    ws.f_vb = (float)rd.bead_vol;
+    ws.d_k = rd.chi * (rd.vol_bin / rd.bead_vol);
+    ws.f_k = (float)ws.d_k;
+    ws.f_lim = (float)rd.vf_limit;
+    ws.d_inv_vol = inverse_or_zero(rd.vol_bin);
+  } else {
+    #pragma unroll 1
+    for (int b = 0; b < CG_MAX_BINDERS; b++) {
+      ws.f_pref[b] = (float)rd.pref[b];
+      ws.f_me[b] = (float)(rd.mu[b] > 0 ? rd.mu[b] * (-rd.mu_adjust + 2) : rd.mu[b] * rd.mu_adjust);
+      ws.f_intra[b] = (float)rd.intra[b];
+    }
+    #pragma unroll 1
+    for (int b = 0; b < CG_MAX_BINDERS * CG_MAX_BINDERS; b++) ws.f_xpref[b] = (float)rd.xpref[b];
   }
 }
+
+static __device__ __noinline__ void setup_part(WarpShared& ws, int part) { setup_body(ws, part); }
 
 // ---------------------------------------------------------------- hash insert
 // Add d to column `col` of a hash entry.  Global-memory tables take one 64-bit

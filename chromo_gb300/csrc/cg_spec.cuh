@@ -2083,9 +2083,19 @@ __global__ void __maxnreg__(sizeof(Pos) == 4 ? 128 : 168) spec_kernel(KArgs a) {
     }
   }
   __syncthreads();
+  // the constants: the lean FP32 form by the warps' first threads (kernel only, 256
+  // chains of 2,000-20,000 beads, 20 steps: 9.27 -> 9.18 ms, one 10,000-bead chain
+  // 2.04 -> 2.02); in the other forms the call cost the main loop registers (FP64 and
+  // SSTWLC chains 0.9 % slower), and one thread takes them
+  constexpr bool kSpreadSetup = sizeof(Pos) == 4 && LEAN;
+  if (kSpreadSetup && lane == 0)
+    #pragma unroll 1
+    for (int part = warp; part < kSetupParts; part += (int)(blockDim.x >> 5)) setup_part(sh.ws, part);
   if (tid == 0) {
     const RepDev& rd0 = sh.ws.rd;
-    setup_f32(sh.ws);
+    if (!kSpreadSetup)
+#pragma unroll
+      for (int part = 0; part < kSetupParts; part++) setup_body(sh.ws, part);
     sh.t0 = sh.start[0] = rd0.draw_pos;
     sh.tlog = rd0.draw_pos;
     sh.run_dE = rd0.run_dE;
