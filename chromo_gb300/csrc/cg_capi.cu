@@ -696,7 +696,8 @@ static int steric_run(cg_sim* s, int rep, long long ind0, long long indf, const 
   double* trial = r_trial ? rows + n + 32 : nullptr;
   double* total = rows + n + 32 + 3 * m;
   if (trial) CUDA_TRY(cudaMemcpy(trial, r_trial, 8 * 3 * m, cudaMemcpyHostToDevice));
-  cg_launch_steric(s->args(), s->fp64 != 0, rep, n, r_trial ? m : n, ind0, indf, trial, e, V0, rows, total, 0);
+  cg_launch_steric(s->args(), s->fp64 != 0, rep, n, r_trial ? m : n, ind0, indf, trial, e, V0, rows, total,
+                   s->n_sm, 0);
   CUDA_TRY(cudaGetLastError());
   CUDA_TRY(cudaMemcpy(out, total, 8, cudaMemcpyDeviceToHost));
   return CG_OK;

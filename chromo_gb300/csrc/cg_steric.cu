@@ -19,14 +19,13 @@
 // us), with the near pairs listed per tile 51 us (86 us).
 #include <cuda_runtime.h>
 
-#include <algorithm>
-
 #include "cg_kernels.h"
+#include "cg_steric_tiles.h"
 
 namespace cg {
 
-constexpr int kRows = 32;       // rows of a tile
-constexpr int kStericThr = 256; // threads of a tile
+constexpr int kRows = CG_STERIC_ROWS;          // rows of a tile
+constexpr int kStericThr = CG_STERIC_THREADS;  // threads of a tile
 constexpr int kGroup = 8;       // rows between two tests
 constexpr int kList = 1024;     // near pairs a CTA lists (5 bits of row, 10 of column)
 static_assert(kRows == 32 && kRows % kGroup == 0, "a bit per row, groups of whole rows");
@@ -252,10 +251,7 @@ __global__ void __launch_bounds__(kStericThr) steric_sum_kernel(const double* pa
 
 }  // namespace cg
 
-// parts holds at least n_beads + 32 doubles.  Columns in chunks of 1,024 (a pass
-// of a tile's threads), more where there would be over 32 chunks; in chunks of 256,
-// a column a thread, where fewer than two CTAs per SM would run: the FP64 terms of
-// the few near pairs, ~4 k cycles each, are then spread over more warps.
+// parts holds at least n_beads + 32 doubles (the split: cg_steric_tiles.h).
 template <typename Pos>
 static void launch_tiles(const cg::KArgs& a, dim3 grid, int rep, long long n_rows, long long ind0, long long indf,
                          long long chunk, const double* trial, double e, double V0, double* parts, cudaStream_t s) {
@@ -268,15 +264,13 @@ static void launch_tiles(const cg::KArgs& a, dim3 grid, int rep, long long n_row
 }
 void cg_launch_steric(const cg::KArgs& a, bool fp64, int rep, long long n_beads, long long n_rows, long long ind0,
                       long long indf, const double* trial, double e, double V0, double* parts, double* out,
-                      cudaStream_t s) {
+                      int n_sm, cudaStream_t s) {
   const long long tiles = (n_rows + cg::kRows - 1) / cg::kRows;
-  long long chunk =
-      std::max<long long>(1024, ((n_beads + 31) / 32 + cg::kStericThr - 1) / cg::kStericThr * cg::kStericThr);
-  const long long narrow = (n_beads + cg::kStericThr - 1) / cg::kStericThr;
-  if (tiles * ((n_beads + chunk - 1) / chunk) < 304 && tiles * narrow <= n_beads + 32) chunk = cg::kStericThr;
+  const long long chunk = cg_steric_chunk(n_beads, tiles, n_sm);
   const long long chunks = (n_beads + chunk - 1) / chunk;
   const dim3 grid((unsigned)tiles, (unsigned)chunks);
   if (fp64) launch_tiles<double>(a, grid, rep, n_rows, ind0, indf, chunk, trial, e, V0, parts, s);
   else launch_tiles<float>(a, grid, rep, n_rows, ind0, indf, chunk, trial, e, V0, parts, s);
+  if (cudaPeekAtLastError() != cudaSuccess) return;  // the caller reports it; no sums to add
   cg::steric_sum_kernel<<<1, cg::kStericThr, 0, s>>>(parts, tiles * chunks, out);
 }
