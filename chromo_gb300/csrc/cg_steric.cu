@@ -143,8 +143,9 @@ __global__ void __launch_bounds__(kStericThr)
     __syncthreads();
     const float ef = (float)e;
     const float reach = ef + 4e-6f * (ef + 2.0f * far_sh) + 1e-30f;
-    // beyond FP32's squares every pair takes the FP64 distance (NaN: no d2 is >= thr)
-    const bool all = !(reach < 1e18f);
+    // beyond FP32's squares, and where they lose bits below its normal numbers, every
+    // pair takes the FP64 distance (NaN: no d2 is >= thr)
+    const bool all = !(reach > 1e-18f && reach < 1e18f);
     const float thr = all ? __int_as_float(0x7FFFFFFF) : reach * reach * 1.00001f;
     #pragma unroll 1
     for (long long jb = c0; jb < c1; jb += COLS * kStericThr) {
