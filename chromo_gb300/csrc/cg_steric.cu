@@ -30,10 +30,20 @@ constexpr int kGroup = 8;       // rows between two tests
 constexpr int kList = 1024;     // near pairs a CTA lists (5 bits of row, 10 of column)
 static_assert(kRows == 32 && kRows % kGroup == 0, "a bit per row, groups of whole rows");
 
+// The powers of f = e / d are products whose rounding errors (one FMA each) are
+// carried along and added at the end: the product of products alone is off by up to
+// 5 units in the last place, twelve multiplications' worth, where pow is off by
+// one.
 __device__ __forceinline__ double clash_energy(double d, double e, double V0) {
   if (!(d < e)) return 0.0;
-  const double f = e / d, f2 = f * f, f6 = f2 * f2 * f2;
-  return V0 * (f6 * f6 - 2 * f6 + 1);
+  const double f = e / d;
+  const double f2 = f * f, r2 = __fma_rn(f, f, -f2);
+  const double f4 = f2 * f2, r4 = __fma_rn(2 * f2, r2, __fma_rn(f2, f2, -f4));
+  const double f6 = f4 * f2, r6 = __fma_rn(f4, f2, -f6) + __fma_rn(f4, r2, r4 * f2);
+  const double f12 = f6 * f6, r12 = __fma_rn(2 * f6, r6, __fma_rn(f6, f6, -f12));
+  const double c = r12 - 2 * r6;
+  const double t = f12 - 2 * f6 + 1;
+  return V0 * (isfinite(c) ? t + c : t);
 }
 
 __device__ __forceinline__ double dist3(const double a[3], const double b[3]) {
