@@ -657,7 +657,8 @@ __global__ void __cluster_dims__(kSumCtas, 1, 1) __launch_bounds__(kSumThreads)
         a, rd, rank,
         [&](long long, const long long (&row)[4]) {
           if (row[0] > gmax) return;
-          if ((unsigned long long)row[0] >> 52) {
+          // the rows that add_row gives to its FP64 sums
+          if ((unsigned long long)(row[0] | row[1] | row[2] | row[3]) >> 52) {
             sx = __fma_rn((double)row[0], (double)row[0], sx);
             return;
           }
