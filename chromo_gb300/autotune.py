@@ -21,6 +21,8 @@ so a problem is tuned once per GPU model.
 The reference has no counterpart: its loop runs one move at a time on one
 core (chromo/mc/mc_sim.pyx:88-182).
 """
+import functools
+import hashlib
 import json
 import math
 import os
@@ -41,16 +43,30 @@ def cache_path() -> Path:
     return Path(p) if p else Path.home() / ".cache" / "chromo_gb300" / "autotune.json"
 
 
+@functools.lru_cache(maxsize=1)
+def kernel_version() -> str:
+    """Digest of the kernels' sources and of this module's candidates: a shape
+    tuned for other kernels, or from other candidates, is timed again."""
+    h = hashlib.sha256()
+    here = Path(__file__).resolve()
+    for p in sorted((here.parent / "csrc").glob("*.cu*")) + sorted((here.parent / "csrc").glob("*.h")) + [here]:
+        h.update(p.name.encode())
+        h.update(p.read_bytes())
+    return h.hexdigest()[:16]
+
+
 def problem_key(n_beads: Sequence[int], grid_dims: Sequence, n_binders: int, pos_fp64: bool,
                 n_sm: int, device_name: str, extra: str = "") -> str:
     """Signature of a tuning problem: device, replica count, chain-length
-    quantiles, distinct grids, binders and storage precision."""
+    quantiles, distinct grids, binders, storage precision and the kernels that
+    were timed."""
     lengths = np.asarray(n_beads, dtype=np.int64)
     q = [int(np.quantile(lengths, f)) for f in (0.0, 0.5, 1.0)]
     grids = sorted({tuple(int(x) for x in g) for g in np.asarray(grid_dims).reshape(-1, 3)})
     return json.dumps({"device": device_name, "sm": int(n_sm), "R": int(len(lengths)), "len_q": q,
                        "grids": grids[:4], "n_grids": len(grids), "nb": int(n_binders),
-                       "fp64": bool(pos_fp64), "extra": extra}, sort_keys=True)
+                       "fp64": bool(pos_fp64), "extra": extra, "kernels": kernel_version()},
+                      sort_keys=True)
 
 
 def candidates(n_replicas: int, n_sm: int, pos_fp64: bool, warps_per_sm: Dict[int, int]) -> List[Shape]:

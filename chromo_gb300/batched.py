@@ -102,9 +102,21 @@ class ReplicaBatch:
             from . import autotune as at
             (warps_per_block, lanes_per_move), self.tuning = at.tune(
                 self._make_sim, [p.num_beads for p in self.polymers],
-                [_grid_dims(f) for f in self.fields], nb, self._fp64)
+                [_grid_dims(f) for f in self.fields], nb, self._fp64, extra_key=self._kernel_features())
         self.sim = self._make_sim(warps_per_block, lanes_per_move)
         self.rebaseline()
+
+    def _kernel_features(self) -> str:
+        """What of this batch, beyond its sizes, the MC kernel's time depends on:
+        the kernel's form (SSTWLC twist, fast_field) and how far moves get
+        (fields, confinement)."""
+        out = set()
+        for p, f in zip(self.polymers, self.fields):
+            fp = _field_struct(p, f)
+            out.add("/".join([f"field{fp.field_kind}", f"confine{fp.confine_kind}"]
+                             + ["twist"] * hasattr(p, "twist_parameters") + ["fast"] * bool(fp.fast_field)
+                             + ["access"] * self._nonuni))
+        return " ".join(sorted(out))
 
     def _make_sim(self, warps_per_block: int, lanes_per_move: int) -> "nat.Sim":
         """A resident simulation of this batch's chains, fields and controllers."""
