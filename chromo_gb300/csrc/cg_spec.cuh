@@ -1059,11 +1059,19 @@ __device__ __forceinline__ typename AccOf<Pos>::type rotate_tangent(const KArgs&
 // move finds the earlier moves that rotate its beads or their neighbours by
 // three look-ups a bead instead of comparing lists.  A move's staging, index
 // list and draws fit a quarter of a slot's region for up to 16 beads, half of it
-// for up to 32 (longer ones take the path of 32 lanes).  One 10,000-bead chain,
+// for up to 32.  One 10,000-bead chain,
 // 10 MC steps, kernel only: 2.83 -> 2.62 ms; 64 SSTWLC chains of 2,000 beads,
 // whose FP64 twist terms fill their warps' lanes: 10.4 -> 9.1 ms (with the
 // phases' state kept in the plans); 9-16 beads on 16 lanes instead of 8, one
 // pass instead of two: 256 chains 9.90 -> 9.53 ms, the SSTWLC chains 8.46 -> 7.60.
+//
+// Without twist, an amplitude above 16, or a large one for the chain's length
+// (amp^2 > 3/4 N), takes the path of 32 lanes: on 16 lanes over 16 beads need two
+// passes, and beads drawn twice, likely there, are redrawn by one lane.  80
+// rotations on each of 256 chains: 1,000 beads, up to 16 / 32 of them, 230 / 716 us
+// here against 262 / 406 there; 50 beads, up to 16, 578 against 417.  The FP64 twist
+// terms outweigh that up to 32 beads and amp^2 = 8 N (64 SSTWLC chains of 200 / 50
+// beads, up to 32: 2.08 / 2.55 ms against 2.17 / 2.21).
 //
 // Moves in flight: kShortSpan sqrt(N) / (amp + 1), at which about two of them
 // meet an earlier accepted one (3 and 4 measured alike, 6 and 9 were slower on
@@ -2126,7 +2134,10 @@ __global__ void __maxnreg__(sizeof(Pos) == 4 ? 128 : 168) spec_kernel(KArgs a) {
           // in flight as are likely to stand (a later move meets the ~3/2 (amp + 1)
           // beads of each earlier accepted one with probability ~3/8 (amp + 1)^2 / N)
           constexpr bool kShort = G == 32 && sizeof(Pos) == 4;
-          const bool brief = kShort && kind == CG_TANGENT_ROTATION && c.amp_bead >= 1 && c.amp_bead <= 32;
+          const bool twist = !LEAN && sh.ws.rd.twist;
+          const bool brief = kShort && kind == CG_TANGENT_ROTATION && c.amp_bead >= 1 &&
+                             c.amp_bead <= (twist ? 32 : 16) &&
+                             4 * c.amp_bead * c.amp_bead <= (twist ? 32 : 3) * sh.ws.rd.n_beads;
           const int gs = c.amp_bead <= 8 ? 8 : 16, cap = c.amp_bead <= 16 ? 16 : 32;  // of a short rotation
           int most = kind <= CG_SLIDE ? sh.limit[kind] : Sn;
           if (brief) {
