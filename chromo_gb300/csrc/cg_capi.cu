@@ -381,52 +381,62 @@ static int moves_in_flight(const cg_sim* s, int w_req, int W, int G) {
   return (3 * W + 3) / 4;
 }
 
+// One CTA per replica with W warps of 32 / G moves each.  The CTAs that can be
+// resident per SM -- those every replica needs to run at once, or fewer when the
+// register file holds fewer CTAs of W warps (the replicas then run in waves) --
+// share the SM's shared memory; each move slot gets the largest voxel table that
+// then fits.  A shape of the library's own leaves room for a pooled table: with
+// fewer warps and, of one warp, with fewer CTAs per SM than would otherwise run,
+// since without it moves of more than ~16 beads go to tables in global memory (2 MC
+// steps of 1,216 chains of 50 beads: 1 warp 1.24 ms, 2 warps without a table 2.38; of
+// 2,432 chains of 200 beads: fewer CTAs per SM 2.75 ms, all without a table 5.01).
 static int choose_shape(cg_sim* s, int w_req, int g_req) {
-  // One CTA per replica with W warps of 32 / G moves each.  The CTAs that can
-  // be resident per SM -- those every replica needs to run at once, or fewer
-  // when the register file holds fewer CTAs of W warps (the replicas then run
-  // in waves) -- share the SM's shared memory; each move slot gets the
-  // largest voxel table that then fits.
   const size_t smem_per_sm = 227 * 1024;
-  long long ctas_per_sm = (s->R + s->n_sm - 1) / std::max(1, s->n_sm);
-  if (ctas_per_sm < 1) ctas_per_sm = 1;
   const int G = default_lanes(s, g_req);
   int W = w_req > 0 ? w_req : default_warps(s, G);
   if (W > cg::kMaxW) W = cg::kMaxW;
   if (W * (32 / G) > cg::kMaxS) W = cg::kMaxS / (32 / G);
-  const int S = moves_in_flight(s, w_req, W, G);
-  const long long reg_ctas = std::max(1, cg_spec_warps_per_sm(s->fp64 != 0, G) / W);
-  if (ctas_per_sm > reg_ctas) ctas_per_sm = reg_ctas;
-  const size_t budget = std::min<size_t>(smem_per_sm / ctas_per_sm - 1024, 220 * 1024);
-  // block voxel table: moves in flight touch ~50 voxels each, so 1,024 entries
-  // serve 6 of them at a load of 0.25, but 12 at 0.55 (10,000-bead chain, 10 MC
-  // steps: 2.59 ms against 2.42 with 2,048; 4,096 would halve the pool of two
-  // binders on one CTA per SM)
-  const int lhb = S > 8 ? 11 : 10;
+  long long ctas_per_sm = std::max<long long>(1, (s->R + s->n_sm - 1) / std::max(1, s->n_sm));
   const long long sc = G == 32 ? 48 : 32;
-  // the position moves of a batch share one pooled voxel table (keys voxel *
-  // 32 + slot: grids below 2^26 voxels), as large as fits; the slots keep small
-  // tables for binding moves.  FP32 storage: up to 4,096 entries and 64-entry
-  // slot tables.  FP64 storage: up to 2,048 entries (its moves in flight touch
-  // ~50 voxels each) and, where they fit beside a pool of at least 1,024, slot
-  // tables of up to 256 entries.
   int lhp = 0, lh = 6;
-  if (s->max_vox < (1LL << 26)) {
-    for (int t = s->fp64 ? 11 : 12; t >= 8 && lhp == 0; t--)
-      for (int l = s->fp64 && t >= 10 ? 8 : 6; l >= 6 && lhp == 0; l--) {
-        s->layout(l, sc);
-        if (s->cta_layout(lhb, W, G, S, t) <= budget) { lhp = t; lh = l; }
+  for (;;) {
+    const int S = moves_in_flight(s, w_req, W, G);
+    ctas_per_sm = std::min<long long>(ctas_per_sm, std::max(1, cg_spec_warps_per_sm(s->fp64 != 0, G) / W));
+    const size_t budget = std::min<size_t>(smem_per_sm / ctas_per_sm - 1024, 220 * 1024);
+    // block voxel table: moves in flight touch ~50 voxels each, so 1,024 entries
+    // serve 6 of them at a load of 0.25, but 12 at 0.55 (10,000-bead chain, 10 MC
+    // steps: 2.59 ms against 2.42 with 2,048; 4,096 would halve the pool of two
+    // binders on one CTA per SM)
+    const int lhb = S > 8 ? 11 : 10;
+    // the position moves of a batch share one pooled voxel table (keys voxel *
+    // 32 + slot: grids below 2^26 voxels), as large as fits; the slots keep small
+    // tables for binding moves.  FP32 storage: up to 4,096 entries and 64-entry
+    // slot tables.  FP64 storage: up to 2,048 entries (its moves in flight touch
+    // ~50 voxels each) and, where they fit beside a pool of at least 1,024, slot
+    // tables of up to 256 entries.
+    if (s->max_vox < (1LL << 26)) {
+      for (int t = s->fp64 ? 11 : 12; t >= 8 && lhp == 0; t--)
+        for (int l = s->fp64 && t >= 10 ? 8 : 6; l >= 6 && lhp == 0; l--) {
+          s->layout(l, sc);
+          if (s->cta_layout(lhb, W, G, S, t) <= budget) { lhp = t; lh = l; }
+        }
+      if (lhp == 0 && w_req == 0 && (W > 1 || ctas_per_sm > 1)) {
+        if (W > 1) W--;
+        else ctas_per_sm--;
+        continue;
       }
-  }
-  if (lhp == 0) {
-    lh = 10;  // at most 1,024 slots: the 32-bit split counters of a shared table cannot overflow
-    for (; lh > 6; lh--) {
-      s->layout(lh, sc);
-      if (s->cta_layout(lhb, W, G, S) <= budget) break;
     }
+    if (lhp == 0) {
+      lh = 10;  // at most 1,024 slots: the 32-bit split counters of a shared table cannot overflow
+      for (; lh > 6; lh--) {
+        s->layout(lh, sc);
+        if (s->cta_layout(lhb, W, G, S) <= budget) break;
+      }
+    }
+    s->layout(lh, sc);
+    s->spec_bytes = s->cta_layout(lhb, W, G, S, lhp);
+    break;
   }
-  s->layout(lh, sc);
-  s->spec_bytes = s->cta_layout(lhb, W, G, S, lhp);
   s->wpb = 1;
   cudaError_t e = cg_set_spec_smem(s->fp64 != 0, G, (int)s->spec_bytes);
   if (e == cudaSuccess) e = cg_set_mc_smem(s->fp64 != 0, (int)(s->spec_off_warps + s->warp_smem));
@@ -481,13 +491,9 @@ int cg_create(const cg_config* cfg, cg_sim** out) {
     cg_destroy(s);
     return fail(CG_ERR_ARG, "warps_per_block must be in 0..12");
   }
-  {
-    const int G = default_lanes(s, cfg->lanes_per_move);
-    int W = cfg->warps_per_block > 0 ? cfg->warps_per_block : default_warps(s, G);
-    if (W * (32 / G) > cg::kMaxS) W = cg::kMaxS / (32 / G);
-    s->spec_w = W;
-    s->spec_g = G;
-    s->spec_s = moves_in_flight(s, cfg->warps_per_block, W, G);
+  if (int rc = choose_shape(s, cfg->warps_per_block, cfg->lanes_per_move)) {
+    cg_destroy(s);
+    return rc;
   }
   const long long RW = (long long)s->R * s->spec_s;
   // tangent-rotation bitmaps: one per (replica, move slot)
@@ -582,8 +588,6 @@ int cg_create(const cg_config* cfg, cg_sim** out) {
   cudaMemcpy(s->reps, rd.data(), sizeof(RepDev) * s->R, cudaMemcpyHostToDevice);
   e = cudaGetLastError();
   if (e != cudaSuccess) { cg_destroy(s); return fail(CG_ERR_CUDA, cudaGetErrorString(e)); }
-  int rc = choose_shape(s, cfg->warps_per_block, s->spec_g);
-  if (rc) { cg_destroy(s); return rc; }
   *out = s;
   return CG_OK;
 }
