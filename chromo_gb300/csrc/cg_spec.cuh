@@ -1669,79 +1669,82 @@ __device__ void evaluate_move(const KArgs& a, SpecShared& sh, int rep, int s, in
     const unsigned long long axis_base = g.pos;
     V4<Pos>* stage = reinterpret_cast<V4<Pos>*>(S.stage);
     Acc part = acc_zero<Acc>();
-    bool by_axes = false;
-    if constexpr (sizeof(Pos) == 8 && G == 32)
-      if (LEAN || !rd.twist) {
-        // FP64: four lanes a bead, 8 beads a pass (~110 FP64 operations instead of
-        // ~300): the sines of the sphere's angles and of the rotation, the rows of
-        // the rotation, and the two bonds' energies before and after it (1,000
-        // beads, 300 moves, kernel only, with block_deposit's bonds: 5.07 -> 4.66 ms)
-        by_axes = true;
-        #pragma unroll 1
-        for (int k0 = 0; k0 < m; k0 += 8) {
-          const int lane = gl, quad = lane & 28, ax = lane & 3, j = ax < 3 ? ax : 2;
-          const bool on = k0 + (lane >> 2) < m;
-          const int k = on ? k0 + (lane >> 2) : 0;
-          const long long i = idx[k], in = ax & 2 ? i + 1 : i - 1;
-          const unsigned xa = g.word(axis_base + 2 * k), xb = g.word(axis_base + 2 * k + 1);
-          const double u = uni<double>(ax == 0 ? xa : xb);
-          const double phi = u * (2.0 * 3.141592653589793), theta = acos(u * 2 - 1);
-          double sn, cs;
-          sincos(ax == 0 ? phi : ax == 1 ? theta : (double)ang, &sn, &cs);
-          const double st1 = __shfl_sync(kFull, sn, quad + 1);
-          const double axis[3] = {__shfl_sync(kFull, cs, quad) * st1, __shfl_sync(kFull, sn, quad) * st1,
-                                  __shfl_sync(kFull, cs, quad + 1)};
-          const double none[3] = {0, 0, 0};
-          double R[4], r[3], t3[3], t2[3];
-          rotation_row(axis, none, __shfl_sync(kFull, sn, quad + 2), __shfl_sync(kFull, cs, quad + 2), j, R);
-          const double m0 = j == 0 ? R[0] : j == 1 ? R[2] : R[1], m1 = j == 0 ? R[1] : j == 1 ? R[0] : R[2],
-                       m2 = j == 0 ? R[2] : j == 1 ? R[1] : R[0];
-          const V4<double>* q4 = reinterpret_cast<const V4<double>*>(a.t34) + rd.bead_off;
-          ld3(reinterpret_cast<const V4<double>*>(r4), i, r);
-          ld3(q4, i, t3);
-          ld3(reinterpret_cast<const V4<double>*>(a.t24) + rd.bead_off, i, t2);
-          const double tt3 = m0 * t3[0] + m1 * t3[1] + m2 * t3[2], tt2 = m0 * t2[0] + m1 * t2[1] + m2 * t2[2];
-          if (on) {
-            double* q = reinterpret_cast<double*>(stage + 3 * k);
-            q[4 + ax] = ax < 3 ? tt3 : 0.0;
-            q[8 + ax] = ax < 3 ? tt2 : 0.0;
-          }
-          double mine[3];  // the bead's tangent, before (even lanes) or after
-          for (int q = 0; q < 3; q++) {
-            const double moved = __shfl_sync(kFull, tt3, quad + q);
-            mine[q] = ax & 1 ? moved : t3[q];
-          }
-          double e = 0.0;
-          if (in >= 0 && in < N) {
-            const bool left = !(ax & 2);
-            double rn[3], tn[3], ra[3], rb[3], ta[3], tb[3];
-            ld3(reinterpret_cast<const V4<double>*>(r4), in, rn);
-            ld3(q4, in, tn);
-            for (int q = 0; q < 3; q++) {
-              ra[q] = left ? rn[q] : r[q];
-              rb[q] = left ? r[q] : rn[q];
-              ta[q] = left ? tn[q] : mine[q];
-              tb[q] = left ? mine[q] : tn[q];
-            }
-            e = bond_e(load_bond<double>(a.bonds + rd.bead_off * 6, left ? in : i), ra, rb, ta, tb);
-          }
-          const double d = __shfl_xor_sync(kFull, e, 1) - e;          // lanes 0 and 2 of four
-          const double de = d + __shfl_down_sync(kFull, d, 2);        // lane 0
-          const double of = __shfl_sync(kFull, de, 4 * (lane & 7));   // bead k0 + (lane & 7)
-          if ((lane >> 3) == ((k0 >> 3) & 3) && k0 + (lane & 7) < m) acc_add(part, of);
-        }
-      }
-    if (!by_axes) {
+    // FP64 without twist: the last rotations of up to 16 by four lanes a bead, 8 beads
+    // a pass (~110 FP64 operations instead of ~300): the sines of the sphere's angles
+    // and of the rotation, the rows of the rotation, and the two bonds' energies
+    // before and after it, the bead's dE on the lane that a whole pass has it on
+    // (1,000 beads, 300 moves, kernel only, with block_deposit's bonds: 5.07 -> 4.66
+    // ms).  Three such passes take longer than one of 32 beads (80 rotations of up
+    // to 100 beads: 4.51 ms by such passes alone, 3.29 by whole ones, 3.17 mixed).
+    constexpr bool kQuads = sizeof(Pos) == 8 && G == 32;
+    int whole = m;
+    if (kQuads && (LEAN || !rd.twist) && (m & 31) <= 16) whole = m & ~31;
+    if (whole > 0) {
       Real sa, ca;
       rsincos(ang, &sa, &ca);
       #pragma unroll 1
-      for (long long k = gl; k < m; k += G) {
+      for (long long k = gl; k < whole; k += G) {
         const unsigned xa = g.word(axis_base + 2 * k), xb = g.word(axis_base + 2 * k + 1);
         Real tt3[3], tt2[3];
         const Acc de = rotate_tangent<Pos, LEAN>(a, rd, idx[k], xa, xb, sa, ca, tt3, tt2);
         stage[3 * k + 1] = V4<Pos>{(Pos)tt3[0], (Pos)tt3[1], (Pos)tt3[2], (Pos)0};
         stage[3 * k + 2] = V4<Pos>{(Pos)tt2[0], (Pos)tt2[1], (Pos)tt2[2], (Pos)0};
         acc_add(part, de);
+      }
+    }
+    if constexpr (kQuads) {
+      #pragma unroll 1
+      for (int k0 = whole; k0 < m; k0 += 8) {
+        const int lane = gl, quad = lane & 28, ax = lane & 3, j = ax < 3 ? ax : 2;
+        const bool on = k0 + (lane >> 2) < m;
+        const int k = on ? k0 + (lane >> 2) : 0;
+        const long long i = idx[k], in = ax & 2 ? i + 1 : i - 1;
+        const unsigned xa = g.word(axis_base + 2 * k), xb = g.word(axis_base + 2 * k + 1);
+        const double u = uni<double>(ax == 0 ? xa : xb);
+        const double phi = u * (2.0 * 3.141592653589793), theta = acos(u * 2 - 1);
+        double sn, cs;
+        sincos(ax == 0 ? phi : ax == 1 ? theta : (double)ang, &sn, &cs);
+        const double st1 = __shfl_sync(kFull, sn, quad + 1);
+        const double axis[3] = {__shfl_sync(kFull, cs, quad) * st1, __shfl_sync(kFull, sn, quad) * st1,
+                                __shfl_sync(kFull, cs, quad + 1)};
+        const double none[3] = {0, 0, 0};
+        double R[4], r[3], t3[3], t2[3];
+        rotation_row(axis, none, __shfl_sync(kFull, sn, quad + 2), __shfl_sync(kFull, cs, quad + 2), j, R);
+        const double m0 = j == 0 ? R[0] : j == 1 ? R[2] : R[1], m1 = j == 0 ? R[1] : j == 1 ? R[0] : R[2],
+                     m2 = j == 0 ? R[2] : j == 1 ? R[1] : R[0];
+        const V4<double>* q4 = reinterpret_cast<const V4<double>*>(a.t34) + rd.bead_off;
+        ld3(reinterpret_cast<const V4<double>*>(r4), i, r);
+        ld3(q4, i, t3);
+        ld3(reinterpret_cast<const V4<double>*>(a.t24) + rd.bead_off, i, t2);
+        const double tt3 = m0 * t3[0] + m1 * t3[1] + m2 * t3[2], tt2 = m0 * t2[0] + m1 * t2[1] + m2 * t2[2];
+        if (on) {
+          double* q = reinterpret_cast<double*>(stage + 3 * k);
+          q[4 + ax] = ax < 3 ? tt3 : 0.0;
+          q[8 + ax] = ax < 3 ? tt2 : 0.0;
+        }
+        double mine[3];  // the bead's tangent, before (even lanes) or after
+        for (int q = 0; q < 3; q++) {
+          const double moved = __shfl_sync(kFull, tt3, quad + q);
+          mine[q] = ax & 1 ? moved : t3[q];
+        }
+        double e = 0.0;
+        if (in >= 0 && in < N) {
+          const bool left = !(ax & 2);
+          double rn[3], tn[3], ra[3], rb[3], ta[3], tb[3];
+          ld3(reinterpret_cast<const V4<double>*>(r4), in, rn);
+          ld3(q4, in, tn);
+          for (int q = 0; q < 3; q++) {
+            ra[q] = left ? rn[q] : r[q];
+            rb[q] = left ? r[q] : rn[q];
+            ta[q] = left ? tn[q] : mine[q];
+            tb[q] = left ? mine[q] : tn[q];
+          }
+          e = bond_e(load_bond<double>(a.bonds + rd.bead_off * 6, left ? in : i), ra, rb, ta, tb);
+        }
+        const double d = __shfl_xor_sync(kFull, e, 1) - e;          // lanes 0 and 2 of four
+        const double de = d + __shfl_down_sync(kFull, d, 2);        // lane 0
+        const double of = __shfl_sync(kFull, de, 4 * (lane & 7));   // bead k0 + (lane & 7)
+        if ((lane >> 3) == ((k0 >> 3) & 3) && k0 + (lane & 7) < m) acc_add(part, of);
       }
     }
     g.pos = axis_base + 2 * (unsigned long long)m;
