@@ -84,6 +84,7 @@ struct SpecShared {
   int stop;
   unsigned accmask;
   int npool;  // entries of the pooled voxel table in use
+  int short_amp;  // largest amplitude of the short path of tangent rotations
   // conflicts among the position moves of a batch, by kind (see batch_limit):
   // decayed counts of batches cut short and of the pairs of moves they tested,
   // and the moves in flight chosen from them

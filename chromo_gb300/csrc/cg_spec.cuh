@@ -2117,6 +2117,8 @@ __global__ void __maxnreg__(sizeof(Pos) == 4 ? 128 : 168) spec_kernel(KArgs a) {
     }
     sh.stop = 0;
     sh.npool = 0;
+    const float n = (float)rd0.n_beads;
+    sh.short_amp = !LEAN && rd0.twist ? (int)fminf(32.0f, sqrtf(8.0f * n)) : (int)fminf(16.0f, sqrtf(0.75f * n));
   }
   __syncthreads();
 
@@ -2137,11 +2139,8 @@ __global__ void __maxnreg__(sizeof(Pos) == 4 ? 128 : 168) spec_kernel(KArgs a) {
           // in flight as are likely to stand (a later move meets the ~3/2 (amp + 1)
           // beads of each earlier accepted one with probability ~3/8 (amp + 1)^2 / N)
           constexpr bool kShort = G == 32 && sizeof(Pos) == 4;
-          const bool twist = !LEAN && sh.ws.rd.twist;
-          const bool brief = kShort && kind == CG_TANGENT_ROTATION && c.amp_bead >= 1 &&
-                             c.amp_bead <= (twist ? 32 : 16) &&
-                             4 * c.amp_bead * c.amp_bead <= (twist ? 32 : 3) * sh.ws.rd.n_beads;
-          const int gs = c.amp_bead <= 8 ? 8 : 16, cap = c.amp_bead <= 16 ? 16 : 32;  // of a short rotation
+          const bool brief = kShort && kind == CG_TANGENT_ROTATION && c.amp_bead >= 1 && c.amp_bead <= sh.short_amp;
+          const int gs = c.amp_bead <= 8 ? 8 : 16, cap = LEAN || c.amp_bead <= 16 ? 16 : 32;  // of a short rotation
           int most = kind <= CG_SLIDE ? sh.limit[kind] : Sn;
           if (brief) {
             const int room = min(min(kMaxS, Sn * (64 / cap)), (int)blockDim.x / gs);
