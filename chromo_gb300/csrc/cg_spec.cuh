@@ -22,9 +22,10 @@
 // rejected move changes nothing; an accepted move only changes its own
 // footprint), for every W and G: each attempted move takes its random numbers
 // from its own Philox4x32-10 sub-stream, indexed by (replica, move number,
-// draw number), and the FP32 path sums dE exactly in fixed point, so neither
-// the spread of beads and voxels over lanes nor the order of hash claims
-// changes a bit.  Acceptance statistics and the controllers' amplitude updates
+// draw number), and dE is summed exactly in fixed point (FP32 storage: every term;
+// FP64 storage: the field's, whose number and order of voxels vary, the bonds' in a
+// fixed order), so neither the spread of beads and voxels over lanes nor the order
+// of hash claims changes a bit.  Acceptance statistics and the controllers' amplitude updates
 // are applied in move order as in the one-move-at-a-time loop
 // (chromo/mc/mc_sim.pyx:88-182).
 //
@@ -46,6 +47,7 @@
 #include <cuda_runtime.h>
 
 #include "cg_device.cuh"
+#include "cg_exact.h"
 #include "cg_kernels.h"
 #include "cg_move.cuh"
 
@@ -654,40 +656,52 @@ __device__ __forceinline__ void pool_voxel_dE(const WarpShared& ws, const KArgs&
   voxel_dE_f64(ws, a, row, v, d, true, part, huge);
 }
 
-// Add the warp's field terms to their moves' plans (s: this lane's move, -1 for
-// none).  Fixed point: q = l2 2^40 + l1 2^20 + l0 with l0, l1 in [0, 2^20);
-// the limbs of at most 4,096 entries sum within 32 bits (|q| < 2^51), so each
-// lane adds its own with four 32-bit shared atomics (a warp's entries belong to
-// a handful of moves; reducing them move by move first took longer: the field
-// phase of a batch of ~5 moves on 256 chains 12.0 k -> 8.5 k cycles).  FP64: a
-// warp reduces each move's terms first.
+// FP64 storage: a move's field dE is summed exactly (cg_exact.h), so that it does not
+// depend on the order of its voxels, which the claims of a table, the warps of a pass
+// and an overflow to another table change.  Terms beyond the limbs' range, 2^-108 ..
+// 2^32, are added in FP64 to `beyond`, order-dependent in their last place.  The limbs
+// are in the move slot's draw buffer, whose last draw was taken when the move was
+// proposed.  (FP64 reductions of a warp's terms, and an FP64 shared atomic each, took
+// 1.90 ms against 1.81 for 200 moves of each of 64 chains of 1,000 beads.)
+static_assert(CGX_LIMBS <= kDrawCache && CGX_LIMBS <= 32, "the limbs share a slot's draw buffer, a lane clears one");
+__device__ __forceinline__ int* move_limbs(const KArgs& a, SpecShared& sh, int s) {
+  return reinterpret_cast<int*>(reinterpret_cast<unsigned char*>(&sh) + a.spec_off_warps +
+                                (size_t)s * a.warp_smem + a.off_draws);
+}
+__device__ __forceinline__ void add_exact(int* L, double* beyond, double x) {
+  int v[4];
+  const int i = cgx_split((unsigned long long)__double_as_longlong(x), v);
+  if (i < 0) {
+    if (!is_zero64(x)) atomicAdd(beyond, x);
+    return;
+  }
+#pragma unroll
+  for (int k = 0; k < 4; k++) atomicAdd(L + i + k, v[k]);
+}
+
+// Add a lane's field term to its move's plan (s; -1: none).  Fixed point: q = l2
+// 2^40 + l1 2^20 + l0 with l0, l1 in [0, 2^20); the limbs of at most 4,096 entries
+// sum within 32 bits (|q| < 2^51), so each lane adds its own with four 32-bit
+// shared atomics (a warp's entries belong to a handful of moves; reducing them move
+// by move first took longer: the field phase of a batch of ~5 moves on 256 chains
+// 12.0 k against 8.5 k cycles).
 __device__ __forceinline__ void add_plan_part(MovePlan& P, const Fx& part) {
   atomicAdd(&P.fl0, (unsigned)(part.q & 0xFFFFF));
   atomicAdd(&P.fl1, (unsigned)((part.q >> 20) & 0xFFFFF));
   atomicAdd(&P.fl2, (int)(part.q >> 40));
   if (!is_zero64(part.hard)) atomicAdd(&P.fh, part.hard);
 }
-__device__ __forceinline__ void add_pool_part(SpecShared& sh, int s, const Fx& part) {
+__device__ __forceinline__ void add_pool_part(const KArgs&, SpecShared& sh, int s, const Fx& part) {
   if (s < 0) return;
   MovePlan& P = sh.plan[s];
   add_plan_part(P, part);
   atomicAdd(&P.fn, 1);
 }
-__device__ __forceinline__ void add_pool_part(SpecShared& sh, int s, double part) {
-  const int lane = (int)(threadIdx.x & 31u);
-  unsigned todo = __ballot_sync(kFull, s >= 0);
-  while (todo) {
-    const int leader = __ffs((int)todo) - 1;
-    const int sl = __shfl_sync(kFull, s, leader);
-    const bool mine = s == sl;
-    const double sum = warp_sum(mine ? part : 0.0);
-    const unsigned who = __ballot_sync(kFull, mine);
-    if (lane == leader) {
-      atomicAdd(&sh.plan[sl].fh, sum);
-      atomicAdd(&sh.plan[sl].fn, __popc(who));
-    }
-    todo &= ~who;
-  }
+__device__ __forceinline__ void add_pool_part(const KArgs& a, SpecShared& sh, int s, double part) {
+  if (s < 0) return;
+  MovePlan& P = sh.plan[s];
+  add_exact(move_limbs(a, sh, s), &P.fh, part);
+  atomicAdd(&P.fn, 1);
 }
 
 // Field dE and conflict registration of the batch's pooled voxel entries, by
@@ -749,7 +763,7 @@ static __device__ void block_field_pool(const KArgs& a, SpecShared& sh, unsigned
       pool_voxel_dE(ws, a, row, v, pvals + (long long)slot * a.hcol, part, hp);
       if (hp) atomicAdd(reinterpret_cast<unsigned long long*>(&P.fH), (unsigned long long)hp);
     }
-    add_pool_part(sh, s, part);
+    add_pool_part(a, sh, s, part);
   }
 }
 
@@ -815,12 +829,15 @@ static __device__ __noinline__ void log_move(const KArgs& a, int rep, unsigned l
 }
 
 // A move's field dE from its plan: fixed point into `soft` (FP32 storage) or
-// FP64 into `hard`.
-__device__ __forceinline__ void plan_field(const MovePlan& P, Fx& soft, double&) {
+// FP64 into `hard` (limbs: move_limbs).
+__device__ __forceinline__ void plan_field(const MovePlan& P, const int*, Fx& soft, double&) {
   soft.q = P.fq + (long long)P.fl2 * 1099511627776LL + (long long)P.fl1 * 1048576LL + (long long)P.fl0;
   soft.hard = P.fh;
 }
-__device__ __forceinline__ void plan_field(const MovePlan& P, double&, double& hard) { hard = P.fh; }
+__device__ __forceinline__ void plan_field(const MovePlan& P, const int* limbs, double&, double& hard) {
+  hard = cgx_value(limbs);
+  if (!is_zero64(P.fh)) hard += P.fh;
+}
 
 // Scratch of move slot `slot`: its shared-memory region, or its region of the
 // global scratch (tables, staging and lists of any size the move can have).
@@ -850,9 +867,49 @@ __device__ __forceinline__ SlotScratch global_slot(const KArgs& a, int rep, int 
   return S;
 }
 
+// Field dE over a move's own table (nu entries, slot s) by its group: fixed point
+// into `soft` (FP32 storage), or into the move's limbs and P.fh (FP64 storage; the
+// limbs and P.fh are zero).
+template <int G>
+__device__ __forceinline__ void own_field(const KArgs& a, SpecShared& sh, int s, const SlotScratch& S, int nu, int gl,
+                                          bool split, long long& nvox, Fx& soft, long long& huge) {
+  double hard = 0;
+  field_dE_voxels<G>(sh.ws, a, a.hcol, S.keys, S.used, S.vals, nu, gl, nvox, soft, hard, huge, split);
+}
+template <int G>
+__device__ __forceinline__ void own_field(const KArgs& a, SpecShared& sh, int s, const SlotScratch& S, int nu, int gl,
+                                          bool split, long long& nvox, double&, long long& huge) {
+  static_assert(G == 32, "a move of FP64 storage has a warp");
+  const long long* grid = a.grid + sh.ws.rd.vox_off * a.ncol;
+  int* limbs = move_limbs(a, sh, s);
+  long long hp = 0;
+  int room = CGX_TERMS;  // terms that the limbs still hold
+  #pragma unroll 1
+  for (int i0 = 0; i0 < nu; i0 += 32) {
+    const int i = i0 + gl;
+    if (i < nu) {
+      const int slot = S.used[i], v = S.keys[slot];
+      long long row[4];
+      load_row(grid + (long long)v * a.ncol, a.ncol, row);
+      double part = 0;
+      voxel_dE_f64(sh.ws, a, row, v, S.vals + (long long)slot * a.hcol, split, part, hp);
+      add_exact(limbs, &sh.plan[s].fh, part);
+    }
+    room -= 32;
+    if (room < 32) {
+      __syncwarp();
+      if (gl == 0) cgx_carry(limbs);
+      __syncwarp();
+      room = CGX_TERMS;
+    }
+  }
+  nvox = nu;
+  huge += gsum<32>(hp);
+  __syncwarp();
+}
 // Field terms of a move left in its plan by own_path.
-__device__ __forceinline__ void store_field(MovePlan& P, const Fx& soft, double) { P.fq = soft.q; P.fh = soft.hard; }
-__device__ __forceinline__ void store_field(MovePlan& P, double, double hard) { P.fh = hard; }
+__device__ __forceinline__ void store_field(MovePlan& P, const Fx& soft) { P.fq = soft.q; P.fh = soft.hard; }
+__device__ __forceinline__ void store_field(MovePlan&, double) {}
 
 // A position move taken by its own group: its deposit (`dep`: the CTA did not
 // deposit it, or it overflowed the shared table it was deposited in) in its
@@ -948,13 +1005,12 @@ static __device__ __noinline__ void own_path(const KArgs& a, SpecShared& sh, int
   oob = gsum<G>(oob);
   __syncwarp();
   Acc soft = acc_zero<Acc>();
-  double hard = 0;
   long long huge = 0, nvox = 0;
   unsigned cmb = 0;
   int regfail = 0;
   if (density) {
     const int nu = run ? *nused : 0;
-    field_dE_voxels<G>(sh.ws, a, hcol, S.keys, S.used, S.vals, nu, gl, nvox, soft, hard, huge, !gtab);
+    own_field<G>(a, sh, s, S, nu, gl, !gtab, nvox, soft, huge);
     // register the touched voxels for the conflict test: the moves that
     // registered a voxel first are this move's conflicts if earlier in the
     // batch; a later move that registered it first learns of this one through
@@ -991,7 +1047,7 @@ static __device__ __noinline__ void own_path(const KArgs& a, SpecShared& sh, int
     P.gtab = gtab;
     P.fn = (int)nvox;
     P.fH = huge;
-    store_field(P, soft, hard);
+    store_field(P, soft);
     if (cmb) atomicOr(&P.cmask, cmb);
     P.freg = regfail;
   }
@@ -1292,7 +1348,7 @@ static __device__ __noinline__ void short_tangent_twist(const KArgs& a, SpecShar
     MovePlan& P = sh.plan[threadIdx.x];
     Fx part;
     double none = 0.0;
-    plan_field(P, part, none);
+    plan_field(P, nullptr, part, none);
     bool dec = false;
     if (!P.err) dec = decide(P.xm, part, Fx{0, 0.0}, 0.0, P.dq, P.dE);
     P.dec = dec ? 1 : 0;
@@ -1456,6 +1512,10 @@ __device__ void propose_position(const KArgs& a, SpecShared& sh, int rep, int s,
   // the Metropolis draw, taken now: the plan holds all of the move's state from here
   unsigned xm = 0;
   if (live && !err && !empty) xm = g.next();
+  if constexpr (sizeof(Pos) == 8) {  // the field sum's limbs
+    __syncwarp();
+    if (live && gl < CGX_LIMBS) move_limbs(a, sh, s)[gl] = 0;
+  }
   if (m > a.stage_cap) gstage = 1;
   // voxel table: the CTA's pooled table for every move of up to
   // kPoolMaxBeads beads, optimistically (a pool past 3/4 load sends the move
@@ -1547,7 +1607,7 @@ __device__ __forceinline__ void decide_position(const KArgs& a, SpecShared& sh, 
   if (P.m > 0) {
     acc_add(dEp, load_acc<Acc>(P.pq[0], P.ph[0]));
     acc_add(dEp, load_acc<Acc>(P.pq[1], P.ph[1]));
-    plan_field(P, dEs, dEh);
+    plan_field(P, move_limbs(a, sh, s), dEs, dEh);
     const int oo = P.oob;
     dEH = P.fH + (((long long)(oo >> 16) - (long long)(oo & 0xFFFF)) << 40);
     err |= P.derr & ~E_OVF;
@@ -1603,6 +1663,7 @@ __device__ void evaluate_move(const KArgs& a, SpecShared& sh, int rep, int s, in
   long long dEH = 0;  // the exact 1e99 penalties, in kHugeUnit units
   int nvox = 0;
   const bool empty = !live;
+  unsigned xm = 0;  // the decision's draw
   int gtab = 0, gstage = 0, regfail = 0;
   const int Hs = 1 << a.logH;
 
@@ -1769,6 +1830,13 @@ __device__ void evaluate_move(const KArgs& a, SpecShared& sh, int rep, int s, in
       if (!err) segment_of(b0, b1, N, ind0, indf);
     }
     m = (!live || err) ? 0 : indf - ind0;
+    if constexpr (sizeof(Pos) == 8) {  // the decision's draw, then the field sum's limbs in the buffer
+      if (live) xm = g.word(g.pos);
+      __syncwarp();
+      if (live && gl < CGX_LIMBS) move_limbs(a, sh, s)[gl] = 0;
+      if (live && gl == 0) P.fh = 0;
+      __syncwarp();
+    }
     const int nt = rd.sites[bsel];
     if (m > a.stage_cap) gstage = 1;
     if (8 * m > Hs) gtab = 1;
@@ -1832,7 +1900,8 @@ __device__ void evaluate_move(const KArgs& a, SpecShared& sh, int rep, int s, in
     __syncwarp();
     if (density) {
       long long nv = 0;
-      field_dE_voxels<G>(ws, a, hcol, S.keys, S.used, S.vals, *nused, gl, nv, dEs, dEh, dEH, !gtab);
+      own_field<G>(a, sh, s, S, *nused, gl, !gtab, nv, dEs, dEH);
+      if constexpr (sizeof(Pos) == 8) plan_field(P, move_limbs(a, sh, s), dEs, dEh);
       nvox = (int)nv;
       if (m > 0) add_intra(ws, bsel, ddb, dEs, dEh);
     }
@@ -1855,7 +1924,10 @@ __device__ void evaluate_move(const KArgs& a, SpecShared& sh, int rep, int s, in
   long long dq = 0;
   double dh = 0;
   if (live && !err && !empty) {
-    dec = decide(g.next(), dEp, dEs, with_huge(dEh, dEH), dq, dh);
+    const bool taken = sizeof(Pos) == 8 && kind != CG_TANGENT_ROTATION;
+    if (taken) g.pos++;
+    else xm = g.next();
+    dec = decide(xm, dEp, dEs, with_huge(dEh, dEH), dq, dh);
   }
   if (gl == 0 && live) {
     P.dq = dq;
