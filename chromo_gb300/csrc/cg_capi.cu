@@ -385,9 +385,9 @@ static int moves_in_flight(const cg_sim* s, int w_req, int W, int G) {
 // resident per SM -- those every replica needs to run at once, or fewer when the
 // register file holds fewer CTAs of W warps (the replicas then run in waves) --
 // share the SM's shared memory; each move slot gets the largest voxel table that
-// then fits.  A shape of the library's own leaves room for a pooled table: with
-// fewer warps and, of one warp, with fewer CTAs per SM than would otherwise run,
-// since without it moves of more than ~16 beads go to tables in global memory (2 MC
+// then fits.  Shapes leave room for a pooled table: the library's own with fewer
+// warps, then, as a caller's, with fewer CTAs per SM than would otherwise run, since
+// without it moves of more than ~16 beads go to tables in global memory (2 MC
 // steps of 1,216 chains of 50 beads: 1 warp 1.24 ms, 2 warps without a table 2.38; of
 // 2,432 chains of 200 beads: fewer CTAs per SM 2.75 ms, all without a table 5.01).
 static int choose_shape(cg_sim* s, int w_req, int g_req) {
@@ -420,8 +420,8 @@ static int choose_shape(cg_sim* s, int w_req, int g_req) {
           s->layout(l, sc);
           if (s->cta_layout(lhb, W, G, S, t) <= budget) { lhp = t; lh = l; }
         }
-      if (lhp == 0 && w_req == 0 && (W > 1 || ctas_per_sm > 1)) {
-        if (W > 1) W--;
+      if (lhp == 0 && ((w_req == 0 && W > 1) || ctas_per_sm > 1)) {
+        if (w_req == 0 && W > 1) W--;
         else ctas_per_sm--;
         continue;
       }
