@@ -487,13 +487,20 @@ int cg_create(const cg_config* cfg, cg_sim** out) {
     cg_destroy(s);
     return fail(CG_ERR_ARG, "lanes_per_move must be 8, 16 or 32 (32 with FP64 storage)");
   }
-  if (cfg->warps_per_block < 0 || cfg->warps_per_block > cg::kUserMaxW) {
+  const int w_req = cfg->warps_per_block;
+  if (w_req < 0 || w_req > cg::kMaxW) {
     cg_destroy(s);
-    return fail(CG_ERR_ARG, "warps_per_block must be in 0..12");
+    return fail(CG_ERR_ARG, "warps_per_block must be in 0..12, or the library's own choice");
   }
-  if (int rc = choose_shape(s, cfg->warps_per_block, cfg->lanes_per_move)) {
+  // more than kUserMaxW warps: only as cg_get_launch_shape reports the library's own
+  // choice for such a simulation, and then that shape
+  if (int rc = choose_shape(s, w_req > cg::kUserMaxW ? 0 : w_req, cfg->lanes_per_move)) {
     cg_destroy(s);
     return rc;
+  }
+  if (w_req > cg::kUserMaxW && w_req != s->spec_w) {
+    cg_destroy(s);
+    return fail(CG_ERR_ARG, "warps_per_block must be in 0..12, or the library's own choice");
   }
   const long long RW = (long long)s->R * s->spec_s;
   // tangent-rotation bitmaps: one per (replica, move slot)

@@ -102,7 +102,10 @@ typedef struct {
     int32_t n_replicas;
     int32_t pos_fp64;          /* 1: positions stored in FP64, 0: in FP32 */
     int32_t n_binders;         /* 1..CG_MAX_BINDERS (same for every replica) */
-    int32_t warps_per_block;   /* 0: chosen by the library */
+    int32_t warps_per_block;   /* 1..12, with warps * 32 / lanes moves in flight (at most 32);
+                                  0, or the number that cg_get_launch_shape reports for it
+                                  where that is above 12: chosen by the library, with FP32
+                                  storage and 32 lanes fewer moves in flight than warps */
     const int64_t *n_beads;    /* [n_replicas] */
     const int32_t *grid_dims;  /* [n_replicas * 3] voxels in x, y, z (1,1,1 without a field) */
     int64_t max_segment;       /* largest bead amplitude of a segment move + 1 */
@@ -326,9 +329,13 @@ int cg_get_launch_info(cg_sim *sim, int32_t *warps_per_block, int32_t *hash_slot
                        int64_t *kernels_launched);
 
 /* Launch shape of the MC kernel: warps per replica CTA, lanes per move, moves
- * in flight per replica (warps * 32 / lanes) and shared voxel-table slots per
- * move.  No counterpart in the reference (its loop runs one move at a time);
- * the autotuner (chromo_gb300.autotune) reads it. */
+ * in flight per replica (warps * 32 / lanes, at most 32, for warps_per_block 1..12;
+ * 3/4 of the warps for the library's own shape with FP32 storage and 32 lanes) and
+ * shared voxel-table slots.  The warps and lanes reported are accepted by cg_create;
+ * a shape of the library's own with up to 12 warps is had again only with
+ * warps_per_block 0, since the number itself asks for as many moves as warps.  No
+ * counterpart in the reference (its loop runs one move at a time); the autotuner
+ * (chromo_gb300.autotune) reads it. */
 int cg_get_launch_shape(cg_sim *sim, int32_t *warps_per_block, int32_t *lanes_per_move,
                         int32_t *moves_in_flight, int32_t *hash_slots);
 
