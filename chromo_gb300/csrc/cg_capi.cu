@@ -1171,7 +1171,7 @@ int cg_gradient(cg_sim* s, float* dEdr, double* terms) {
   if (!s) return fail(CG_ERR_ARG, "null sim");
   if (int rc = ensure_derivative_buffers(s)) return rc;
   KArgs a = s->args();
-  if (dEdr) cg_launch_gradient(a, s->fp64 != 0, s->grad, s->max_beads, 0);
+  if (dEdr) cg_launch_gradient(a, s->fp64 != 0, s->grad, s->max_beads, s->n_sm, 0);
   if (terms) cg_launch_terms(a, s->terms, nullptr, 0);
   CUDA_TRY(cudaGetLastError());
   if (dEdr) CUDA_TRY(cudaMemcpy(dEdr, s->grad, sizeof(float) * 3 * s->total_beads, cudaMemcpyDeviceToHost));
@@ -1207,7 +1207,8 @@ int cg_gradient_device(cg_sim* s, double* dEdr, double* dEdt3, void* stream) {
   if (!s) return fail(CG_ERR_ARG, "null sim");
   if (!dEdr) return fail(CG_ERR_ARG, "dEdr is required");
   if (dEdt3 && s->twist) return fail(CG_ERR_ARG, "dE/dt3 does not include SSTWLC twist terms");
-  cg_launch_gradient64(s->args(), s->fp64 != 0, dEdr, dEdt3, s->max_beads, (cudaStream_t)stream);
+  cg_launch_gradient64(s->args(), s->fp64 != 0, dEdr, dEdt3, s->max_beads, s->n_sm,
+                       (cudaStream_t)stream);
   CUDA_TRY(cudaGetLastError());
   return CG_OK;
 }

@@ -336,23 +336,25 @@ __global__ void __cluster_dims__(kSumCtas, 1, 1) __launch_bounds__(kSumThreads)
 // wave of CTAs (5 per SM) remains, up to 8: a CTA's constants take ~200 FP64
 // operations, a pass ~170 a warp.  64 chains of 5,000 beads with the read-back:
 // one pass a warp 210 us, two waves of CTAs 195, one 183.
-static dim3 gradient_grid(const cg::KArgs& a, long long max_beads) {
+static dim3 gradient_grid(const cg::KArgs& a, long long max_beads, int n_sm) {
   const long long passes = (max_beads + 29) / 30;
-  const long long per = std::min<long long>(8, std::max<long long>(1, passes * a.n_reps / (4 * 5 * 152)));
+  const long long per =
+      std::min<long long>(8, std::max<long long>(1, passes * a.n_reps / (4 * 5 * std::max(1, n_sm))));
   long long bx = (passes + 4 * per - 1) / (4 * per);
   if (bx < 1) bx = 1;
   return dim3((unsigned)bx, (unsigned)a.n_reps);
 }
 
-void cg_launch_gradient(const cg::KArgs& a, bool fp64, float* out, long long max_beads, cudaStream_t s) {
-  const dim3 grid = gradient_grid(a, max_beads);
+void cg_launch_gradient(const cg::KArgs& a, bool fp64, float* out, long long max_beads, int n_sm,
+                        cudaStream_t s) {
+  const dim3 grid = gradient_grid(a, max_beads, n_sm);
   if (fp64) cg::gradient_kernel<double, float><<<grid, 128, 0, s>>>(a, out, nullptr);
   else cg::gradient_kernel<float, float><<<grid, 128, 0, s>>>(a, out, nullptr);
 }
 
 void cg_launch_gradient64(const cg::KArgs& a, bool fp64, double* out, double* out_t3, long long max_beads,
-                          cudaStream_t s) {
-  const dim3 grid = gradient_grid(a, max_beads);
+                          int n_sm, cudaStream_t s) {
+  const dim3 grid = gradient_grid(a, max_beads, n_sm);
   if (fp64) cg::gradient_kernel<double, double><<<grid, 128, 0, s>>>(a, out, out_t3);
   else cg::gradient_kernel<float, double><<<grid, 128, 0, s>>>(a, out, out_t3);
 }

@@ -202,9 +202,10 @@ namespace cg {
 constexpr int kTerms = 14;                                // energy terms per replica (cg_grad.cu)
 constexpr int kAccPerRep = kTerms + kTerms * kTerms + 1;  // running sums of T, T T^T, count
 }
-void cg_launch_gradient(const cg::KArgs& a, bool fp64, float* out, long long max_beads, cudaStream_t s);
+void cg_launch_gradient(const cg::KArgs& a, bool fp64, float* out, long long max_beads, int n_sm,
+                        cudaStream_t s);
 void cg_launch_gradient64(const cg::KArgs& a, bool fp64, double* out, double* out_t3, long long max_beads,
-                          cudaStream_t s);
+                          int n_sm, cudaStream_t s);
 void cg_launch_host_load(const cg::KArgs& a, bool fp64, const void* tab, int R, long long max_beads, int nb,
                          unsigned* flag, int mode, cudaStream_t s);
 void cg_launch_host_store(const cg::KArgs& a, bool fp64, const void* tab, int R, long long max_beads, int nb,
