@@ -54,6 +54,7 @@ struct cg_sim {
   std::vector<long long> n_beads, bead_off, n_vox, vox_off, picked_off;
   std::vector<int> dims;
   long long total_beads = 0, total_vox = 0, total_picked = 0;
+  long long work_max = 0, work_sum = 0;  // of the energies' sums: 32 per bead, 1 per voxel
   long long max_segment = 0, max_tangent = 0, max_beads = 0, max_vox = 0;
   int n_ctl = 5;
   long long kernels = 0;
@@ -247,6 +248,22 @@ struct cg_sim {
     a.mu_swaps = mu_swaps; a.mu_swap_attempts = mu_swap_attempts;
     a.lean = n_full == 0 ? 1 : 0;
     return a;
+  }
+
+  // CTAs per replica of the sums over beads and voxels, as a power of two: a replica's
+  // part takes a CTA ~8 us before its first bead, so a replica is split only as far
+  // as its share of the work asks for on ~5/4 CTAs per SM, and into parts of some
+  // size (4,096 voxels, or as much, 16,384 where the parts outnumber the SMs).
+  // Energies, us, with 1 / 2 / 4 / 8 CTAs per replica: 2,000 chains of 30 beads and
+  // 4^3 voxels 75 / 158 / 297 / 630 (98 before the clusters), 256 of 2,000 and 30^3
+  // 74 / 86 / 111 / 160, 64 of 5,000 and 40^3 127 / 76 / 53 / 63, one of 20,000 and
+  // 60^3 297 / 156 / 86 / 51.
+  int sum_log() const {
+    int log = 0;
+    while (log < 3 && (work_max >> log) * 5 * n_sm > 4 * work_sum &&
+           work_max >> (log + 1) >= ((long long)R << (log + 1) > n_sm ? 16384 : 4096))
+      log++;
+    return log;
   }
 
   // Region of one move slot for voxel-table capacity 2^lh and staging
@@ -479,6 +496,8 @@ int cg_create(const cg_config* cfg, cg_sim** out) {
     s->total_picked += (n + 31) / 32;
     s->max_beads = std::max(s->max_beads, n);
     s->max_vox = std::max(s->max_vox, (long long)nx * ny * nz);
+    s->work_max = std::max(s->work_max, 32 * n + (long long)nx * ny * nz);
+    s->work_sum += 32 * n + (long long)nx * ny * nz;
   }
   s->g_logH = next_log2(32 * s->max_segment);
   s->g_stage_cap = std::max(s->max_segment, s->max_tangent);
@@ -1138,7 +1157,7 @@ int cg_run_audit(cg_sim* s, int rep, int64_t n_steps, const uint32_t* draws, int
 int cg_energy(cg_sim* s, int rep, double* out) {
   if (int rc = check_rep(s, rep)) return rc;
   KArgs a = s->args();
-  cg_launch_energy(a, s->fp64, s->eout, 0);
+  cg_launch_energy(a, s->fp64, s->sum_log(), s->eout, 0);
   CUDA_TRY(cudaGetLastError());
   double buf[5];
   CUDA_TRY(cudaMemcpy(buf, s->eout + 5 * rep, sizeof buf, cudaMemcpyDeviceToHost));
@@ -1150,7 +1169,7 @@ int cg_energies(cg_sim* s, double* out, void* stream) {
   if (!s || !out) return fail(CG_ERR_ARG, "null argument");
   cudaStream_t st = (cudaStream_t)stream;
   KArgs a = s->args();
-  cg_launch_energy(a, s->fp64, s->eout, st);
+  cg_launch_energy(a, s->fp64, s->sum_log(), s->eout, st);
   CUDA_TRY(cudaGetLastError());
   CUDA_TRY(cudaMemcpyAsync(out, s->eout, sizeof(double) * 5 * s->R, cudaMemcpyDeviceToHost, st));
   CUDA_TRY(cudaStreamSynchronize(st));
@@ -1172,7 +1191,7 @@ int cg_gradient(cg_sim* s, float* dEdr, double* terms) {
   if (int rc = ensure_derivative_buffers(s)) return rc;
   KArgs a = s->args();
   if (dEdr) cg_launch_gradient(a, s->fp64 != 0, s->grad, s->max_beads, s->n_sm, 0);
-  if (terms) cg_launch_terms(a, s->terms, nullptr, 0);
+  if (terms) cg_launch_terms(a, s->sum_log(), s->terms, nullptr, 0);
   CUDA_TRY(cudaGetLastError());
   if (dEdr) CUDA_TRY(cudaMemcpy(dEdr, s->grad, sizeof(float) * 3 * s->total_beads, cudaMemcpyDeviceToHost));
   if (terms) CUDA_TRY(cudaMemcpy(terms, s->terms, sizeof(double) * cg::kTerms * s->R, cudaMemcpyDeviceToHost));
@@ -1198,7 +1217,7 @@ int cg_deposit_async(cg_sim* s, void* stream) {
 
 int cg_energies_device(cg_sim* s, double* out, void* stream) {
   if (!s || !out) return fail(CG_ERR_ARG, "null argument");
-  cg_launch_energy(s->args(), s->fp64, out, (cudaStream_t)stream);
+  cg_launch_energy(s->args(), s->fp64, s->sum_log(), out, (cudaStream_t)stream);
   CUDA_TRY(cudaGetLastError());
   return CG_OK;
 }
@@ -1216,7 +1235,7 @@ int cg_gradient_device(cg_sim* s, double* dEdr, double* dEdt3, void* stream) {
 int cg_sample_terms(cg_sim* s, void* stream) {
   if (!s) return fail(CG_ERR_ARG, "null sim");
   if (int rc = ensure_derivative_buffers(s)) return rc;
-  cg_launch_terms(s->args(), nullptr, s->acc, (cudaStream_t)stream);
+  cg_launch_terms(s->args(), s->sum_log(), nullptr, s->acc, (cudaStream_t)stream);
   CUDA_TRY(cudaGetLastError());
   return CG_OK;
 }
@@ -1252,7 +1271,7 @@ int cg_reset_tally(cg_sim* s) {
 
 static int enqueue_exchange(cg_sim* s, int n_rungs, long long round, uint64_t seed, cudaStream_t st) {
   KArgs a = s->args();
-  cg_launch_chi_sum(a, s->eout, st);
+  cg_launch_chi_sum(a, s->sum_log(), s->eout, st);
   cg_launch_exchange(a, s->eout, n_rungs, round, seed, st);
   return CG_OK;
 }

@@ -73,80 +73,151 @@ __device__ __forceinline__ void voxel_energy(const KArgs& a, const RepDev& rd, l
 
 // ---------------------------------------------------------------- sums of one replica
 // The energies, the exchange's S and the derivative terms are sums over one
-// replica's beads and voxels.  A replica is taken by a cluster of kSumCtas
-// CTAs, whose partial sums meet in distributed shared memory and are added in
-// rank order: no workspace, the same bits every time, and 8 x R CTAs in flight
-// (one CTA per replica left most of the GPU idle below 152 replicas).  FP64
-// runs at 1/64 of the FP32 rate here, so the loops hold only the FP64
-// operations the sums need: rows of empty voxels are skipped (two thirds of a
-// 40^3 grid of a 5,000-bead chain), the volume factors are applied once to the
-// sums of products of fixed-point values (uniform volumes), vf > vf_limit is an
-// integer comparison, products are FMAs, and each bond's bead before it comes
-// from the neighbouring lane, already converted.  Upload, deposit and energies
-// of 256 chains of 2,000-20,000 beads: 7.06 -> 2.90 ms (the energies alone took
-// 4.6 ms with one CTA per replica and five divisions a voxel).
-constexpr int kSumCtas = 8;
+// replica's beads and voxels.  A replica is taken by a cluster of 1 to 8 CTAs
+// (cg_sim::sum_log), whose partial sums meet in distributed shared memory and are
+// added in rank order: no workspace, the same bits every time.  FP64 runs at 1/64 of
+// the FP32 rate here, so the loops hold only the FP64 operations the sums need: rows
+// of empty voxels are skipped (two thirds of a 40^3 grid of a 5,000-bead chain), the
+// volume factors are applied once to the sums of products of fixed-point values
+// (uniform volumes), vf > vf_limit is an integer comparison, products are FMAs, and
+// each bond's bead before it comes from the neighbouring lane, already converted (64
+// chains of 5,000 beads: energies 53 us, 2.05 ms with a CTA per replica and five
+// divisions a voxel).
 constexpr int kSumThreads = 256;
+
+// A CTA's replica and its part of the replica's beads or voxels: one of 2^log_ctas.
+struct SumPart {
+  int rep, rank, log_ctas;
+  explicit __device__ __forceinline__ SumPart(int log)
+      : rep((int)(blockIdx.x >> log)), rank((int)(blockIdx.x & ((1u << log) - 1u))), log_ctas(log) {}
+  __device__ __forceinline__ void of(long long n, long long& lo, long long& hi) const {
+    const long long per = (n + (1 << log_ctas) - 1) >> log_ctas;
+    lo = rank * per;
+    hi = lo + per < n ? lo + per : n;
+  }
+};
+
+// Launch of one of the sum kernels: a cluster of 2^log_ctas CTAs per replica.
+template <class... P, class... A>
+static void launch_sums(void (*kernel)(KArgs, int, P...), const KArgs& a, int log_ctas, cudaStream_t s, A... args) {
+  cudaLaunchAttribute at{};
+  at.id = cudaLaunchAttributeClusterDimension;
+  at.val.clusterDim.x = 1u << log_ctas;
+  at.val.clusterDim.y = at.val.clusterDim.z = 1;
+  cudaLaunchConfig_t c{};
+  c.gridDim = dim3((unsigned)a.n_reps << log_ctas);
+  c.blockDim = dim3(kSumThreads);
+  c.stream = s;
+  c.attrs = &at;
+  c.numAttrs = log_ctas > 0 ? 1 : 0;
+  cudaLaunchKernelEx(&c, kernel, a, log_ctas, P(args)...);
+}
+
+// The warps' sums in sh added in warp order, then the CTAs' in rank order, valid in the
+// first 16 threads of rank 0.
+__device__ __forceinline__ double over_ctas(double (*sh)[16]) {
+  namespace cgr = cooperative_groups;
+  cgr::cluster_group cl = cgr::this_cluster();
+  double t = 0;
+  if (threadIdx.x < 16)
+    #pragma unroll 1
+    for (int w = 0; w < kSumThreads / 32; w++)
+      if (!is_zero64(sh[w][threadIdx.x])) t += sh[w][threadIdx.x];
+  if (cl.num_blocks() == 1) return t;
+  if (threadIdx.x < 16) sh[0][threadIdx.x] = t;
+  cl.sync();
+  if (cl.block_rank() == 0 && threadIdx.x < 16)
+    #pragma unroll 1
+    for (int r = 1; r < (int)cl.num_blocks(); r++) t += cl.map_shared_rank(&sh[0][0], r)[threadIdx.x];
+  cl.sync();  // no CTA leaves while its sums are read
+  return t;
+}
 
 // 16 sums over the CTAs of a cluster, valid in the first 16 threads of rank 0
 // (thread k: sum k).  Every thread of the cluster calls it.  Within a warp the
 // lanes halve the set of sums they carry at each step (16 FP64 additions
 // instead of 80).
 __device__ __forceinline__ double cluster_sums(double (&v)[16], double (*sh)[16]) {
-  namespace cgr = cooperative_groups;
-  cgr::cluster_group cl = cgr::this_cluster();
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  bool any = false;  // of few beads or voxels most warps hold zeros
 #pragma unroll
-  for (int h = 8, o = 16; h >= 1; h >>= 1, o >>= 1) {
-    const bool up = lane & o;
+  for (int k = 0; k < 16; k++) any = any || !is_zero64(v[k]);
+  if (__any_sync(kFull, any)) {
 #pragma unroll
-    for (int k = 0; k < h; k++) {
-      const double keep = up ? v[k + h] : v[k], give = up ? v[k] : v[k + h];
-      v[k] = keep + __shfl_xor_sync(kFull, give, o);
+    for (int h = 8, o = 16; h >= 1; h >>= 1, o >>= 1) {
+      const bool up = lane & o;
+#pragma unroll
+      for (int k = 0; k < h; k++) {
+        const double keep = up ? v[k + h] : v[k], give = up ? v[k] : v[k + h];
+        v[k] = keep + __shfl_xor_sync(kFull, give, o);
+      }
     }
+    v[0] += __shfl_xor_sync(kFull, v[0], 1);
+  } else {
+    v[0] = 0.0;
   }
-  v[0] += __shfl_xor_sync(kFull, v[0], 1);
   // lane l holds sum (bits 4, 3, 2, 1 of l as bits 3, 2, 1, 0)
   if (!(lane & 1)) sh[warp][lane >> 1] = v[0];
   __syncthreads();
-  double t = 0;
-  if (threadIdx.x < 16) {
-    for (int w = 0; w < kSumThreads / 32; w++) t += sh[w][threadIdx.x];
-    sh[0][threadIdx.x] = t;
-  }
-  cl.sync();
-  if (cl.block_rank() == 0 && threadIdx.x < 16)
-    for (int r = 1; r < kSumCtas; r++) t += cl.map_shared_rank(&sh[0][0], r)[threadIdx.x];
-  cl.sync();  // no CTA leaves while its sums are read
-  return t;
+  return over_ctas(sh);
+}
+// The sum of one number over the CTAs of a cluster, by the additions of cluster_sums,
+// valid in thread 0 of rank 0.
+__device__ __forceinline__ double cluster_sum(double v, double (*sh)[16]) {
+  const bool any = !is_zero64(v);
+  if (__any_sync(kFull, any))
+#pragma unroll
+    for (int o = 16; o >= 1; o >>= 1) v += __shfl_xor_sync(kFull, v, o);
+  else
+    v = 0.0;
+  if ((threadIdx.x & 31) < 16) sh[threadIdx.x >> 5][threadIdx.x & 31] = v;
+  __syncthreads();
+  return over_ctas(sh);
 }
 
-// Largest fixed-point bead weight of a voxel whose volume fraction, as the
-// FP64 expression of voxel_energy gives it, is not above vf_limit (that
-// expression does not decrease with the weight).  Uniform volumes.
-__device__ __forceinline__ long long weight_at_limit(const RepDev& rd) {
-  auto over = [&](long long n) { return ((double)n * kFxInv) / rd.vol_bin * rd.bead_vol > rd.vf_limit; };
+// The line of vf_limit in fixed-point bead weights, uniform volumes: the volume
+// fraction, as the FP64 expression of voxel_energy gives it, is not above the limit
+// for weights up to `sure` and above it beyond `over`; the few between take the
+// expression itself (it does not decrease with the weight).
+struct Limit {
+  long long sure, over;
+};
+__device__ __forceinline__ bool weight_is_over(const RepDev& rd, long long n) {
+  return ((double)n * kFxInv) / rd.vol_bin * rd.bead_vol > rd.vf_limit;
+}
+__device__ __forceinline__ Limit limit_of(const RepDev& rd) {
   const double est = rd.vf_limit / rd.bead_vol * rd.vol_bin * kFxScale;
-  if (!(est < 4e18)) return 0x7FFFFFFFFFFFFFFFLL;
-  if (!(est > 0)) return over(0) ? -1 : 0;  // limits of 0 and below: only empty voxels, or none
-  long long lo = (long long)(est * (1 - 4e-15)) - 2, hi = (long long)(est * (1 + 4e-15)) + 2;
-  if (lo < 0) lo = 0;
-  while (hi - lo > 1) {
-    const long long mid = lo + (hi - lo) / 2;
-    if (over(mid)) hi = mid;
-    else lo = mid;
+  if (!(est < 4e18)) return Limit{0x7FFFFFFFFFFFFFFFLL, 0x7FFFFFFFFFFFFFFFLL};
+  if (!(est > 0)) {  // limits of 0 and below: only empty voxels, or none
+    const long long w = weight_is_over(rd, 0) ? -1 : 0;
+    return Limit{w, w};
   }
-  return lo;
+  const long long lo = (long long)(est * (1 - 4e-15)) - 2, hi = (long long)(est * (1 + 4e-15)) + 2;
+  return Limit{lo < 0 ? 0 : lo, hi};
+}
+static __device__ __noinline__ bool near_limit(const RepDev& rd, long long n) { return weight_is_over(rd, n); }
+__device__ __forceinline__ bool above_limit(const RepDev& rd, const Limit& lim, long long n) {
+  return n > lim.sure && (n > lim.over || near_limit(rd, n));
+}
+// The largest weight not above the limit.
+__device__ __forceinline__ long long weight_at_limit(const RepDev& rd) {
+  Limit l = limit_of(rd);
+  while (l.over - l.sure > 1) {
+    const long long mid = l.sure + (l.over - l.sure) / 2;
+    if (weight_is_over(rd, mid)) l.over = mid;
+    else l.sure = mid;
+  }
+  return l.sure;
 }
 
 // One CTA's part of a replica's voxels: f(voxel, row) for its thread's rows, or
 // (SKIP) for those of them that are not empty; g() after every kRowsInFlight.
 constexpr int kRowsInFlight = 4;
 template <bool SKIP, class F, class G>
-__device__ __forceinline__ void for_each_row(const KArgs& a, const RepDev& rd, int rank, const F& f, const G& g) {
+__device__ __forceinline__ void for_each_row(const KArgs& a, const RepDev& rd, SumPart part, const F& f, const G& g) {
   const long long* grid = a.grid + rd.vox_off * a.ncol;
-  const long long per = (rd.n_vox + kSumCtas - 1) / kSumCtas;
-  const long long v0 = rank * per, v1 = v0 + per < rd.n_vox ? v0 + per : rd.n_vox;
+  long long v0, v1;
+  part.of(rd.n_vox, v0, v1);
   constexpr int U = kRowsInFlight;
   for (long long v = v0 + threadIdx.x; v < v1; v += U * kSumThreads) {
     long long row[U][4];
@@ -164,8 +235,8 @@ __device__ __forceinline__ void for_each_row(const KArgs& a, const RepDev& rd, i
   }
 }
 template <bool SKIP, class F>
-__device__ __forceinline__ void for_each_row(const KArgs& a, const RepDev& rd, int rank, const F& f) {
-  for_each_row<SKIP>(a, rd, rank, f, [] {});
+__device__ __forceinline__ void for_each_row(const KArgs& a, const RepDev& rd, SumPart part, const F& f) {
+  for_each_row<SKIP>(a, rd, part, f, [] {});
 }
 
 // Non-uniform volumes: an empty voxel adds nothing, unless its volume is not
@@ -204,6 +275,7 @@ __device__ __forceinline__ void fx_product(FxSum& s, unsigned l0, unsigned h0, u
 // The sum in FP64 (one conversion, of its leading 64 bits); `shift` is 26, or 27
 // for squares.
 __device__ __forceinline__ double fx_value(const FxSum& s, int shift) {
+  if (!(s.ll | s.lh | s.hh)) return 0.0;
   unsigned long long lo = s.ll, hi = s.lh >> (64 - shift), t = s.lh << shift;
   lo += t;
   hi += lo < t ? 1 : 0;
@@ -287,12 +359,12 @@ __device__ __forceinline__ void drain_sums(int nb, GridSums& s, RestSums& rest) 
   s.rest = true;
 }
 // The sums of one CTA's part of a replica: out[kRest00 .. kRestVf].
-__device__ __forceinline__ void grid_sums(const KArgs& a, const RepDev& rd, int rank, long long gmax, RestSums& rest,
+__device__ __forceinline__ void grid_sums(const KArgs& a, const RepDev& rd, SumPart part, long long gmax, RestSums& rest,
                                           double (&out)[kRests]) {
   GridSums s;
   init_sums(s, rest);
   const int nb = rd.nb;
-  for_each_row<true>(a, rd, rank, [&](long long, const long long (&row)[4]) { add_row(rd, gmax, row, s, rest); },
+  for_each_row<true>(a, rd, part, [&](long long, const long long (&row)[4]) { add_row(rd, gmax, row, s, rest); },
                      [&] { drain_sums(nb, s, rest); });
   out[kRestOver] = out[kRestVf] = 0.0;
   sum_values(s, nb, [&](int k, double x) { out[k] = x; });
@@ -323,14 +395,14 @@ __device__ __forceinline__ double bond_energy(const double* b, const double r0[3
 // bound beyond max_binders.  A warp takes 31 bonds a pass: lane l holds bead
 // i0 + l, converted once, and its bond to lane l - 1's bead.
 template <typename Pos>
-__device__ __forceinline__ void bead_sums(const KArgs& a, const RepDev& rd, int rank, const double* bf, double& el,
+__device__ __forceinline__ void bead_sums(const KArgs& a, const RepDev& rd, SumPart part, const double* bf, double& el,
                                           double& bi, int (&dbl)[CG_MAX_BINDERS], long long& excess) {
   const V4<Pos>* r4 = reinterpret_cast<const V4<Pos>*>(a.r4) + rd.bead_off;
   const V4<Pos>* t34 = reinterpret_cast<const V4<Pos>*>(a.t34) + rd.bead_off;
   const V4<Pos>* t24 = reinterpret_cast<const V4<Pos>*>(a.t24) + rd.bead_off;
   const double* bonds = a.bonds + rd.bead_off * 6;
-  const long long N = rd.n_beads, per = (N + kSumCtas - 1) / kSumCtas;
-  const long long b0 = rank * per, b1 = b0 + per < N ? b0 + per : N;
+  long long b0, b1;
+  part.of(rd.n_beads, b0, b1);
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   // lane 0's bead is the one before the pass's first
   for (long long i0 = b0 - 1 + 31LL * warp; i0 + 1 < b1; i0 += 31LL * (kSumThreads / 32)) {

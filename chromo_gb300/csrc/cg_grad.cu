@@ -256,13 +256,14 @@ __global__ void __launch_bounds__(128) gradient_kernel(KArgs a, Out* out, Out* o
 // [7..9] #(state_b == 2), [10..12] sum_i s_ib, [13] sum_v (W / V)^2 with W the
 // bead weight of the voxel.  acc (or null): running sums [T, T T^T, count].
 // A cluster per replica (see cg_energy.cuh).
-__global__ void __cluster_dims__(kSumCtas, 1, 1) __launch_bounds__(kSumThreads)
-    terms_kernel(KArgs a, double* terms, double* acc) {
+__global__ void __launch_bounds__(kSumThreads)
+    terms_kernel(KArgs a, int log_ctas, double* terms, double* acc) {
   __shared__ double sh[kSumThreads / 32][16];
   __shared__ double T[16];
   __shared__ RestSums rest;
   __shared__ long long gmax_sh;
-  const int rep = blockIdx.x / kSumCtas, rank = blockIdx.x % kSumCtas;
+  const SumPart part(log_ctas);
+  const int rep = part.rep, rank = part.rank;
   const RepDev& rd = a.reps[rep];
   const bool field = rd.field_kind == 2, uniform = field && !rd.has_access;
   if (threadIdx.x == 0) gmax_sh = uniform ? weight_at_limit(rd) : 0;
@@ -271,9 +272,9 @@ __global__ void __cluster_dims__(kSumCtas, 1, 1) __launch_bounds__(kSumThreads)
   long long sum[CG_MAX_BINDERS] = {0, 0, 0};
   {
     const unsigned* st = a.states + rd.bead_off;
-    const long long per = (rd.n_beads + kSumCtas - 1) / kSumCtas;
-    const long long b1 = (rank + 1) * per < rd.n_beads ? (rank + 1) * per : rd.n_beads;
-    for (long long i = rank * per + threadIdx.x; i < b1; i += blockDim.x) {
+    long long b0, b1;
+    part.of(rd.n_beads, b0, b1);
+    for (long long i = b0 + threadIdx.x; i < b1; i += blockDim.x) {
       const unsigned sw = st[i];
 #pragma unroll
       for (int b = 0; b < CG_MAX_BINDERS; b++)
@@ -286,9 +287,9 @@ __global__ void __cluster_dims__(kSumCtas, 1, 1) __launch_bounds__(kSumThreads)
   }
   double g[kRests] = {}, dens2 = 0;
   if (uniform) {
-    grid_sums(a, rd, rank, gmax_sh, rest, g);
+    grid_sums(a, rd, part, gmax_sh, rest, g);
   } else if (field) {
-    for_each_row<false>(a, rd, rank, [&](long long v, const long long (&row)[4]) {
+    for_each_row<false>(a, rd, part, [&](long long v, const long long (&row)[4]) {
       if (empty_voxel(a, rd, v, row)) return;
       const double V = a.access_vol[rd.vox_off + v];
       double rho[CG_MAX_BINDERS] = {0, 0, 0};
@@ -383,6 +384,6 @@ void cg_launch_store_chains(const cg::KArgs& a, bool fp64, long long total, cons
   else cg::store_chains_kernel<float><<<(unsigned)blocks, 256, 0, s>>>(a, total, r, t3);
 }
 
-void cg_launch_terms(const cg::KArgs& a, double* terms, double* acc, cudaStream_t s) {
-  cg::terms_kernel<<<a.n_reps * cg::kSumCtas, cg::kSumThreads, 0, s>>>(a, terms, acc);
+void cg_launch_terms(const cg::KArgs& a, int log_ctas, double* terms, double* acc, cudaStream_t s) {
+  cg::launch_sums(cg::terms_kernel, a, log_ctas, s, terms, acc);
 }

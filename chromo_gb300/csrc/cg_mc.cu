@@ -576,13 +576,14 @@ __device__ __forceinline__ double chi_free_sum(const RepDev& rd, double s00) {
 }
 
 template <typename Pos>
-__global__ void __cluster_dims__(kSumCtas, 1, 1) __launch_bounds__(kSumThreads)
-    energy_kernel(KArgs a, double* out) {
+__global__ void __launch_bounds__(kSumThreads)
+    energy_kernel(KArgs a, int log_ctas, double* out) {
   __shared__ double sh[kSumThreads / 32][16];
   __shared__ double bf[CG_MAX_BINDERS * (CG_MAX_MARK + 1) * (CG_MAX_MARK + 1)];
   __shared__ RestSums rest;
   __shared__ long long gmax_sh;
-  const int rep = blockIdx.x / kSumCtas, rank = blockIdx.x % kSumCtas;
+  const SumPart part(log_ctas);
+  const int rep = part.rep, rank = part.rank;
   const RepDev& rd = a.reps[rep];
   fill_bind_table(rd, bf);
   const bool field = rd.field_kind == 2, uniform = field && !rd.has_access;
@@ -599,11 +600,11 @@ __global__ void __cluster_dims__(kSumCtas, 1, 1) __launch_bounds__(kSumThreads)
   #pragma unroll 1
   for (int phase = 0; phase < 2; phase++) {
     if (((threadIdx.x >> 5) ^ phase) & 1) {
-      bead_sums<Pos>(a, rd, rank, bf, el, bi, dbl, excess);
+      bead_sums<Pos>(a, rd, part, bf, el, bi, dbl, excess);
     } else if (uniform) {
-      grid_sums(a, rd, rank, gmax_sh, rest, g);
+      grid_sums(a, rd, part, gmax_sh, rest, g);
     } else if (field) {
-      for_each_row<false>(a, rd, rank, [&](long long v, const long long (&row)[4]) {
+      for_each_row<false>(a, rd, part, [&](long long v, const long long (&row)[4]) {
         if (!empty_voxel(a, rd, v, row)) voxel_energy(a, rd, v, p);
       });
     }
@@ -639,24 +640,25 @@ __global__ void __cluster_dims__(kSumCtas, 1, 1) __launch_bounds__(kSumThreads)
 // The chi-free sums S_r alone (the input of the exchange): the same rows in the
 // same order as energy_kernel's out[5 r + 4], so the values are identical; and
 // with a mu ladder the bound sites of its binder (an exact integer sum).
-__global__ void __cluster_dims__(kSumCtas, 1, 1) __launch_bounds__(kSumThreads)
-    chi_sum_kernel(KArgs a, double* out) {
+__global__ void __launch_bounds__(kSumThreads)
+    chi_sum_kernel(KArgs a, int log_ctas, double* out) {
   __shared__ double sh[kSumThreads / 32][16];
-  __shared__ long long gmax_sh;
-  const int rep = blockIdx.x / kSumCtas, rank = blockIdx.x % kSumCtas;
+  __shared__ Limit lim_sh;
+  const SumPart part(log_ctas);
+  const int rep = part.rep, rank = part.rank;
   const RepDev& rd = a.reps[rep];
   const bool field = rd.field_kind == 2, uniform = field && !rd.has_access;
-  if (threadIdx.x == 0) gmax_sh = uniform ? weight_at_limit(rd) : 0;
+  if (threadIdx.x == 0 && uniform) lim_sh = limit_of(rd);
   __syncthreads();
   double sx = 0;
   if (uniform) {
-    const long long gmax = gmax_sh;
+    const Limit lim = lim_sh;
     FxSum s{};
     int left = kFxRows / kRowsInFlight;
     for_each_row<true>(
-        a, rd, rank,
+        a, rd, part,
         [&](long long, const long long (&row)[4]) {
-          if (row[0] > gmax) return;
+          if (above_limit(rd, lim, row[0])) return;
           // the rows that add_row gives to its FP64 sums
           if ((unsigned long long)(row[0] | row[1] | row[2] | row[3]) >> 52) {
             sx = __fma_rn((double)row[0], (double)row[0], sx);
@@ -675,7 +677,7 @@ __global__ void __cluster_dims__(kSumCtas, 1, 1) __launch_bounds__(kSumThreads)
     sx += fx_value(s, 27);
   } else if (field) {
     EnergyParts p{0.0, 0.0, 0.0, 0.0, {0, 0, 0}};
-    for_each_row<false>(a, rd, rank, [&](long long v, const long long (&row)[4]) {
+    for_each_row<false>(a, rd, part, [&](long long v, const long long (&row)[4]) {
       if (!empty_voxel(a, rd, v, row)) voxel_energy(a, rd, v, p);
     });
     sx = p.sx;
@@ -684,15 +686,17 @@ __global__ void __cluster_dims__(kSumCtas, 1, 1) __launch_bounds__(kSumThreads)
   if (a.mu_rungs > 1) {
     const unsigned* st = a.states + rd.bead_off;
     const int sh8 = 8 * a.mu_binder;
-    const long long per = (rd.n_beads + kSumCtas - 1) / kSumCtas;
-    const long long b1 = (rank + 1) * per < rd.n_beads ? (rank + 1) * per : rd.n_beads;
-    for (long long i = rank * per + threadIdx.x; i < b1; i += blockDim.x) nbl += (st[i] >> sh8) & 0xFFu;
+    long long b0, b1;
+    part.of(rd.n_beads, b0, b1);
+    for (long long i = b0 + threadIdx.x; i < b1; i += blockDim.x) nbl += (st[i] >> sh8) & 0xFFu;
   }
-  double v[16] = {sx, (double)nbl};
-  const double t = cluster_sums(v, sh);
-  if (rank != 0) return;
-  if (threadIdx.x == 0) out[rep * 5 + 4] = uniform ? chi_free_sum(rd, t) : t;
-  if (threadIdx.x == 1 && a.mu_rungs > 1) a.nbound[rep] = t;
+  const double t = cluster_sum(sx, sh);
+  if (rank == 0 && threadIdx.x == 0) out[rep * 5 + 4] = uniform ? chi_free_sum(rd, t) : t;
+  if (a.mu_rungs > 1) {
+    __syncthreads();
+    const double n = cluster_sum((double)nbl, sh);
+    if (rank == 0 && threadIdx.x == 0) a.nbound[rep] = n;
+  }
 }
 
 // ---------------------------------------------------------------- replica exchange
@@ -825,14 +829,13 @@ void cg_launch_deposit(const cg::KArgs& a, bool fp64, int rep, int n_reps_launch
   else cg::deposit_kernel<float><<<grid, 256, 0, s>>>(a, rep);
 }
 
-void cg_launch_energy(const cg::KArgs& a, bool fp64, double* out, cudaStream_t s) {
-  const int blocks = a.n_reps * cg::kSumCtas;
-  if (fp64) cg::energy_kernel<double><<<blocks, cg::kSumThreads, 0, s>>>(a, out);
-  else cg::energy_kernel<float><<<blocks, cg::kSumThreads, 0, s>>>(a, out);
+void cg_launch_energy(const cg::KArgs& a, bool fp64, int log_ctas, double* out, cudaStream_t s) {
+  if (fp64) cg::launch_sums(cg::energy_kernel<double>, a, log_ctas, s, out);
+  else cg::launch_sums(cg::energy_kernel<float>, a, log_ctas, s, out);
 }
 
-void cg_launch_chi_sum(const cg::KArgs& a, double* out, cudaStream_t s) {
-  cg::chi_sum_kernel<<<a.n_reps * cg::kSumCtas, cg::kSumThreads, 0, s>>>(a, out);
+void cg_launch_chi_sum(const cg::KArgs& a, int log_ctas, double* out, cudaStream_t s) {
+  cg::launch_sums(cg::chi_sum_kernel, a, log_ctas, s, out);
 }
 
 void cg_launch_exchange(const cg::KArgs& a, const double* eout, int n_rungs, long long round,
