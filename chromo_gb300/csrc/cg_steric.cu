@@ -30,25 +30,29 @@ constexpr int kGroup = 8;       // rows between two tests
 constexpr int kList = 1024;     // near pairs a CTA lists (5 bits of row, 10 of column)
 static_assert(kRows == 32 && kRows % kGroup == 0, "a bit per row, groups of whole rows");
 
-// The powers of f = e / d are products whose rounding errors (one FMA each) are
-// carried along and added at the end: the product of products alone is off by up to
-// 5 units in the last place, twelve multiplications' worth, where pow is off by
-// one.
-__device__ __forceinline__ double clash_energy(double d, double e, double V0) {
-  if (!(d < e)) return 0.0;
-  const double f = e / d;
-  const double f2 = f * f, r2 = __fma_rn(f, f, -f2);
-  const double f4 = f2 * f2, r4 = __fma_rn(2 * f2, r2, __fma_rn(f2, f2, -f4));
-  const double f6 = f4 * f2, r6 = __fma_rn(f4, f2, -f6) + __fma_rn(f4, r2, r4 * f2);
-  const double f12 = f6 * f6, r12 = __fma_rn(2 * f6, r6, __fma_rn(f6, f6, -f12));
-  const double c = r12 - 2 * r6;
-  const double t = f12 - 2 * f6 + 1;
-  return V0 * (isfinite(c) ? t + c : t);
+// The pair energy from the squared distance: the powers of (e / d)^2, one quotient of
+// squares (e2 = e^2; 0 where squares leave FP64's range, with the square root).  The
+// roundings of the root and of e / d count twelvefold in (e / d)^12, those of the
+// squares and their quotient sixfold: the error is 0.7 of that of pow(e / d, 12), at
+// half the FP64 operations.
+__device__ __forceinline__ double clash_energy(double d2, double e, double e2, double V0) {
+  double f2;
+  if (!is_zero64(e2)) {
+    if (!(d2 < e2)) return 0.0;
+    f2 = e2 / d2;
+  } else {
+    const double d = sqrt(d2);
+    if (!(d < e)) return 0.0;
+    const double f = e / d;
+    f2 = f * f;
+  }
+  const double f6 = f2 * f2 * f2;
+  return V0 * (f6 * f6 - 2 * f6 + 1);
 }
 
-__device__ __forceinline__ double dist3(const double a[3], const double b[3]) {
+__device__ __forceinline__ double square3(const double a[3], const double b[3]) {
   const double x = a[0] - b[0], y = a[1] - b[1], z = a[2] - b[2];
-  return sqrt(x * x + y * y + z * z);
+  return x * x + y * y + z * z;
 }
 
 // Offset of a position from the tile's origin, rounded to FP32.  Pairs closer
@@ -87,17 +91,17 @@ __device__ __forceinline__ double tile_total(double v, double* sh) {
 // The FP64 term of beads i (a row) and j.
 template <typename Pos, bool TRIAL>
 static __device__ __noinline__ double pair_term(const V4<Pos>* r4, long long i, long long j, long long ind0,
-                                                long long indf, const double* trial, double e, double V0) {
+                                                long long indf, const double* trial, double e, double e2, double V0) {
   double ri[3], rj[3];
   ld3(r4, i, ri);
   ld3(r4, j, rj);
-  const double before = clash_energy(dist3(ri, rj), e, V0);
+  const double before = clash_energy(square3(ri, rj), e, e2, V0);
   if (!TRIAL) return before;
   const double* ti = trial + 3 * (i - ind0);
   const double t0[3] = {ti[0], ti[1], ti[2]};
   if (j >= ind0 && j < indf)
     for (int q = 0; q < 3; q++) rj[q] = trial[3 * (j - ind0) + q];
-  return clash_energy(dist3(t0, rj), e, V0) - before;
+  return clash_energy(square3(t0, rj), e, e2, V0) - before;
 }
 
 // Rows [kRows blockIdx.x, ...) against columns [blockIdx.y chunk, ...): the
@@ -112,7 +116,7 @@ static __device__ __noinline__ double pair_term(const V4<Pos>* r4, long long i, 
 template <typename Pos, bool TRIAL, int COLS>
 __global__ void __launch_bounds__(kStericThr)
     steric_tile_kernel(KArgs a, int rep, long long n_rows, long long ind0, long long indf, long long chunk,
-                       const double* trial, double e, double V0, double* parts) {
+                       const double* trial, double e, double e2, double V0, double* parts) {
   __shared__ float4 cur[kRows], tri[TRIAL ? kRows : 1];
   __shared__ float far_sh;
   __shared__ int found[kStericThr / 32];
@@ -234,13 +238,13 @@ __global__ void __launch_bounds__(kStericThr)
           if (v == u) hit[v] &= hit[v] - 1;
         cnt--;
         if (listed) list[at++] = (unsigned short)((u * kStericThr + (int)threadIdx.x) << 5 | k);
-        else part += pair_term<Pos, TRIAL>(r4, row0 + k, j0 + u * kStericThr, ind0, indf, trial, e, V0);
+        else part += pair_term<Pos, TRIAL>(r4, row0 + k, j0 + u * kStericThr, ind0, indf, trial, e, e2, V0);
       }
       __syncthreads();
       if (listed)
         #pragma unroll 1
         for (int q = threadIdx.x; q < total; q += kStericThr)
-          part += pair_term<Pos, TRIAL>(r4, row0 + (list[q] & 31), jb + (list[q] >> 5), ind0, indf, trial, e, V0);
+          part += pair_term<Pos, TRIAL>(r4, row0 + (list[q] & 31), jb + (list[q] >> 5), ind0, indf, trial, e, e2, V0);
       __syncthreads();  // the list is read
     }
   }
@@ -266,8 +270,9 @@ __global__ void __launch_bounds__(kStericThr) steric_sum_kernel(const double* pa
 template <typename Pos>
 static void launch_tiles(const cg::KArgs& a, dim3 grid, int rep, long long n_rows, long long ind0, long long indf,
                          long long chunk, const double* trial, double e, double V0, double* parts, cudaStream_t s) {
+  const double e2 = e > 1e-150 && e < 1e150 ? e * e : 0.0;
   auto run = [&](auto kernel) {
-    kernel<<<grid, cg::kStericThr, 0, s>>>(a, rep, n_rows, ind0, indf, chunk, trial, e, V0, parts);
+    kernel<<<grid, cg::kStericThr, 0, s>>>(a, rep, n_rows, ind0, indf, chunk, trial, e, e2, V0, parts);
   };
   const bool one = chunk == cg::kStericThr;
   if (trial) run(one ? cg::steric_tile_kernel<Pos, true, 1> : cg::steric_tile_kernel<Pos, true, 4>);
