@@ -104,7 +104,7 @@ static __device__ __noinline__ double pair_term(const V4<Pos>* r4, long long i, 
   return clash_energy(square3(t0, rj), e, e2, V0) - before;
 }
 
-// Rows [kRows blockIdx.x, ...) against columns [blockIdx.y chunk, ...): the
+// Rows [height blockIdx.x, ...) (at most kRows) against columns [blockIdx.y chunk, ...): the
 // pairs i < j of the resident chain, or (TRIAL) with positions `trial` of the
 // beads [ind0, indf) (m x 3) the change of the pairs of the moved beads, those of
 // two moved beads counted once (j < i).  parts: one sum per tile, by row tile and
@@ -116,7 +116,7 @@ static __device__ __noinline__ double pair_term(const V4<Pos>* r4, long long i, 
 template <typename Pos, bool TRIAL, int COLS>
 __global__ void __launch_bounds__(kStericThr)
     steric_tile_kernel(KArgs a, int rep, long long n_rows, long long ind0, long long indf, long long chunk,
-                       const double* trial, double e, double e2, double V0, double* parts) {
+                       int height, const double* trial, double e, double e2, double V0, double* parts) {
   __shared__ float4 cur[kRows], tri[TRIAL ? kRows : 1];
   __shared__ float far_sh;
   __shared__ int found[kStericThr / 32];
@@ -126,8 +126,8 @@ __global__ void __launch_bounds__(kStericThr)
   const V4<Pos>* r4 = reinterpret_cast<const V4<Pos>*>(a.r4) + rd.bead_off;
   const long long N = rd.n_beads;
   const int lane = (int)(threadIdx.x & 31u), warp = (int)(threadIdx.x >> 5);
-  const long long k0 = (long long)blockIdx.x * kRows, row0 = (TRIAL ? ind0 : 0) + k0;  // bead of row 0
-  const int rows = (int)(n_rows - k0 < kRows ? n_rows - k0 : kRows);
+  const long long k0 = (long long)blockIdx.x * height, row0 = (TRIAL ? ind0 : 0) + k0;  // bead of row 0
+  const int rows = (int)(n_rows - k0 < height ? n_rows - k0 : height);
   long long c0 = (long long)blockIdx.y * chunk;
   const long long c1 = c0 + chunk < N ? c0 + chunk : N;
   if (!TRIAL && c0 < k0 + 1) c0 = k0 + 1;  // pairs above the diagonal
@@ -269,10 +269,11 @@ __global__ void __launch_bounds__(kStericThr) steric_sum_kernel(const double* pa
 // parts holds at least n_beads + 32 doubles (the split: cg_steric_tiles.h).
 template <typename Pos>
 static void launch_tiles(const cg::KArgs& a, dim3 grid, int rep, long long n_rows, long long ind0, long long indf,
-                         long long chunk, const double* trial, double e, double V0, double* parts, cudaStream_t s) {
+                         long long chunk, int height, const double* trial, double e, double V0, double* parts,
+                         cudaStream_t s) {
   const double e2 = e > 1e-150 && e < 1e150 ? e * e : 0.0;
   auto run = [&](auto kernel) {
-    kernel<<<grid, cg::kStericThr, 0, s>>>(a, rep, n_rows, ind0, indf, chunk, trial, e, e2, V0, parts);
+    kernel<<<grid, cg::kStericThr, 0, s>>>(a, rep, n_rows, ind0, indf, chunk, height, trial, e, e2, V0, parts);
   };
   const bool one = chunk == cg::kStericThr;
   if (trial) run(one ? cg::steric_tile_kernel<Pos, true, 1> : cg::steric_tile_kernel<Pos, true, 4>);
@@ -281,12 +282,13 @@ static void launch_tiles(const cg::KArgs& a, dim3 grid, int rep, long long n_row
 void cg_launch_steric(const cg::KArgs& a, bool fp64, int rep, long long n_beads, long long n_rows, long long ind0,
                       long long indf, const double* trial, double e, double V0, double* parts, double* out,
                       int n_sm, cudaStream_t s) {
-  const long long tiles = (n_rows + cg::kRows - 1) / cg::kRows;
-  const long long chunk = cg_steric_chunk(n_beads, tiles, n_sm);
+  int height;
+  const long long chunk = cg_steric_split(n_beads, n_rows, n_sm, &height);
+  const long long tiles = (n_rows + height - 1) / height;
   const long long chunks = (n_beads + chunk - 1) / chunk;
   const dim3 grid((unsigned)tiles, (unsigned)chunks);
-  if (fp64) launch_tiles<double>(a, grid, rep, n_rows, ind0, indf, chunk, trial, e, V0, parts, s);
-  else launch_tiles<float>(a, grid, rep, n_rows, ind0, indf, chunk, trial, e, V0, parts, s);
+  if (fp64) launch_tiles<double>(a, grid, rep, n_rows, ind0, indf, chunk, height, trial, e, V0, parts, s);
+  else launch_tiles<float>(a, grid, rep, n_rows, ind0, indf, chunk, height, trial, e, V0, parts, s);
   if (cudaPeekAtLastError() != cudaSuccess) return;  // the caller reports it; no sums to add
   cg::steric_sum_kernel<<<1, cg::kStericThr, 0, s>>>(parts, tiles * chunks, out);
 }

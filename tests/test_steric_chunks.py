@@ -15,11 +15,11 @@ HDR = Path(__file__).resolve().parents[1] / "chromo_gb300" / "csrc" / "cg_steric
 @pytest.fixture(scope="module")
 def chunk(tmp_path_factory):
     d = tmp_path_factory.mktemp("steric")
-    (d / "t.c").write_text(f'#include "{HDR}"\nlong long chunk(long long n, long long t, int sm)'
-                           "{ return cg_steric_chunk(n, t, sm); }\n")
+    (d / "t.c").write_text(f'#include "{HDR}"\nlong long chunk(long long n, long long m, int sm, int* rows)'
+                           "{ return cg_steric_split(n, m, sm, rows); }\n")
     subprocess.check_call(["gcc", "-O1", "-shared", "-fPIC", "-o", str(d / "t.so"), str(d / "t.c")])
     f = ctypes.CDLL(str(d / "t.so")).chunk
-    f.argtypes = [ctypes.c_longlong, ctypes.c_longlong, ctypes.c_int]
+    f.argtypes = [ctypes.c_longlong, ctypes.c_longlong, ctypes.c_int, ctypes.c_void_p]
     f.restype = ctypes.c_longlong
     return f
 
@@ -29,9 +29,10 @@ def test_chunks_fit_the_grid_and_the_sums(chunk, n):
     for m in sorted({1, 32, 33, 288, 289, 320, n}):
         if m > n:
             continue
-        tiles = (m + 31) // 32
-        c = chunk(n, tiles, 152)
-        chunks = (n + c - 1) // c
+        rows = ctypes.c_int()
+        c = chunk(n, m, 152, ctypes.byref(rows))
+        tiles, chunks = (m + rows.value - 1) // rows.value, (n + c - 1) // c
+        assert rows.value in (1, 2, 4, 8, 16, 32)
         assert c % 256 == 0 and (c == 256 or c >= 1024)
         assert chunks <= 65535 and tiles <= 2 ** 31 - 1
         assert tiles * chunks <= n + 32
