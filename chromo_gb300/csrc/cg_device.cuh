@@ -443,8 +443,8 @@ __device__ __forceinline__ void rotation_row(const double a[3], const double p[3
   R[3] += (pu * (1 - uu) - u * (pv * v + pw * w)) * oc;
 }
 
-// (double)x, of normal numbers and zeros by their bits: a conversion holds the
-// FP64 pipe for ~65 cycles a warp.
+// (double)x, of normal numbers by their bits (others by a conversion, which holds
+// the FP64 pipe for ~65 cycles a warp).
 __device__ __forceinline__ double widen(float x) {
   const unsigned u = __float_as_uint(x), m = u & 0x7FFFFFFFu;
   if (m - 0x00800000u < 0x7F000000u)

@@ -179,9 +179,7 @@ __device__ __forceinline__ void claim_slots(int* keys, U* used, int* nused, int 
   }
   // linear probing of the displaced claims, one loop for all of a lane's: a
   // warp nearly always holds a few, and a call per claim took 2.4 k cycles a
-  // pass with the claims (256 chains, 20 MC steps: 16.4 -> 14.1 ms together
-  // with the branch-free wrap of voxel_axes and the state times split halves of
-  // add_corner)
+  // pass with the claims
   const int mask = (1 << logH) - 1;
   #pragma unroll 1
   for (int it = 1; pend; it++) {

@@ -39,10 +39,8 @@
 //
 // Loops of run-time length are not unrolled: the kernel is large and few warps
 // share an SM, and a fifth of its instruction fetches missed the first cache
-// (256 chains of 2,000-20,000 beads, 20 MC steps, kernel only: 11.5 -> 10.4 ms;
-// one 10,000-bead chain, 10 steps: 2.62 -> 2.44 ms with the larger block table
-// above 8 moves in flight).  Exceptions, measured: the binder columns of
-// add_corner.
+// with them unrolled (a tenth of the kernel's time on 256 chains).  Exceptions,
+// measured: the binder columns of add_corner.
 #pragma once
 #include <cuda_runtime.h>
 
@@ -389,14 +387,13 @@ template <> __device__ __forceinline__ double load_acc<double>(long long, double
 // the cells go round by shuffles and each lane adds two corners (old weights
 // out, new weights in) to the voxel table.  The last warp also takes the
 // moves' boundary bonds, one per lane.  (Four lanes per bead for the whole
-// task, each repeating the bead's transform and cells, issued three times the
-// instructions; the bonds, taken by the lanes of a segment's end beads, were
-// executed by nearly every warp.  256 chains of 2,000-20,000 beads, 20 MC steps
-// and the read-back: 20.9 -> 18.5 ms; one 10,000-bead chain, 10 steps: 3.71 ->
-// 3.46 ms; 64 SSTWLC chains of 2,000 beads, whose FP64 twist terms of a batch's
-// bonds now share their warp's issue, 10 steps: 18.2 -> 11.8 ms.)  The table is the CTA's pooled table (FP32
-// storage: keys voxel * 32 + slot, one used list) or the slot's own table.  The
-// bond terms, confinement counts and error bits go to the move's plan.  A move
+// task, each repeating the bead's transform and cells, issue three times the
+// instructions; bonds on the lanes of a segment's end beads are executed by
+// nearly every warp: together a ninth of a pass over 256 chains, and a third of
+// one over SSTWLC chains, whose FP64 twist terms of a batch's bonds so share their
+// warp's issue.)  The table is the CTA's pooled table (keys voxel * 32 + slot,
+// one used list) or the slot's own table.  The bond terms, confinement counts
+// and error bits go to the move's plan.  A move
 // whose optimistic table overflows (E_OVF: a pool or a table past 3/4 load) is
 // skipped from then on; its group deposits it again in its global table.
 // Called by every thread.
@@ -918,9 +915,7 @@ __device__ __forceinline__ void store_field(MovePlan&, double) {}
 // only when they are long (over kPoolMaxBeads) or overflowed the pool; chains
 // in no density field take it for the bond terms.  Out of line: with the pooled
 // table it is rare, and inline it cost every batch ~3.6 k cycles of empty
-// passes and reductions (256 chains, 20 MC steps: 18.5 -> 16.4 ms with the
-// field sums in 32-bit limbs; 1,000 beads in FP64, whose moves over 64
-// beads took it before the pool served FP64: 9.7 -> 6.9 ms).  Called by the whole warp; `run` is false for groups
+// passes and reductions.  Called by the whole warp; `run` is false for groups
 // without such a move.
 template <typename Pos, int G, bool LEAN>
 static __device__ __noinline__ void own_path(const KArgs& a, SpecShared& sh, int rep, int s, int gl, bool run,
