@@ -169,17 +169,19 @@ struct cg_sim {
   int direct_host = 0;
   void* hio_tab = nullptr;
   unsigned* hio_flag = nullptr;
-  // replicas using SSTWLC twist or fast_field (the MC kernel's full form); with
-  // none, launches take its lean form
-  std::vector<unsigned char> full_of;
-  long long n_full = 0;
+  // replicas using SSTWLC twist (the MC kernel's full form) or fast_field (its lean
+  // form with the sub-bin weights); with none, launches take its lean form
+  std::vector<unsigned char> features;  // bit 0: twist, bit 1: fast_field
+  long long n_twist = 0, n_fast = 0;
+  int form() const { return n_twist > 0 ? 0 : n_fast > 0 ? 2 : 1; }
   void note_features(int rep, const RepDev& d) {
-    const unsigned char f = d.twist != 0 || d.fast_n > 0;
-    if (f == full_of[rep]) return;
-    const bool was_lean = n_full == 0;
-    n_full += f ? 1 : -1;
-    full_of[rep] = f;
-    if (was_lean != (n_full == 0)) drop_graph();  // the captured launches' form changes
+    const unsigned char f = (d.twist != 0 ? 1 : 0) | (d.fast_n > 0 ? 2 : 0), old = features[rep];
+    if (f == old) return;
+    const int was = form();
+    n_twist += (f & 1) - (old & 1);
+    n_fast += (f >> 1) - (old >> 1);
+    features[rep] = f;
+    if (was != form()) drop_graph();  // the captured launches' form changes
   }
   // device staging arrays of a direct upload (resident layout; allocated on
   // the first upload, hio_stage_failed when there was no room)
@@ -246,7 +248,7 @@ struct cg_sim {
     a.xround = xround;
     a.mu_rungs = mu_rungs; a.mu_binder = mu_binder; a.nbound = nbound;
     a.mu_swaps = mu_swaps; a.mu_swap_attempts = mu_swap_attempts;
-    a.lean = n_full == 0 ? 1 : 0;
+    a.lean = form();
     return a;
   }
 
@@ -468,7 +470,7 @@ int cg_create(const cg_config* cfg, cg_sim** out) {
     return fail(CG_ERR_ARG, "n_binders must be in 1..3");
   cg_sim* s = new cg_sim();
   s->R = cfg->n_replicas;
-  s->full_of.assign(s->R, 0);
+  s->features.assign(s->R, 0);
   s->nb = cfg->n_binders;
   s->ncol = cfg->n_binders + 1 <= 2 ? 2 : 4;
   s->fp64 = cfg->pos_fp64 ? 1 : 0;

@@ -138,8 +138,8 @@ struct KArgs {
   // voxel * 32 + move slot, shared by the position moves of a batch
   int pool_on, pool_logH, off_pkeys, off_pused, off_pvals;
   unsigned long long seed;
-  // the MC kernel's lean form: no replica uses SSTWLC twist or fast_field and the move log
-  // is off
+  // the MC kernel's form: 1 no replica uses SSTWLC twist or fast_field and the move
+  // log is off, 2 some use fast_field, 0 any
   int lean;
   // audit mode
   int audit_rep;

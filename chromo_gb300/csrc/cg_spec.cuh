@@ -201,7 +201,7 @@ __device__ __forceinline__ void load_transform(const MovePlan& P, Pos (&M)[3][4]
 // Elastic dE of one boundary bond of a position move: the bond to the fixed
 // neighbour left of the segment (side 0) or right of it (side 1); zero where the
 // segment ends the chain.  The move's plan holds its segment and transform.
-template <typename Pos, typename Acc, bool LEAN>
+template <typename Pos, typename Acc, int LEAN>
 static __device__ __forceinline__ Acc boundary_term(const KArgs& a, const RepDev& rd, const MovePlan& P, int kind,
                                                  int side) {
   const ChainView<Pos> cv(a, rd, LEAN);
@@ -291,7 +291,7 @@ struct BeadCells {
 // stages its new vectors for the commit, counts the confinement crossings and
 // finds its cells.  Returns false (and E_NONFINITE in e) for a position that
 // is not finite.
-template <typename Pos, bool LEAN>
+template <typename Pos, int LEAN>
 __device__ __forceinline__ bool place_bead(const RepDev& rd, const GridF& gf, const ChainView<Pos>& cv, int kind,
                                            const Pos (&M)[3][4], long long i, V4<Pos>* stage, bool density,
                                            bool conf, BeadCells<Pos>& c, unsigned& e, int& oob) {
@@ -316,10 +316,10 @@ __device__ __forceinline__ bool place_bead(const RepDev& rd, const GridF& gf, co
   }
   if (density) {
     int lo[3], hi[3];
-    move_axes<LEAN>(rd, gf, r, c.wl0, lo, hi);
+    move_axes<LEAN == 1>(rd, gf, r, c.wl0, lo, hi);
     c.v0 = lo[0] + gf.nx * lo[1] + gf.nxy * lo[2];
     c.wrap0 = (hi[0] == 0 ? 1u : 0u) | (hi[1] == 0 ? 2u : 0u) | (hi[2] == 0 ? 4u : 0u);
-    move_axes<LEAN>(rd, gf, tr, c.wl1, lo, hi);
+    move_axes<LEAN == 1>(rd, gf, tr, c.wl1, lo, hi);
     c.v1 = lo[0] + gf.nx * lo[1] + gf.nxy * lo[2];
     c.wrap1 = (hi[0] == 0 ? 1u : 0u) | (hi[1] == 0 ? 2u : 0u) | (hi[2] == 0 ? 4u : 0u);
   }
@@ -397,7 +397,7 @@ template <> __device__ __forceinline__ double load_acc<double>(long long, double
 // whose optimistic table overflows (E_OVF: a pool or a table past 3/4 load) is
 // skipped from then on; its group deposits it again in its global table.
 // Called by every thread.
-template <typename Pos, bool LEAN>
+template <typename Pos, int LEAN>
 __device__ void block_deposit(const KArgs& a, SpecShared& sh, int rep, int B, int kind) {
   using Acc = typename AccOf<Pos>::type;
   unsigned char* smem = reinterpret_cast<unsigned char*>(&sh);
@@ -502,7 +502,7 @@ __device__ void block_deposit(const KArgs& a, SpecShared& sh, int rep, int B, in
         stage[ax] = ax < 3 ? tr : 0.0;
       }
       const unsigned bad = __ballot_sync(kFull, !isfinite(tr)) >> quad & 15u;
-      const bool fast = !LEAN && rd.fast_n > 0;
+      const bool fast = LEAN != 1 && rd.fast_n > 0;
       double t[3] = {0, 0, 0};
       if (conf || fast)
         for (int q = 0; q < 3; q++) t[q] = __shfl_sync(kFull, tr, quad + q);
@@ -917,7 +917,7 @@ __device__ __forceinline__ void store_field(MovePlan&, double) {}
 // table it is rare, and inline it cost every batch ~3.6 k cycles of empty
 // passes and reductions.  Called by the whole warp; `run` is false for groups
 // without such a move.
-template <typename Pos, int G, bool LEAN>
+template <typename Pos, int G, int LEAN>
 static __device__ __noinline__ void own_path(const KArgs& a, SpecShared& sh, int rep, int s, int gl, bool run,
                                              int kind, int* bkeys, unsigned* bmask) {
   using Acc = typename AccOf<Pos>::type;
@@ -1052,7 +1052,7 @@ static __device__ __noinline__ void own_path(const KArgs& a, SpecShared& sh, int
 // Tangent rotation of bead i about the axis of draws xa, xb (sine sa, cosine
 // ca): its new frame and the dE of its two bonds, the neighbours' frames as they
 // are.  Lean: without the twist terms.
-template <typename Pos, bool LEAN>
+template <typename Pos, int LEAN>
 __device__ __forceinline__ typename AccOf<Pos>::type rotate_tangent(const KArgs& a, const RepDev& rd, long long i,
                                                                     unsigned xa, unsigned xb, Pos sa, Pos ca,
                                                                     Pos (&tt3)[3], Pos (&tt2)[3]) {
@@ -1174,7 +1174,7 @@ __device__ __forceinline__ unsigned block_find(const int* bkeys, const unsigned*
 }
 
 // Evaluate the batch's B moves (one per group of GS lanes) into their plans.
-template <bool LEAN>
+template <int LEAN>
 __device__ void short_tangent_evaluate(const KArgs& a, SpecShared& sh, int rep, const ShortTangent& T, int B,
                                        const cg_move_ctl& c, int* bkeys, unsigned* bmask) {
   const RepDev& rd = sh.ws.rd;
@@ -1402,7 +1402,7 @@ __device__ __forceinline__ void segment_of(long long b0, long long b1, long long
 // its segment and transform, its table and its Metropolis draw go to its plan.
 // `live` is false for the groups of a partly filled batch.  Called by the whole
 // warp.
-template <typename Pos, int G, bool LEAN>
+template <typename Pos, int G, int LEAN>
 __device__ void propose_position(const KArgs& a, SpecShared& sh, int rep, int s, int gl, bool live, int kind,
                                  const cg_move_ctl& c, unsigned long long t) {
   using Real = Pos;
@@ -1589,7 +1589,7 @@ __device__ __forceinline__ void bead_conflicts(SpecShared& sh, int s, int gl, bo
 }
 
 // The decision on a position move from the results in its plan.
-template <typename Pos, int G, bool LEAN>
+template <typename Pos, int G, int LEAN>
 __device__ __forceinline__ void decide_position(const KArgs& a, SpecShared& sh, int s, int gl, bool live) {
   using Acc = typename AccOf<Pos>::type;
   if (!live) return;
@@ -1628,7 +1628,7 @@ __device__ __forceinline__ void decide_position(const KArgs& a, SpecShared& sh, 
 // Evaluate tangent rotation or binding move t of the batch in slot s (group
 // lanes gl = 0..G-1); `live` is false for the groups of a partly filled batch.
 // Called by the whole warp.
-template <typename Pos, int G, bool LEAN>
+template <typename Pos, int G, int LEAN>
 __device__ void evaluate_move(const KArgs& a, SpecShared& sh, int rep, int s, int gl, bool live, int kind,
                               const cg_move_ctl& c, unsigned long long t, int* bkeys, unsigned* bmask) {
   using Real = Pos;
@@ -1866,7 +1866,7 @@ __device__ void evaluate_move(const KArgs& a, SpecShared& sh, int rep, int s, in
           Real p[3], wl[3], w;
           int lo[3], hi[3];
           ld3(r4, i, p);
-          move_axes<LEAN>(rd, gf, p, wl, lo, hi);
+          move_axes<LEAN == 1>(rd, gf, p, wl, lo, hi);
           voxel_corner(gf, wl, lo, hi, cl, w, vq[0]);
           q = q40(w) * (long long)(s_new - s_old);
           want[0] = true;
@@ -2120,10 +2120,12 @@ __device__ __forceinline__ int batch_limit(float met, float pairs, int most) {
 // moves in flight (the block-wide phases use them all).  At 168 registers and 12
 // warps: 256 chains, 20 MC steps, kernel only, 10.3 against 9.95 ms, one
 // 10,000-bead chain, 10 steps, 2.40 against 2.23.  FP64 storage: 168 registers.
-// LEAN: the instantiation for launches with no SSTWLC or fast_field replica and
-// no move log, whose code for those is left out (the host picks it per launch,
-// a.lean).
-template <typename Pos, int G, bool LEAN>
+// LEAN (the host picks it per launch, a.lean): 1, the instantiation for launches with
+// no SSTWLC or fast_field replica and no move log, whose code for those is left out; 2,
+// the same with fast_field; 0, any launch.  The full form's spills cost fast_field
+// replicas ~10 % (one 1,000-bead chain, 80 moves: rotations of up to 60 beads 373 us in
+// form 2, 410 in form 0; binding moves 93 and 103; cranks of up to 30 beads 147 and 164).
+template <typename Pos, int G, int LEAN>
 __global__ void __maxnreg__(sizeof(Pos) == 4 ? 128 : 168) spec_kernel(KArgs a) {
   extern __shared__ __align__(32) unsigned char smem[];
   constexpr int GPW = 32 / G;  // move groups per warp
@@ -2383,24 +2385,26 @@ __global__ void __maxnreg__(sizeof(Pos) == 4 ? 128 : 168) spec_kernel(KArgs a) {
 }  // namespace cg
 
 // Launch, shared-memory opt-in and register count of one storage / lanes
-// pair (both its lean and full forms).
+// pair (all its forms).
 #define CG_SPEC_INSTANTIATE(Pos, G, NAME)                                                          \
   void cg_launch_spec_##NAME(const cg::KArgs& a, size_t smem, cudaStream_t s) {                    \
-    if (a.lean)                                                                                    \
-      cg::spec_kernel<Pos, G, true><<<a.n_reps, 32 * a.spec_w, smem, s>>>(a);                      \
-    else                                                                                           \
-      cg::spec_kernel<Pos, G, false><<<a.n_reps, 32 * a.spec_w, smem, s>>>(a);                     \
+    auto* kernel = a.lean == 1 ? cg::spec_kernel<Pos, G, 1>                                        \
+                   : a.lean == 2 ? cg::spec_kernel<Pos, G, 2> : cg::spec_kernel<Pos, G, 0>;        \
+    kernel<<<a.n_reps, 32 * a.spec_w, smem, s>>>(a);                                               \
   }                                                                                                \
   cudaError_t cg_spec_smem_##NAME(int bytes) {                                                     \
-    cudaError_t e = cudaFuncSetAttribute(cg::spec_kernel<Pos, G, false>,                           \
-                                         cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);      \
-    if (e != cudaSuccess) return e;                                                                \
-    return cudaFuncSetAttribute(cg::spec_kernel<Pos, G, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, \
-                                bytes);                                                            \
+    for (auto* kernel : {cg::spec_kernel<Pos, G, 0>, cg::spec_kernel<Pos, G, 1>, cg::spec_kernel<Pos, G, 2>}) { \
+      const cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes); \
+      if (e != cudaSuccess) return e;                                                              \
+    }                                                                                              \
+    return cudaSuccess;                                                                            \
   }                                                                                                \
   int cg_spec_regs_##NAME() {                                                                      \
-    cudaFuncAttributes at, bt;                                                                     \
-    if (cudaFuncGetAttributes(&at, cg::spec_kernel<Pos, G, false>) != cudaSuccess) return 0;       \
-    if (cudaFuncGetAttributes(&bt, cg::spec_kernel<Pos, G, true>) != cudaSuccess) return 0;        \
-    return at.numRegs > bt.numRegs ? at.numRegs : bt.numRegs;                                      \
+    int regs = 0;                                                                                  \
+    for (auto* kernel : {cg::spec_kernel<Pos, G, 0>, cg::spec_kernel<Pos, G, 1>, cg::spec_kernel<Pos, G, 2>}) { \
+      cudaFuncAttributes at;                                                                       \
+      if (cudaFuncGetAttributes(&at, kernel) != cudaSuccess) return 0;                             \
+      if (at.numRegs > regs) regs = at.numRegs;                                                    \
+    }                                                                                              \
+    return regs;                                                                                   \
   }
