@@ -383,10 +383,16 @@ static int default_lanes(const cg_sim* s, int g_req) {
 
 // Warps per replica: the largest W <= kMaxW for which every replica's CTA is
 // resident at once (ceil(R / SMs) CTAs per SM, W warps each, within the
-// register file), and at most 32 moves in flight.
+// register file), and at most 32 moves in flight.  With 8 or 16 lanes per move, where
+// a warp has several moves, 12 warps per SM: 32 moves of 16 lanes overflow the pooled
+// table that 24 fit, and meet more conflicts (80 cranks of up to 300 beads of a
+// 10,000-bead chain 2.93 ms with 16 warps, 0.83 with 12; 80 end pivots of up to 100 on
+// 304 chains of 300 beads 3.24 with 8 each, 1.20 with 6; rotations 1.1-1.3 times as long).
 static int default_warps(const cg_sim* s, int G) {
   const long long ctas = (s->R + s->n_sm - 1) / std::max(1, s->n_sm);
-  const long long W = cg_spec_warps_per_sm(s->fp64 != 0, G) / std::max(1LL, ctas);
+  const int per_sm = G == 32 ? cg_spec_warps_per_sm(s->fp64 != 0, G)
+                             : std::min(cg::kUserMaxW, cg_spec_warps_per_sm(s->fp64 != 0, G));
+  const long long W = per_sm / std::max(1LL, ctas);
   const long long wmax = std::min<long long>(cg::kMaxW, cg::kMaxS / (32 / G));
   return (int)std::min<long long>(wmax, std::max<long long>(1, W));
 }
