@@ -1116,13 +1116,18 @@ __device__ __forceinline__ typename AccOf<Pos>::type rotate_tangent(const KArgs&
 // phases' state kept in the plans); 9-16 beads on 16 lanes instead of 8, one
 // pass instead of two: 256 chains 9.90 -> 9.53 ms, the SSTWLC chains 8.46 -> 7.60.
 //
-// Without twist, an amplitude above 16, or a large one for the chain's length
-// (amp^2 > 3/4 N), takes the path of 32 lanes: on 16 lanes over 16 beads need two
-// passes, and beads drawn twice, likely there, are redrawn by one lane.  80
-// rotations on each of 256 chains: 1,000 beads, up to 16 / 32 of them, 230 / 716 us
-// here against 262 / 406 there; 50 beads, up to 16, 578 against 417.  The FP64 twist
-// terms outweigh that up to 32 beads and amp^2 = 8 N (64 SSTWLC chains of 200 / 50
-// beads, up to 32: 2.08 / 2.55 ms against 2.17 / 2.21).
+// Without twist, amplitudes above 16 + N S / 4000 (S moves in flight) and those with
+// amp^2 > 5.4 sqrt(N S) take the path of 32 lanes: on 16 lanes over 16 beads need two
+// passes, which pays where more moves stand than the S of 32 lanes, and beads drawn
+// twice, likely on short chains, are redrawn by one lane.  320 rotations here / there,
+// us: 64 chains (S = 12) of 50 beads, up to 10 / 13 / 16: 1,160 / 1,454 / 1,747 and
+// 1,401 / 1,468 / 1,538; of 1,000, up to 17 / 24 / 32: 644 / 1,137 / 1,819 and 832 /
+// 1,084 / 1,288; of 5,000: 374 / 555 / 883 and 539 / 700 / 856; 32 of 50,000: 232 / 306 /
+// 395 and 411 / 468 / 544.  256 chains (S = 6) of 50 beads, up to 8 / 10 / 13: 928 /
+// 1,132 / 1,358 and 1,088 / 1,161 / 1,182; of 5,000, up to 17 / 24 / 32: 432 / 698 / 943
+// and 563 / 665 / 795.  The FP64 twist terms outweigh that up to 32 beads and amp^2 =
+// 8 N (64 SSTWLC chains of 200 / 50 beads, up to 32, 80 rotations: 2.08 / 2.55 ms here,
+// 2.17 / 2.21 there).
 //
 // Moves in flight: kShortSpan sqrt(N) / (amp + 1), at which about two of them
 // meet an earlier accepted one (3 and 4 measured alike, 6 and 9 were slower on
@@ -2187,7 +2192,9 @@ __global__ void __maxnreg__(sizeof(Pos) == 4 ? 128 : 168) spec_kernel(KArgs a) {
     sh.stop = 0;
     sh.npool = 0;
     const float n = (float)rd0.n_beads;
-    sh.short_amp = !LEAN && rd0.twist ? (int)fminf(32.0f, sqrtf(8.0f * n)) : (int)fminf(16.0f, sqrtf(0.75f * n));
+    sh.short_amp = !LEAN && rd0.twist ? (int)fminf(32.0f, sqrtf(8.0f * n))
+                                          : (int)fminf(fminf(32.0f, sqrtf(5.4f * sqrtf(n * (float)Sn))),
+                                                       16.0f + n * (float)Sn * (1.0f / 4000.0f));
   }
   __syncthreads();
 
@@ -2209,7 +2216,7 @@ __global__ void __maxnreg__(sizeof(Pos) == 4 ? 128 : 168) spec_kernel(KArgs a) {
           // beads of each earlier accepted one with probability ~3/8 (amp + 1)^2 / N)
           constexpr bool kShort = G == 32 && sizeof(Pos) == 4;
           const bool brief = kShort && kind == CG_TANGENT_ROTATION && c.amp_bead >= 1 && c.amp_bead <= sh.short_amp;
-          const int gs = c.amp_bead <= 8 ? 8 : 16, cap = LEAN || c.amp_bead <= 16 ? 16 : 32;  // of a short rotation
+          const int gs = c.amp_bead <= 8 ? 8 : 16, cap = c.amp_bead <= 16 ? 16 : 32;  // of a short rotation
           int most = kind <= CG_SLIDE ? sh.limit[kind] : Sn;
           if (brief) {
             const int room = min(min(kMaxS, Sn * (64 / cap)), (int)blockDim.x / gs);
