@@ -255,15 +255,15 @@ struct cg_sim {
   // CTAs per replica of the sums over beads and voxels, as a power of two: a replica's
   // part takes a CTA ~8 us before its first bead, so a replica is split only as far
   // as its share of the work asks for on ~5/4 CTAs per SM, and into parts of some
-  // size (4,096 voxels, or as much, 16,384 where the parts outnumber the SMs).
-  // Energies, us, with 1 / 2 / 4 / 8 CTAs per replica: 2,000 chains of 30 beads and
-  // 4^3 voxels 75 / 158 / 297 / 630 (98 before the clusters), 256 of 2,000 and 30^3
-  // 74 / 86 / 111 / 160, 64 of 5,000 and 40^3 127 / 76 / 53 / 63, one of 20,000 and
-  // 60^3 297 / 156 / 86 / 51.
+  // size (4,096 voxels, or as much, 8,192 where the parts outnumber the SMs).
+  // Energies, us, with 1 / 2 / 4 / 8 CTAs per replica: 600 chains of 50 beads and 8^3
+  // voxels 29 / 53 / 96 / 188, 256 of 3,000 and 30^3 95 / 105 / 123 / 157, 64 of 1,000
+  // and 20^3 27 / 23 / 21 / 31, 64 of 5,000 and 40^3 136 / 82 / 56 / 63, 30 of 3,000 and
+  // 30^3 55 / 37 / 26 / 23, one of 20,000 and 60^3 306 / 174 / 93 / 57.
   int sum_log() const {
     int log = 0;
     while (log < 3 && (work_max >> log) * 5 * n_sm > 4 * work_sum &&
-           work_max >> (log + 1) >= ((long long)R << (log + 1) > n_sm ? 16384 : 4096))
+           work_max >> (log + 1) >= ((long long)R << (log + 1) > n_sm ? 8192 : 4096))
       log++;
     return log;
   }
@@ -1547,7 +1547,7 @@ int cg_load_state(cg_sim* s, const void* buf, int64_t bytes) {
     off += p.bytes;
   }
   if (s->guard_every) CUDA_TRY(cudaMemset(s->guard_init, 0, sizeof(int) * s->R));  // new reference energies
-  {  // the restored replicas' twist chooses the MC kernel's form
+  {  // the restored replicas' twist and fast_field choose the MC kernel's form
     std::vector<RepDev> rd(s->R);
     CUDA_TRY(cudaMemcpy(rd.data(), s->reps, sizeof(RepDev) * s->R, cudaMemcpyDeviceToHost));
     for (int r = 0; r < s->R; r++) s->note_features(r, rd[r]);

@@ -97,9 +97,11 @@ struct SumPart {
   }
 };
 
-// Launch of one of the sum kernels: a cluster of 2^log_ctas CTAs per replica.
+// Launch of one of the sum kernels, instantiated for whole replicas (a CTA each) and for
+// replicas split over a cluster of 2^log_ctas CTAs.
 template <class... P, class... A>
-static void launch_sums(void (*kernel)(KArgs, int, P...), const KArgs& a, int log_ctas, cudaStream_t s, A... args) {
+static void launch_sums(void (*whole)(KArgs, int, P...), void (*split)(KArgs, int, P...), const KArgs& a, int log_ctas,
+                        cudaStream_t s, A... args) {
   cudaLaunchAttribute at{};
   at.id = cudaLaunchAttributeClusterDimension;
   at.val.clusterDim.x = 1u << log_ctas;
@@ -110,25 +112,43 @@ static void launch_sums(void (*kernel)(KArgs, int, P...), const KArgs& a, int lo
   c.stream = s;
   c.attrs = &at;
   c.numAttrs = log_ctas > 0 ? 1 : 0;
-  cudaLaunchKernelEx(&c, kernel, a, log_ctas, P(args)...);
+  cudaLaunchKernelEx(&c, log_ctas > 0 ? split : whole, a, log_ctas, P(args)...);
 }
 
-// The warps' sums in sh added in warp order, then the CTAs' in rank order, valid in the
-// first 16 threads of rank 0.
+// The warps' sums in sh added in warp order, then (SPLIT) the CTAs' in rank order, valid
+// in the first 16 threads of rank 0.  Without SPLIT many replicas share the FP64 pipes,
+// and zero sums are left out; with it few CTAs run, and loads and additions without
+// branches are sooner done (derivative terms of one 1,000-bead chain, 8 CTAs: 12.3 us,
+// 14.4 with the branches).
+template <bool SPLIT>
 __device__ __forceinline__ double over_ctas(double (*sh)[16]) {
+  constexpr int kWarps = kSumThreads / 32;
+  double t = 0;
+  if (!SPLIT) {
+    if (threadIdx.x < 16)
+      #pragma unroll 1
+      for (int w = 0; w < kWarps; w++)
+        if (!is_zero64(sh[w][threadIdx.x])) t += sh[w][threadIdx.x];
+    return t;
+  }
   namespace cgr = cooperative_groups;
   cgr::cluster_group cl = cgr::this_cluster();
-  double t = 0;
-  if (threadIdx.x < 16)
-    #pragma unroll 1
-    for (int w = 0; w < kSumThreads / 32; w++)
-      if (!is_zero64(sh[w][threadIdx.x])) t += sh[w][threadIdx.x];
-  if (cl.num_blocks() == 1) return t;
-  if (threadIdx.x < 16) sh[0][threadIdx.x] = t;
+  constexpr int kMaxCtas = 8;
+  const int ctas = (int)cl.num_blocks();
+  if (threadIdx.x < 16) {
+#pragma unroll
+    for (int w = 0; w < kWarps; w++) t += sh[w][threadIdx.x];
+    sh[0][threadIdx.x] = t;
+  }
   cl.sync();
-  if (cl.block_rank() == 0 && threadIdx.x < 16)
-    #pragma unroll 1
-    for (int r = 1; r < (int)cl.num_blocks(); r++) t += cl.map_shared_rank(&sh[0][0], r)[threadIdx.x];
+  if (cl.block_rank() == 0 && threadIdx.x < 16) {
+    double part[kMaxCtas];
+#pragma unroll
+    for (int r = 1; r < kMaxCtas; r++) part[r] = r < ctas ? cl.map_shared_rank(&sh[0][0], r)[threadIdx.x] : 0.0;
+#pragma unroll
+    for (int r = 1; r < kMaxCtas; r++)
+      if (r < ctas) t += part[r];
+  }
   cl.sync();  // no CTA leaves while its sums are read
   return t;
 }
@@ -137,12 +157,13 @@ __device__ __forceinline__ double over_ctas(double (*sh)[16]) {
 // (thread k: sum k).  Every thread of the cluster calls it.  Within a warp the
 // lanes halve the set of sums they carry at each step (16 FP64 additions
 // instead of 80).
+template <bool SPLIT>
 __device__ __forceinline__ double cluster_sums(double (&v)[16], double (*sh)[16]) {
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  bool any = false;  // of few beads or voxels most warps hold zeros
+  bool any = SPLIT;  // of few beads or voxels most warps hold zeros
 #pragma unroll
   for (int k = 0; k < 16; k++) any = any || !is_zero64(v[k]);
-  if (__any_sync(kFull, any)) {
+  if (SPLIT || __any_sync(kFull, any)) {
 #pragma unroll
     for (int h = 8, o = 16; h >= 1; h >>= 1, o >>= 1) {
       const bool up = lane & o;
@@ -159,20 +180,21 @@ __device__ __forceinline__ double cluster_sums(double (&v)[16], double (*sh)[16]
   // lane l holds sum (bits 4, 3, 2, 1 of l as bits 3, 2, 1, 0)
   if (!(lane & 1)) sh[warp][lane >> 1] = v[0];
   __syncthreads();
-  return over_ctas(sh);
+  return over_ctas<SPLIT>(sh);
 }
 // The sum of one number over the CTAs of a cluster, by the additions of cluster_sums,
 // valid in thread 0 of rank 0.
+template <bool SPLIT>
 __device__ __forceinline__ double cluster_sum(double v, double (*sh)[16]) {
   const bool any = !is_zero64(v);
-  if (__any_sync(kFull, any))
+  if (SPLIT || __any_sync(kFull, any))
 #pragma unroll
     for (int o = 16; o >= 1; o >>= 1) v += __shfl_xor_sync(kFull, v, o);
   else
     v = 0.0;
   if ((threadIdx.x & 31) < 16) sh[threadIdx.x >> 5][threadIdx.x & 31] = v;
   __syncthreads();
-  return over_ctas(sh);
+  return over_ctas<SPLIT>(sh);
 }
 
 // The line of vf_limit in fixed-point bead weights, uniform volumes: the volume
@@ -274,8 +296,9 @@ __device__ __forceinline__ void fx_product(FxSum& s, unsigned l0, unsigned h0, u
 }
 // The sum in FP64 (one conversion, of its leading 64 bits); `shift` is 26, or 27
 // for squares.
+template <bool SPLIT>
 __device__ __forceinline__ double fx_value(const FxSum& s, int shift) {
-  if (!(s.ll | s.lh | s.hh)) return 0.0;
+  if (!SPLIT && !(s.ll | s.lh | s.hh)) return 0.0;
   unsigned long long lo = s.ll, hi = s.lh >> (64 - shift), t = s.lh << shift;
   lo += t;
   hi += lo < t ? 1 : 0;
@@ -307,14 +330,14 @@ __device__ __forceinline__ void init_sums(GridSums& s, RestSums& rest) {
   for (int k = 0; k < kRests; k++) rest[k][threadIdx.x] = 0.0;
 }
 // The integer sums as FP64, in the order of kRest00 .. kRestX + 2.
-template <class F>
+template <bool SPLIT, class F>
 __device__ __forceinline__ void sum_values(const GridSums& s, int nb, const F& f) {
-  f(kRest00, fx_value(s.s00, 27));
+  f(kRest00, fx_value<SPLIT>(s.s00, 27));
 #pragma unroll
-  for (int b = 0; b < CG_MAX_BINDERS; b++) f(kRestBB + b, b < nb ? fx_value(s.sbb[b], 27) : 0.0);
-  f(kRestX, nb > 1 ? fx_value(s.sx[0], 26) : 0.0);
-  f(kRestX + 1, nb > 2 ? fx_value(s.sx[1], 26) : 0.0);
-  f(kRestX + 2, nb > 2 ? fx_value(s.sx[2], 26) : 0.0);
+  for (int b = 0; b < CG_MAX_BINDERS; b++) f(kRestBB + b, b < nb ? fx_value<SPLIT>(s.sbb[b], 27) : 0.0);
+  f(kRestX, nb > 1 ? fx_value<SPLIT>(s.sx[0], 26) : 0.0);
+  f(kRestX + 1, nb > 2 ? fx_value<SPLIT>(s.sx[1], 26) : 0.0);
+  f(kRestX + 2, nb > 2 ? fx_value<SPLIT>(s.sx[2], 26) : 0.0);
 }
 static __device__ __noinline__ void add_row_f64(RestSums& rest, long long gmax, double vol, double bead_vol,
                                                 long long r0, long long r1, long long r2, long long r3) {
@@ -351,23 +374,25 @@ __device__ __forceinline__ void add_row(const RepDev& rd, long long gmax, const 
   }
 }
 // Called after every outer iteration: empties full integer sums.
+template <bool SPLIT>
 __device__ __forceinline__ void drain_sums(int nb, GridSums& s, RestSums& rest) {
   if (--s.left) return;
-  sum_values(s, nb, [&](int k, double x) { rest[k][threadIdx.x] += x; });
+  sum_values<SPLIT>(s, nb, [&](int k, double x) { rest[k][threadIdx.x] += x; });
   s = GridSums{};
   s.left = kFxRows / kRowsInFlight;
   s.rest = true;
 }
 // The sums of one CTA's part of a replica: out[kRest00 .. kRestVf].
+template <bool SPLIT>
 __device__ __forceinline__ void grid_sums(const KArgs& a, const RepDev& rd, SumPart part, long long gmax, RestSums& rest,
                                           double (&out)[kRests]) {
   GridSums s;
   init_sums(s, rest);
   const int nb = rd.nb;
   for_each_row<true>(a, rd, part, [&](long long, const long long (&row)[4]) { add_row(rd, gmax, row, s, rest); },
-                     [&] { drain_sums(nb, s, rest); });
+                     [&] { drain_sums<SPLIT>(nb, s, rest); });
   out[kRestOver] = out[kRestVf] = 0.0;
-  sum_values(s, nb, [&](int k, double x) { out[k] = x; });
+  sum_values<SPLIT>(s, nb, [&](int k, double x) { out[k] = x; });
   if (s.rest)
 #pragma unroll
     for (int k = 0; k < kRests; k++) out[k] += rest[k][threadIdx.x];

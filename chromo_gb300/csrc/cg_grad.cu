@@ -255,7 +255,8 @@ __global__ void __launch_bounds__(128) gradient_kernel(KArgs a, Out* out, Out* o
 // [1..3] sum_v rho_b^2, [4..6] sum_v rho_0 rho_1, rho_0 rho_2, rho_1 rho_2,
 // [7..9] #(state_b == 2), [10..12] sum_i s_ib, [13] sum_v (W / V)^2 with W the
 // bead weight of the voxel.  acc (or null): running sums [T, T T^T, count].
-// A cluster per replica (see cg_energy.cuh).
+// A CTA or (SPLIT) a cluster per replica (see cg_energy.cuh).
+template <bool SPLIT>
 __global__ void __launch_bounds__(kSumThreads)
     terms_kernel(KArgs a, int log_ctas, double* terms, double* acc) {
   __shared__ double sh[kSumThreads / 32][16];
@@ -287,7 +288,7 @@ __global__ void __launch_bounds__(kSumThreads)
   }
   double g[kRests] = {}, dens2 = 0;
   if (uniform) {
-    grid_sums(a, rd, part, gmax_sh, rest, g);
+    grid_sums<SPLIT>(a, rd, part, gmax_sh, rest, g);
   } else if (field) {
     for_each_row<false>(a, rd, part, [&](long long v, const long long (&row)[4]) {
       if (empty_voxel(a, rd, v, row)) return;
@@ -309,7 +310,7 @@ __global__ void __launch_bounds__(kSumThreads)
   double v[16] = {g[kRest00], g[kRestBB], g[kRestBB + 1], g[kRestBB + 2], g[kRestX], g[kRestX + 1], g[kRestX + 2],
                   (double)dbl[0], (double)dbl[1], (double)dbl[2], (double)sum[0], (double)sum[1], (double)sum[2],
                   uniform ? g[kRest00] + g[kRestOver] : dens2, 0.0, 0.0};
-  double t = cluster_sums(v, sh);
+  double t = cluster_sums<SPLIT>(v, sh);
   if (rank != 0) return;
   if (threadIdx.x < kTerms) {
     const int k = threadIdx.x;
@@ -385,5 +386,5 @@ void cg_launch_store_chains(const cg::KArgs& a, bool fp64, long long total, cons
 }
 
 void cg_launch_terms(const cg::KArgs& a, int log_ctas, double* terms, double* acc, cudaStream_t s) {
-  cg::launch_sums(cg::terms_kernel, a, log_ctas, s, terms, acc);
+  cg::launch_sums(cg::terms_kernel<false>, cg::terms_kernel<true>, a, log_ctas, s, terms, acc);
 }

@@ -566,7 +566,7 @@ __global__ void deposit_kernel(KArgs a, int rep_only) {
 }
 
 // ---------------------------------------------------------------- FP64 energies
-// A cluster per replica (see cg_energy.cuh).
+// A CTA or (SPLIT) a cluster per replica (see cg_energy.cuh).
 //
 // S and the chi term of a replica with uniform voxel volumes: c the volume
 // fraction per fixed-point unit, S = (V / Vb) c^2 sum g0^2.
@@ -575,7 +575,7 @@ __device__ __forceinline__ double chi_free_sum(const RepDev& rd, double s00) {
   return (rd.vol_bin / rd.bead_vol) * (c * c) * s00;
 }
 
-template <typename Pos>
+template <typename Pos, bool SPLIT>
 __global__ void __launch_bounds__(kSumThreads)
     energy_kernel(KArgs a, int log_ctas, double* out) {
   __shared__ double sh[kSumThreads / 32][16];
@@ -602,7 +602,7 @@ __global__ void __launch_bounds__(kSumThreads)
     if (((threadIdx.x >> 5) ^ phase) & 1) {
       bead_sums<Pos>(a, rd, part, bf, el, bi, dbl, excess);
     } else if (uniform) {
-      grid_sums(a, rd, part, gmax_sh, rest, g);
+      grid_sums<SPLIT>(a, rd, part, gmax_sh, rest, g);
     } else if (field) {
       for_each_row<false>(a, rd, part, [&](long long v, const long long (&row)[4]) {
         if (!empty_voxel(a, rd, v, row)) voxel_energy(a, rd, v, p);
@@ -611,7 +611,7 @@ __global__ void __launch_bounds__(kSumThreads)
   }
   double v[16] = {el, bi, uniform ? g[kRest00] : p.sx, uniform ? g[kRestVf] : p.fe, g[kRestBB], g[kRestBB + 1],
                   g[kRestBB + 2], g[kRestX], g[kRestX + 1], g[kRestX + 2], (double)dbl[0], (double)dbl[1], (double)dbl[2], (double)excess, 0.0, 0.0};
-  const double t = cluster_sums(v, sh);
+  const double t = cluster_sums<SPLIT>(v, sh);
   if (rank != 0 || threadIdx.x >= 32) return;
   double s[16];
   for (int k = 0; k < 16; k++) s[k] = __shfl_sync(kFull, t, k);
@@ -640,6 +640,7 @@ __global__ void __launch_bounds__(kSumThreads)
 // The chi-free sums S_r alone (the input of the exchange): the same rows in the
 // same order as energy_kernel's out[5 r + 4], so the values are identical; and
 // with a mu ladder the bound sites of its binder (an exact integer sum).
+template <bool SPLIT>
 __global__ void __launch_bounds__(kSumThreads)
     chi_sum_kernel(KArgs a, int log_ctas, double* out) {
   __shared__ double sh[kSumThreads / 32][16];
@@ -670,11 +671,11 @@ __global__ void __launch_bounds__(kSumThreads)
         },
         [&] {
           if (--left) return;
-          sx += fx_value(s, 27);
+          sx += fx_value<SPLIT>(s, 27);
           s = FxSum{};
           left = kFxRows / kRowsInFlight;
         });
-    sx += fx_value(s, 27);
+    sx += fx_value<SPLIT>(s, 27);
   } else if (field) {
     EnergyParts p{0.0, 0.0, 0.0, 0.0, {0, 0, 0}};
     for_each_row<false>(a, rd, part, [&](long long v, const long long (&row)[4]) {
@@ -690,11 +691,11 @@ __global__ void __launch_bounds__(kSumThreads)
     part.of(rd.n_beads, b0, b1);
     for (long long i = b0 + threadIdx.x; i < b1; i += blockDim.x) nbl += (st[i] >> sh8) & 0xFFu;
   }
-  const double t = cluster_sum(sx, sh);
+  const double t = cluster_sum<SPLIT>(sx, sh);
   if (rank == 0 && threadIdx.x == 0) out[rep * 5 + 4] = uniform ? chi_free_sum(rd, t) : t;
   if (a.mu_rungs > 1) {
     __syncthreads();
-    const double n = cluster_sum((double)nbl, sh);
+    const double n = cluster_sum<SPLIT>((double)nbl, sh);
     if (rank == 0 && threadIdx.x == 0) a.nbound[rep] = n;
   }
 }
@@ -830,12 +831,12 @@ void cg_launch_deposit(const cg::KArgs& a, bool fp64, int rep, int n_reps_launch
 }
 
 void cg_launch_energy(const cg::KArgs& a, bool fp64, int log_ctas, double* out, cudaStream_t s) {
-  if (fp64) cg::launch_sums(cg::energy_kernel<double>, a, log_ctas, s, out);
-  else cg::launch_sums(cg::energy_kernel<float>, a, log_ctas, s, out);
+  if (fp64) cg::launch_sums(cg::energy_kernel<double, false>, cg::energy_kernel<double, true>, a, log_ctas, s, out);
+  else cg::launch_sums(cg::energy_kernel<float, false>, cg::energy_kernel<float, true>, a, log_ctas, s, out);
 }
 
 void cg_launch_chi_sum(const cg::KArgs& a, int log_ctas, double* out, cudaStream_t s) {
-  cg::launch_sums(cg::chi_sum_kernel, a, log_ctas, s, out);
+  cg::launch_sums(cg::chi_sum_kernel<false>, cg::chi_sum_kernel<true>, a, log_ctas, s, out);
 }
 
 void cg_launch_exchange(const cg::KArgs& a, const double* eout, int n_rungs, long long round,
