@@ -44,6 +44,8 @@
 #pragma once
 #include <cuda_runtime.h>
 
+#include <atomic>
+
 #include "cg_device.cuh"
 #include "cg_exact.h"
 #include "cg_kernels.h"
@@ -2406,12 +2408,15 @@ __global__ void __maxnreg__(sizeof(Pos) == 4 ? 128 : 168) spec_kernel(KArgs a) {
     }                                                                                              \
     return cudaSuccess;                                                                            \
   }                                                                                                \
-  int cg_spec_regs_##NAME() {                                                                      \
-    int regs = 0;                                                                                  \
+  int cg_spec_regs_##NAME() { /* of the code, the same on every device: asked for once */          \
+    static std::atomic<int> known{0};                                                              \
+    int regs = known.load(std::memory_order_relaxed);                                              \
+    if (regs > 0) return regs;                                                                     \
     for (auto* kernel : {cg::spec_kernel<Pos, G, 0>, cg::spec_kernel<Pos, G, 1>, cg::spec_kernel<Pos, G, 2>}) { \
       cudaFuncAttributes at;                                                                       \
       if (cudaFuncGetAttributes(&at, kernel) != cudaSuccess) return 0;                             \
       if (at.numRegs > regs) regs = at.numRegs;                                                    \
     }                                                                                              \
+    known.store(regs, std::memory_order_relaxed);                                                  \
     return regs;                                                                                   \
   }
