@@ -1128,8 +1128,9 @@ __device__ __forceinline__ typename AccOf<Pos>::type rotate_tangent(const KArgs&
 // 395 and 411 / 468 / 544.  256 chains (S = 6) of 50 beads, up to 8 / 10 / 13: 928 /
 // 1,132 / 1,358 and 1,088 / 1,161 / 1,182; of 5,000, up to 17 / 24 / 32: 432 / 698 / 943
 // and 563 / 665 / 795.  The FP64 twist terms outweigh that up to 32 beads and amp^2 =
-// 8 N (64 SSTWLC chains of 200 / 50 beads, up to 32, 80 rotations: 2.08 / 2.55 ms here,
-// 2.17 / 2.21 there).
+// 16 N (200 rotations on each of 64 SSTWLC chains of 20 beads, up to 16 / 20: 3,052 /
+// 5,464 and 4,978 / 4,760; of 50, up to 26 / 32: 3,811 / 4,787 and 4,360 / 4,247; of
+// 200, up to 32: 3,678 and 4,052).
 //
 // Moves in flight: kShortSpan sqrt(N) / (amp + 1), at which about two of them
 // meet an earlier accepted one (3 and 4 measured alike, 6 and 9 were slower on
@@ -2194,7 +2195,7 @@ __global__ void __maxnreg__(sizeof(Pos) == 4 ? 128 : 168) spec_kernel(KArgs a) {
     sh.stop = 0;
     sh.npool = 0;
     const float n = (float)rd0.n_beads;
-    sh.short_amp = !LEAN && rd0.twist ? (int)fminf(32.0f, sqrtf(8.0f * n))
+    sh.short_amp = !LEAN && rd0.twist ? (int)fminf(32.0f, 4.0f * sqrtf(n))
                                           : (int)fminf(fminf(32.0f, sqrtf(5.4f * sqrtf(n * (float)Sn))),
                                                        16.0f + n * (float)Sn * (1.0f / 4000.0f));
   }

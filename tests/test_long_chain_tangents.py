@@ -6,6 +6,7 @@ import pytest
 
 from chromo_gb300 import workloads as wl
 from chromo_gb300.device import move_ctl
+from test_short_tangents import _run
 
 pytestmark = pytest.mark.gpu
 
@@ -25,4 +26,12 @@ def test_rotations_equal_one_at_a_time(n, amp):
         out.append(sim.get_chain(0) + (sim.tally(0),))
         sim.close()
     for a, b in zip(*out):
+        np.testing.assert_array_equal(a, b)
+
+
+@pytest.mark.parametrize("n,amp", [(16, 16), (20, 17), (20, 18), (64, 32), (63, 32)])
+def test_twisted_rotations_equal_eight_lanes(n, amp):
+    want = _run(n, amp, True, 2, 8)
+    assert want[-2][3, 1] > 0
+    for a, b in zip(want, _run(n, amp, True, 0, 32)):
         np.testing.assert_array_equal(a, b)
